@@ -29,6 +29,7 @@
 #include "kf_pointwise.cuh"
 #include "kf_poisson.cuh"
 #include "kf_stretch.cuh"
+#include "kf_zprod.cuh"
 
 using namespace kf;
 
@@ -93,6 +94,11 @@ struct kf_ctx {
     void *kv = nullptr, *SV = nullptr, *PF = nullptr, *tw = nullptr;
     double *q2 = nullptr;
     int *pb = nullptr;  // x-pass 2/3-rule bounds per (j, kz) column (dealias_bounds)
+    // the kept part of a masked half spectrum (AxTrunc; tr_nkz 0: its bounds
+    // do not hold on this grid and every pass is AX_FULL)
+    int tr_nkz = 0, tr_nt = 0;
+    double tr_ball = 0., tr_disc = 0.;  // elements kept; elements of the active columns
+    int *tr_jb = nullptr, *tr_tl = nullptr;
     double *stage64 = nullptr;
     std::vector<LevelBuf> lv;
     double *partial = nullptr;
@@ -354,6 +360,40 @@ std::vector<int> dealias_bounds(const std::vector<double> &q2, int n, double thr
             pb[(size_t)j * nzc + k] = ok ? b : -2;
         }
     return pb;
+}
+
+// The kept part of a masked half spectrum from its x-pass bounds pb: nkz and
+// jb[kz] such that the column (j, kz) has a kept element exactly when kz < nkz
+// and min(j, n - j) <= jb[kz], and the x-pass tiles of tc columns that cover
+// those columns.  nkz = 0 when some column does not fit that form.
+struct TruncTab {
+    int nkz = 0;
+    std::vector<int> jb, tl;
+};
+TruncTab trunc_table(const std::vector<int> &pb, int n, int tc) {
+    const int nzc = n / 2 + 1;
+    TruncTab t;
+    std::vector<int> jb(nzc, -1);
+    int nkz = 0;
+    for (int k = 0; k < nzc; ++k) {
+        for (int m = 0; m <= n / 2; ++m)
+            if (pb[(size_t)m * nzc + k] >= 0) jb[k] = m;
+        if (jb[k] >= 0) nkz = k + 1;
+    }
+    for (int j = 0; j < n; ++j)
+        for (int k = 0; k < nzc; ++k) {
+            const int b = pb[(size_t)j * nzc + k];
+            if (b == -2 || (b >= 0) != ((j <= n / 2 ? j : n - j) <= jb[k])) return t;
+        }
+    t.nkz = nkz;
+    t.jb = jb;
+    for (int j = 0; j < n; ++j) {
+        int last = -1;
+        for (int k = 0; k < nkz; ++k)
+            if (pb[(size_t)j * nzc + k] >= 0) last = k;
+        for (int k = 0; k <= last; k += tc) t.tl.push_back((j << 16) | k);
+    }
+    return t;
 }
 
 // ------------------------------------------------------------------ Poisson driver
@@ -780,7 +820,8 @@ double read_max_slots(kf_ctx *c) {
 }
 
 // The colour-split copy of c->rho that the finest half sweeps read: made at
-// the start of every FAS solve, so it follows whatever wrote c->rho.
+// the start of a FAS solve, unless the pass that wrote c->rho (k_z_rho) wrote
+// it as well.
 void rho_split(kf_ctx *c) {
     if (!c->rho_cs) return;
     const int n = c->n;
@@ -789,8 +830,9 @@ void rho_split(kf_ctx *c) {
     CK(cudaGetLastError());
 }
 
-// Poisson solve on c->phi with source c->rho.  Returns KF_OK or KF_ERR_NOT_CONVERGED.
-int poisson(kf_ctx *c) {
+// Poisson solve on c->phi with source c->rho; split: whoever wrote c->rho wrote
+// its colour-split copy too.  Returns KF_OK or KF_ERR_NOT_CONVERGED.
+int poisson(kf_ctx *c, bool split = false) {
     NvtxRange nv("kf Poisson solve");
     const kf_config &cf = c->cfg;
     c->diag.solves++;
@@ -838,7 +880,7 @@ int poisson(kf_ctx *c) {
     } else if (!(cf.res_tol > 0.)) {
         // fixed number of V-cycles: the result is a smooth function of rho
         // and of the initial guess (no data-dependent stopping)
-        rho_split(c);
+        if (!split) rho_split(c);
         for (int cyc = 0; cyc < cf.max_cycles; ++cyc) run_vcycle(c);
         const double r = max_residual(c, L0, c->phi, c->rho, true);
         c->diag.last_iterations = cf.max_cycles;
@@ -849,7 +891,7 @@ int poisson(kf_ctx *c) {
     } else if (c->lv.size() > 1) {
         // test after each cycle's pre-smoothing on the residual the cycle
         // computes anyway; the rest of the cycle only when it fails
-        rho_split(c);
+        if (!split) rho_split(c);
         double r = 0.;
         int cyc = 0;
         for (;;) {
@@ -870,7 +912,7 @@ int poisson(kf_ctx *c) {
             rc = 1;
         }
     } else {
-        rho_split(c);
+        if (!split) rho_split(c);
         double r = max_residual(c, L0, c->phi, c->rho, true);
         int cyc = 0;
         while (r > cf.res_tol && cyc < cf.max_cycles) {
@@ -925,7 +967,6 @@ void poisson_captured(kf_ctx *c) {
     }
     LevelBuf &L0 = c->lv[0];
     const bool fixed = !(cf.res_tol > 0.);
-    rho_split(c);
     c->head_kernels = 0;
     if (!fixed && c->lv.size() > 1) {
         // WHILE { head of the cycle (pre-smoothing, residual with its max);
@@ -1077,11 +1118,15 @@ template <typename T, int N> struct Impl {
         CK(cudaFuncSetAttribute(k_axis_pipe<T, N, +1, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_c2r<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_r2c<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        CK(cudaFuncSetAttribute(k_zprod<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        CK(cudaFuncSetAttribute(k_z_rho<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        CK(cudaFuncSetAttribute(k_z_phi<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_xfwd_assemble<T, N, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_xfwd_assemble<T, N, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     }
 
-    static double job_bytes(kf_ctx *c, int off, int njobs) {
+    // distinct inputs and outputs of a launch, each as far as the mode moves it
+    static double job_bytes(kf_ctx *c, int off, int njobs, int mode = AX_FULL) {
         std::vector<const void *> u;
         for (int j = 0; j < njobs; ++j) {
             const void *p = c->hj[off + j].in;
@@ -1089,7 +1134,11 @@ template <typename T, int N> struct Impl {
             for (auto q : u) seen |= q == p;
             if (!seen) u.push_back(p);
         }
-        return (double)(u.size() + njobs) * c->Nc * sizeof(T2);
+        double fin = (double)c->Nc, fout = fin;
+        if (c->tr_nkz && mode == AX_XM) fin = c->tr_ball, fout = c->tr_disc;
+        if (c->tr_nkz && mode == AX_YI) fin = c->tr_disc, fout = (double)N * N * c->tr_nkz;
+        if (c->tr_nkz && mode == AX_YF) fin = (double)N * N * c->tr_nkz, fout = c->tr_disc;
+        return (u.size() * fin + njobs * fout) * sizeof(T2);
     }
     // resident blocks per SM x SMs of the pipelined pass (its grid)
     template <int V> static int pipe_grid(int sign) {
@@ -1108,25 +1157,41 @@ template <typename T, int N> struct Impl {
         }
         return v;
     }
-    template <int V> static void axis_v(kf_ctx *c, int off, int njobs, int ax, int sign) {
-        const int ntiles = ax == 0 ? (N * NZC + TC - 1) / TC : N * ((NZC + TC - 1) / TC);
+    // AX_FULL when the grid's 2/3 rule has no truncated form (tr_nkz == 0)
+    static AxTrunc trunc(kf_ctx *c, int mode) {
+        AxTrunc A{AX_FULL, NZC, 0.f, nullptr, nullptr};
+        if (mode == AX_FULL || !c->tr_nkz) return A;
+        A.mode = mode;
+        A.nkz = c->tr_nkz;
+        A.itpp = 1.f / (float)((c->tr_nkz + TC - 1) / TC);
+        A.jb = c->tr_jb;
+        A.tl = c->tr_tl;
+        return A;
+    }
+    // kz extent of a z pass over masked fields
+    static int nkz(kf_ctx *c, bool masked) { return masked && c->tr_nkz ? c->tr_nkz : NZC; }
+    template <int V> static void axis_v(kf_ctx *c, int off, int njobs, int ax, int sign, int mode) {
+        const AxTrunc A = trunc(c, mode);
+        const int ntiles = A.mode == AX_XM ? c->tr_nt
+                           : ax == 0       ? (N * NZC + TC - 1) / TC
+                                           : N * ((A.nkz + TC - 1) / TC);
         const int total = njobs * ntiles, grid = std::min(total, pipe_grid<V>(sign));
         const size_t smem = axis_pipe_smem<T, N>(njobs);
         if (sign < 0)
             k_axis_pipe<T, N, -1, V><<<grid, TC * PV<V>, smem, c->st>>>(c->dj + off, njobs, ax, geo(c),
-                                                                      (const T2 *)c->tw, total);
+                                                                      (const T2 *)c->tw, total, A);
         else
             k_axis_pipe<T, N, +1, V><<<grid, TC * PV<V>, smem, c->st>>>(c->dj + off, njobs, ax, geo(c),
-                                                                      (const T2 *)c->tw, total);
+                                                                      (const T2 *)c->tw, total, A);
     }
-    static void axis(kf_ctx *c, int off, int njobs, int ax, int sign) {
-        Launch L_(c, sign > 0 ? KC_AXIS_INV : KC_AXIS_FWD, job_bytes(c, off, njobs));
+    static void axis(kf_ctx *c, int off, int njobs, int ax, int sign, int mode = AX_FULL) {
+        Launch L_(c, sign > 0 ? KC_AXIS_INV : KC_AXIS_FWD, job_bytes(c, off, njobs, mode));
         if (c->fftv)
-            axis_v<1>(c, off, njobs, ax, sign);
+            axis_v<1>(c, off, njobs, ax, sign, mode);
         else
-            axis_v<0>(c, off, njobs, ax, sign);
+            axis_v<0>(c, off, njobs, ax, sign, mode);
     }
-    static double z_bytes(kf_ctx *c, int off, int njobs, bool c2r) {
+    static double z_bytes(kf_ctx *c, int off, int njobs, bool c2r, bool masked) {
         std::vector<const void *> u;
         int outs = 0;
         for (int j = 0; j < njobs; ++j) {
@@ -1139,32 +1204,35 @@ template <typename T, int N> struct Impl {
             }
             outs += (z.outA ? 1 : 0) + (z.outB ? 1 : 0);
         }
-        const double cb = (double)c->Nc * sizeof(T2), rb = (double)c->N * sizeof(T);
+        const double cb = (double)N * N * nkz(c, masked) * sizeof(T2), rb = (double)c->N * sizeof(T);
         return c2r ? u.size() * cb + outs * rb : u.size() * rb + outs * cb;
     }
     // scale < 0: the 1/N of c2r; otherwise the given factor (1 for transposes)
-    static void zc2r(kf_ctx *c, int off, int njobs, double scale = -1.) {
+    // masked: the half spectra come from masked x / y passes (zero from kz = nkz on)
+    static void zc2r(kf_ctx *c, int off, int njobs, bool masked = false, double scale = -1.) {
         const int nrows = N * N;
         const int ntiles = (nrows + LZ - 1) / LZ;
         const size_t smem = ZSmem<T, N, true>::bytes;
-        Launch L_(c, KC_Z_C2R, z_bytes(c, off, njobs, true));
+        Launch L_(c, KC_Z_C2R, z_bytes(c, off, njobs, true, masked));
         const T sc = (T)(scale < 0. ? 1. / ((double)N * N * N) : scale);
         if (c->fftv)
             k_z_c2r<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        (const T2 *)c->tw, sc);
+                                                                        (const T2 *)c->tw, sc, nkz(c, masked));
         else
             k_z_c2r<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        (const T2 *)c->tw, sc);
+                                                                        (const T2 *)c->tw, sc, nkz(c, masked));
     }
-    static void zr2c(kf_ctx *c, int off, int njobs) {
+    static void zr2c(kf_ctx *c, int off, int njobs, bool masked = false) {
         const int nrows = N * N;
         const int ntiles = (nrows + LZ - 1) / LZ;
         const size_t smem = ZSmem<T, N, false>::bytes;
-        Launch L_(c, KC_Z_R2C, z_bytes(c, off, njobs, false));
+        Launch L_(c, KC_Z_R2C, z_bytes(c, off, njobs, false, masked));
         if (c->fftv)
-            k_z_r2c<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, (const T2 *)c->tw);
+            k_z_r2c<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, (const T2 *)c->tw,
+                                                                        nkz(c, masked));
         else
-            k_z_r2c<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, (const T2 *)c->tw);
+            k_z_r2c<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, (const T2 *)c->tw,
+                                                                        nkz(c, masked));
     }
     static RhsArgs<T> rargs(kf_ctx *c) {
         RhsArgs<T> a;
@@ -1180,19 +1248,75 @@ template <typename T, int N> struct Impl {
         return a;
     }
 
-    // rounds A (P s, d_x s, d_y s and s_d = c2r(P s)), the Poisson solve and
-    // B (phi^ = r2c(phi)), shared by both right-hand sides
-    // Round D's jobs on u' and s (the first 6 x, 9 y and 8 z jobs of its
-    // lists): every input is the stage state or round A's output.
+    // Round D's passes on u' (the first 6 x and 9 y jobs of its lists): every
+    // input is the stage state.
     static void round_D_us(kf_ctx *c) {
-        axis(c, c->jD_x, 6, 0, +1);
-        axis(c, c->jD_y, 9, 1, +1);
-        zc2r(c, c->zD, 8);
+        axis(c, c->jD_x, 6, 0, +1, AX_XM);
+        axis(c, c->jD_y, 9, 1, +1, AX_YI);
+    }
+
+    // rho = exp(c2r(P s)) + n_d (and its colour-split copy) from round A's P s
+    // in CY[0]; sd: also s_d itself
+    static void rho_pass(kf_ctx *c, T *sd) {
+        const int nb = (N * N / 2 + LZ - 1) / LZ;
+        const size_t smem = (size_t)LZ * PadLen<N>::value * sizeof(T2);
+        const T sc = (T)(1. / ((double)N * N * N));
+        Launch L_(c, KC_RHO, (double)N * N * nkz(c, true) * sizeof(T2) + (double)c->N * (c->rho_cs ? 24 : 16));
+        if (c->fftv)
+            k_z_rho<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, c->rho, c->rho_cs,
+                                                              (const T2 *)c->tw, sc, nkz(c, true));
+        else
+            k_z_rho<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, c->rho, c->rho_cs,
+                                                              (const T2 *)c->tw, sc, nkz(c, true));
+        CK(cudaGetLastError());
+    }
+
+    // CX[8] = z r2c of phi in the bulk precision
+    static void phi_pass(kf_ctx *c) {
+        const int nb = (N * N / 2 + LZ - 1) / LZ;
+        const size_t smem = (size_t)LZ * PadLen<N>::value * sizeof(T2);
+        Launch L_(c, KC_Z_R2C, (double)c->N * 8 + (double)c->Nc * sizeof(T2));
+        if (c->fftv)
+            k_z_phi<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>(c->phi, (T2 *)c->CX[8], (const T2 *)c->tw, NZC);
+        else
+            k_z_phi<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>(c->phi, (T2 *)c->CX[8], (const T2 *)c->tw, NZC);
+        CK(cudaGetLastError());
+    }
+
+    // rounds D (z), E and the z part of F: k_zprod -> CX[0..3]
+    static void zprod(kf_ctx *c, bool pen) {
+        ZProdArgs<T> a{};
+        a.s0 = (const T2 *)c->CY[0];
+        a.sy = (const T2 *)c->CY[1];
+        a.sx = (const T2 *)c->CY[2];
+        for (int q = 0; q < 3; ++q) {
+            a.u[q] = (const T2 *)c->CY[3 + 3 * q];
+            a.uy[q] = (const T2 *)c->CY[4 + 3 * q];
+            a.ux[q] = (const T2 *)c->CY[5 + 3 * q];
+        }
+        for (int q = 0; q < 4; ++q) {
+            a.out[q] = (T2 *)c->CX[q];
+            a.rl[q] = (const T *)c->R[16 + q];
+        }
+        a.H = (const T *)c->H;
+        a.M = (T)c->cfg.M;
+        a.eta = (T)c->cfg.pen_eta;
+        a.scale = (T)(1. / ((double)N * N * N));
+        a.terms = c->cfg.terms;
+        a.nkz = nkz(c, true);
+        a.nko = nkz(c, pen);
+        const size_t smem = ZProdSmem<T, N>::bytes;
+        Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko) + (pen ? 5. * c->N * sizeof(T) : 0.));
+        if (c->fftv)
+            k_zprod<T, N, 1><<<N * N / ZP_ROWS, ZP_LINES * PV<1>, smem, c->st>>>(a, (const T *)c->kv, (const T2 *)c->tw);
+        else
+            k_zprod<T, N, 0><<<N * N / ZP_ROWS, ZP_LINES * PV<0>, smem, c->st>>>(a, (const T *)c->kv, (const T2 *)c->tw);
+        CK(cudaGetLastError());
     }
 
     // In a captured step, fork round_D_us onto st_side after round A; rhs
-    // joins it before the products.  The branch writes CX[2..7], CY[3..11]
-    // and R[1..15], which nothing between the fork and the join touches (the
+    // joins it before the products.  The branch writes CX[2..7] and CY[3..11],
+    // which nothing between the fork and the join touches (the
     // Poisson solve, round B in CX[8] / CY[12], k_lin, round D's LIN part).
     // (Measured at 256^3 FP32 bulk: +1 to +2.4 % per step; the Poisson chain
     // at a higher stream priority than the branch was slower than equal
@@ -1217,26 +1341,27 @@ template <typename T, int N> struct Impl {
         return true;
     }
 
-    static bool rounds_AB(kf_ctx *c, bool fork = false) {
+    // rounds A (P s, d_x s, d_y s, the Poisson source and, with keep_sd, s_d
+    // in R[0]), the Poisson solve and B (phi^ = r2c(phi)), shared by both
+    // right-hand sides
+    static bool rounds_AB(kf_ctx *c, bool fork, bool keep_sd) {
         const int Tm = c->cfg.terms;
-        const bool pen = Tm & T_PENALIZATION;
         const bool pois = (Tm & T_POISSON) && (Tm & T_E_INT);
         // A
-        axis(c, c->jA_x, 2, 0, +1);
-        axis(c, c->jA_y, 3, 1, +1);
-        if (pois || pen) zc2r(c, c->zA, 1);
+        axis(c, c->jA_x, 2, 0, +1, AX_XM);
+        axis(c, c->jA_y, 3, 1, +1, AX_YI);
+        const bool solve = pois && !c->phi_given;
+        if (solve)
+            rho_pass(c, keep_sd ? (T *)c->R[0] : nullptr);
+        else if (keep_sd)
+            zc2r(c, c->zA, 1, true);
         const bool forked = fork && fork_D(c);
-        if (pois && !c->phi_given) {
-            {
-                Launch L_(c, KC_RHO, (double)c->N * (sizeof(T) + 16));
-                k_rho<T><<<nblk(c->N, 256), 256, 0, c->st>>>((const T *)c->R[0], c->nd, c->rho, c->N);
-            }
-            CK(cudaGetLastError());
+        if (solve) {
             if (c->capturing) {
                 poisson_captured(c);
             } else {
                 const bool newtime = phi_guess(c);
-                int rc = poisson(c);
+                int rc = poisson(c, true);
                 if (rc) throw KfError{KF_ERR_NOT_CONVERGED, "Poisson solve did not reach its tolerance"};
                 if (c->cfg.phi_extrap && newtime) {
                     c->nhist = c->nhist < 2 ? c->nhist + 1 : 2;
@@ -1248,11 +1373,7 @@ template <typename T, int N> struct Impl {
         if (c->capturing && c->capture_wait_u && c->stage_idx == 0)
             CK(cudaStreamWaitEvent(c->st, c->ev_u, cudaEventWaitExternal));
         if (Tm & T_E_INT) {
-            if (c->fp32) {
-                Launch L_(c, KC_MISC, (double)c->N * (8 + sizeof(T)));
-                k_from_f64<T><<<nblk(c->N, 256), 256, 0, c->st>>>((T *)c->phiT, c->phi, c->N);
-            }
-            zr2c(c, c->zB, 1);
+            phi_pass(c);
             axis(c, c->jB_y, 1, 1, -1);
             axis(c, c->jB_x, 1, 0, -1);
         }
@@ -1263,7 +1384,7 @@ template <typename T, int N> struct Impl {
     static void rhs(kf_ctx *c) {
         const int Tm = c->cfg.terms;
         const bool pen = Tm & T_PENALIZATION;
-        const bool forked = rounds_AB(c, true);
+        const bool forked = rounds_AB(c, true, false);
         // C
         if (pen) {
             Launch L_(c, KC_LIN, (double)c->Nc * (9 * sizeof(T2) + 2 * sizeof(T)));
@@ -1271,56 +1392,31 @@ template <typename T, int N> struct Impl {
                                                                (T2 *)c->LIN[2], (T2 *)c->LIN[3]);
         }
         // D: the u', s part (unless forked) and the linear terms' part
-        if (!forked) {
-            axis(c, c->jD_x, pen ? 10 : 6, 0, +1);
-            axis(c, c->jD_y, pen ? 13 : 9, 1, +1);
-            zc2r(c, c->zD, pen ? 10 : 8);
-        } else {
-            if (pen) {
-                axis(c, c->jD_x + 6, 4, 0, +1);
-                axis(c, c->jD_y + 9, 4, 1, +1);
-                zc2r(c, c->zD + 8, 2);
-            }
-            CK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
+        if (!forked) round_D_us(c);
+        if (pen) {
+            axis(c, c->jD_x + 6, 4, 0, +1);
+            axis(c, c->jD_y + 9, 4, 1, +1);
+            zc2r(c, c->zD + 8, 2);
         }
-        // E
-        ProdArgs<T> pa;
-        for (int q = 0; q < 3; ++q) {
-            pa.U[q] = (const T *)c->R[1 + q];
-            pa.ds[q] = (const T *)c->R[13 + q];
-            for (int d = 0; d < 3; ++d) pa.dU[q][d] = (const T *)c->R[4 + 3 * q + d];
-        }
-        for (int q = 0; q < 4; ++q) {
-            pa.rl[q] = (const T *)c->R[16 + q];
-            pa.out[q] = (T *)c->R[20 + q];
-        }
-        pa.sd = (const T *)c->R[0];
-        pa.H = (const T *)c->H;
-        pa.M = (T)c->cfg.M;
-        pa.eta = (T)c->cfg.pen_eta;
-        pa.terms = Tm;
-        pa.N = c->N;
-        {
-            Launch L_(c, KC_PROD, (double)c->N * sizeof(T) * (19 + (pen ? 6 : 0)));
-            k_products<T><<<nblk(c->N, 256), 256, 0, c->st>>>(pa);
-        }
-        // F
-        zr2c(c, c->zF, 2);
-        axis(c, c->jF_y, 4, 1, -1);
-        const int ntiles = (N * NZC + TC - 1) / TC;
+        if (forked) CK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
+        // z part of D, E, z part of F (with penalization only what the 2/3 rule keeps is formed)
+        zprod(c, pen);
+        axis(c, c->jF_y, 4, 1, -1, pen ? AX_YF : AX_FULL);
+        const AxTrunc A = trunc(c, pen ? AX_XM : AX_FULL);
+        const int ntiles = A.mode == AX_XM ? c->tr_nt : (N * NZC + TC - 1) / TC;
         {
             const double cb = (double)c->Nc * sizeof(T2), rb = (double)c->Nc * sizeof(T);
-            Launch L_(c, KC_XASM, pen ? 8 * cb : 8 * cb + 4 * cb + ((Tm & T_E_INT) ? cb : 0.) + 2 * rb);
+            Launch L_(c, KC_XASM, A.mode == AX_XM ? 4. * (c->tr_disc + c->tr_ball) * sizeof(T2) : pen ? 8 * cb : 8 * cb + 4 * cb + ((Tm & T_E_INT) ? cb : 0.) + 2 * rb);
             const size_t sm = (size_t)N * TC * sizeof(T2);
             const AxisJob *j = c->dj + c->jF_x;
             if (c->fftv && pen)
-                k_xfwd_assemble<T, N, 1, true><<<ntiles, TC * PV<1>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw);
+                k_xfwd_assemble<T, N, 1, true><<<ntiles, TC * PV<1>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw, A);
             else if (c->fftv)
-                k_xfwd_assemble<T, N, 1, false><<<ntiles, TC * PV<1>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw);
+                k_xfwd_assemble<T, N, 1, false><<<ntiles, TC * PV<1>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw, A);
             else if (pen)
-                k_xfwd_assemble<T, N, 0, true><<<ntiles, TC * PV<0>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw);
+                k_xfwd_assemble<T, N, 0, true><<<ntiles, TC * PV<0>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw, A);
             else
-                k_xfwd_assemble<T, N, 0, false><<<ntiles, TC * PV<0>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw);
+                k_xfwd_assemble<T, N, 0, false><<<ntiles, TC * PV<0>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw, A);
         }
         CK(cudaGetLastError());
     }
@@ -1339,16 +1435,16 @@ template <typename T, int N> struct Impl {
         const bool pen = Tm & T_PENALIZATION;
         const long Nc = c->Nc, Nr = c->N;
         const double cb = (double)Nc * sizeof(T2), rb = (double)Nr * sizeof(T);
-        rounds_AB(c);
+        rounds_AB(c, false, pen);
         {  // C'
             Launch L_(c, KC_LIN, 4 * cb + 6 * cb + 2 * rb);
             k_sl_lin<T><<<nblk(Nc, 256), 256, 0, c->st>>>(rargs(c), geo(c), (T2 *)c->LIN[0], (T2 *)c->LIN[1],
                                                             (T2 *)c->LIN[2], (T2 *)c->LIN[3], (T2 *)c->CX[10]);
         }
         // D'
-        axis(c, c->jS_Dx, 8, 0, +1);
-        axis(c, c->jS_Dy, 12, 1, +1);
-        zc2r(c, c->zS_D, 10);
+        axis(c, c->jS_Dx, 8, 0, +1, AX_XM);
+        axis(c, c->jS_Dy, 12, 1, +1, AX_YI);
+        zc2r(c, c->zS_D, 10, true);
         {  // E'
             ScaleArgs<T> sa;
             for (int j = 0; j < 15; ++j) sa.f[j] = (T *)c->R[4 + j];
@@ -1365,9 +1461,9 @@ template <typename T, int N> struct Impl {
         const bool prod = Tm & (T_ADVECTION | T_CONTINUITY);
         if (prod) {
             // G'
-            axis(c, c->jS_Gx, 12, 0, +1);
-            axis(c, c->jS_Gy, 12, 1, +1);
-            zc2r(c, c->zS_G, 6);
+            axis(c, c->jS_Gx, 12, 0, +1, AX_XM);
+            axis(c, c->jS_Gy, 12, 1, +1, AX_YI);
+            zc2r(c, c->zS_G, 6, true);
             {  // H'
                 ProdArgs<T> pa{};
                 for (int q = 0; q < 3; ++q) {
@@ -1448,17 +1544,19 @@ template <typename T, int N> struct Impl {
     static void adj_pass(kf_ctx *c, int which) {
         switch (which) {
             case 0:  // forward intermediates s_d, U_c, d_d U_c, d_d s of the stage input in Ys
-                axis(c, c->jA_x, 2, 0, +1);
-                axis(c, c->jA_y, 3, 1, +1);
-                zc2r(c, c->zA, 1);
-                axis(c, c->jD_x, 6, 0, +1);
-                axis(c, c->jD_y, 9, 1, +1);
-                zc2r(c, c->zD, 8);
+                axis(c, c->jA_x, 2, 0, +1, AX_XM);
+                axis(c, c->jA_y, 3, 1, +1, AX_YI);
+                zc2r(c, c->zA, 1, true);
+                round_D_us(c);
+                zc2r(c, c->zD, 8, true);
                 break;
             case 1:  // f_bar = r2c^T(P Kbar) = c2r_unscaled(P Kbar / w)
-                axis(c, c->jV_x, 4, 0, +1);
-                axis(c, c->jV_y, 4, 1, +1);
-                zc2r(c, c->zV, 2, 1.);
+            {
+                const bool pen = c->cfg.terms & T_PENALIZATION;  // masked then (build_adj_jobs)
+                axis(c, c->jV_x, 4, 0, +1, pen ? AX_XM : AX_FULL);
+                axis(c, c->jV_y, 4, 1, +1, pen ? AX_YI : AX_FULL);
+                zc2r(c, c->zV, 2, pen, 1.);
+            }
                 break;
             case 2:  // r2c of the physical cotangents
                 zr2c(c, c->zW, c->nWz);
@@ -1468,7 +1566,7 @@ template <typename T, int N> struct Impl {
             case 3:  // phi_bar = r2c^T(phihat_bar)
                 axis(c, c->jP_x, 1, 0, +1);
                 axis(c, c->jP_y, 1, 1, +1);
-                zc2r(c, c->zP, 1, 1.);
+                zc2r(c, c->zP, 1, false, 1.);
                 break;
             case 4:  // r2c of s_d_bar
                 zr2c(c, c->zS, 1);
@@ -1478,13 +1576,13 @@ template <typename T, int N> struct Impl {
             case 5:  // r2c^T of the s cotangent, and c2r of the state's s
                 axis(c, c->jQ_x, 2, 0, +1);
                 axis(c, c->jQ_y, 2, 1, +1);
-                zc2r(c, c->zQ, 1, 1.);
+                zc2r(c, c->zQ, 1, false, 1.);
                 zc2r(c, c->zQ + 1, 1);
                 break;
             case 6:  // s_d only (the Poisson source of the state in Ys)
-                axis(c, c->jA_x, 2, 0, +1);
-                axis(c, c->jA_y, 3, 1, +1);
-                zc2r(c, c->zA, 1);
+                axis(c, c->jA_x, 2, 0, +1, AX_XM);
+                axis(c, c->jA_y, 3, 1, +1, AX_YI);
+                zc2r(c, c->zA, 1, true);
                 break;
         }
         CK(cudaGetLastError());
@@ -1631,6 +1729,20 @@ void build_tables(kf_ctx *c) {
         const std::vector<int> pb = dealias_bounds(q2, n, dealias_threshold());
         c->pb = dalloc<int>(c, sizeof(int) * pb.size());
         CK(cudaMemcpy(c->pb, pb.data(), sizeof(int) * pb.size(), cudaMemcpyHostToDevice));
+        const TruncTab t = trunc_table(pb, n, c->fp32 ? Tile<float>::TC : Tile<double>::TC);
+        if (t.nkz > 0 && !t.tl.empty()) {
+            c->tr_nkz = t.nkz;
+            c->tr_nt = (int)t.tl.size();
+            for (int b : pb)
+                if (b >= 0) {
+                    c->tr_ball += 2 * b + 1;
+                    c->tr_disc += n;
+                }
+            c->tr_jb = dalloc<int>(c, sizeof(int) * t.jb.size());
+            c->tr_tl = dalloc<int>(c, sizeof(int) * t.tl.size());
+            CK(cudaMemcpy(c->tr_jb, t.jb.data(), sizeof(int) * t.jb.size(), cudaMemcpyHostToDevice));
+            CK(cudaMemcpy(c->tr_tl, t.tl.data(), sizeof(int) * t.tl.size(), cudaMemcpyHostToDevice));
+        }
     }
     if (c->fp32) {
         std::vector<float> kvf(n), SVf(c->Nc), PFf(c->Nc), twf(2 * n);
@@ -1989,6 +2101,7 @@ void create(kf_ctx *c) {
     for (int q = 0; q < 4; ++q) {
         CK(cudaMemset(c->Y[q], 0, cb));
         CK(cudaMemset(c->Ys[q], 0, cb));
+        CK(cudaMemset(c->K[q], 0, cb));  // k_xfwd_assemble writes only what the 2/3 rule keeps
     }
     c->npartial = 1184;
     c->partial = dalloc<double>(c, sizeof(double) * KF_RED * c->npartial);

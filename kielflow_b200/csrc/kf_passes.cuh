@@ -121,13 +121,14 @@ template <typename T> struct AxisTile {
     T2 *out;
     int base, rstride;  // element indices: n * n * (n/2 + 1) < 2^31 for every supported n
     int jj, kk, mul;
+    int lb, sb;  // rows r with min(r, N - r) <= lb are loaded (the others are zero), <= sb stored
     bool valid;
 };
 
 // Tile `tile` of job `job` (global tile index tile * njobs + job), column c.
 template <typename T, int N>
 __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ jobs, int job, int tile, int axis,
-                                                 int c) {
+                                                 int c, const AxTrunc &A, const Geo<T> &g) {
     typedef typename C2<T>::type T2;
     constexpr int TC = Tile<T>::TC, n = N, nzc = N / 2 + 1;
     AxisTile<T> G;
@@ -137,23 +138,49 @@ __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ job
     G.mul = J.mul;
     G.jj = 0;
     G.kk = 0;
+    G.lb = G.sb = N / 2;
     if (axis == 0) {
-        const int col = tile * TC + c;
-        G.valid = col < n * nzc;
-        G.base = col;
         G.rstride = n * nzc;
-        G.jj = col / nzc;
-        G.kk = col - G.jj * nzc;
+        if (A.mode == AX_XM) {
+            const int w = A.tl[tile];
+            G.jj = w >> 16;
+            G.kk = (w & 0xffff) + c;
+            G.base = G.jj * nzc + G.kk;
+            G.lb = G.kk < A.nkz ? g.pb[G.base] : -1;
+            G.valid = G.lb >= 0;
+        } else {
+            const int col = tile * TC + c;
+            G.valid = col < n * nzc;
+            G.base = col;
+            G.jj = col / nzc;
+            G.kk = col - G.jj * nzc;
+        }
     } else {
         constexpr int tpp = (nzc + TC - 1) / TC;
-        const int plane = tile / tpp;
-        G.kk = (tile - plane * tpp) * TC + c;
-        G.valid = G.kk < nzc;
+        int plane;
+        if (A.mode == AX_FULL) {
+            plane = tile / tpp;
+            G.kk = (tile - plane * tpp) * TC + c;
+            G.valid = G.kk < nzc;
+        } else {
+            const int tq = (A.nkz + TC - 1) / TC;
+            plane = __float2int_rd(((float)tile + 0.5f) * A.itpp);  // tile / tq (exact: tile < 2^13)
+            G.kk = (tile - plane * tq) * TC + c;
+            G.valid = G.kk < A.nkz;
+            const int b = G.valid ? A.jb[G.kk] : -1;
+            if (A.mode == AX_YI)
+                G.lb = b;
+            else
+                G.sb = b;
+        }
         G.base = plane * n * nzc + G.kk;
         G.rstride = nzc;
     }
     return G;
 }
+
+// min(r, N - r), the |frequency| of row r
+template <int N> __device__ __forceinline__ int row_freq(int r) { return r <= N / 2 ? r : N - r; }
 
 // Resident blocks per SM that the transform kernels ask the register
 // allocator for: as many as their shared memory allows (TILES tiles of
@@ -204,7 +231,7 @@ template <typename T, int N, int SIGN, int V = 0>
 __global__ void __launch_bounds__(Tile<T>::TC * PlanV<N, V>::P,
                                   (KF_PIPE_MINB ? PipeMinBlocks<T, N, V, 1 + KF_PIPE_DEPTH, (KF_PIPE_MINB > 0 ? KF_PIPE_MINB : 1), 64>::value : 1))
 k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
-            const typename C2<T>::type *__restrict__ tw, int total) {
+            const typename C2<T>::type *__restrict__ tw, int total, AxTrunc A) {
     typedef typename C2<T>::type T2;
     constexpr int TC = Tile<T>::TC, P = PlanV<N, V>::P, E = N / P;
     constexpr int D = KF_PIPE_DEPTH;
@@ -233,13 +260,13 @@ k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
     // cp.async.wait_group D - 1 always leaves the current tile complete.
     auto prefetch = [&](int slot) {
         if (ptt < total) {
-            const AxisTile<T> G = axis_tile<T, N>(jobs, pj, pt, axis, c);
+            const AxisTile<T> G = axis_tile<T, N>(jobs, pj, pt, axis, c, A, g);
             T2 *st = stg0 + slot * (N * TC);
 #pragma unroll
             for (int q = 0; q < E; ++q) {
                 const int row = reg_row<N, P, PlanV<N, V>::R1>(p, q);
                 T2 *dst = st + row * TC + c;
-                if (G.valid)
+                if (G.valid && row_freq<N>(row) <= G.lb)
                     cp_async_copy(dst, G.in + G.base + row * G.rstride);
                 else
                     *dst = mk<T2>((T)0, (T)0);
@@ -253,12 +280,12 @@ k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
     for (int d = 0; d < D; ++d) prefetch(d);
     for (int it = 0; t < total; t += GS, ++it) {
         const int slot = it % D;
-        const AxisTile<T> cur = axis_tile<T, N>(jobs, cj, ct, axis, c);
+        const AxisTile<T> cur = axis_tile<T, N>(jobs, cj, ct, axis, c, A, g);
         adv(cj, ct);
-        // the 2/3 rule of this column as an index bound (one table read per tile)
-        const int pbnd = cur.valid && (cur.mul == MUL_P || cur.mul == MUL_P_IK)
-                             ? dealias_bound(g.pb, cur.jj, cur.kk, g.nzc)
-                             : -2;
+        // the 2/3 rule of this column as an index bound (one table read per
+        // tile); a masked pass has staged zeros outside it already
+        const bool mask = (cur.mul == MUL_P || cur.mul == MUL_P_IK) && A.mode == AX_FULL;
+        const int pbnd = cur.valid && mask ? dealias_bound(g.pb, cur.jj, cur.kk, g.nzc) : -2;
         cp_async_wait<D - 1>();
         const T2 *stg = stg0 + slot * (N * TC);
         T2 v[E];
@@ -266,7 +293,7 @@ k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
         for (int q = 0; q < E; ++q) {
             const int row = reg_row<N, P, PlanV<N, V>::R1>(p, q);
             T2 x = stg[row * TC + c];
-            if (cur.mul == MUL_P || cur.mul == MUL_P_IK) {
+            if (mask) {
                 if (!dealias_keep_b(g.q2, g.thr, pbnd, g.n, row, cur.jj, cur.kk)) x = mk<T2>((T)0, (T)0);
             }
             if (cur.mul == MUL_P_IK || cur.mul == MUL_IK) x = mul_ik(x, g.kv[row]);
@@ -278,7 +305,7 @@ k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
 #pragma unroll
             for (int q = 0; q < E; ++q) {
                 const int row = reg_row<N, P, PlanV<N, V>::RL>(p, q);
-                cur.out[cur.base + row * cur.rstride] = v[q];
+                if (row_freq<N>(row) <= cur.sb) cur.out[cur.base + row * cur.rstride] = v[q];
             }
         }
     }
@@ -309,7 +336,7 @@ template <typename T, int N, bool C2R> struct ZSmem {
 template <typename T, int N, int V = 0>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P, (sizeof(T) == 4 && KF_ZC2R_MINB > 0 ? KF_ZC2R_MINB : 1))
 k_z_c2r(const ZJob *__restrict__ jobs, int njobs, int nrows, Geo<T> g,
-        const typename C2<T>::type *__restrict__ tw, T scale) {
+        const typename C2<T>::type *__restrict__ tw, T scale, int nkz) {
     typedef typename C2<T>::type T2;
     constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1;
     constexpr int LS = PadLen<N>::value;  // padded line of the exchange buffer
@@ -321,33 +348,51 @@ k_z_c2r(const ZJob *__restrict__ jobs, int njobs, int nrows, Geo<T> g,
     const int r0 = tile * LZ;
     const T2 *inA = static_cast<const T2 *>(J.inA);
     const T2 *inB = static_cast<const T2 *>(J.inB);
+    const int p = threadIdx.x % P, l = threadIdx.x / P;
     // raw half spectra -> shared memory with asynchronous copies (all of a
     // thread's loads in flight at once); the multipliers are applied below.
-    // The tile's LZ rows of a half spectrum are one contiguous run of
-    // LZ * NZC elements from row r0.
     const int lim = (nrows - r0) * NZC;  // elements of the run inside the field
     const long off = (long)r0 * NZC;
-    for (int e = threadIdx.x; e < LZ * NZC; e += blockDim.x) {
-        if (e < lim) {
-            cp_async_copy(half + e, inA + off + e);
-            if (inB)
-                cp_async_copy(half + LZ * NZC + e, inB + off + e);
-            else
+    if (nkz == NZC) {
+        // the tile's LZ rows of a half spectrum are one contiguous run of
+        // LZ * NZC elements from row r0
+        for (int e = threadIdx.x; e < LZ * NZC; e += blockDim.x) {
+            if (e < lim) {
+                cp_async_copy(half + e, inA + off + e);
+                if (inB)
+                    cp_async_copy(half + LZ * NZC + e, inB + off + e);
+                else
+                    half[LZ * NZC + e] = mk<T2>((T)0, (T)0);
+            } else {
+                half[e] = mk<T2>((T)0, (T)0);
                 half[LZ * NZC + e] = mk<T2>((T)0, (T)0);
-        } else {
-            half[e] = mk<T2>((T)0, (T)0);
-            half[LZ * NZC + e] = mk<T2>((T)0, (T)0);
+            }
+        }
+    } else {
+        // spectra that are zero from kz = nkz on: only that part of each row
+        for (int k = p; k < nkz; k += P) {
+            const int e = l * NZC + k;
+            if (e < lim) {
+                cp_async_copy(half + e, inA + off + e);
+                if (inB)
+                    cp_async_copy(half + LZ * NZC + e, inB + off + e);
+                else
+                    half[LZ * NZC + e] = mk<T2>((T)0, (T)0);
+            } else {
+                half[e] = mk<T2>((T)0, (T)0);
+                half[LZ * NZC + e] = mk<T2>((T)0, (T)0);
+            }
         }
     }
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
-    const int p = threadIdx.x % P, l = threadIdx.x / P;
     const T2 *hA = half + l * NZC;
     const T2 *hB = half + LZ * NZC + l * NZC;
     // staged element kk (0 <= kk < NZC) times its job's multiplier, with the
     // imaginary parts of the kz = 0 and kz = n/2 bins dropped
     auto staged = [&](const T2 *h, int kk, int mul) {
+        if (kk >= nkz) return mk<T2>((T)0, (T)0);
         T2 x = h[kk];
         if (mul == MUL_IK) x = mul_ik(x, g.kv[kk]);
         if (mul == MUL_HALF && kk > 0 && 2 * kk < N) x = mk<T2>((T)0.5 * x.x, (T)0.5 * x.y);
@@ -389,7 +434,7 @@ k_z_c2r(const ZJob *__restrict__ jobs, int njobs, int nrows, Geo<T> g,
 template <typename T, int N, int V = 0>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
 k_z_r2c(const ZJob *__restrict__ jobs, int njobs, int nrows,
-        const typename C2<T>::type *__restrict__ tw) {
+        const typename C2<T>::type *__restrict__ tw, int nkz) {
     typedef typename C2<T>::type T2;
     constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1;
     constexpr int LS = PadLen<N>::value;
@@ -420,18 +465,25 @@ k_z_r2c(const ZJob *__restrict__ jobs, int njobs, int nrows,
 #pragma unroll
     for (int q = 0; q < E; ++q) line[pa(reg_row<N, P, PlanV<N, V>::RL>(p, q))] = v[q];
     __syncthreads();
-    // the tile's LZ output rows of a half spectrum are one contiguous run of
-    // LZ * NZC elements from row r0
     const int lim = (nrows - r0) * NZC;
     T2 *oA = static_cast<T2 *>(J.outA) + (long)r0 * NZC;
     T2 *oB = J.outB ? static_cast<T2 *>(J.outB) + (long)r0 * NZC : nullptr;
-    for (int idx = threadIdx.x; idx < LZ * NZC && idx < lim; idx += blockDim.x) {
-        const int ll = idx / NZC, k = idx - ll * NZC;
+    auto put = [&](int idx, int ll, int k) {
         const T2 zk = xch[ll * LS + pa(k)];
         const T2 zm = xch[ll * LS + pa(k == 0 ? 0 : N - k)];
         const T cr = zm.x, ci = -zm.y;  // conj(Z[N-k])
         oA[idx] = mk<T2>((T)0.5 * (zk.x + cr), (T)0.5 * (zk.y + ci));
         if (oB) oB[idx] = mk<T2>((T)0.5 * (zk.y - ci), (T)-0.5 * (zk.x - cr));
+    };
+    if (nkz == NZC) {
+        // the tile's LZ output rows of a half spectrum are one contiguous run
+        // of LZ * NZC elements from row r0
+        for (int idx = threadIdx.x; idx < LZ * NZC && idx < lim; idx += blockDim.x) {
+            const int ll = idx / NZC;
+            put(idx, ll, idx - ll * NZC);
+        }
+    } else {  // only kz < nkz is used by what follows
+        for (int k = p; k < nkz && l * NZC + k < lim; k += P) put(l * NZC + k, l, k);
     }
 }
 
@@ -523,7 +575,7 @@ template <typename T, int N, int V = 0, bool PEN = false>
 __global__ void __launch_bounds__(Tile<T>::TC * PlanV<N, V>::P,
                                   (PEN ? PipeMinBlocks<T, N, V, 1, sizeof(T) == 4 ? 4 : 2, 64>::value : 1))
 k_xfwd_assemble(const AxisJob *__restrict__ jobs, Geo<T> g, RhsArgs<T> a,
-                const typename C2<T>::type *__restrict__ tw) {
+                const typename C2<T>::type *__restrict__ tw, AxTrunc A) {
     typedef typename C2<T>::type T2;
     constexpr int TC = Tile<T>::TC, P = PlanV<N, V>::P, E = N / P;
     extern __shared__ __align__(16) unsigned char kf_smem[];
@@ -531,10 +583,20 @@ k_xfwd_assemble(const AxisJob *__restrict__ jobs, Geo<T> g, RhsArgs<T> a,
     const int tile = blockIdx.x;
     const int c = threadIdx.x % TC, p = threadIdx.x / TC;
     const int n = g.n, nzc = g.nzc;
-    const int col = tile * TC + c;
-    const bool valid = col < n * nzc;
+    // A.mode AX_XM (penalization form only): the columns the 2/3 rule keeps,
+    // and of K the rows it keeps (K is zero elsewhere since its allocation)
+    const bool act = PEN && A.mode == AX_XM;
+    int col = tile * TC + c;
+    bool valid = col < n * nzc;
+    int jj = col / nzc, kk = col - jj * nzc;
+    if (act) {
+        const int w = A.tl[tile];
+        jj = w >> 16;
+        kk = (w & 0xffff) + c;
+        col = jj * nzc + kk;
+        valid = kk < A.nkz && g.pb[col] >= 0;
+    }
     const long rstride = (long)n * nzc;
-    const int jj = col / nzc, kk = col - jj * nzc;
     const int b = valid ? dealias_bound(g.pb, jj, kk, nzc) : -2;
     for (int q = 0; q < 4; ++q) {
         const T2 *__restrict__ in = static_cast<const T2 *>(jobs[q].in);
@@ -554,6 +616,7 @@ k_xfwd_assemble(const AxisJob *__restrict__ jobs, Geo<T> g, RhsArgs<T> a,
                 T2 F = v[e];
                 T2 K;
                 if constexpr (PEN) {
+                    if (act && row_freq<N>(i) > b) continue;
                     K = dealias_keep_b(g.q2, g.thr, b, N, i, jj, kk) ? F : mk<T2>((T)0, (T)0);
                 } else {
                     T2 fb = lin_term(a, g, q, i, jj, kk, idx, b);

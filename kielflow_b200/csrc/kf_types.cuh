@@ -52,6 +52,25 @@ template <typename T> struct Geo {
     const int *pb;     // per (j, kz) column: the 2/3 rule along i as a bound (dealias_bounds), or nullptr
 };
 
+// Which part of a half spectrum an x / y pass moves (uniform over a launch).
+// The 2/3 rule keeps a ball of radius n/3: 16 % of a half spectrum, the columns
+// (j, kz) of a disc (35 %) once x is transformed, kz < nkz (67 %) once y is.
+// A pass over a masked field reads, transforms and writes only those parts; the
+// next pass knows that the rest is zero and does not read it.
+enum AxMode : int {
+    AX_FULL = 0,  // everything
+    AX_XM = 1,    // x pass, masked input: active columns, rows within the column's bound -> every row
+    AX_YI = 2,    // y pass after AX_XM: columns kz < nkz, rows j within jb[kz] -> every row
+    AX_YF = 3,    // forward y pass whose x pass needs only active columns: every row -> rows within jb[kz]
+};
+struct AxTrunc {
+    int mode;
+    int nkz;        // columns kz < nkz are active
+    float itpp;     // 1 / column tiles per plane of AX_YI, AX_YF
+    const int *jb;  // per kz < nkz: largest min(j, n - j) of an active column
+    const int *tl;  // active x-pass tiles: (j << 16) | first kz
+};
+
 // sqrt is correctly rounded and monotone, so sqrt(s) < 2/3 holds exactly when
 // s < thr for the smallest double thr with sqrt(thr) >= 2/3: the 2/3 rule of
 // rhs_standard.cpp:22 on |k~| (OP_dealiasing.hpp:28) without a square root.

@@ -1,0 +1,257 @@
+// kf_zprod.cuh -- the z-local middle of the right-hand side in one kernel: the
+// inverse z transforms of u', s and their derivatives, the physical-space
+// products (k_products' terms) and the forward z transform of the four results.
+//
+// Everything between the y passes is local to a z line (i, j), so the 16 real
+// fields of round D never go to memory.  A block of 8 groups of P threads (a
+// group carries one packed complex line) takes ZP_ROWS rows in turn: per row the 16
+// real lines are 8 packed c2r lines,
+//   lines 0-2: U_c + i d_z U_c        lines 3-5: d_y U_c + i d_x U_c
+//   line  6  : d_y s + i d_x s        line  7  : s_d + i d_z s
+// whose 8 groups transform them at once; the products of the row's z points
+// give 4 real lines = 2 packed lines, kept in shared memory for one forward
+// transform of all rows' results at the end.
+//
+// 256^3 FP32, one right-hand side: the three passes it replaces (k_z_c2r 491 us,
+// k_products 305 us, k_z_r2c 74 us) wrote and read 40 real fields on the way.
+#pragma once
+
+#include "kf_passes.cuh"
+#include "kf_types.cuh"
+
+namespace kf {
+
+// Two rows at a time leave half of the groups idle in the forward transform but
+// fit 8 blocks per SM where 4 rows fit 6 (256^3 FP32: 497 us against 553 us).
+constexpr int ZP_ROWS = 2, ZP_LINES = 8;
+
+// Resident blocks per SM asked of the register allocator: 64 registers a thread
+// in FP32, 128 in FP64, what the shared memory of a 256-point block allows as
+// well.  The kernel is bound by latency (a third of the issue slots used without
+// the request), so residency is time.  256^3, products without penalization:
+// FP32 861 us with 159 registers and 3 blocks, 497 us with 64 and 8; FP64 1657 us
+// with 226 and 2, 1031 us with 128 and 4.
+template <typename T, int N, int V> struct ZProdMinBlocks {
+    static constexpr int by_regs = (sizeof(T) == 4 ? 1024 : 512) / (ZP_LINES * PlanV<N, V>::P);
+    static constexpr int value = by_regs < 12 ? by_regs : 12;
+};
+
+template <typename T> struct ZProdArgs {
+    typedef typename C2<T>::type T2;
+    const T2 *s0, *sy, *sx;             // y-passed spectra of P s, d_y s, d_x s
+    const T2 *u[3], *uy[3], *ux[3];     // of U_c, d_y U_c, d_x U_c
+    T2 *out[4];                         // z-transformed results, half spectra
+    const T *rl[4];                     // c2r(-lin_q)   (penalization only)
+    const T *H;                         // mask          (penalization only)
+    T M, eta, scale;                    // scale: the 1/N of the c2r
+    int terms;
+    int nkz;  // the inputs are zero from kz = nkz on
+    int nko;  // outputs are needed for kz < nko
+};
+
+template <typename T, int N> struct ZProdSmem {
+    typedef typename C2<T>::type T2;
+    static constexpr int LS = PadLen<N>::value;
+    // exchange / line buffers, and the packed results of ZP_ROWS rows
+    static constexpr size_t bytes = (size_t)(ZP_LINES * LS + 2 * ZP_ROWS * N) * sizeof(T2);
+};
+
+template <typename T, int N, int V>
+__global__ void __launch_bounds__(ZP_LINES * PlanV<N, V>::P, ZProdMinBlocks<T, N, V>::value)
+k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
+        const typename C2<T>::type *__restrict__ tw) {
+    typedef typename C2<T>::type T2;
+    constexpr int P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1, LS = PadLen<N>::value;
+    constexpr int NT = ZP_LINES * P;
+    extern __shared__ __align__(16) unsigned char kf_smem[];
+    T2 *xch = reinterpret_cast<T2 *>(kf_smem);  // [ZP_LINES][LS]
+    T2 *res = xch + ZP_LINES * LS;              // [2 ZP_ROWS][N]
+    const int p = threadIdx.x % P, l = threadIdx.x / P;
+    const int r0 = blockIdx.x * ZP_ROWS;
+    // this group's line: half spectra A and B (B == nullptr: i kz A)
+    const T2 *__restrict__ inA = l < 3 ? a.u[l] : l < 6 ? a.uy[l - 3] : l == 6 ? a.sy : a.s0;
+    const T2 *__restrict__ inB = l < 3 ? nullptr : l < 6 ? a.ux[l - 3] : l == 6 ? a.sx : nullptr;
+    T2 *line = xch + l * LS;
+    const PadAddr pa;
+    const bool adv = a.terms & T_ADVECTION, cont = a.terms & T_CONTINUITY, pen = a.terms & T_PENALIZATION;
+#pragma unroll 1
+    for (int rr = 0; rr < ZP_ROWS; ++rr) {
+        const long off = (long)(r0 + rr) * NZC;
+        T2 v[E];
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            const int k = reg_row<N, P, PlanV<N, V>::R1>(p, q);
+            const int kk = k < NZC ? k : N - k;
+            T2 x = mk<T2>((T)0, (T)0), y = x;
+            if (kk < a.nkz) {
+                x = __ldg(inA + off + kk);
+                y = inB ? __ldg(inB + off + kk) : mul_ik(x, kv[kk]);
+            }
+            if (kk == 0 || 2 * kk == N) x.y = y.y = (T)0;  // as a c2r transform does
+            if (k >= NZC) {
+                x.y = -x.y;
+                y.y = -y.y;
+            }
+            v[q] = mk<T2>(x.x - y.y, x.y + y.x);  // A + iB
+        }
+        PlanV<N, V>::template fft<T2, +1>(v, line, pa, p, tw);  // its last exchange ends with a barrier
+#pragma unroll
+        for (int q = 0; q < E; ++q)
+            line[reg_row<N, P, PlanV<N, V>::RL>(p, q)] = mk<T2>(v[q].x * a.scale, v[q].y * a.scale);
+        __syncthreads();
+        for (int z = threadIdx.x; z < N; z += NT) {
+            const T2 U0 = xch[z], U1 = xch[LS + z], U2 = xch[2 * LS + z];  // (U_c, d_z U_c)
+            const T ux = U0.x, uy = U1.x, uz = U2.x;
+            const T2 S = xch[6 * LS + z], S0 = xch[7 * LS + z];  // (d_y s, d_x s), (s_d, d_z s)
+            T pr[4];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                T s = (T)0;
+                if (adv) {
+                    const T2 d = xch[(3 + c) * LS + z];  // (d_y U_c, d_x U_c)
+                    s = ux * d.y;
+                    s += uy * d.x;
+                    s += uz * (c == 0 ? U0.y : c == 1 ? U1.y : U2.y);
+                }
+                pr[c] = s;
+            }
+            {
+                T s = (T)0;
+                if (cont) {
+                    s = S.y * ux;
+                    s += S.x * uy;
+                    s += S0.y * uz;
+                }
+                pr[3] = s;
+            }
+            if (pen) {
+                const long i = (long)(r0 + rr) * N + z;
+                const T h = a.H[i];
+                const T qd[4] = {ux, uy, uz, S0.x};
+                const T qfix[4] = {-a.M, (T)0, (T)0, (T)-10};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const T r = a.rl[q][i] - pr[q];
+                    pr[q] = ((T)1 - h) * r + h * a.eta * (qd[q] - qfix[q]);
+                }
+            }
+            res[(2 * rr) * N + z] = mk<T2>(pr[0], pr[1]);
+            res[(2 * rr + 1) * N + z] = mk<T2>(pr[2], pr[3]);
+        }
+        __syncthreads();
+    }
+    // forward: group l < 2 ZP_ROWS carries the packed line l & 1 of row l / 2
+    T2 v[E];
+#pragma unroll
+    for (int q = 0; q < E; ++q) v[q] = res[(l % (2 * ZP_ROWS)) * N + reg_row<N, P, PlanV<N, V>::R1>(p, q)];
+    PlanV<N, V>::template fft<T2, -1>(v, line, pa, p, tw);
+#pragma unroll
+    for (int q = 0; q < E; ++q) line[pa(reg_row<N, P, PlanV<N, V>::RL>(p, q))] = v[q];
+    __syncthreads();
+    if (l >= 2 * ZP_ROWS) return;
+    const long off = (long)(r0 + l / 2) * NZC;
+    T2 *oA = a.out[2 * (l & 1)] + off, *oB = a.out[2 * (l & 1) + 1] + off;
+    for (int k = p; k < a.nko; k += P) {
+        const T2 zk = line[pa(k)];
+        const T2 zm = line[pa(k == 0 ? 0 : N - k)];
+        const T cr = zm.x, ci = -zm.y;  // conj(Z[N-k])
+        oA[k] = mk<T2>((T)0.5 * (zk.x + cr), (T)0.5 * (zk.y + ci));
+        oB[k] = mk<T2>((T)0.5 * (zk.y - ci), (T)-0.5 * (zk.x - cr));
+    }
+}
+
+// z pass of one field, two of its rows (2 m, 2 m + 1) packed into a complex
+// line; ZTile<T>::LZ lines per block, n^2 / (2 LZ) blocks.
+//
+// Inverse, with the Poisson source as the epilogue: s_d = c2r(P s^) and
+// rho = e^{s_d} + n_d in FP64 (rhs_standard.cpp:108-111), into rho and, when
+// given, its colour-split copy (k_rho_split's layout); sd is written when given.
+template <typename T, int N, int V>
+__global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
+k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, const double *__restrict__ nd,
+        double *__restrict__ rho, double *__restrict__ rcs, const typename C2<T>::type *__restrict__ tw, T scale,
+        int nkz) {
+    typedef typename C2<T>::type T2;
+    constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1, LS = PadLen<N>::value;
+    extern __shared__ __align__(16) unsigned char kf_smem[];
+    T2 *xch = reinterpret_cast<T2 *>(kf_smem);  // [LZ][LS]
+    const int p = threadIdx.x % P, l = threadIdx.x / P;
+    const int r = 2 * (blockIdx.x * LZ + l);
+    const long off = (long)r * NZC;
+    T2 v[E];
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        const int k = reg_row<N, P, PlanV<N, V>::R1>(p, q);
+        const int kk = k < NZC ? k : N - k;
+        T2 x = mk<T2>((T)0, (T)0), y = x;
+        if (kk < nkz && r < N * N) {
+            x = __ldg(in + off + kk);
+            y = __ldg(in + off + NZC + kk);
+        }
+        if (kk == 0 || 2 * kk == N) x.y = y.y = (T)0;
+        if (k >= NZC) {
+            x.y = -x.y;
+            y.y = -y.y;
+        }
+        v[q] = mk<T2>(x.x - y.y, x.y + y.x);
+    }
+    PlanV<N, V>::template fft<T2, +1>(v, xch + l * LS, PadAddr{}, p, tw);
+    if (r >= N * N) return;
+    const int c0 = (r / N + r % N) & 1;  // colour of z = 0 in row r (row r + 1: the other one)
+    constexpr long half = (long)N * N * (N / 2);
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        const int z = reg_row<N, P, PlanV<N, V>::RL>(p, q);
+        const long ia = (long)r * N + z, ib = ia + N;
+        const T sa = v[q].x * scale, sb = v[q].y * scale;
+        const double ra = exp((double)sa) + nd[ia], rb = exp((double)sb) + nd[ib];
+        if (sd) {
+            sd[ia] = sa;
+            sd[ib] = sb;
+        }
+        rho[ia] = ra;
+        rho[ib] = rb;
+        if (rcs) {
+            const int c = (c0 + z) & 1;
+            rcs[c * half + (ia >> 1)] = ra;
+            rcs[(c ^ 1) * half + (ib >> 1)] = rb;
+        }
+    }
+}
+
+// Forward, of the FP64 potential in the bulk precision: out = the half spectra
+// of phi's rows, kz < nko.
+template <typename T, int N, int V>
+__global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
+k_z_phi(const double *__restrict__ phi, typename C2<T>::type *__restrict__ out,
+        const typename C2<T>::type *__restrict__ tw, int nko) {
+    typedef typename C2<T>::type T2;
+    constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1, LS = PadLen<N>::value;
+    extern __shared__ __align__(16) unsigned char kf_smem[];
+    T2 *xch = reinterpret_cast<T2 *>(kf_smem);  // [LZ][LS]
+    const int p = threadIdx.x % P, l = threadIdx.x / P;
+    const int r = 2 * (blockIdx.x * LZ + l);
+    T2 *line = xch + l * LS;
+    const PadAddr pa;
+    T2 v[E];
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        const long i = (long)r * N + reg_row<N, P, PlanV<N, V>::R1>(p, q);
+        v[q] = r < N * N ? mk<T2>((T)phi[i], (T)phi[i + N]) : mk<T2>((T)0, (T)0);
+    }
+    PlanV<N, V>::template fft<T2, -1>(v, line, pa, p, tw);
+#pragma unroll
+    for (int q = 0; q < E; ++q) line[pa(reg_row<N, P, PlanV<N, V>::RL>(p, q))] = v[q];
+    __syncthreads();
+    if (r >= N * N) return;
+    T2 *oA = out + (long)r * NZC, *oB = oA + NZC;
+    for (int k = p; k < nko; k += P) {
+        const T2 zk = line[pa(k)];
+        const T2 zm = line[pa(k == 0 ? 0 : N - k)];
+        const T cr = zm.x, ci = -zm.y;
+        oA[k] = mk<T2>((T)0.5 * (zk.x + cr), (T)0.5 * (zk.y + ci));
+        oB[k] = mk<T2>((T)0.5 * (zk.y - ci), (T)-0.5 * (zk.x - cr));
+    }
+}
+
+}  // namespace kf

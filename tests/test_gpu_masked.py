@@ -1,0 +1,53 @@
+"""Masked transform passes (only what the 2/3 rule keeps is moved): right-hand
+sides of states whose spectra are full, against the CPU oracle.  White noise
+puts as much into the removed wave numbers as into the kept ones, so a wrong
+bound of a pass, a stale value outside one or a missing edge element shows."""
+import numpy as np
+import pytest
+
+import kielflow_b200 as kf
+from kielflow_b200 import configs as C
+from kielflow_b200 import inputs as I
+from oracle import bind
+
+pytestmark = pytest.mark.gpu
+
+NO_PHI = kf.KF_T_ALL & ~(kf.KF_T_POISSON | kf.KF_T_E_INT)
+
+
+def noise_state(n, seed):
+    rng = np.random.default_rng(seed)
+    return [1e-2 * bind.r2c(rng.standard_normal((n, n, n))) for _ in range(4)]
+
+
+def oracle_rhs(cfg, st, nd, mask):
+    o = bind.Oracle(bind.KfoConfig(*[getattr(cfg, f) for f, _ in bind.KfoConfig._fields_]))
+    o.set_state(st)
+    o.set_sources(nd, mask)
+    o.rhs()
+    return o.get_state()
+
+
+@pytest.mark.parametrize("plan", [0, 1])
+@pytest.mark.parametrize("prec", [kf.KF_FP64, kf.KF_FP32_BULK])
+@pytest.mark.parametrize("pen", [True, False])
+@pytest.mark.parametrize("n", [16, 32, 64, 96, 128])
+def test_full_spectrum_rhs_vs_oracle(n, pen, prec, plan):
+    w = C.WORKLOADS["fas128"]
+    terms = NO_PHI if pen else NO_PHI & ~kf.KF_T_PENALIZATION
+    cfg = C.config_for(w, n=n, precision=prec, terms=terms)
+    nd = I.gauss_charge(n, C.L_BOX, w["Q"], w["sigma"])
+    mask = I.sphere_mask(n, C.L_BOX, 2.0)
+    st = noise_state(n, n)
+    with kf.Context(cfg) as ctx:
+        ctx.set_tuning(plan, 8)
+        ctx.set_state(*noise_state(n, n + 1))  # another state first: whatever it leaves outside the
+        ctx.set_sources(nd, mask)              # bounds must not reach the second result
+        ctx.rhs()
+        ctx.set_state(*st)
+        ctx.rhs()
+        g = ctx.get_state()
+    r = oracle_rhs(cfg, st, nd, mask)
+    scale = max(np.abs(x).max() for x in r)
+    err = max(np.abs(a - b).max() for a, b in zip(g, r)) / scale
+    assert err < (1e-12 if prec == kf.KF_FP64 else 1e-5)
