@@ -5,12 +5,14 @@
 //   A  inverse x/y passes of s^ (P s^, i k_x P s^, i k_y P s^) and the z pass of
 //      P s^  ->  s_d;  rho = exp(s_d) + n_d;  Poisson solve -> phi
 //   B  phi^ = r2c(phi)                                    (E-force, :218-226)
-//   C  (penalization) rl_q = -lin_q in k-space
-//   D  inverse passes generating U_c, d_d U_c, d_d s (and c2r(rl_q))
-//   E  physical-space products (advection, u.grad s) [+ penalization]
-//   F  forward z/y passes, then the forward x pass fused with the assembly
-//      K_q = -(lin_q + F_q)   (or P F_q with penalization)
-// RK4 (RKO4.cpp:50-241) combines four such evaluations with k_rk.
+//   C  -lin_q in k-space (k_lin); with penalization also c2r(-lin_q) on the
+//      window of rows on which the mask is not zero
+//   D  inverse x / y passes generating U_c, d_d U_c, d_d s
+//   E  k_zprod: their inverse z pass, the physical-space products (advection,
+//      u.grad s) [+ penalization] and the forward z pass of the results
+//   F  forward y pass, then the forward x pass fused with the assembly
+//      K_q = -lin_q + F_q (inside the 2/3 rule with penalization) and with the
+//      RK4 stage update (RKO4.cpp:50-241) that uses it
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -94,8 +96,7 @@ struct kf_ctx {
     void *kv = nullptr, *SV = nullptr, *PF = nullptr, *tw = nullptr;
     double *q2 = nullptr;
     int *pb = nullptr;  // x-pass 2/3-rule bounds per (j, kz) column (dealias_bounds)
-    // the kept part of a masked half spectrum (AxTrunc; tr_nkz 0: its bounds
-    // do not hold on this grid and every pass is AX_FULL)
+    // the kept part of a masked half spectrum (AxTrunc)
     int tr_nkz = 0, tr_nt = 0;
     double tr_ball = 0., tr_disc = 0.;  // elements kept; elements of the active columns
     int *tr_jb = nullptr, *tr_tl = nullptr;
@@ -164,6 +165,13 @@ struct kf_ctx {
     int cc_level = -1;         // entry level of k_coarse_cycle, or -1 (cc_setup)
     CoarseCycle ccyc{};
     size_t cc_smem = 0;
+    // window of rows (i, j) on which the penalization mask is not zero
+    // (k_mask_box; bi = 0: none)
+    int bx_i0 = 0, bx_i = 0, bx_j0 = 0, bx_j = 0;
+    int *d_box = nullptr;
+    // what the end of the right-hand side does with K (k_xfwd_stage; 3: store it)
+    int rk_mode = 3;
+    double rk_c = 0.;
     int stage_idx = 0;  // RK stage of the right-hand side being evaluated (0..3)
     // one RK4 step captured as a CUDA graph (FAS or no Poisson, profile off):
     // time / warm-start history and solve statistics live on the device
@@ -218,7 +226,7 @@ enum KCls { KC_AXIS_INV, KC_AXIS_FWD, KC_Z_C2R, KC_Z_R2C, KC_XASM, KC_PROD, KC_L
             KC_MG_COARSE, KC_MARCH, KC_MARCH_RES,
             KC_N };
 const char *const kKClsName[KC_N] = {"k_axis_pass(inverse)", "k_axis_pass(forward)", "k_z_c2r", "k_z_r2c",
-                                     "k_xfwd_assemble", "k_products", "k_lin", "k_rho", "k_rk", "k_jacobi",
+                                     "k_xfwd_stage", "k_zprod/k_products", "k_lin", "k_rho", "k_rk", "k_jacobi",
                                      "k_rbgs", "k_residual", "k_restrict/k_fas_rhs/k_prolong/k_inject",
                                      "k_coarse_solve/k_coarse_cycle", "k_reduce_final", "conversion/diagnostics",
                                      "adjoint pointwise (k_prod_vjp/k_vjp_assemble/k_adj_stage/...)",
@@ -365,7 +373,9 @@ std::vector<int> dealias_bounds(const std::vector<double> &q2, int n, double thr
 // The kept part of a masked half spectrum from its x-pass bounds pb: nkz and
 // jb[kz] such that the column (j, kz) has a kept element exactly when kz < nkz
 // and min(j, n - j) <= jb[kz], and the x-pass tiles of tc columns that cover
-// those columns.  nkz = 0 when some column does not fit that form.
+// those columns.  (q2 grows with |frequency| and is the same for both signs, and
+// rounded sums keep that order, so every column fits this form; a column that
+// did not is an error.)
 struct TruncTab {
     int nkz = 0;
     std::vector<int> jb, tl;
@@ -383,7 +393,8 @@ TruncTab trunc_table(const std::vector<int> &pb, int n, int tc) {
     for (int j = 0; j < n; ++j)
         for (int k = 0; k < nzc; ++k) {
             const int b = pb[(size_t)j * nzc + k];
-            if (b == -2 || (b >= 0) != ((j <= n / 2 ? j : n - j) <= jb[k])) return t;
+            if (b == -2 || (b >= 0) != ((j <= n / 2 ? j : n - j) <= jb[k]))
+                throw KfError{KF_ERR_ARG, "the 2/3 rule has no index bounds on this grid"};
         }
     t.nkz = nkz;
     t.jb = jb;
@@ -1121,8 +1132,7 @@ template <typename T, int N> struct Impl {
         CK(cudaFuncSetAttribute(k_zprod<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_rho<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_phi<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        CK(cudaFuncSetAttribute(k_xfwd_assemble<T, N, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        CK(cudaFuncSetAttribute(k_xfwd_assemble<T, N, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        CK(cudaFuncSetAttribute(k_xfwd_stage<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     }
 
     // distinct inputs and outputs of a launch, each as far as the mode moves it
@@ -1135,9 +1145,11 @@ template <typename T, int N> struct Impl {
             if (!seen) u.push_back(p);
         }
         double fin = (double)c->Nc, fout = fin;
-        if (c->tr_nkz && mode == AX_XM) fin = c->tr_ball, fout = c->tr_disc;
-        if (c->tr_nkz && mode == AX_YI) fin = c->tr_disc, fout = (double)N * N * c->tr_nkz;
-        if (c->tr_nkz && mode == AX_YF) fin = (double)N * N * c->tr_nkz, fout = c->tr_disc;
+        if (mode == AX_XM) fin = c->tr_ball, fout = c->tr_disc;
+        if (mode == AX_YI) fin = c->tr_disc, fout = (double)N * N * c->tr_nkz;
+        if (mode == AX_XB) fout = (double)c->bx_i * N * NZC;
+        if (mode == AX_YB) fin = (double)c->bx_i * N * NZC, fout = (double)c->bx_i * c->bx_j * NZC;
+        if (mode == AX_YF) fin = (double)N * N * c->tr_nkz, fout = c->tr_disc;
         return (u.size() * fin + njobs * fout) * sizeof(T2);
     }
     // resident blocks per SM x SMs of the pipelined pass (its grid)
@@ -1157,10 +1169,15 @@ template <typename T, int N> struct Impl {
         }
         return v;
     }
-    // AX_FULL when the grid's 2/3 rule has no truncated form (tr_nkz == 0)
     static AxTrunc trunc(kf_ctx *c, int mode) {
-        AxTrunc A{AX_FULL, NZC, 0.f, nullptr, nullptr};
-        if (mode == AX_FULL || !c->tr_nkz) return A;
+        AxTrunc A{AX_FULL, NZC, 0.f, nullptr, nullptr, 0, N};
+        if (mode == AX_XB || mode == AX_YB) {
+            A.mode = mode;
+            A.r0 = mode == AX_XB ? c->bx_i0 : c->bx_j0;
+            A.rm = mode == AX_XB ? c->bx_i : c->bx_j;
+            return A;
+        }
+        if (mode == AX_FULL) return A;
         A.mode = mode;
         A.nkz = c->tr_nkz;
         A.itpp = 1.f / (float)((c->tr_nkz + TC - 1) / TC);
@@ -1169,12 +1186,12 @@ template <typename T, int N> struct Impl {
         return A;
     }
     // kz extent of a z pass over masked fields
-    static int nkz(kf_ctx *c, bool masked) { return masked && c->tr_nkz ? c->tr_nkz : NZC; }
+    static int nkz(kf_ctx *c, bool masked) { return masked ? c->tr_nkz : NZC; }
     template <int V> static void axis_v(kf_ctx *c, int off, int njobs, int ax, int sign, int mode) {
         const AxTrunc A = trunc(c, mode);
         const int ntiles = A.mode == AX_XM ? c->tr_nt
                            : ax == 0       ? (N * NZC + TC - 1) / TC
-                                           : N * ((A.nkz + TC - 1) / TC);
+                                           : (A.mode == AX_YB ? c->bx_i : N) * ((A.nkz + TC - 1) / TC);
         const int total = njobs * ntiles, grid = std::min(total, pipe_grid<V>(sign));
         const size_t smem = axis_pipe_smem<T, N>(njobs);
         if (sign < 0)
@@ -1191,7 +1208,7 @@ template <typename T, int N> struct Impl {
         else
             axis_v<0>(c, off, njobs, ax, sign, mode);
     }
-    static double z_bytes(kf_ctx *c, int off, int njobs, bool c2r, bool masked) {
+    static double z_bytes(kf_ctx *c, int off, int njobs, bool c2r, bool masked, int nrows = N * N) {
         std::vector<const void *> u;
         int outs = 0;
         for (int j = 0; j < njobs; ++j) {
@@ -1204,16 +1221,15 @@ template <typename T, int N> struct Impl {
             }
             outs += (z.outA ? 1 : 0) + (z.outB ? 1 : 0);
         }
-        const double cb = (double)N * N * nkz(c, masked) * sizeof(T2), rb = (double)c->N * sizeof(T);
+        const double cb = (double)nrows * nkz(c, masked) * sizeof(T2), rb = (double)nrows * N * sizeof(T);
         return c2r ? u.size() * cb + outs * rb : u.size() * rb + outs * cb;
     }
     // scale < 0: the 1/N of c2r; otherwise the given factor (1 for transposes)
     // masked: the half spectra come from masked x / y passes (zero from kz = nkz on)
-    static void zc2r(kf_ctx *c, int off, int njobs, bool masked = false, double scale = -1.) {
-        const int nrows = N * N;
+    static void zc2r(kf_ctx *c, int off, int njobs, bool masked = false, double scale = -1., int nrows = N * N) {
         const int ntiles = (nrows + LZ - 1) / LZ;
         const size_t smem = ZSmem<T, N, true>::bytes;
-        Launch L_(c, KC_Z_C2R, z_bytes(c, off, njobs, true, masked));
+        Launch L_(c, KC_Z_C2R, z_bytes(c, off, njobs, true, masked, nrows));
         const T sc = (T)(scale < 0. ? 1. / ((double)N * N * N) : scale);
         if (c->fftv)
             k_z_c2r<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
@@ -1299,6 +1315,12 @@ template <typename T, int N> struct Impl {
             a.rl[q] = (const T *)c->R[16 + q];
         }
         a.H = (const T *)c->H;
+        if (pen) {
+            a.i0 = c->bx_i0;
+            a.bi = c->bx_i;
+            a.j0 = c->bx_j0;
+            a.bj = c->bx_j;
+        }
         a.M = (T)c->cfg.M;
         a.eta = (T)c->cfg.pen_eta;
         a.scale = (T)(1. / ((double)N * N * N));
@@ -1306,7 +1328,7 @@ template <typename T, int N> struct Impl {
         a.nkz = nkz(c, true);
         a.nko = nkz(c, pen);
         const size_t smem = ZProdSmem<T, N>::bytes;
-        Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko) + (pen ? 5. * c->N * sizeof(T) : 0.));
+        Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko) + 5. * a.bi * a.bj * N * sizeof(T));
         if (c->fftv)
             k_zprod<T, N, 1><<<N * N / ZP_ROWS, ZP_LINES * PV<1>, smem, c->st>>>(a, (const T *)c->kv, (const T2 *)c->tw);
         else
@@ -1386,38 +1408,50 @@ template <typename T, int N> struct Impl {
         const bool pen = Tm & T_PENALIZATION;
         const bool forked = rounds_AB(c, true, false);
         // C
-        if (pen) {
+        {
             Launch L_(c, KC_LIN, (double)c->Nc * (9 * sizeof(T2) + 2 * sizeof(T)));
             k_lin<T><<<mg_grid(NZC, N), mg_block(), 0, c->st>>>(rargs(c), geo(c), (T2 *)c->LIN[0], (T2 *)c->LIN[1],
                                                                (T2 *)c->LIN[2], (T2 *)c->LIN[3]);
         }
-        // D: the u', s part (unless forked) and the linear terms' part
-        if (!forked) round_D_us(c);
-        if (pen) {
-            axis(c, c->jD_x + 6, 4, 0, +1);
-            axis(c, c->jD_y + 9, 4, 1, +1);
-            zc2r(c, c->zD + 8, 2);
+        if (pen && c->bx_i) {  // c2r(-lin_q) on the mask's window
+            axis(c, c->jD_x + 6, 4, 0, +1, AX_XB);
+            axis(c, c->jD_y + 9, 4, 1, +1, AX_YB);
+            zc2r(c, c->zD + 8, 2, false, -1., c->bx_i * c->bx_j);
         }
-        if (forked) CK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
+        // D: the u', s part, unless forked
+        if (!forked)
+            round_D_us(c);
+        else
+            CK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
         // z part of D, E, z part of F (with penalization only what the 2/3 rule keeps is formed)
         zprod(c, pen);
         axis(c, c->jF_y, 4, 1, -1, pen ? AX_YF : AX_FULL);
+        stage(c, pen);
+    }
+
+    // the end of F: the forward x pass, K and its use in the RK4 stage
+    static void stage(kf_ctx *c, bool pen) {
         const AxTrunc A = trunc(c, pen ? AX_XM : AX_FULL);
-        const int ntiles = A.mode == AX_XM ? c->tr_nt : (N * NZC + TC - 1) / TC;
-        {
-            const double cb = (double)c->Nc * sizeof(T2), rb = (double)c->Nc * sizeof(T);
-            Launch L_(c, KC_XASM, A.mode == AX_XM ? 4. * (c->tr_disc + c->tr_ball) * sizeof(T2) : pen ? 8 * cb : 8 * cb + 4 * cb + ((Tm & T_E_INT) ? cb : 0.) + 2 * rb);
-            const size_t sm = (size_t)N * TC * sizeof(T2);
-            const AxisJob *j = c->dj + c->jF_x;
-            if (c->fftv && pen)
-                k_xfwd_assemble<T, N, 1, true><<<ntiles, TC * PV<1>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw, A);
-            else if (c->fftv)
-                k_xfwd_assemble<T, N, 1, false><<<ntiles, TC * PV<1>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw, A);
-            else if (pen)
-                k_xfwd_assemble<T, N, 0, true><<<ntiles, TC * PV<0>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw, A);
-            else
-                k_xfwd_assemble<T, N, 0, false><<<ntiles, TC * PV<0>, sm, c->st>>>(j, geo(c), rargs(c), (const T2 *)c->tw, A);
+        StageArgs<T> a;
+        for (int q = 0; q < 4; ++q) {
+            a.in[q] = (const T2 *)c->CY[q];
+            a.lin[q] = (const T2 *)c->LIN[q];
+            a.y[q] = (T2 *)c->Y[q];
+            a.acc[q] = (T2 *)c->ACC[q];
+            a.ys[q] = (T2 *)c->Ys[q];
+            a.K[q] = (T2 *)c->K[q];
         }
+        a.c = (T)c->rk_c;
+        a.mode = c->rk_mode;
+        const bool act = A.mode == AX_XM;
+        const int ntiles = act ? c->tr_nt : (N * NZC + TC - 1) / TC;
+        const double use = act ? c->tr_ball : (double)c->Nc;
+        const size_t sm = (size_t)N * TC * sizeof(T2);
+        Launch L_(c, KC_XASM, 4. * sizeof(T2) * ((act ? c->tr_disc : use) + use * (a.mode == 3 ? 2 : a.mode == 0 ? 4 : 5)));
+        if (c->fftv)
+            k_xfwd_stage<T, N, 1><<<4 * ntiles, TC * PV<1>, sm, c->st>>>(a, geo(c), (const T2 *)c->tw, A);
+        else
+            k_xfwd_stage<T, N, 0><<<4 * ntiles, TC * PV<0>, sm, c->st>>>(a, geo(c), (const T2 *)c->tw, A);
         CK(cudaGetLastError());
     }
 
@@ -1730,19 +1764,17 @@ void build_tables(kf_ctx *c) {
         c->pb = dalloc<int>(c, sizeof(int) * pb.size());
         CK(cudaMemcpy(c->pb, pb.data(), sizeof(int) * pb.size(), cudaMemcpyHostToDevice));
         const TruncTab t = trunc_table(pb, n, c->fp32 ? Tile<float>::TC : Tile<double>::TC);
-        if (t.nkz > 0 && !t.tl.empty()) {
-            c->tr_nkz = t.nkz;
-            c->tr_nt = (int)t.tl.size();
-            for (int b : pb)
-                if (b >= 0) {
-                    c->tr_ball += 2 * b + 1;
-                    c->tr_disc += n;
-                }
-            c->tr_jb = dalloc<int>(c, sizeof(int) * t.jb.size());
-            c->tr_tl = dalloc<int>(c, sizeof(int) * t.tl.size());
-            CK(cudaMemcpy(c->tr_jb, t.jb.data(), sizeof(int) * t.jb.size(), cudaMemcpyHostToDevice));
-            CK(cudaMemcpy(c->tr_tl, t.tl.data(), sizeof(int) * t.tl.size(), cudaMemcpyHostToDevice));
-        }
+        c->tr_nkz = t.nkz;
+        c->tr_nt = (int)t.tl.size();
+        for (int b : pb)
+            if (b >= 0) {
+                c->tr_ball += 2 * b + 1;
+                c->tr_disc += n;
+            }
+        c->tr_jb = dalloc<int>(c, sizeof(int) * t.jb.size());
+        c->tr_tl = dalloc<int>(c, sizeof(int) * t.tl.size());
+        CK(cudaMemcpy(c->tr_jb, t.jb.data(), sizeof(int) * t.jb.size(), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(c->tr_tl, t.tl.data(), sizeof(int) * t.tl.size(), cudaMemcpyHostToDevice));
     }
     if (c->fp32) {
         std::vector<float> kvf(n), SVf(c->Nc), PFf(c->Nc), twf(2 * n);
@@ -2101,12 +2133,13 @@ void create(kf_ctx *c) {
     for (int q = 0; q < 4; ++q) {
         CK(cudaMemset(c->Y[q], 0, cb));
         CK(cudaMemset(c->Ys[q], 0, cb));
-        CK(cudaMemset(c->K[q], 0, cb));  // k_xfwd_assemble writes only what the 2/3 rule keeps
+        CK(cudaMemset(c->K[q], 0, cb));  // k_xfwd_stage writes only what the 2/3 rule keeps
     }
     c->npartial = 1184;
     c->partial = dalloc<double>(c, sizeof(double) * KF_RED * c->npartial);
     c->red = dalloc<double>(c, sizeof(double) * 8);
     c->d_sweeps = dalloc<int>(c, sizeof(int) * 4);
+    c->d_box = dalloc<int>(c, sizeof(int) * 4);
     c->d_err = dalloc<int>(c, sizeof(int));
     CK(cudaMemset(c->d_err, 0, sizeof(int)));
     CK(cudaMallocHost(&c->h_err, sizeof(int)));
@@ -2152,6 +2185,26 @@ void copy_state(kf_ctx *c, void *const *dst, void *const *src) {
         CK(cudaMemcpyAsync(dst[q], src[q], c->cs * c->Nc, cudaMemcpyDeviceToDevice, c->st));
 }
 
+// One stage: the right-hand side of Ys and the stage's combination, in the
+// right-hand side's last kernel or (stretched axes) in k_rk on its K.
+void rk_launch(kf_ctx *c, double cdt, int mode);
+void rk_stage(kf_ctx *c, double cdt, int mode) {
+    if (c->stretched) {
+        c->rhs_fn(c);
+        rk_launch(c, cdt, mode);
+        return;
+    }
+    c->rk_mode = mode;
+    c->rk_c = cdt;
+    try {
+        c->rhs_fn(c);
+    } catch (...) {
+        c->rk_mode = 3;
+        throw;
+    }
+    c->rk_mode = 3;
+}
+
 void rk_launch(kf_ctx *c, double cdt, int mode) {
     const long M = c->Nc;
     for (int q = 0; q < 4; ++q) {
@@ -2185,12 +2238,11 @@ void rk4_step(kf_ctx *c, double dt, void *const *X, double *const *PH, double *c
             CK(cudaMemcpyAsync(c->phi, PHin[i], 8 * c->N, cudaMemcpyDeviceToDevice, c->st));
             c->phi_given = true;
         }
-        c->rhs_fn(c);
+        rk_stage(c, cdt[i], mode[i]);
         c->phi_given = false;
         if (PH) CK(cudaMemcpyAsync(PH[i], c->phi, 8 * c->N, cudaMemcpyDeviceToDevice, c->st));
-        rk_launch(c, cdt[i], mode[i]);
     }
-    copy_state(c, c->Ys, c->Y);
+    if (c->stretched) copy_state(c, c->Ys, c->Y);
     c->t = t0 + dt;
 }
 
@@ -2244,10 +2296,9 @@ void capture_step(kf_ctx *c, double dt, bool wait_u, cudaGraphExec_t *out) {
                 k_time<<<1, 32, 0, c->st>>>(c->dtime, xs[i], 0);
             }
             c->stage_idx = i;
-            c->rhs_fn(c);
-            rk_launch(c, cdt[i], mode[i]);
+            rk_stage(c, cdt[i], mode[i]);
         }
-        copy_state(c, c->Ys, c->Y);
+        if (c->stretched) copy_state(c, c->Ys, c->Y);
         {
             Launch L_(c, KC_MISC, 0.);
             k_time<<<1, 32, 0, c->st>>>(c->dtime, dt, 1);
@@ -2395,6 +2446,32 @@ void drop_graphs(kf_ctx *c) {
         cudaGraphExecDestroy(c->adj->graph);
         c->adj->graph = nullptr;
     }
+}
+
+// The mask's window of rows; the captured steps hold it, so a change drops them.
+void mask_box(kf_ctx *c) {
+    const int n = c->n;
+    int b[4] = {n, -1, n, -1};
+    CK(cudaMemcpyAsync(c->d_box, b, sizeof(b), cudaMemcpyHostToDevice, c->st));
+    {
+        Launch L_(c, KC_MISC, (double)c->N * c->es);
+        const dim3 g(1, (n + 7) / 8, n);
+        if (c->fp32)
+            k_mask_box<float><<<g, mg_block(), 0, c->st>>>((const float *)c->H, n, c->d_box);
+        else
+            k_mask_box<double><<<g, mg_block(), 0, c->st>>>((const double *)c->H, n, c->d_box);
+    }
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(b, c->d_box, sizeof(b), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    const bool any = b[1] >= 0;
+    const int i0 = any ? b[0] : 0, bi = any ? b[1] - b[0] + 1 : 0, j0 = any ? b[2] : 0, bj = any ? b[3] - b[2] + 1 : 0;
+    if (i0 == c->bx_i0 && bi == c->bx_i && j0 == c->bx_j0 && bj == c->bx_j) return;
+    c->bx_i0 = i0;
+    c->bx_i = bi;
+    c->bx_j0 = j0;
+    c->bx_j = bj;
+    drop_graphs(c);
 }
 
 // milliseconds per call of f: two untimed calls, then reps calls between
@@ -2586,7 +2663,10 @@ int kf_get_state(kf_ctx *c, double *ux, double *uy, double *uz, double *s) {
 int kf_set_sources(kf_ctx *c, const double *nd, const double *mask) {
     return guarded(c, [&] {
         if (nd) CK(cudaMemcpyAsync(c->nd, nd, 8 * c->N, cudaMemcpyHostToDevice, c->st));
-        if (mask) put_bulk(c, c->H, mask, c->N);
+        if (mask) {
+            put_bulk(c, c->H, mask, c->N);
+            mask_box(c);
+        }
         CK(cudaStreamSynchronize(c->st));
     });
 }

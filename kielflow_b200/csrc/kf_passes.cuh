@@ -100,7 +100,8 @@ k_axis_pass(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
 // beside the exchange buffer).  Every thread stages exactly the elements it
 // later reads, so the staging buffer needs no barrier; the exchange buffer
 // keeps the FFT's own.  Same tiles, multipliers, transforms and stores as
-// k_axis_pass, so the same results.
+// k_axis_pass, so the same results.  The 2/3 rule (MUL_P, MUL_P_IK) is applied
+// by the bounds of AX_XM, the mode of every masked launch.
 __device__ __forceinline__ void cp_async_copy(void *smem, const float2 *g) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(g) : "memory");
@@ -120,7 +121,8 @@ template <typename T> struct AxisTile {
     const T2 *in;
     T2 *out;
     int base, rstride;  // element indices: n * n * (n/2 + 1) < 2^31 for every supported n
-    int jj, kk, mul;
+    int obase;          // of the output (the input's base but for a packed window)
+    int mul;
     int lb, sb;  // rows r with min(r, N - r) <= lb are loaded (the others are zero), <= sb stored
     bool valid;
 };
@@ -136,45 +138,41 @@ __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ job
     G.in = static_cast<const T2 *>(J.in);
     G.out = static_cast<T2 *>(J.out);
     G.mul = J.mul;
-    G.jj = 0;
-    G.kk = 0;
     G.lb = G.sb = N / 2;
     if (axis == 0) {
         G.rstride = n * nzc;
         if (A.mode == AX_XM) {
             const int w = A.tl[tile];
-            G.jj = w >> 16;
-            G.kk = (w & 0xffff) + c;
-            G.base = G.jj * nzc + G.kk;
-            G.lb = G.kk < A.nkz ? g.pb[G.base] : -1;
+            const int kk = (w & 0xffff) + c;
+            G.base = (w >> 16) * nzc + kk;
+            G.lb = kk < A.nkz ? g.pb[G.base] : -1;
             G.valid = G.lb >= 0;
         } else {
-            const int col = tile * TC + c;
-            G.valid = col < n * nzc;
-            G.base = col;
-            G.jj = col / nzc;
-            G.kk = col - G.jj * nzc;
+            G.base = tile * TC + c;
+            G.valid = G.base < n * nzc;
         }
+        G.obase = A.mode == AX_XB ? G.base - A.r0 * n * nzc : G.base;
     } else {
         constexpr int tpp = (nzc + TC - 1) / TC;
-        int plane;
-        if (A.mode == AX_FULL) {
+        int plane, kk;
+        if (A.mode == AX_FULL || A.mode == AX_YB) {
             plane = tile / tpp;
-            G.kk = (tile - plane * tpp) * TC + c;
-            G.valid = G.kk < nzc;
+            kk = (tile - plane * tpp) * TC + c;
+            G.valid = kk < nzc;
         } else {
             const int tq = (A.nkz + TC - 1) / TC;
             plane = __float2int_rd(((float)tile + 0.5f) * A.itpp);  // tile / tq (exact: tile < 2^13)
-            G.kk = (tile - plane * tq) * TC + c;
-            G.valid = G.kk < A.nkz;
-            const int b = G.valid ? A.jb[G.kk] : -1;
+            kk = (tile - plane * tq) * TC + c;
+            G.valid = kk < A.nkz;
+            const int b = G.valid ? A.jb[kk] : -1;
             if (A.mode == AX_YI)
                 G.lb = b;
             else
                 G.sb = b;
         }
-        G.base = plane * n * nzc + G.kk;
+        G.base = plane * n * nzc + kk;
         G.rstride = nzc;
+        G.obase = A.mode == AX_YB ? (plane * A.rm - A.r0) * nzc + kk : G.base;
     }
     return G;
 }
@@ -282,20 +280,13 @@ k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
         const int slot = it % D;
         const AxisTile<T> cur = axis_tile<T, N>(jobs, cj, ct, axis, c, A, g);
         adv(cj, ct);
-        // the 2/3 rule of this column as an index bound (one table read per
-        // tile); a masked pass has staged zeros outside it already
-        const bool mask = (cur.mul == MUL_P || cur.mul == MUL_P_IK) && A.mode == AX_FULL;
-        const int pbnd = cur.valid && mask ? dealias_bound(g.pb, cur.jj, cur.kk, g.nzc) : -2;
         cp_async_wait<D - 1>();
         const T2 *stg = stg0 + slot * (N * TC);
         T2 v[E];
 #pragma unroll
         for (int q = 0; q < E; ++q) {
             const int row = reg_row<N, P, PlanV<N, V>::R1>(p, q);
-            T2 x = stg[row * TC + c];
-            if (mask) {
-                if (!dealias_keep_b(g.q2, g.thr, pbnd, g.n, row, cur.jj, cur.kk)) x = mk<T2>((T)0, (T)0);
-            }
+            T2 x = stg[row * TC + c];  // AX_XM: zeros staged outside the 2/3 rule
             if (cur.mul == MUL_P_IK || cur.mul == MUL_IK) x = mul_ik(x, g.kv[row]);
             v[q] = x;
         }
@@ -305,7 +296,8 @@ k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
 #pragma unroll
             for (int q = 0; q < E; ++q) {
                 const int row = reg_row<N, P, PlanV<N, V>::RL>(p, q);
-                if (row_freq<N>(row) <= cur.sb) cur.out[cur.base + row * cur.rstride] = v[q];
+                const bool st = A.mode >= AX_XB ? (unsigned)(row - A.r0) < (unsigned)A.rm : row_freq<N>(row) <= cur.sb;
+                if (st) cur.out[cur.obase + row * cur.rstride] = v[q];
             }
         }
     }
@@ -487,145 +479,84 @@ k_z_r2c(const ZJob *__restrict__ jobs, int njobs, int nrows,
     }
 }
 
-// --------------------------------------------- spectral linear terms (FB parts)
-// lin_q is the part of rhs_standard's FBuffer_q (the negated right-hand side)
-// that is computed in k-space, in the reference's order of accumulation:
-//   u_c: (tau+SV) u^ [+ D|k|^2 u^] + i k_c (PF phi^ + s^/theta) + M i k_x P u^
-//        (rhs_standard.cpp:119-140, 218-248, 279-295)
-//   s  : SV s^ [+ D|k|^2 s^] + M i k_x P s^ + i k.P u^
-//        (rhs_standard.cpp:135-139, 304-319)
-// b: the column's 2/3-rule bound (dealias_bound), or -2 for the exact test.
-template <typename T>
-__device__ __forceinline__ typename C2<T>::type lin_term(const RhsArgs<T> &a, const Geo<T> &g, int q,
-                                                         int i, int j, int k, long idx, int b) {
+// ------------------------------ forward x pass + assembly + RK4 stage update
+// One block transforms one column tile of one of the four fields and finishes
+// the right-hand side there,
+//   K_q = -lin_q + F_q                             (rhs_standard.cpp:538-560)
+// with -lin_q from k_lin and F_q the transform of the physical part (k_zprod);
+// with penalization F_q and -lin_q are needed inside the 2/3 rule only (the
+// filter after the physical-space penalization, rhs_standard.cpp:491-532): the
+// active columns (A.mode AX_XM), the rows within their bounds, K being zero
+// elsewhere.  What the RK4 stage does with K (RKO4.cpp:140-238) follows in
+// place, so K is neither written nor read back:
+//   mode 0: acc = K,      ys = y + c K
+//   mode 1: acc += 2 K,   ys = y + c K
+//   mode 2: y += c (acc + K), ys = y
+//   mode 3: K itself (a right-hand side on its own)
+// Outside the 2/3 rule K = 0, hence ys = y, which holds from the stage's start.
+template <typename T> struct StageArgs {
     typedef typename C2<T>::type T2;
-    const int Tm = a.terms;
-    const bool P = dealias_keep_b(g.q2, g.thr, b, g.n, i, j, k);
-    const T kx = g.kv[i], ky = g.kv[j], kz = g.kv[k];
-    const T sv = a.SV[idx];
-    T2 fb;
-    if (q < 3) {
-        const T2 u = a.Y[q][idx];
-        const bool diss = Tm & T_DISSIPATION, svo = Tm & T_SVISCOSITY;
-        const T cf = diss && svo ? (a.tau + sv) : diss ? a.tau : svo ? sv : (T)0;
-        fb = mk<T2>(cf * u.x, cf * u.y);
-        if (Tm & T_DIFFUSION) {
-            const T k2 = kx * kx + ky * ky + kz * kz;
-            fb.x += a.D * k2 * u.x;
-            fb.y += a.D * k2 * u.y;
-        }
-        const bool pres = Tm & T_PRESSURE, eint = Tm & T_E_INT;
-        if (pres || eint) {
-            T2 F1 = mk<T2>((T)0, (T)0);
-            if (eint) {
-                F1 = a.phihat[idx];
-                if (pres) { const T pf = a.PF[idx]; F1.x *= pf; F1.y *= pf; }
-            }
-            if (pres) {
-                const T2 s = a.Y[3][idx];
-                F1.x += s.x / a.theta;
-                F1.y += s.y / a.theta;
-            }
-            const T kc = q == 0 ? kx : q == 1 ? ky : kz;
-            const T2 d = mul_ik(F1, kc);
-            fb.x += d.x;
-            fb.y += d.y;
-        }
-        if ((Tm & T_E_EXT) && P) {
-            const T2 d = mul_ik(u, kx);
-            fb.x += a.M * d.x;
-            fb.y += a.M * d.y;
-        }
-    } else {
-        const T2 s = a.Y[3][idx];
-        const T cf = (Tm & T_SVISCOSITY) ? sv : (T)0;
-        fb = mk<T2>(cf * s.x, cf * s.y);
-        if (Tm & T_DIFFUSION) {
-            const T k2 = kx * kx + ky * ky + kz * kz;
-            fb.x += a.D * k2 * s.x;
-            fb.y += a.D * k2 * s.y;
-        }
-        if ((Tm & T_E_EXT) && P) {
-            const T2 d = mul_ik(s, kx);
-            fb.x += a.M * d.x;
-            fb.y += a.M * d.y;
-        }
-        if ((Tm & T_CONTINUITY) && P) {
-            const T2 dx = mul_ik(a.Y[0][idx], kx);
-            const T2 dy = mul_ik(a.Y[1][idx], ky);
-            const T2 dz = mul_ik(a.Y[2][idx], kz);
-            fb.x += dx.x; fb.y += dx.y;
-            fb.x += dy.x; fb.y += dy.y;
-            fb.x += dz.x; fb.y += dz.y;
-        }
-    }
-    return fb;
-}
+    const T2 *in[4], *lin[4];
+    T2 *y[4], *acc[4], *ys[4], *K[4];
+    T c;
+    int mode;
+};
 
-// ------------------------------------ forward x pass + right-hand-side assembly
-// For each of the four output fields the forward x transform of the y-passed
-// product (or penalized) field is formed and combined per element:
-//   penalization off: K_q = -(lin_q + F_q)        (rhs_standard.cpp:538-560)
-//   penalization on : K_q = P(k) F_q              (the 2/3 filter after the
-//                     physical-space penalization, rhs_standard.cpp:491-532)
-// gridDim.x = number of column tiles; jobs[q].in = y-passed field, .out = K_q.
-// PEN: the penalization form (a.terms has T_PENALIZATION), instantiated apart
-// so that its registers do not carry the linear terms'.
-template <typename T, int N, int V = 0, bool PEN = false>
+template <typename T, int N, int V = 0>
 __global__ void __launch_bounds__(Tile<T>::TC * PlanV<N, V>::P,
-                                  (PEN ? PipeMinBlocks<T, N, V, 1, sizeof(T) == 4 ? 4 : 2, 64>::value : 1))
-k_xfwd_assemble(const AxisJob *__restrict__ jobs, Geo<T> g, RhsArgs<T> a,
-                const typename C2<T>::type *__restrict__ tw, AxTrunc A) {
+                                  PipeMinBlocks<T, N, V, 1, sizeof(T) == 4 ? 4 : 2, 64>::value)
+k_xfwd_stage(const __grid_constant__ StageArgs<T> a, Geo<T> g, const typename C2<T>::type *__restrict__ tw, AxTrunc A) {
     typedef typename C2<T>::type T2;
-    constexpr int TC = Tile<T>::TC, P = PlanV<N, V>::P, E = N / P;
+    constexpr int TC = Tile<T>::TC, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1;
     extern __shared__ __align__(16) unsigned char kf_smem[];
     T2 *sm = reinterpret_cast<T2 *>(kf_smem);
-    const int tile = blockIdx.x;
+    const int q = blockIdx.x & 3, tile = blockIdx.x >> 2;
     const int c = threadIdx.x % TC, p = threadIdx.x / TC;
-    const int n = g.n, nzc = g.nzc;
-    // A.mode AX_XM (penalization form only): the columns the 2/3 rule keeps,
-    // and of K the rows it keeps (K is zero elsewhere since its allocation)
-    const bool act = PEN && A.mode == AX_XM;
-    int col = tile * TC + c;
-    bool valid = col < n * nzc;
-    int jj = col / nzc, kk = col - jj * nzc;
-    if (act) {
+    constexpr int rstride = N * NZC;
+    int col = tile * TC + c, b = N / 2;
+    bool valid = col < N * NZC;
+    if (A.mode == AX_XM) {
         const int w = A.tl[tile];
-        jj = w >> 16;
-        kk = (w & 0xffff) + c;
-        col = jj * nzc + kk;
-        valid = kk < A.nkz && g.pb[col] >= 0;
+        const int kk = (w & 0xffff) + c;
+        col = (w >> 16) * NZC + kk;
+        b = kk < A.nkz ? g.pb[col] : -1;
+        valid = b >= 0;
     }
-    const long rstride = (long)n * nzc;
-    const int b = valid ? dealias_bound(g.pb, jj, kk, nzc) : -2;
-    for (int q = 0; q < 4; ++q) {
-        const T2 *__restrict__ in = static_cast<const T2 *>(jobs[q].in);
-        T2 *__restrict__ out = static_cast<T2 *>(jobs[q].out);
-        T2 v[E];
+    const T2 *__restrict__ in = a.in[q];
+    T2 v[E];
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int row = reg_row<N, P, PlanV<N, V>::R1>(p, e);
-            v[e] = valid ? in[col + row * rstride] : mk<T2>((T)0, (T)0);
+    for (int e = 0; e < E; ++e) {
+        const int row = reg_row<N, P, PlanV<N, V>::R1>(p, e);
+        v[e] = valid ? in[col + row * rstride] : mk<T2>((T)0, (T)0);
+    }
+    PlanV<N, V>::template fft<T2, -1>(v, sm + c, StrideAddr{TC}, p, tw);
+    if (!valid) return;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int i = reg_row<N, P, PlanV<N, V>::RL>(p, e);
+        if (row_freq<N>(i) > b) continue;
+        const int idx = col + i * rstride;
+        const T2 l = a.lin[q][idx];
+        const T2 k = mk<T2>(l.x + v[e].x, l.y + v[e].y);
+        if (a.mode == 3) {
+            a.K[q][idx] = k;
+            continue;
         }
-        PlanV<N, V>::template fft<T2, -1>(v, sm + c, StrideAddr{TC}, p, tw);
-        if (valid) {
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                const int i = reg_row<N, P, PlanV<N, V>::RL>(p, e);
-                const long idx = col + i * rstride;
-                T2 F = v[e];
-                T2 K;
-                if constexpr (PEN) {
-                    if (act && row_freq<N>(i) > b) continue;
-                    K = dealias_keep_b(g.q2, g.thr, b, N, i, jj, kk) ? F : mk<T2>((T)0, (T)0);
-                } else {
-                    T2 fb = lin_term(a, g, q, i, jj, kk, idx, b);
-                    K = mk<T2>(-(fb.x + F.x), -(fb.y + F.y));
-                }
-                out[idx] = K;
+        const T2 y = a.y[q][idx];
+        if (a.mode == 2) {
+            const T2 s = a.acc[q][idx];
+            const T2 r = mk<T2>(y.x + a.c * (s.x + k.x), y.y + a.c * (s.y + k.y));
+            a.y[q][idx] = r;
+            a.ys[q][idx] = r;
+        } else {
+            T2 s = k;
+            if (a.mode == 1) {
+                s = a.acc[q][idx];
+                s = mk<T2>(s.x + (T)2 * k.x, s.y + (T)2 * k.y);
             }
+            a.acc[q][idx] = s;
+            a.ys[q][idx] = mk<T2>(y.x + a.c * k.x, y.y + a.c * k.y);
         }
-        __syncthreads();
     }
 }
 

@@ -66,10 +66,15 @@ __global__ void k_products(ProdArgs<T> a) {
     }
 }
 
-// rl_q = -lin_q in k-space (penalization path).  Grid (ceil(nzc/32), n/8, n)
-// of 32 x 8 blocks over (kz, j, i): no index division.  The four outputs of
-// an element share its loads (state, phi^, tables); each is accumulated in the
-// order of lin_term (kf_passes.cuh), so the values are those of lin_term.
+// -lin_q in k-space, lin_q being the part of rhs_standard's FBuffer_q (the
+// negated right-hand side) that is computed there, in the reference's order of
+// accumulation:
+//   u_c: (tau+SV) u^ [+ D|k|^2 u^] + i k_c (PF phi^ + s^/theta) + M i k_x P u^
+//        (rhs_standard.cpp:119-140, 218-248, 279-295)
+//   s  : SV s^ [+ D|k|^2 s^] + M i k_x P s^ + i k.P u^
+//        (rhs_standard.cpp:135-139, 304-319)
+// Grid (ceil(nzc/32), n/8, n) of 32 x 8 blocks over (kz, j, i): no index
+// division; the four outputs of an element share its loads (state, phi^, tables).
 template <typename T>
 __global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *o0,
                                              typename C2<T>::type *o1, typename C2<T>::type *o2,
@@ -143,6 +148,23 @@ __global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2
             fb.x += dz.x; fb.y += dz.y;
         }
         o[3][idx] = mk<T2>(-fb.x, -fb.y);
+    }
+}
+
+// The (i, j) rows on which the penalization mask is not zero, as the window
+// box = {min i, max i, min j, max j} (started from {n, -1, n, -1}): outside it
+// the penalization has no effect, so c2r(-lin_q) is needed on the window only.
+template <typename T>
+__global__ void __launch_bounds__(256) k_mask_box(const T *__restrict__ H, int n, int *__restrict__ box) {
+    const int j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
+    if (j >= n) return;
+    bool any = false;
+    for (int k = threadIdx.x; k < n; k += 32) any |= H[((long)i * n + j) * n + k] != (T)0;
+    if (any) {
+        atomicMin(box + 0, i);
+        atomicMax(box + 1, i);
+        atomicMin(box + 2, j);
+        atomicMax(box + 3, j);
     }
 }
 

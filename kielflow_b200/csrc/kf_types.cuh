@@ -62,6 +62,8 @@ enum AxMode : int {
     AX_XM = 1,    // x pass, masked input: active columns, rows within the column's bound -> every row
     AX_YI = 2,    // y pass after AX_XM: columns kz < nkz, rows j within jb[kz] -> every row
     AX_YF = 3,    // forward y pass whose x pass needs only active columns: every row -> rows within jb[kz]
+    AX_XB = 4,    // x pass of which a window of planes is needed: every row -> rows r0 .. r0 + rm - 1, packed
+    AX_YB = 5,    // y pass after AX_XB (rm0 planes): every row -> rows r0 .. r0 + rm - 1, packed
 };
 struct AxTrunc {
     int mode;
@@ -69,6 +71,7 @@ struct AxTrunc {
     float itpp;     // 1 / column tiles per plane of AX_YI, AX_YF
     const int *jb;  // per kz < nkz: largest min(j, n - j) of an active column
     const int *tl;  // active x-pass tiles: (j << 16) | first kz
+    int r0, rm;     // AX_XB, AX_YB: the window
 };
 
 // sqrt is correctly rounded and monotone, so sqrt(s) < 2/3 holds exactly when
@@ -100,7 +103,7 @@ __device__ __forceinline__ bool dealias_keep_b(const double *__restrict__ q2, do
     return dealias_keep(q2, thr, i, j, k);
 }
 
-// Everything the spectral linear terms and the assembly need.
+// Everything the spectral linear terms need.
 template <typename T> struct RhsArgs {
     typedef typename C2<T>::type T2;
     const T2 *Y[4];     // stage input: u'_x, u'_y, u'_z, s  (half spectra)

@@ -1,6 +1,10 @@
 // kf_zprod.cuh -- the z-local middle of the right-hand side in one kernel: the
 // inverse z transforms of u', s and their derivatives, the physical-space
-// products (k_products' terms) and the forward z transform of the four results.
+// products (k_products' terms) and the forward z transform of the four results,
+//   g_q = -prod_q                                             (H = 0)
+//   g_q = (1-H) (rl_q - prod_q) + H eta (q_d - q_fix) - rl_q   (H != 0)
+// so that the right-hand side is -lin_q + r2c(g_q) with the linear terms left in
+// k-space (rl_q = c2r(-lin_q), needed where the mask H is not zero only).
 //
 // Everything between the y passes is local to a z line (i, j), so the 16 real
 // fields of round D never go to memory.  A block of 8 groups of P threads (a
@@ -41,8 +45,11 @@ template <typename T> struct ZProdArgs {
     const T2 *s0, *sy, *sx;             // y-passed spectra of P s, d_y s, d_x s
     const T2 *u[3], *uy[3], *ux[3];     // of U_c, d_y U_c, d_x U_c
     T2 *out[4];                         // z-transformed results, half spectra
-    const T *rl[4];                     // c2r(-lin_q)   (penalization only)
-    const T *H;                         // mask          (penalization only)
+    // penalization: the mask, the window of rows on which it is not zero
+    // (k_mask_box; bi = 0: none) and c2r(-lin_q) on that window's rows
+    const T *H;
+    const T *rl[4];
+    int i0, bi, j0, bj;
     T M, eta, scale;                    // scale: the 1/N of the c2r
     int terms;
     int nkz;  // the inputs are zero from kz = nkz on
@@ -73,7 +80,7 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
     const T2 *__restrict__ inB = l < 3 ? nullptr : l < 6 ? a.ux[l - 3] : l == 6 ? a.sx : nullptr;
     T2 *line = xch + l * LS;
     const PadAddr pa;
-    const bool adv = a.terms & T_ADVECTION, cont = a.terms & T_CONTINUITY, pen = a.terms & T_PENALIZATION;
+    const bool adv = a.terms & T_ADVECTION, cont = a.terms & T_CONTINUITY;
 #pragma unroll 1
     for (int rr = 0; rr < ZP_ROWS; ++rr) {
         const long off = (long)(r0 + rr) * NZC;
@@ -99,6 +106,8 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
         for (int q = 0; q < E; ++q)
             line[reg_row<N, P, PlanV<N, V>::RL>(p, q)] = mk<T2>(v[q].x * a.scale, v[q].y * a.scale);
         __syncthreads();
+        const int bi = (r0 + rr) / N - a.i0, bj = (r0 + rr) % N - a.j0, brow = bi * a.bj + bj;
+        const bool box = (unsigned)bi < (unsigned)a.bi && (unsigned)bj < (unsigned)a.bj;
         for (int z = threadIdx.x; z < N; z += NT) {
             const T2 U0 = xch[z], U1 = xch[LS + z], U2 = xch[2 * LS + z];  // (U_c, d_z U_c)
             const T ux = U0.x, uy = U1.x, uz = U2.x;
@@ -124,16 +133,18 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
                 }
                 pr[3] = s;
             }
-            if (pen) {
-                const long i = (long)(r0 + rr) * N + z;
-                const T h = a.H[i];
+            const T h = box ? a.H[(long)(r0 + rr) * N + z] : (T)0;
+            if (h != (T)0) {
                 const T qd[4] = {ux, uy, uz, S0.x};
                 const T qfix[4] = {-a.M, (T)0, (T)0, (T)-10};
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const T r = a.rl[q][i] - pr[q];
-                    pr[q] = ((T)1 - h) * r + h * a.eta * (qd[q] - qfix[q]);
+                    const T l = a.rl[q][(long)brow * N + z], r = l - pr[q];
+                    pr[q] = (((T)1 - h) * r + h * a.eta * (qd[q] - qfix[q])) - l;
                 }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) pr[q] = -pr[q];
             }
             res[(2 * rr) * N + z] = mk<T2>(pr[0], pr[1]);
             res[(2 * rr + 1) * N + z] = mk<T2>(pr[2], pr[3]);

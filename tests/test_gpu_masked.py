@@ -51,3 +51,36 @@ def test_full_spectrum_rhs_vs_oracle(n, pen, prec, plan):
     scale = max(np.abs(x).max() for x in r)
     err = max(np.abs(a - b).max() for a, b in zip(g, r)) / scale
     assert err < (1e-12 if prec == kf.KF_FP64 else 1e-5)
+
+
+MASKS = {
+    "none": lambda n: np.zeros((n, n, n)),
+    "one point": lambda n: np.eye(1, n ** 3, 5 * n * n + 3 * n + n - 1).reshape(n, n, n),
+    "ball": lambda n: I.sphere_mask(n, C.L_BOX, 2.0),
+    "across the box edge": lambda n: np.roll(I.sphere_mask(n, C.L_BOX, 2.0), (n // 2, n // 2, n // 3), (0, 1, 2)),
+    "smooth, everywhere": lambda n: np.random.default_rng(n).uniform(0.0, 1.0, (n, n, n)),
+}
+
+
+@pytest.mark.parametrize("prec", [kf.KF_FP64, kf.KF_FP32_BULK])
+@pytest.mark.parametrize("kind", list(MASKS))
+def test_penalization_masks_vs_oracle(kind, prec):
+    """The linear terms are transformed on the mask's window of rows only."""
+    n, w = 32, C.WORKLOADS["fas128"]
+    cfg = C.config_for(w, n=n, precision=prec, terms=NO_PHI)
+    nd = I.gauss_charge(n, C.L_BOX, w["Q"], w["sigma"])
+    st, dt = noise_state(n, 7), 1e-3
+    o = bind.Oracle(bind.KfoConfig(*[getattr(cfg, f) for f, _ in bind.KfoConfig._fields_]))
+    with kf.Context(cfg) as ctx:
+        for k in ("ball", kind):  # the window changes under a captured step
+            ctx.set_sources(nd, MASKS[k](n))
+            ctx.set_state(*st)
+            ctx.rk4(dt, 2)
+        g = ctx.get_state()
+    o.set_state(st)
+    o.set_sources(nd, MASKS[kind](n))
+    o.rk4(dt, 2)
+    r = o.get_state()
+    scale = max(np.abs(x).max() for x in r)
+    err = max(np.abs(a - b).max() for a, b in zip(g, r)) / scale
+    assert err < (1e-12 if prec == kf.KF_FP64 else 1e-5)
