@@ -26,6 +26,7 @@
 #include "../../include/kielflow_b200.h"
 #include "kf_adjoint.cuh"
 #include "kf_graph.cuh"
+#include "kf_jacobi.cuh"
 #include "kf_march.cuh"
 #include "kf_passes.cuh"
 #include "kf_pointwise.cuh"
@@ -51,10 +52,11 @@ struct KfError {
 struct LevelBuf {
     int n = 0;
     double *dd = nullptr, *dp = nullptr, *dm = nullptr, *ip = nullptr, *im = nullptr, *gam = nullptr;
+    double *rp = nullptr, *rm = nullptr;
     double *phi = nullptr, *rho = nullptr, *r = nullptr, *phi0 = nullptr;
     double *t = nullptr;  // second potential of the streaming smoother (k_rbgs_march), n >= MT_TK
     std::shared_ptr<AxTab> tab;  // host copy of dd, ip, im for k_rbgs_t (n <= KF_TAB_N)
-    Lev lev() const { return Lev{n, dd, dp, dm, ip, im}; }
+    Lev lev() const { return Lev{n, dd, dp, dm, ip, im, rp, rm}; }
 };
 
 constexpr int RBS = 256;  // reduction block size
@@ -70,6 +72,17 @@ constexpr int RBS = 256;  // reduction block size
 #define KF_RBGS_TAB 1
 #endif
 
+
+// Sweeps in the body of the Jacobi loop's WHILE node (even: they alternate
+// between the two potentials).
+constexpr int JC_UNROLL = 16;
+
+// The sweep loop of one level and stop rule, captured on first use.
+struct JacGraph {
+    const double *phi, *tmp, *rho;
+    JacStop stop;
+    cudaGraphExec_t exec;
+};
 
 struct AdjState;  // discrete-adjoint buffers (allocated by the first kf_adjoint_run)
 struct OutState;  // output buffers of kf_run / kf_get_output (allocated on first use)
@@ -128,9 +141,10 @@ struct kf_ctx {
     double *vol = nullptr;  // dS per index (cell widths / h) for the diagnostics
     int jS_Dx = 0, jS_Dy = 0, zS_D = 0, zS_F = 0, jS_Fy = 0, jS_Fx = 0, jS_Gx = 0, jS_Gy = 0, zS_G = 0;
     int zS_I = 0, jS_Iy = 0, jS_Ix = 0, jS_Kx = 0, jS_Ky = 0, zS_K = 0, zS_Kf = 0, jS_Kfy = 0, jS_Kfx = 0;
-    // Jacobi state carried between sweeps and solves (solver_poisson_jacobi_nlin.hpp:66-95)
-    double norm_max = 0., norm_sum = 0., norm_max_old = -1., norm_sum_old = -1.;
-    double sup = 0., inf = 0., omega = 1.;
+    // Jacobi state carried between solves (solver_poisson_jacobi_nlin.hpp:66-95)
+    double norm_max = 0., norm_sum = 0.;
+    JacState *d_js = nullptr, *h_js = nullptr;
+    std::vector<JacGraph> jac;
     kf_diag_out diag{};
     // kernel profiling (CUDA events around each launch, when enabled)
     bool prof = false;
@@ -228,7 +242,7 @@ enum KCls { KC_AXIS_INV, KC_AXIS_FWD, KC_Z_C2R, KC_Z_R2C, KC_XASM, KC_PROD, KC_L
 const char *const kKClsName[KC_N] = {"k_axis_pass(inverse)", "k_axis_pass(forward)", "k_z_c2r", "k_z_r2c",
                                      "k_xfwd_stage", "k_zprod/k_products", "k_lin", "k_rho", "k_rk", "k_jacobi",
                                      "k_rbgs", "k_residual", "k_restrict/k_fas_rhs/k_prolong/k_inject",
-                                     "k_coarse_solve/k_coarse_cycle", "k_reduce_final", "conversion/diagnostics",
+                                     "k_coarse_solve/k_coarse_cycle", "-", "conversion/diagnostics",
                                      "adjoint pointwise (k_prod_vjp/k_vjp_assemble/k_adj_stage/...)",
                                      "adjoint Poisson (linear multigrid)",
                                      "FAS levels below the finest (k_rbgs/k_residual/transfers)",
@@ -408,16 +422,6 @@ TruncTab trunc_table(const std::vector<int> &pb, int n, int tc) {
 }
 
 // ------------------------------------------------------------------ Poisson driver
-void reduce_read(kf_ctx *c, int nb) {
-    {
-        Launch L_(c, KC_REDUCE, 0.);
-        k_reduce_final<RBS><<<1, RBS, 0, c->st>>>(c->partial, nb, c->red);
-    }
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(c->h_red, c->red, sizeof(double) * KF_RED, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-}
-
 int red_blocks(long N) {
     long nb = (N + RBS - 1) / RBS;
     return (int)(nb < 1184 ? nb : 1184);
@@ -471,54 +475,111 @@ double max_residual(kf_ctx *c, const LevelBuf &L, const double *phi, const doubl
     return r;
 }
 
+// One Jacobi sweep of level L, in -> out.
+void jacobi_sweep(kf_ctx *c, const LevelBuf &L, const double *in, double *out, const double *rho, const JacStop &S,
+                  int cond, cudaGraphConditionalHandle h) {
+    const long N = (long)L.n * L.n * L.n;
+    Launch L_(c, KC_JACOBI, 24. * N);
+    k_jacobi<RBS><<<red_blocks(N), RBS, 0, c->st>>>(in, out, rho, L.lev(), S, c->partial, c->d_js, cond, h);
+}
+
+// The captured sweep loop: WHILE { JC_UNROLL sweeps phi -> tmp -> phi ... }, then
+// the result into phi.
+cudaGraphExec_t jacobi_graph(kf_ctx *c, const LevelBuf &L, double *phi, double *tmp, const double *rho,
+                             const JacStop &S) {
+    for (const JacGraph &g : c->jac)
+        if (g.phi == phi && g.tmp == tmp && g.rho == rho && g.stop.max_it == S.max_it &&
+            g.stop.resstop == S.resstop && g.stop.limit == S.limit && g.stop.tol == S.tol)
+            return g.exec;
+    const long N = (long)L.n * L.n * L.n;
+    const long long l0 = c->launches;
+    cudaStream_t outer = c->st;
+    cudaGraph_t g = nullptr;
+    CK(cudaStreamBeginCapture(outer, cudaStreamCaptureModeThreadLocal));
+    try {
+        cudaStreamCaptureStatus cs;
+        cudaGraph_t cg = nullptr;
+        const cudaGraphNode_t *deps = nullptr;
+        size_t ndeps = 0;
+        CK(cudaStreamGetCaptureInfo(outer, &cs, nullptr, &cg, &deps, &ndeps));
+        cudaGraphConditionalHandle h;
+        CK(cudaGraphConditionalHandleCreate(&h, cg, 1, cudaGraphCondAssignDefault));
+        cudaGraphNodeParams wp = {cudaGraphNodeTypeConditional};
+        wp.conditional.handle = h;
+        wp.conditional.type = cudaGraphCondTypeWhile;
+        wp.conditional.size = 1;
+        cudaGraphNode_t wnode;
+        CK(cudaGraphAddNode(&wnode, cg, deps, ndeps, &wp));
+        CK(cudaStreamUpdateCaptureDependencies(outer, &wnode, 1, cudaStreamSetCaptureDependencies));
+        c->st = c->st_body;
+        CK(cudaStreamBeginCaptureToGraph(c->st, wp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                         cudaStreamCaptureModeThreadLocal));
+        cudaGraph_t body = nullptr;
+        try {
+            for (int s = 0; s < JC_UNROLL; ++s)
+                jacobi_sweep(c, L, s & 1 ? tmp : phi, s & 1 ? phi : tmp, rho, S, s + 1 == JC_UNROLL, h);
+        } catch (...) {
+            cudaStreamEndCapture(c->st, &body);
+            throw;
+        }
+        CK(cudaStreamEndCapture(c->st, &body));
+        c->st = outer;
+        Launch L_(c, KC_JACOBI, 0.);
+        k_jacobi_out<<<nblk(N, 256), 256, 0, c->st>>>(phi, tmp, c->d_js, N);
+    } catch (...) {
+        c->st = outer;
+        cudaStreamEndCapture(outer, &g);
+        if (g) cudaGraphDestroy(g);
+        c->launches = l0;
+        throw;
+    }
+    CK(cudaStreamEndCapture(outer, &g));
+    JacGraph J{phi, tmp, rho, S, nullptr};
+    const cudaError_t e = cudaGraphInstantiate(&J.exec, g, 0);
+    cudaGraphDestroy(g);
+    CK(e);
+    c->launches = l0;
+    c->jac.push_back(J);
+    return J.exec;
+}
+
 // solver_poisson_jacobi_nlin::solve (:50-108) on one level; phi, tmp: level-sized.
 int jacobi_solve(kf_ctx *c, const LevelBuf &L, double *phi, double *tmp, const double *rho, int max_it,
                  double limit_max, bool resstop, double tol) {
     const long N = (long)L.n * L.n * L.n;
-    const int nb = red_blocks(N);
-    c->sup = 0.;
-    c->inf = 0.;
-    int iteration = 0;
-    c->omega = 1.;
-    bool converged = false;
-    c->norm_sum_old = -1.;
-    if (max_it < 0) max_it = 1000;
-    double *cur = phi, *oth = tmp;
-    double rlast = 0.;
-    while (!converged && iteration < max_it) {
-        iteration++;
-        c->norm_sum_old = c->norm_sum;
-        c->norm_max_old = c->norm_max;
-        {
-            Launch L_(c, KC_JACOBI, 24. * N);
-            k_jacobi<RBS><<<nb, RBS, 0, c->st>>>(cur, oth, rho, L.lev(), c->omega, c->partial);
+    const JacStop S{max_it < 0 ? 1000 : max_it, resstop, limit_max, tol};
+    JacState &js = *c->h_js;
+    js = JacState{};
+    js.norm_max = c->norm_max;
+    js.norm_sum = c->norm_sum;
+    js.omega = 1.;
+    if (S.max_it > 0) {
+        cudaGraphExec_t exec = c->prof ? nullptr : jacobi_graph(c, L, phi, tmp, rho, S);
+        CK(cudaMemcpyAsync(c->d_js, &js, sizeof(JacState), cudaMemcpyHostToDevice, c->st));
+        if (exec) {
+            CK(cudaGraphLaunch(exec, c->st));
+        } else {  // one sweep at a time, for the per-launch profile
+            for (int s = 0; !js.done; ++s) {
+                jacobi_sweep(c, L, s & 1 ? tmp : phi, s & 1 ? phi : tmp, rho, S, 0, 0);
+                CK(cudaGetLastError());
+                CK(cudaMemcpyAsync(&js, c->d_js, sizeof(JacState), cudaMemcpyDeviceToHost, c->st));
+                CK(cudaStreamSynchronize(c->st));
+            }
+            Launch L_(c, KC_JACOBI, 0.);
+            k_jacobi_out<<<nblk(N, 256), 256, 0, c->st>>>(phi, tmp, c->d_js, N);
         }
-        reduce_read(c, nb);
-        std::swap(cur, oth);
-        c->norm_max = c->h_red[0];
-        c->norm_sum = c->h_red[1];
-        c->sup = c->h_red[2];
-        c->inf = c->h_red[3];
-        rlast = c->h_red[4];
-        if (rlast != rlast || c->norm_max != c->norm_max) throw KfError{KF_ERR_NAN, "NaN in the Jacobi sweep"};
-        // Carre's over-relaxation factor (:237-252)
-        c->norm_sum = c->norm_sum / ((double)N);
-        if ((c->norm_max < c->norm_max_old) && (iteration > 1)) {
-            double lambda = c->norm_sum / c->norm_sum_old;
-            c->omega = 2. / (1. + sqrt(1. - pow(lambda + c->omega - 1., 2.) / (lambda * pow(c->omega, 2.))));
-        } else {
-            c->omega = .5;
-        }
-        if (c->omega != c->omega) c->omega = .5;
-        bool conv_rel = c->norm_max < limit_max * (c->sup - c->inf);
-        converged = resstop ? (rlast <= tol) : conv_rel;
+        CK(cudaMemcpyAsync(&js, c->d_js, sizeof(JacState), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+        if (exec) c->launches += js.iteration + 1;
     }
-    if (cur != phi) CK(cudaMemcpyAsync(phi, cur, sizeof(double) * N, cudaMemcpyDeviceToDevice, c->st));
-    c->diag.last_iterations = iteration;
-    c->diag.total_iterations += iteration;
-    c->diag.last_residual = rlast;
-    if (!converged) c->diag.not_converged++;
-    return converged ? 0 : 1;
+    c->norm_max = js.norm_max;
+    c->norm_sum = js.norm_sum;
+    if (js.nan) throw KfError{KF_ERR_NAN, "NaN in the Jacobi sweep"};
+    c->diag.last_iterations = js.iteration;
+    c->diag.total_iterations += js.iteration;
+    c->diag.last_residual = js.rlast;
+    if (!js.converged) c->diag.not_converged++;
+    return js.converged ? 0 : 1;
 }
 
 // over-relaxation factor of the FAS smoother's Newton step (0 selects 1)
@@ -1838,7 +1899,7 @@ void build_levels(kf_ctx *c) {
         const int n = c->n >> l;
         L.n = n;
         const double Lb = cf.L;
-        std::vector<double> H(n + 1), dd(n), dp(n), dm(n), ip(n), im(n), gam(n, 0.);
+        std::vector<double> H(n + 1), dd(n), dp(n), dm(n), ip(n), im(n), rp(n), rm(n), gam(n, 0.);
         const double sm = cf.stretch_m;
         for (int i = 0; i < n + 1; ++i) H[i] = val_at(i, n, Lb, sm) - val_at(i - 1, n, Lb, sm);  // H_create (:112-126)
         for (int i = 0; i < n; ++i) {
@@ -1847,6 +1908,8 @@ void build_levels(kf_ctx *c) {
             dm[i] = H[i] * (H[i + 1] + H[i]);
             ip[i] = 2. / dp[i];
             im[i] = 2. / dm[i];
+            rp[i] = 1. / dp[i];
+            rm[i] = 1. / dm[i];
         }
         for (int m = 1; m < n; m += 2) {  // OP_hto2h gamma on this (fine) axis
             const double x1 = val_at(m - 1, n, Lb, sm), x2 = val_at(m + 1, n, Lb, sm), x = val_at(m, n, Lb, sm);
@@ -1858,6 +1921,10 @@ void build_levels(kf_ctx *c) {
         L.gam = dalloc<double>(c, 8 * n);
         L.ip = dalloc<double>(c, 8 * n);
         L.im = dalloc<double>(c, 8 * n);
+        L.rp = dalloc<double>(c, 8 * n);
+        L.rm = dalloc<double>(c, 8 * n);
+        CK(cudaMemcpy(L.rp, rp.data(), 8 * n, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(L.rm, rm.data(), 8 * n, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(L.ip, ip.data(), 8 * n, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(L.im, im.data(), 8 * n, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(L.dd, dd.data(), 8 * n, cudaMemcpyHostToDevice));
@@ -2147,6 +2214,8 @@ void create(kf_ctx *c) {
     CK(cudaMallocHost(&c->h_max, 64 * sizeof(unsigned long long)));
     if (cf.phi_extrap) c->phi_a = dalloc<double>(c, 8 * c->N);
     CK(cudaMallocHost(&c->h_red, sizeof(double) * 8));
+    c->d_js = dalloc<JacState>(c, sizeof(JacState));
+    CK(cudaMallocHost(&c->h_js, sizeof(JacState)));
     c->dtime = dalloc<DevTime>(c, sizeof(DevTime));
     c->dpois = dalloc<DevPois>(c, sizeof(DevPois));
     CK(cudaMemset(c->dtime, 0, sizeof(DevTime)));
@@ -2612,6 +2681,8 @@ int kf_ctx_destroy(kf_ctx *c) {
     adj_release(c);
     out_release(c);
     for (void *p : c->allocs) cudaFree(p);
+    for (auto &g : c->jac) cudaGraphExecDestroy(g.exec);
+    if (c->h_js) cudaFreeHost(c->h_js);
     if (c->h_red) cudaFreeHost(c->h_red);
     if (c->h_max) cudaFreeHost(c->h_max);
     if (c->h_err) cudaFreeHost(c->h_err);

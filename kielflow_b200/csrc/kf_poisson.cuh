@@ -22,6 +22,8 @@ struct Lev {
     const double *dm;  // H[i]   (H[i+1] + H[i])
     const double *ip;  // 2/dp  (FAS cycle weights)
     const double *im;  // 2/dm
+    const double *rp;  // 1/dp  (k_jacobi's division)
+    const double *rm;  // 1/dm
 };
 
 __device__ __forceinline__ int wrapi(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
@@ -74,100 +76,12 @@ __device__ __forceinline__ double f_point(double A, double D, double x) {
     return __dsub_rn(__dsub_rn(A, __dmul_rn(D, x)), exp(x));
 }
 
-// newton_method::solve (newton_method.hpp:16-63), eps 0.05, Nmax 20, g 0.8
-__device__ __forceinline__ double newton_point(double x, double A, double D) {
-    const double g = 0.8;
-    double omega = 1.;
-    double dx = 0.;
-    double ex = exp(x);
-    double dx_alt = __dsub_rn(__dsub_rn(A, __dmul_rn(D, x)), ex) / __dsub_rn(-D, ex);
-    int i = 0;
-    do {
-        x = __dsub_rn(x, __dmul_rn(omega, dx));
-        ex = exp(x);
-        dx = __dsub_rn(__dsub_rn(A, __dmul_rn(D, x)), ex) / __dsub_rn(-D, ex);
-        omega = fabs(dx) > fabs(dx_alt) ? __dmul_rn(g, omega) : __dadd_rn(__dmul_rn(1. - g, omega), g * 1.);
-        dx_alt = dx;
-        ++i;
-    } while (fabs(dx) > 0.05 && i < 20);
-    return __dsub_rn(x, dx);
-}
-
 // ------------------------------------------------------------ reductions
-// Block partials of the Jacobi sweep statistics; slot layout per block:
-// [0] max|dP|, [1] sum|dP|, [2] max P_new, [3] min P_new, [4] max|f(P_old)|
-constexpr int KF_RED = 5;
+constexpr int KF_RED = 5;  // slots of a block's partials (kf_jacobi.cuh)
 
 // NaN-propagating max / min (fmax alone would drop a NaN)
 __device__ __forceinline__ double nmax(double a, double b) { return (a != a || b != b) ? a + b : fmax(a, b); }
 __device__ __forceinline__ double nmin(double a, double b) { return (a != a || b != b) ? a + b : fmin(a, b); }
-
-template <int BS>
-__device__ __forceinline__ void block_reduce5(double v[KF_RED], double *sh, double *out) {
-    // sh: [KF_RED][BS]
-    for (int s = 0; s < KF_RED; ++s) sh[s * BS + threadIdx.x] = v[s];
-    __syncthreads();
-    for (int w = BS / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            double *a = sh + threadIdx.x, *b = sh + threadIdx.x + w;
-            a[0] = nmax(a[0], b[0]);
-            a[BS] = __dadd_rn(a[BS], b[BS]);
-            a[2 * BS] = nmax(a[2 * BS], b[2 * BS]);
-            a[3 * BS] = nmin(a[3 * BS], b[3 * BS]);
-            a[4 * BS] = nmax(a[4 * BS], b[4 * BS]);
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int s = 0; s < KF_RED; ++s) out[s] = sh[s * BS];
-}
-
-// Jacobi sweep (iteration_loop, solver_poisson_jacobi_nlin.cpp:140-235)
-template <int BS>
-__global__ void __launch_bounds__(BS) k_jacobi(const double *__restrict__ in, double *__restrict__ out,
-                                               const double *__restrict__ rho, Lev L, double omega,
-                                               double *__restrict__ partial) {
-    __shared__ double sh[KF_RED * BS];
-    const int n = L.n;
-    const long N = (long)n * n * n;
-    double v[KF_RED] = {0., 0., -INFINITY, INFINITY, 0.};
-    if (blockIdx.x == 0 && threadIdx.x == 0) v[2] = v[3] = in[0];  // supremum = infinum = in.val[0] (:158-159)
-    for (long id = (long)blockIdx.x * BS + threadIdx.x; id < N; id += (long)gridDim.x * BS) {
-        const int k = (int)(id % n);
-        const long r = id / n;
-        const int j = (int)(r % n), i = (int)(r / n);
-        double A, D;
-        point_coeffs(in, rho, L, i, j, k, A, D);
-        const double P_old = in[id];
-        const double f0 = f_point(A, D, P_old);
-        const double P_new = newton_point(P_old, A, D);
-        const double delta = fabs(__dsub_rn(P_new, P_old));
-        out[id] = __dadd_rn(__dmul_rn(1. - omega, P_old), __dmul_rn(omega, P_new));
-        v[0] = nmax(v[0], delta);
-        v[1] = __dadd_rn(v[1], delta);
-        v[2] = nmax(v[2], P_new);
-        v[3] = nmin(v[3], P_new);
-        v[4] = nmax(v[4], fabs(f0));
-    }
-    block_reduce5<BS>(v, sh, partial + (long)blockIdx.x * KF_RED);
-}
-
-// Final fixed-order reduction of nb block partials into out[0..4].
-template <int BS>
-__global__ void __launch_bounds__(BS) k_reduce_final(const double *__restrict__ partial, int nb,
-                                                     double *__restrict__ out) {
-    __shared__ double sh[KF_RED * BS];
-    double v[KF_RED] = {0., 0., -INFINITY, INFINITY, 0.};
-    for (int b = threadIdx.x; b < nb; b += BS) {
-        const double *p = partial + (long)b * KF_RED;
-        v[0] = nmax(v[0], p[0]);
-        v[1] = __dadd_rn(v[1], p[1]);
-        v[2] = nmax(v[2], p[2]);
-        v[3] = nmin(v[3], p[3]);
-        v[4] = nmax(v[4], p[4]);
-    }
-    block_reduce5<BS>(v, sh, out);
-}
 
 // Launch geometry of the multigrid kernels: block (32, 8), grid
 // (ceil(nx/32), ceil(n/8), n) over (k or k/2, j, i) -- no index division.
