@@ -1887,6 +1887,10 @@ void build_levels(kf_ctx *c) {
     for (int l = 1; l < nl; ++l)
         if ((c->n >> l) < 2 || ((c->n >> (l - 1)) % 2))
             throw KfError{KF_ERR_ARG, "too many multigrid levels for this grid"};
+    // a red-black order needs even grids: with an odd level the half sweeps read
+    // and write past the level's end
+    if (cf.poisson_mode == KF_PS_FAS && (c->n >> (nl - 1)) % 2)
+        throw KfError{KF_ERR_ARG, "an FAS level with an odd number of points per axis; fewer levels needed"};
     if (cf.poisson_mode == KF_PS_CASCADIC && c->n % 8) throw KfError{KF_ERR_ARG, "cascadic plan needs n % 8 == 0"};
     if (cf.poisson_mode == KF_PS_FAS && ((long)(c->n >> (nl - 1)) * (c->n >> (nl - 1)) * (c->n >> (nl - 1)) > 8192))
         throw KfError{KF_ERR_ARG, "coarsest FAS level above 8192 points (shared-memory solve); add levels"};

@@ -91,3 +91,12 @@ def test_load_rejects_another_grid(tmp_path):
         assert e.value.code == -1
         with pytest.raises(kf.KfError):
             b.load(str(tmp_path / "missing.kfh"))
+
+
+def test_odd_multigrid_level_is_refused():
+    """96^3 with six levels would end at 3^3; five end at 6^3."""
+    with pytest.raises(kf.KfError) as e:
+        kf.Context(kf.Config.make(96, C.L_BOX, 0.8, poisson_mode=kf.KF_PS_FAS, mg_levels=6))
+    assert e.value.code == -1  # KF_ERR_ARG
+    with kf.Context(kf.Config.make(96, C.L_BOX, 0.8, poisson_mode=kf.KF_PS_FAS, mg_levels=5)):
+        pass
