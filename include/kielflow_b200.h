@@ -280,12 +280,13 @@ int kf_autotune(kf_ctx *ctx, int reps, kf_tune_out *out);
  * applied to every instance of a sweep).  KF_ERR_ARG for other values. */
 int kf_set_tuning(kf_ctx *ctx, int fft_plan, int rbgs_rows);
 
-/* Levels of at most 16^3 points below the finest, in FAS V-cycles that reach
- * a level below them (the 16^3 and 8^3 levels of the 6-level 256^3 cycle):
- * on = 1 (the default) runs them, with the correction they return, as one
- * block with the levels in shared memory (one launch instead of 16 kernels
- * that each last about their launch latency); on = 0 level by level.  The
- * potentials are the same bit for bit.  KF_ERR_ARG for other values. */
+/* The levels of at most 32^3 points below the finest, in FAS V-cycles (and in
+ * the adjoint's linear ones): on = 1 (the default) runs them, with the
+ * correction they return, in one thread-block cluster with the levels in its
+ * shared memory (one launch instead of a dozen kernels a level that each last
+ * about their launch latency, and a coarsest solve on one SM); on = 0 level by
+ * level.  The potentials are the same bit for bit.  KF_ERR_ARG for other
+ * values. */
 int kf_set_coarse_block(kf_ctx *ctx, int on);
 
 /* In the captured step (kf_rk4_steps, kf_step_host, kf_batch_rk4_steps), the

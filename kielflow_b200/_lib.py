@@ -357,9 +357,9 @@ class Context:
         self._check(self.L.kf_set_tuning(self.h, fft_plan, rbgs_rows))
 
     def set_coarse_block(self, on: bool):
-        """kf_set_coarse_block: run the V-cycle's levels of at most 16^3 points
-        (when a level lies below them) as one shared-memory block (True, the
-        default) or level by level (False); bit-identical potentials."""
+        """kf_set_coarse_block: run the V-cycle's levels of at most 32^3 points
+        below the finest in one thread-block cluster (True, the default) or
+        level by level (False); bit-identical potentials."""
         self._check(self.L.kf_set_coarse_block(self.h, 1 if on else 0))
 
     def set_overlap(self, on: bool):

@@ -264,14 +264,18 @@ void avcycle(kf_ctx *c, int l) {
         Launch L_(c, KC_ADJ_MG, 8. * N + 32. * Nc3);
         k_restrict<<<mg_grid(Lc.n, Lc.n), mg_block(), 0, c->st>>>(A.r, A.psi, n, C.r, C.psi, C.phi0);
     }
-    {
-        Launch L_(c, KC_ADJ_MG, 32. * Nc3);
-        k_fas_rhs_lin<<<mg_grid(Lc.n, Lc.n), mg_block(), 0, c->st>>>(C.psi, C.r, C.cc, Lc.lev(), C.b);
-    }
-    avcycle(c, l + 1);
-    {
-        Launch L_(c, KC_ADJ_MG, 24. * Nc3);
-        k_correction<<<mg_grid(Lc.n, Lc.n), mg_block(), 0, c->st>>>(C.psi, C.phi0, Lc.n);
+    if (l + 1 == c->cc_level) {
+        coarse_cluster<true>(c, C.psi, C.phi0, C.r, &c->adj->cl, kAdjCoarseRtol, 400, KC_ADJ_MG);
+    } else {
+        {
+            Launch L_(c, KC_ADJ_MG, 32. * Nc3);
+            k_fas_rhs_lin<<<mg_grid(Lc.n, Lc.n), mg_block(), 0, c->st>>>(C.psi, C.r, C.cc, Lc.lev(), C.b);
+        }
+        avcycle(c, l + 1);
+        {
+            Launch L_(c, KC_ADJ_MG, 24. * Nc3);
+            k_correction<<<mg_grid(Lc.n, Lc.n), mg_block(), 0, c->st>>>(C.psi, C.phi0, Lc.n);
+        }
     }
     {
         Launch L_(c, KC_ADJ_MG, 16. * N + 8. * Nc3);

@@ -25,6 +25,7 @@
 
 #include "../../include/kielflow_b200.h"
 #include "kf_adjoint.cuh"
+#include "kf_cluster.cuh"
 #include "kf_graph.cuh"
 #include "kf_jacobi.cuh"
 #include "kf_march.cuh"
@@ -175,10 +176,10 @@ struct kf_ctx {
     int fftv = 0;     // radix-plan variant of the transform kernels (kf_autotune)
     int rbgs_by = 8;  // smoother variant (kf_autotune): k_rbgs rows per block, or 0 for k_rbgs_march
     bool march_maps = false;  // the driver's tensor-map encoder is available
-    bool coarse_block = true;  // levels <= 16^3 of a V-cycle in one k_coarse_cycle block (kf_set_coarse_block)
-    int cc_level = -1;         // entry level of k_coarse_cycle, or -1 (cc_setup)
-    CoarseCycle ccyc{};
-    size_t cc_smem = 0;
+    bool coarse_block = true;  // the coarse levels of a V-cycle in one k_cc cluster (kf_set_coarse_block)
+    int cc_level = -1;         // entry level of k_cc, or -1 (cc_setup)
+    int cc_ctas = 0;           // its cluster size
+    ClusterCycle ccyc{};
     // window of rows (i, j) on which the penalization mask is not zero
     // (k_mask_box; bi = 0: none)
     int bx_i0 = 0, bx_i = 0, bx_j0 = 0, bx_j = 0;
@@ -242,7 +243,7 @@ enum KCls { KC_AXIS_INV, KC_AXIS_FWD, KC_Z_C2R, KC_Z_R2C, KC_XASM, KC_PROD, KC_L
 const char *const kKClsName[KC_N] = {"k_axis_pass(inverse)", "k_axis_pass(forward)", "k_z_c2r", "k_z_r2c",
                                      "k_xfwd_stage", "k_zprod/k_products", "k_lin", "k_rho", "k_rk", "k_jacobi",
                                      "k_rbgs", "k_residual", "k_restrict/k_fas_rhs/k_prolong/k_inject",
-                                     "k_coarse_solve/k_coarse_cycle", "-", "conversion/diagnostics",
+                                     "k_coarse_solve/k_cc", "-", "conversion/diagnostics",
                                      "adjoint pointwise (k_prod_vjp/k_vjp_assemble/k_adj_stage/...)",
                                      "adjoint Poisson (linear multigrid)",
                                      "FAS levels below the finest (k_rbgs/k_residual/transfers)",
@@ -729,6 +730,34 @@ void smooth_plain(kf_ctx *c, LevelBuf &L, double *phi, const double *rho, const 
         }
 }
 
+// The coarse levels' cycle (k_cc) from the injected potential, its copy and the
+// restricted residual of the entry level.  LIN: the adjoint's linear system with
+// e^phi in cc, its coarsest relaxation tested every 4 sweeps and not over-relaxed
+// (k_coarse_solve_lin).
+template <bool LIN>
+void coarse_cluster(kf_ctx *c, double *phi, double *phi0, const double *r, const std::vector<double *> *cc,
+                    double rtol, int max_sweeps, int cls) {
+    const kf_config &cf = c->cfg;
+    ClusterCycle C = c->ccyc;
+    if (LIN)
+        for (int m = 0; m < C.nl; ++m) C.cc[m] = (*cc)[c->cc_level + m];
+    const long N = (long)C.n[0] * C.n[0] * C.n[0];
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(c->cc_ctas);
+    lc.blockDim = dim3(CC_THREADS);
+    lc.dynamicSmemBytes = cc_smem(C, c->cc_ctas, LIN);
+    lc.stream = c->st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = c->cc_ctas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    Launch L_(c, cls, 40. * N);
+    CK(cudaLaunchKernelEx(&lc, k_cc<LIN>, phi, phi0, r, C, cf.mg_pre, cf.mg_post, LIN ? 0. : cf.coarse_tol, rtol,
+                          max_sweeps, LIN ? 4 : 1, mg_omega(cf), LIN ? 1. : mg_omega(cf), c->d_sweeps));
+}
+
 void vcycle(kf_ctx *c, int l);
 
 // First part of a V-cycle on level l (not the coarsest): pre-smoothing and the
@@ -793,10 +822,8 @@ void vcycle_tail(kf_ctx *c, int l) {
         k_restrict<<<mg_grid(Lc.n, Lc.n), mg_block(), 0, c->st>>>(L.r, L.phi, n, Lc.r, Lc.phi, Lc.phi0);
     }
     if (l + 1 == c->cc_level) {
-        // the levels from l + 1 down in one block: FAS right-hand side, cycle, correction
-        Launch L_(c, KC_COARSE, 40. * Nc3);
-        k_coarse_cycle<<<1, 1024, c->cc_smem, c->st>>>(Lc.phi, Lc.phi0, Lc.r, c->ccyc, cf.mg_pre, cf.mg_post,
-                                                       cf.coarse_tol, 1000, mg_omega(cf), c->d_sweeps);
+        // the levels from l + 1 down: FAS right-hand side, cycle, correction
+        coarse_cluster<false>(c, Lc.phi, Lc.phi0, Lc.r, nullptr, 1e-4, 1000, KC_COARSE);
     } else {
         {
             Launch L_(c, l == 0 ? KC_TRANSFER : KC_MG_COARSE, 24. * Nc3);
@@ -1959,22 +1986,27 @@ void build_levels(kf_ctx *c) {
             L.phi0 = dalloc<double>(c, bytes);
         }
     }
-    CK(cudaFuncSetAttribute(k_coarse_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    for (const void *k : {(const void *)k_cc<false>, (const void *)k_cc<true>}) {
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CC_SMEM_MAX));
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
     cc_setup(c);
 }
 
-// The entry level of k_coarse_cycle: the first level below the finest with
-// n <= 16 that has at least one level below it, when the levels from it down
-// fit the kernel (KF_CC_LEVELS, 200 KB of shared memory); -1 otherwise or
-// with the block switched off.
+// The coarse levels that k_cc takes: from the first level below the finest with
+// n <= 32 down, in a cluster of as many CTAs as divide the coarsest n (one plane
+// of it each at 16^3: the chain of sweeps there is what the size serves), as long
+// as the levels fit the kernel and the device can hold such a cluster; -1 with
+// the switch off.  (From 64^3 down a cluster's 16 SMs would be slower than the
+// whole chip with its launches.)
 void cc_setup(kf_ctx *c) {
     c->cc_level = -1;
     const int nl = (int)c->lv.size();
-    if (!c->coarse_block || c->cfg.poisson_mode != KF_PS_FAS) return;
+    if (!c->coarse_block || c->cfg.poisson_mode != KF_PS_FAS || nl < 2) return;
     int lb = 1;
-    while (lb < nl && c->lv[lb].n > 16) ++lb;
-    if (lb >= nl - 1 || nl - lb > KF_CC_LEVELS) return;
-    CoarseCycle C{};
+    while (lb < nl - 1 && (c->lv[lb].n > CC_MAX_N || nl - lb > CC_LEVELS)) ++lb;
+    if (c->lv[lb].n > CC_MAX_N) return;
+    ClusterCycle C{};
     C.nl = nl - lb;
     for (int m = 0; m < C.nl; ++m) {
         const LevelBuf &L = c->lv[lb + m];
@@ -1984,11 +2016,31 @@ void cc_setup(kf_ctx *c) {
         C.im[m] = L.im;
         C.gam[m] = L.gam;
     }
-    const size_t b = coarse_cycle_smem(C);
-    if (b > 200 * 1024) return;
-    c->ccyc = C;
-    c->cc_smem = b;
-    c->cc_level = lb;
+    const int nc = c->lv[nl - 1].n;
+    for (int cl = std::min(nc, CC_MAX_CTAS); cl >= 1; --cl) {
+        const size_t sm = cc_smem(C, cl, true);
+        if (nc % cl || sm > (size_t)CC_SMEM_MAX) continue;
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3(cl);
+        lc.blockDim = dim3(CC_THREADS);
+        lc.dynamicSmemBytes = sm;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = cl;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, k_cc<true>, &lc) != cudaSuccess) {
+            cudaGetLastError();
+            fit = 0;
+        }
+        if (fit < 1) continue;
+        c->ccyc = C;
+        c->cc_ctas = cl;
+        c->cc_level = lb;
+        return;
+    }
 }
 
 void build_jobs(kf_ctx *c) {

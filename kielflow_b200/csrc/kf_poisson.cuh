@@ -576,134 +576,6 @@ __global__ void __launch_bounds__(256) k_prolong_add(double *__restrict__ phi, c
     prolong_cell(phi, e, gam, nf, I, J, K);
 }
 
-// ------------------------------------------------------------ coarse levels in one block
-// Levels of at most 16^3 points hold at most 4096 points: the kernels of one
-// V-cycle there (half-sweeps, residual, restriction, FAS right-hand side,
-// coarsest solve, correction, prolongation: 14 launches from the 16^3 level
-// down to 8^3) each run for about the time of their launch.  k_coarse_cycle
-// runs all of it in one block with every level in shared memory, from the
-// entry level's injected potential and restricted residual (k_restrict) to
-// its correction e = phi - phi0 (left in phi0 for k_prolong_add), with the
-// per-point arithmetic of the level-by-level kernels, so the potentials are
-// the same bit for bit.
-constexpr int KF_CC_LEVELS = 4;
-
-struct CoarseCycle {
-    int nl;  // levels held: 0 = the entry level, nl - 1 = the coarsest (2 <= nl <= KF_CC_LEVELS)
-    int n[KF_CC_LEVELS];
-    const double *dd[KF_CC_LEVELS], *ip[KF_CC_LEVELS], *im[KF_CC_LEVELS];
-    const double *gam[KF_CC_LEVELS];  // fine-axis gammas of level m (prolongation from m + 1)
-};
-
-// Shared memory of k_coarse_cycle: per level phi, rho, r, phi0 (n^3 each) and
-// four axis tables (n each).
-inline size_t coarse_cycle_smem(const CoarseCycle &C) {
-    size_t b = 0;
-    for (int m = 0; m < C.nl; ++m) b += 8 * (4 * (size_t)C.n[m] * C.n[m] * C.n[m] + 4 * (size_t)C.n[m]);
-    return b;
-}
-
-// Level m of the shared-memory layout of k_coarse_cycle.
-struct CcLevel {
-    double *P, *R, *F, *P0;  // phi, rho, r, phi0
-    Lev L;                   // n and the tables dd, ip, im (in shared memory)
-    double *G;               // gammas (in shared memory)
-};
-__device__ __forceinline__ CcLevel cc_level(const CoarseCycle &C, double *sm, int m) {
-    for (int l = 0; l < m; ++l) sm += 4 * (C.n[l] * C.n[l] * C.n[l] + C.n[l]);
-    const int n = C.n[m], N = n * n * n;
-    double *t = sm + 4 * N;
-    return CcLevel{sm, sm + N, sm + 2 * N, sm + 3 * N, Lev{n, t, nullptr, nullptr, t + n, t + 2 * n}, t + 3 * n};
-}
-
-__global__ void __launch_bounds__(1024) k_coarse_cycle(double *__restrict__ phi, double *__restrict__ phi0,
-                                                       const double *__restrict__ r, CoarseCycle C, int pre,
-                                                       int post, double tol, int max_sweeps, double om,
-                                                       int *__restrict__ sweeps_out) {
-    extern __shared__ __align__(16) double cc_sm[];
-    __shared__ double sh[32];
-    for (int m = 0; m < C.nl; ++m) {
-        const CcLevel V = cc_level(C, cc_sm, m);
-        double *dd = const_cast<double *>(V.L.dd), *ip = const_cast<double *>(V.L.ip);
-        double *im = const_cast<double *>(V.L.im);
-        for (int t = threadIdx.x; t < V.L.n; t += blockDim.x) {
-            dd[t] = C.dd[m][t];
-            ip[t] = C.ip[m][t];
-            im[t] = C.im[m][t];
-            V.G[t] = C.gam[m] ? C.gam[m][t] : 0.;
-        }
-    }
-    {
-        const CcLevel V = cc_level(C, cc_sm, 0);
-        const int N = C.n[0] * C.n[0] * C.n[0];
-        for (int id = threadIdx.x; id < N; id += blockDim.x) {
-            V.P[id] = phi[id];
-            V.R[id] = r[id];
-        }
-    }
-    __syncthreads();
-    // the entry level's FAS right-hand side (k_fas_rhs) in place of its r;
-    // on the levels below, the restriction leaves r in R the same way
-    for (int m = 0; m < C.nl; ++m) {
-        const CcLevel V = cc_level(C, cc_sm, m);
-        const int n = V.L.n, N = n * n * n;
-        for (int id = threadIdx.x; id < N; id += blockDim.x) {
-            const int k = id % n, j = (id / n) % n, i = id / (n * n);
-            V.R[id] = fas_rho_point(V.P, V.R[id], V.L, i, j, k);
-        }
-        __syncthreads();
-        if (m + 1 == C.nl) break;
-        // pre-smoothing, residual (k_residual<true>), restriction and injection (k_restrict)
-        for (int s = 0; s < pre; ++s) {
-            block_half_sweep(V.P, V.R, V.L, 0, om);
-            block_half_sweep(V.P, V.R, V.L, 1, om);
-        }
-        for (int id = threadIdx.x; id < N; id += blockDim.x) {
-            const int k = id % n, j = (id / n) % n, i = id / (n * n);
-            double A, D;
-            point_coeffs_fast(V.P, V.R, V.L, i, j, k, A, D);
-            V.F[id] = f_point(A, D, V.P[id]);
-        }
-        __syncthreads();
-        const CcLevel W = cc_level(C, cc_sm, m + 1);
-        const int nc = n / 2, Ncc = nc * nc * nc;
-        for (int id = threadIdx.x; id < Ncc; id += blockDim.x) {
-            const int k = id % nc, j = (id / nc) % nc, i = id / (nc * nc);
-            W.R[id] = fw_point(V.F, n, i, j, k);
-            const double p = V.P[lidx(2 * i, 2 * j, 2 * k, n)];
-            W.P[id] = p;
-            W.P0[id] = p;
-        }
-        __syncthreads();
-    }
-    const CcLevel Vc = cc_level(C, cc_sm, C.nl - 1);
-    const int s = block_coarse_relax(Vc.P, Vc.R, Vc.L, tol, max_sweeps, om, sh);
-    for (int m = C.nl - 2; m >= 0; --m) {
-        // correction (k_correction), prolongation (k_prolong_add), post-smoothing
-        const CcLevel V = cc_level(C, cc_sm, m), W = cc_level(C, cc_sm, m + 1);
-        const int n = V.L.n, nc = n / 2, Ncc = nc * nc * nc;
-        for (int id = threadIdx.x; id < Ncc; id += blockDim.x) W.P0[id] = __dsub_rn(W.P[id], W.P0[id]);
-        __syncthreads();
-        for (int id = threadIdx.x; id < Ncc; id += blockDim.x) {
-            const int K = id % nc, J = (id / nc) % nc, I = id / (nc * nc);
-            prolong_cell(V.P, W.P0, V.G, n, I, J, K);
-        }
-        __syncthreads();
-        for (int t = 0; t < post; ++t) {
-            block_half_sweep(V.P, V.R, V.L, 0, om);
-            block_half_sweep(V.P, V.R, V.L, 1, om);
-        }
-    }
-    const CcLevel V0 = cc_level(C, cc_sm, 0);
-    const int N = C.n[0] * C.n[0] * C.n[0];
-    for (int id = threadIdx.x; id < N; id += blockDim.x) {
-        const double p = V0.P[id];
-        phi[id] = p;
-        phi0[id] = __dsub_rn(p, phi0[id]);
-    }
-    if (threadIdx.x == 0 && sweeps_out) *sweeps_out = s;
-}
-
 // Strided injection (OP_2htoh_lvl0 / OP_4htoh / OP_8htoh)
 __global__ void __launch_bounds__(256) k_inject(const double *__restrict__ in, int nf, int step,
                                                 double *__restrict__ out) {
