@@ -32,6 +32,7 @@
 #include "kf_passes.cuh"
 #include "kf_pointwise.cuh"
 #include "kf_poisson.cuh"
+#include "kf_split.cuh"
 #include "kf_stretch.cuh"
 #include "kf_zprod.cuh"
 
@@ -56,16 +57,18 @@ struct LevelBuf {
     double *rp = nullptr, *rm = nullptr;
     double *phi = nullptr, *rho = nullptr, *r = nullptr, *phi0 = nullptr;
     double *t = nullptr;  // second potential of the streaming smoother (k_rbgs_march), n >= MT_TK
+    // colour-split form (kf_split.cuh): sp says that the half-sweep cycle keeps the
+    // level's phi, rho, r and phi0 in split order; ph, rh are phi and rho so kept
+    // (the finest level's are buffers of their own)
+    bool sp = false;
+    double *ddk = nullptr, *ipk = nullptr, *imk = nullptr;
+    double *ph = nullptr, *rh = nullptr;
+    SLev slev() const { return SLev{n, dd, ip, im, ddk, ipk, imk}; }
     std::shared_ptr<AxTab> tab;  // host copy of dd, ip, im for k_rbgs_t (n <= KF_TAB_N)
     Lev lev() const { return Lev{n, dd, dp, dm, ip, im, rp, rm}; }
 };
 
 constexpr int RBS = 256;  // reduction block size
-
-// Colour-split copy of the finest rho for the half sweeps (0: they read rho).
-#ifndef KF_RHO_CS
-#define KF_RHO_CS 1
-#endif
 
 // Half sweeps with the i and j axis tables passed as a kernel parameter
 // (k_rbgs_t; 0: k_rbgs reads them from global memory).
@@ -105,7 +108,7 @@ struct kf_ctx {
     void *Y[4] = {}, *Ys[4] = {}, *ACC[4] = {}, *K[4] = {};
     void *CX[12] = {}, *CY[16] = {}, *R[24] = {}, *phihat = nullptr, *LIN[4] = {};
     double *phi = nullptr, *rho = nullptr, *nd = nullptr;
-    double *rho_cs = nullptr;  // colour-split copy of rho for the finest half sweeps (rho_split)
+    double *rho_cs = nullptr, *phi_cs = nullptr;  // the finest rho and phi in split order
     void *H = nullptr, *phiT = nullptr;
     void *kv = nullptr, *SV = nullptr, *PF = nullptr, *tw = nullptr;
     double *q2 = nullptr;
@@ -704,14 +707,6 @@ void smooth_plain(kf_ctx *c, LevelBuf &L, double *phi, const double *rho, const 
                     k_rbgs_lin<16><<<g, b, 0, c->st>>>(phi, rho, cc, L.lev(), color, om);
                 else
                     k_rbgs_lin<8><<<g, b, 0, c->st>>>(phi, rho, cc, L.lev(), color, om);
-            } else if (L.tab && rho == c->rho && c->rho_cs) {
-                // the finest level reads the colour-split copy (rho_split at the solve's start)
-                if (by == 4)
-                    k_rbgs_t<4, true><<<g, b, 0, c->st>>>(phi, c->rho_cs, L.lev(), color, om, *L.tab);
-                else if (by == 16)
-                    k_rbgs_t<16, true><<<g, b, 0, c->st>>>(phi, c->rho_cs, L.lev(), color, om, *L.tab);
-                else
-                    k_rbgs_t<8, true><<<g, b, 0, c->st>>>(phi, c->rho_cs, L.lev(), color, om, *L.tab);
             } else if (L.tab) {
                 if (by == 4)
                     k_rbgs_t<4><<<g, b, 0, c->st>>>(phi, rho, L.lev(), color, om, *L.tab);
@@ -758,6 +753,40 @@ void coarse_cluster(kf_ctx *c, double *phi, double *phi0, const double *r, const
                           max_sweeps, LIN ? 4 : 1, mg_omega(cf), LIN ? 1. : mg_omega(cf), c->d_sweeps));
 }
 
+// Whether level l's cycle runs in split order (not with the streaming smoother)
+bool split_on(const kf_ctx *c, int l) { return c->lv[l].sp && c->rbgs_by != 0; }
+
+// Blocks of the split-order kernels: 64 threads where the level streams from
+// memory, 128 where it lies in L2 (split_pair), halved or doubled by rbgs_rows 4, 16.
+dim3 split_block(const kf_ctx *c, int n) {
+    const int want = std::min(128, (n >= 256 ? 8 : 16) * c->rbgs_by), tx = n / 4;
+    return dim3(tx, std::max(1, want / tx));
+}
+
+// `sweeps` red-black sweeps in split order
+void smooth_split(kf_ctx *c, const LevelBuf &L, double *ph, const double *rh, int sweeps, int cls) {
+    const int n = L.n;
+    const dim3 b = split_block(c, n), g(1, (n + b.y - 1) / b.y, n);
+    for (int s = 0; s < sweeps; ++s)
+        for (int color = 0; color < 2; ++color) {
+            Launch L_(c, cls, 16. * n * n * n);
+            k_rbgs_s<<<g, b, 0, c->st>>>(ph, rh, L.slev(), color, mg_omega(c->cfg), *L.tab);
+        }
+}
+
+// r = residual in split order, its max |r| into the d_max slots with_max
+void residual_split(kf_ctx *c, const LevelBuf &L, bool with_max, int cls) {
+    const int n = L.n;
+    const int Z = with_max ? (n >= 128 ? 4 : 2) : (n >= 128 ? 2 : 1);
+    const dim3 b = split_block(c, n), g(1, (n + b.y - 1) / b.y, 2 * n / Z);
+    if (with_max) CK(cudaMemsetAsync(c->d_max, 0, 64 * sizeof(unsigned long long), c->st));
+    Launch L_(c, cls, 24. * n * n * n);
+    if (with_max)
+        k_residual_s<true><<<g, b, 0, c->st>>>(L.ph, L.rh, L.slev(), L.r, c->d_max, Z, *L.tab);
+    else
+        k_residual_s<false><<<g, b, 0, c->st>>>(L.ph, L.rh, L.slev(), L.r, nullptr, Z, *L.tab);
+}
+
 void vcycle(kf_ctx *c, int l);
 
 // First part of a V-cycle on level l (not the coarsest): pre-smoothing and the
@@ -767,6 +796,11 @@ void vcycle_head(kf_ctx *c, int l, bool with_max) {
     const kf_config &cf = c->cfg;
     const int n = L.n;
     const long N = (long)n * n * n;
+    if (split_on(c, l)) {
+        smooth_split(c, L, L.ph, L.rh, cf.mg_pre, l == 0 ? KC_RBGS : KC_MG_COARSE);
+        residual_split(c, L, with_max, l == 0 ? KC_RESID : KC_MG_COARSE);
+        return;
+    }
     if (march_ok(c, L) && cf.mg_pre >= 1) {
         // the last pre-smoothing sweep fused with the residual (and its max):
         // the sweeps before it leave the potential in L.t
@@ -817,6 +851,36 @@ void vcycle_tail(kf_ctx *c, int l) {
     const long N = (long)n * n * n;
     LevelBuf &Lc = c->lv[l + 1];
     const long Nc3 = (long)Lc.n * Lc.n * Lc.n;
+    if (split_on(c, l)) {
+        const int cls = l == 0 ? KC_TRANSFER : KC_MG_COARSE;
+        const bool cs = split_on(c, l + 1), cl = l + 1 == c->cc_level;
+        const dim3 g = mg_grid(Lc.n, Lc.n);
+        {
+            Launch L_(c, cls, 8. * N + 24. * Nc3);
+            if (cl)
+                k_restrict_s<false, false><<<g, mg_block(), 0, c->st>>>(L.r, L.ph, n, Lc.lev(), Lc.r, Lc.phi, Lc.phi0);
+            else if (cs)
+                k_restrict_s<true, true><<<g, mg_block(), 0, c->st>>>(L.r, L.ph, n, Lc.lev(), Lc.rho, Lc.phi, Lc.phi0);
+            else
+                k_restrict_s<false, true><<<g, mg_block(), 0, c->st>>>(L.r, L.ph, n, Lc.lev(), Lc.rho, Lc.phi, Lc.phi0);
+        }
+        if (cl)
+            coarse_cluster<false>(c, Lc.phi, Lc.phi0, Lc.r, nullptr, 1e-4, 1000, KC_COARSE);
+        else
+            vcycle(c, l + 1);
+        {
+            Launch L_(c, cls, 16. * N + (cl ? 8. : 16.) * Nc3);
+            if (cl)
+                k_prolong_s<false, true><<<g, mg_block(), 0, c->st>>>(L.ph, Lc.phi, Lc.phi0, L.gam, n);
+            else if (cs)
+                k_prolong_s<true, false><<<g, mg_block(), 0, c->st>>>(L.ph, Lc.phi, Lc.phi0, L.gam, n);
+            else
+                k_prolong_s<false, false><<<g, mg_block(), 0, c->st>>>(L.ph, Lc.phi, Lc.phi0, L.gam, n);
+        }
+        smooth_split(c, L, L.ph, L.rh, cf.mg_post, l == 0 ? KC_RBGS : KC_MG_COARSE);
+        CK(cudaGetLastError());
+        return;
+    }
     {
         Launch L_(c, l == 0 ? KC_TRANSFER : KC_MG_COARSE, 8. * N + 32. * Nc3);
         k_restrict<<<mg_grid(Lc.n, Lc.n), mg_block(), 0, c->st>>>(L.r, L.phi, n, Lc.r, Lc.phi, Lc.phi0);
@@ -918,14 +982,22 @@ double read_max_slots(kf_ctx *c) {
     return r;
 }
 
-// The colour-split copy of c->rho that the finest half sweeps read: made at
-// the start of a FAS solve, unless the pass that wrote c->rho (k_z_rho) wrote
-// it as well.
-void rho_split(kf_ctx *c) {
-    if (!c->rho_cs) return;
-    const int n = c->n;
+// The finest level in and out of split order around a solve.  rho: unless the
+// pass that wrote c->rho (k_z_rho) wrote its split copy as well.
+void split_field(kf_ctx *c, const double *x, double *s) {
     Launch L_(c, KC_RHO, 16. * c->N);
-    k_rho_split<<<mg_grid(n / 2, n), mg_block(), 0, c->st>>>(c->rho, c->rho_cs, n);
+    k_split<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(x, s, c->n);
+    CK(cudaGetLastError());
+}
+void solve_begin(kf_ctx *c, bool rho_done) {
+    if (!split_on(c, 0)) return;
+    if (!rho_done) split_field(c, c->rho, c->rho_cs);
+    split_field(c, c->phi, c->phi_cs);
+}
+void solve_end(kf_ctx *c) {
+    if (!split_on(c, 0)) return;
+    Launch L_(c, KC_RHO, 16. * c->N);
+    k_unsplit<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(c->phi_cs, c->phi, c->n);
     CK(cudaGetLastError());
 }
 
@@ -979,8 +1051,9 @@ int poisson(kf_ctx *c, bool split = false) {
     } else if (!(cf.res_tol > 0.)) {
         // fixed number of V-cycles: the result is a smooth function of rho
         // and of the initial guess (no data-dependent stopping)
-        if (!split) rho_split(c);
+        solve_begin(c, split);
         for (int cyc = 0; cyc < cf.max_cycles; ++cyc) run_vcycle(c);
+        solve_end(c);
         const double r = max_residual(c, L0, c->phi, c->rho, true);
         c->diag.last_iterations = cf.max_cycles;
         c->diag.total_iterations += cf.max_cycles;
@@ -990,7 +1063,7 @@ int poisson(kf_ctx *c, bool split = false) {
     } else if (c->lv.size() > 1) {
         // test after each cycle's pre-smoothing on the residual the cycle
         // computes anyway; the rest of the cycle only when it fails
-        if (!split) rho_split(c);
+        solve_begin(c, split);
         double r = 0.;
         int cyc = 0;
         for (;;) {
@@ -1001,6 +1074,7 @@ int poisson(kf_ctx *c, bool split = false) {
             run_vcycle_tail(c);
             ++cyc;
         }
+        solve_end(c);
         c->diag.last_iterations = cyc;
         c->diag.stage_cycles[c->stage_idx & 3] += cyc;
         c->diag.total_iterations += cyc;
@@ -1011,7 +1085,7 @@ int poisson(kf_ctx *c, bool split = false) {
             rc = 1;
         }
     } else {
-        if (!split) rho_split(c);
+        solve_begin(c, split);
         double r = max_residual(c, L0, c->phi, c->rho, true);
         int cyc = 0;
         while (r > cf.res_tol && cyc < cf.max_cycles) {
@@ -1056,9 +1130,15 @@ bool phi_guess(kf_ctx *c) {
 void poisson_captured(kf_ctx *c) {
     const kf_config &cf = c->cfg;
     const bool extrap = cf.phi_extrap != 0;
-    if (extrap) {
+    const bool sp = split_on(c, 0);
+    if (extrap && sp) {
+        Launch L_(c, KC_MISC, 32. * c->N);
+        k_guess_s<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(c->phi, c->phi_a, c->phi_cs, c->dtime, c->n);
+    } else if (extrap) {
         Launch L_(c, KC_MISC, 24. * c->N);
         k_guess<<<nblk(c->N, 256), 256, 0, c->st>>>(c->phi, c->phi_a, c->dtime, c->N);
+    } else if (sp) {
+        split_field(c, c->phi, c->phi_cs);
     }
     if (extrap) {
         Launch L_(c, KC_MISC, 0.);
@@ -1129,6 +1209,7 @@ void poisson_captured(kf_ctx *c) {
         c->st = outer;
         CK(e);
         c->cycle_kernels = c->launches - l0;
+        solve_end(c);
         if (extrap) {
             Launch L_(c, KC_MISC, 0.);
             k_hist_post<<<1, 32, 0, c->st>>>(c->dtime);
@@ -1137,6 +1218,10 @@ void poisson_captured(kf_ctx *c) {
         return;
     }
     auto resmax = [&](cudaStream_t st) {
+        if (sp) {
+            residual_split(c, L0, true, KC_RESID);
+            return;
+        }
         CK(cudaMemsetAsync(c->d_max, 0, 64 * sizeof(unsigned long long), st));
         Launch L_(c, KC_RESID, 16. * c->N);
         dim3 g = mg_grid(L0.n, L0.n);
@@ -1184,6 +1269,7 @@ void poisson_captured(kf_ctx *c) {
     c->st = outer;
     CK(e);
     c->cycle_kernels = c->launches - l0;
+    solve_end(c);
     if (extrap) {
         Launch L_(c, KC_MISC, 0.);
         k_hist_post<<<1, 32, 0, c->st>>>(c->dtime);
@@ -1985,6 +2071,27 @@ void build_levels(kf_ctx *c) {
             L.rho = dalloc<double>(c, bytes);
             L.phi0 = dalloc<double>(c, bytes);
         }
+        // above the sizes that the cluster takes, where bandwidth counts
+        L.sp = cf.poisson_mode == KF_PS_FAS && nl > 1 && l + 1 < nl && n > CC_MAX_N && n % 16 == 0 && L.tab;
+        if (L.sp) {
+            std::vector<double> t(3 * n);
+            for (int k = 0; k < n; ++k) {
+                const int e = (k & 1) * (n / 2) + k / 2;
+                t[e] = dd[k];
+                t[n + e] = ip[k];
+                t[2 * n + e] = im[k];
+            }
+            L.ddk = dalloc<double>(c, 8 * t.size());
+            L.ipk = L.ddk + n;
+            L.imk = L.ipk + n;
+            CK(cudaMemcpy(L.ddk, t.data(), 8 * t.size(), cudaMemcpyHostToDevice));
+            if (l == 0) {
+                c->phi_cs = dalloc<double>(c, bytes);
+                c->rho_cs = dalloc<double>(c, bytes);
+            }
+            L.ph = l == 0 ? c->phi_cs : L.phi;
+            L.rh = l == 0 ? c->rho_cs : L.rho;
+        }
     }
     for (const void *k : {(const void *)k_cc<false>, (const void *)k_cc<true>}) {
         CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CC_SMEM_MAX));
@@ -2244,8 +2351,6 @@ void create(kf_ctx *c) {
     c->phihat = dalloc<void>(c, cb);
     c->phi = dalloc<double>(c, 8 * c->N);
     c->rho = dalloc<double>(c, 8 * c->N);
-    if (KF_RHO_CS && c->cfg.poisson_mode == KF_PS_FAS && c->n >= 64 && c->n <= KF_TAB_N)
-        c->rho_cs = dalloc<double>(c, 8 * c->N);
     c->nd = dalloc<double>(c, 8 * c->N);
     c->H = dalloc<void>(c, rb);
     c->phiT = c->fp32 ? dalloc<void>(c, rb) : (void *)c->phi;
@@ -2660,8 +2765,7 @@ void autotune(kf_ctx *c, int reps, kf_tune_out *o) {
         double *tmp = nullptr;
         CK(cudaMalloc(&tmp, 8 * (size_t)c->N));
         try {
-            CK(cudaMemcpyAsync(tmp, c->phi, 8 * (size_t)c->N, cudaMemcpyDeviceToDevice, c->st));
-            rho_split(c);  // the finest half sweeps read the colour-split copy
+            if (c->phi_cs) split_field(c, c->rho, c->rho_cs);
             int best = -1;
             for (int k = 0; k < 4; ++k) {
                 c->rbgs_by = rows[k];
@@ -2669,8 +2773,17 @@ void autotune(kf_ctx *c, int reps, kf_tune_out *o) {
                     r.rbgs_ms[k] = -1.;
                     continue;
                 }
-                r.rbgs_ms[k] =
-                    0.5 * time_candidate(c, reps, [&] { smooth(c, L0, tmp, c->rho, nullptr, 2, KC_RBGS); });
+                const bool sp = split_on(c, 0);
+                if (sp)
+                    split_field(c, c->phi, tmp);
+                else
+                    CK(cudaMemcpyAsync(tmp, c->phi, 8 * (size_t)c->N, cudaMemcpyDeviceToDevice, c->st));
+                r.rbgs_ms[k] = 0.5 * time_candidate(c, reps, [&] {
+                                   if (sp)
+                                       smooth_split(c, L0, tmp, c->rho_cs, 2, KC_RBGS);
+                                   else
+                                       smooth(c, L0, tmp, c->rho, nullptr, 2, KC_RBGS);
+                               });
                 if (best < 0 || r.rbgs_ms[k] < r.rbgs_ms[best]) best = k;
             }
             r.rbgs_rows = rows[best];

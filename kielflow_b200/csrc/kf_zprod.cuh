@@ -176,7 +176,7 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
 //
 // Inverse, with the Poisson source as the epilogue: s_d = c2r(P s^) and
 // rho = e^{s_d} + n_d in FP64 (rhs_standard.cpp:108-111), into rho and, when
-// given, its colour-split copy (k_rho_split's layout); sd is written when given.
+// given, its colour-split copy (k_split's layout); sd is written when given.
 template <typename T, int N, int V>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
 k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, const double *__restrict__ nd,
