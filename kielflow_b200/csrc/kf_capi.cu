@@ -110,7 +110,8 @@ struct kf_ctx {
     double *phi = nullptr, *rho = nullptr, *nd = nullptr;
     double *rho_cs = nullptr, *phi_cs = nullptr;  // the finest rho and phi in split order
     void *H = nullptr, *phiT = nullptr;
-    void *kv = nullptr, *SV = nullptr, *PF = nullptr, *tw = nullptr;
+    void *kv = nullptr, *SV = nullptr, *PF = nullptr;
+    void *tw[2] = {};  // twiddles of the two radix plans (plan_twiddles)
     double *q2 = nullptr;
     int *pb = nullptr;  // x-pass 2/3-rule bounds per (j, kz) column (dealias_bounds)
     // the kept part of a masked half spectrum (AxTrunc)
@@ -1283,6 +1284,8 @@ template <typename T, int N> struct Impl {
     static constexpr int TC = Tile<T>::TC, LZ = ZTile<T>::LZ, NZC = N / 2 + 1;
     template <int V> static constexpr int PV = PlanV<N, V>::P;
 
+    static const T2 *tw(kf_ctx *c) { return (const T2 *)c->tw[c->fftv]; }
+
     static Geo<T> geo(kf_ctx *c) {
         return Geo<T>{c->n, c->nzc, (const T *)c->kv, c->q2, dealias_threshold(), c->pb};
     }
@@ -1370,10 +1373,10 @@ template <typename T, int N> struct Impl {
         const size_t smem = axis_pipe_smem<T, N>(njobs);
         if (sign < 0)
             k_axis_pipe<T, N, -1, V><<<grid, TC * PV<V>, smem, c->st>>>(c->dj + off, njobs, ax, geo(c),
-                                                                      (const T2 *)c->tw, total, A);
+                                                                      tw(c), total, A);
         else
             k_axis_pipe<T, N, +1, V><<<grid, TC * PV<V>, smem, c->st>>>(c->dj + off, njobs, ax, geo(c),
-                                                                      (const T2 *)c->tw, total, A);
+                                                                      tw(c), total, A);
     }
     static void axis(kf_ctx *c, int off, int njobs, int ax, int sign, int mode = AX_FULL) {
         Launch L_(c, sign > 0 ? KC_AXIS_INV : KC_AXIS_FWD, job_bytes(c, off, njobs, mode));
@@ -1407,10 +1410,10 @@ template <typename T, int N> struct Impl {
         const T sc = (T)(scale < 0. ? 1. / ((double)N * N * N) : scale);
         if (c->fftv)
             k_z_c2r<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        (const T2 *)c->tw, sc, nkz(c, masked));
+                                                                        tw(c), sc, nkz(c, masked));
         else
             k_z_c2r<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        (const T2 *)c->tw, sc, nkz(c, masked));
+                                                                        tw(c), sc, nkz(c, masked));
     }
     static void zr2c(kf_ctx *c, int off, int njobs, bool masked = false) {
         const int nrows = N * N;
@@ -1418,10 +1421,10 @@ template <typename T, int N> struct Impl {
         const size_t smem = ZSmem<T, N, false>::bytes;
         Launch L_(c, KC_Z_R2C, z_bytes(c, off, njobs, false, masked));
         if (c->fftv)
-            k_z_r2c<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, (const T2 *)c->tw,
+            k_z_r2c<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c),
                                                                         nkz(c, masked));
         else
-            k_z_r2c<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, (const T2 *)c->tw,
+            k_z_r2c<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c),
                                                                         nkz(c, masked));
     }
     static RhsArgs<T> rargs(kf_ctx *c) {
@@ -1454,10 +1457,10 @@ template <typename T, int N> struct Impl {
         Launch L_(c, KC_RHO, (double)N * N * nkz(c, true) * sizeof(T2) + (double)c->N * (c->rho_cs ? 24 : 16));
         if (c->fftv)
             k_z_rho<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, c->rho, c->rho_cs,
-                                                              (const T2 *)c->tw, sc, nkz(c, true));
+                                                              tw(c), sc, nkz(c, true));
         else
             k_z_rho<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, c->rho, c->rho_cs,
-                                                              (const T2 *)c->tw, sc, nkz(c, true));
+                                                              tw(c), sc, nkz(c, true));
         CK(cudaGetLastError());
     }
 
@@ -1467,9 +1470,9 @@ template <typename T, int N> struct Impl {
         const size_t smem = (size_t)LZ * PadLen<N>::value * sizeof(T2);
         Launch L_(c, KC_Z_R2C, (double)c->N * 8 + (double)c->Nc * sizeof(T2));
         if (c->fftv)
-            k_z_phi<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>(c->phi, (T2 *)c->CX[8], (const T2 *)c->tw, NZC);
+            k_z_phi<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>(c->phi, (T2 *)c->CX[8], tw(c), NZC);
         else
-            k_z_phi<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>(c->phi, (T2 *)c->CX[8], (const T2 *)c->tw, NZC);
+            k_z_phi<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>(c->phi, (T2 *)c->CX[8], tw(c), NZC);
         CK(cudaGetLastError());
     }
 
@@ -1504,9 +1507,9 @@ template <typename T, int N> struct Impl {
         const size_t smem = ZProdSmem<T, N>::bytes;
         Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko) + 5. * a.bi * a.bj * N * sizeof(T));
         if (c->fftv)
-            k_zprod<T, N, 1><<<N * N / ZP_ROWS, ZP_LINES * PV<1>, smem, c->st>>>(a, (const T *)c->kv, (const T2 *)c->tw);
+            k_zprod<T, N, 1><<<N * N / ZP_ROWS, ZP_LINES * PV<1>, smem, c->st>>>(a, (const T *)c->kv, tw(c));
         else
-            k_zprod<T, N, 0><<<N * N / ZP_ROWS, ZP_LINES * PV<0>, smem, c->st>>>(a, (const T *)c->kv, (const T2 *)c->tw);
+            k_zprod<T, N, 0><<<N * N / ZP_ROWS, ZP_LINES * PV<0>, smem, c->st>>>(a, (const T *)c->kv, tw(c));
         CK(cudaGetLastError());
     }
 
@@ -1623,9 +1626,9 @@ template <typename T, int N> struct Impl {
         const size_t sm = (size_t)N * TC * sizeof(T2);
         Launch L_(c, KC_XASM, 4. * sizeof(T2) * ((act ? c->tr_disc : use) + use * (a.mode == 3 ? 2 : a.mode == 0 ? 4 : 5)));
         if (c->fftv)
-            k_xfwd_stage<T, N, 1><<<4 * ntiles, TC * PV<1>, sm, c->st>>>(a, geo(c), (const T2 *)c->tw, A);
+            k_xfwd_stage<T, N, 1><<<4 * ntiles, TC * PV<1>, sm, c->st>>>(a, geo(c), tw(c), A);
         else
-            k_xfwd_stage<T, N, 0><<<4 * ntiles, TC * PV<0>, sm, c->st>>>(a, geo(c), (const T2 *)c->tw, A);
+            k_xfwd_stage<T, N, 0><<<4 * ntiles, TC * PV<0>, sm, c->st>>>(a, geo(c), tw(c), A);
         CK(cudaGetLastError());
     }
 
@@ -1850,6 +1853,17 @@ void plan_info(int n, int rad[2][4], int thr[2]) {
     }
 }
 
+std::vector<double> plan_tw(int n, int v) {
+    switch (n) {
+        case 16: return v ? plan_twiddles<16, 1>() : plan_twiddles<16, 0>();
+        case 32: return v ? plan_twiddles<32, 1>() : plan_twiddles<32, 0>();
+        case 64: return v ? plan_twiddles<64, 1>() : plan_twiddles<64, 0>();
+        case 96: return v ? plan_twiddles<96, 1>() : plan_twiddles<96, 0>();
+        case 128: return v ? plan_twiddles<128, 1>() : plan_twiddles<128, 0>();
+        default: return v ? plan_twiddles<256, 1>() : plan_twiddles<256, 0>();
+    }
+}
+
 // FP64 sums of the charge density e^s - e^phi + n_d and the kinetic energy
 // density 0.5 e^s |M e_x + u'|^2 (block partials in slots 0 and 1).
 template <typename T>
@@ -1923,14 +1937,6 @@ void build_tables(kf_ctx *c) {
                 const double kq = sqrt(pow(kx / kmax, 2.) + pow(ky / kmax, 2.) + pow(kz / kzq, 2.));
                 PF[ijk] = exp(-2000. * pow(kq, 15.));
             }
-    // twiddles W_N^m = exp(-2 pi i m / N), long double
-    std::vector<double> tw(2 * n);
-    const long double twopi = 6.283185307179586476925286766559005768L;
-    for (int m = 0; m < n; ++m) {
-        long double a = twopi * (long double)m / (long double)n;
-        tw[2 * m] = (double)cosl(a);
-        tw[2 * m + 1] = (double)(-sinl(a));
-    }
     c->q2 = dalloc<double>(c, sizeof(double) * n);
     CK(cudaMemcpy(c->q2, q2.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
     {
@@ -1951,27 +1957,32 @@ void build_tables(kf_ctx *c) {
         CK(cudaMemcpy(c->tr_tl, t.tl.data(), sizeof(int) * t.tl.size(), cudaMemcpyHostToDevice));
     }
     if (c->fp32) {
-        std::vector<float> kvf(n), SVf(c->Nc), PFf(c->Nc), twf(2 * n);
+        std::vector<float> kvf(n), SVf(c->Nc), PFf(c->Nc);
         for (int i = 0; i < n; ++i) kvf[i] = (float)kv[i];
         for (long i = 0; i < c->Nc; ++i) { SVf[i] = (float)SV[i]; PFf[i] = (float)PF[i]; }
-        for (int i = 0; i < 2 * n; ++i) twf[i] = (float)tw[i];
         c->kv = dalloc<void>(c, 4 * n);
         c->SV = dalloc<void>(c, 4 * c->Nc);
         c->PF = dalloc<void>(c, 4 * c->Nc);
-        c->tw = dalloc<void>(c, 8 * n);
         CK(cudaMemcpy(c->kv, kvf.data(), 4 * n, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(c->SV, SVf.data(), 4 * c->Nc, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(c->PF, PFf.data(), 4 * c->Nc, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(c->tw, twf.data(), 8 * n, cudaMemcpyHostToDevice));
     } else {
         c->kv = dalloc<void>(c, 8 * n);
         c->SV = dalloc<void>(c, 8 * c->Nc);
         c->PF = dalloc<void>(c, 8 * c->Nc);
-        c->tw = dalloc<void>(c, 16 * n);
         CK(cudaMemcpy(c->kv, kv.data(), 8 * n, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(c->SV, SV.data(), 8 * c->Nc, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(c->PF, PF.data(), 8 * c->Nc, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(c->tw, tw.data(), 16 * n, cudaMemcpyHostToDevice));
+    }
+    for (int v = 0; v < 2; ++v) {
+        const std::vector<double> w = plan_tw(n, v);
+        c->tw[v] = dalloc<void>(c, c->es * w.size());
+        if (c->fp32) {
+            const std::vector<float> wf(w.begin(), w.end());
+            CK(cudaMemcpy(c->tw[v], wf.data(), 4 * w.size(), cudaMemcpyHostToDevice));
+        } else {
+            CK(cudaMemcpy(c->tw[v], w.data(), 8 * w.size(), cudaMemcpyHostToDevice));
+        }
     }
     if (c->stretched) {
         const std::vector<double> met = metric_table(n, L, c->cfg.stretch_m, dealias_threshold());

@@ -10,11 +10,16 @@
 // registers and the last stage leaves its outputs in registers, so that
 //   input  v[b*R1 + t]  is element  p + b*P + t*N/R1,
 //   output v[b*RL + t]  is element  p + b*P + t*N/RL.
-// Twiddles W_N^m = exp(SIGN*2*pi*i*m/N) come from a per-N table (host-computed
-// in long double), SIGN = -1 forward, +1 backward, as FFTW's r2c/c2r.
+// Twiddles W_N^m = exp(SIGN*2*pi*i*m/N) come from a per-plan table (host-computed
+// in long double; plan_twiddles), SIGN = -1 forward, +1 backward, as FFTW's
+// r2c/c2r: stage s holds W_N^(t*k*N/(Ns*R)) at its offset + t*Ns + k, so that
+// the lanes of a line, which differ in k, read one contiguous run per t.
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <cmath>
+#include <vector>
 
 namespace kf {
 
@@ -145,9 +150,13 @@ template <int SIGN> struct DFT<16, SIGN> : DFT2F<4, 4, SIGN> {};
 // Shared-memory addressing of element r of a line.
 struct StrideAddr {  // columns interleaved: r * stride (+ the column offset in the base pointer)
     int s;
+    // a line's threads lie in several warps
+    static __device__ __forceinline__ void sync() { __syncthreads(); }
     __device__ __forceinline__ int operator()(int r) const { return r * s; }
 };
 struct PadAddr {  // one line contiguous, a pad word every 16: avoids the radix-16 scatter conflicts
+    // a line's P threads (P divides 32, threadIdx.x = p + P l) lie in one warp
+    static __device__ __forceinline__ void sync() { __syncwarp(); }
     __device__ __forceinline__ int operator()(int r) const { return r + (r >> 4); }
 };
 template <int N> struct PadLen { static constexpr int value = N + N / 16 + 1; };
@@ -158,17 +167,9 @@ template <int... Rs> struct Last;
 template <int R> struct Last<R> { static constexpr int value = R; };
 template <int R, int R2, int... Rest> struct Last<R, R2, Rest...> { static constexpr int value = Last<R2, Rest...>::value; };
 
-// Twiddle table W_N^m: in global memory (read through the read-only path) or
-// staged in shared memory by a persistent kernel.
-template <typename T2> __device__ __forceinline__ T2 tw_load(const T2 *__restrict__ tw, int m) { return __ldg(tw + m); }
-template <typename T2> struct SharedTw {
-    const T2 *p;
-};
-template <typename T2> __device__ __forceinline__ T2 tw_load(SharedTw<T2> tw, int m) { return tw.p[m]; }
-
 // Stages of one line.  v: E registers; sm: this line's shared-memory column
-// (element r at sm[r*stride]); tw: W_N table (global, read through L1, or a
-// SharedTw).
+// (element r at sm[addr(r)]); tw: the plan's twiddles from this stage on (global
+// memory, read through L1).
 template <typename T2, int N, int P, int SIGN, int Ns, int R, int... Rest>
 struct Stages {
     static constexpr int E = N / P;
@@ -183,8 +184,7 @@ struct Stages {
             if (Ns > 1) {
 #pragma unroll
                 for (int t = 1; t < R; ++t) {
-                    const int m = (t * k * (N / (Ns * R))) % N;
-                    T2 w = tw_load(tw, m);
+                    T2 w = __ldg(tw + t * Ns + k);
                     if (SIGN > 0) w.y = -w.y;
                     v[b * R + t] = cmul(v[b * R + t], w);
                 }
@@ -200,15 +200,15 @@ struct Stages {
 #pragma unroll
                 for (int t = 0; t < R; ++t) sm[addr(idxD + t * Ns)] = v[b * R + t];
             }
-            __syncthreads();
+            A::sync();
             constexpr int R2 = First<Rest...>::value;
             constexpr int NB2 = N / (P * R2);
 #pragma unroll
             for (int b = 0; b < NB2; ++b)
 #pragma unroll
                 for (int t = 0; t < R2; ++t) v[b * R2 + t] = sm[addr(p + b * P + t * (N / R2))];
-            __syncthreads();
-            Stages<T2, N, P, SIGN, Ns * R, Rest...>::run(v, sm, addr, p, tw);
+            A::sync();
+            Stages<T2, N, P, SIGN, Ns * R, Rest...>::run(v, sm, addr, p, Ns > 1 ? tw + Ns * R : tw);
         }
     }
 };
@@ -254,5 +254,24 @@ KF_PLAN(256, 0, 16, 16, 16, 16, 16)
 KF_PLAN(256, 1, 32, 8, 4, 8, 8, 4)
 #undef KF_PLAN
 template <int N> using Plan = PlanV<N, 0>;
+
+// The twiddles of a plan's stages after the first, as (re, im) pairs.
+template <int N, int V> inline std::vector<double> plan_twiddles() {
+    std::vector<double> w;
+    const long double twopi = 6.283185307179586476925286766559005768L;
+    int Ns = PlanV<N, V>::radix[0];
+    for (int s = 1; s < 4 && PlanV<N, V>::radix[s]; ++s) {
+        const int R = PlanV<N, V>::radix[s];
+        for (int t = 0; t < R; ++t)
+            for (int k = 0; k < Ns; ++k) {
+                const int m = (t * k * (N / (Ns * R))) % N;
+                const long double a = twopi * (long double)m / (long double)N;
+                w.push_back((double)cosl(a));
+                w.push_back((double)(-sinl(a)));
+            }
+        Ns *= R;
+    }
+    return w;
+}
 
 }  // namespace kf

@@ -89,11 +89,10 @@ int fail(int code, const std::string &msg) {
 template <int N>
 cudaError_t run(const double *in, double *out, unsigned char *scratch, cudaStream_t st) {
     NoallocParams p;
-    const long double twopi = 6.283185307179586476925286766559005768L;
-    for (int m = 0; m < N; ++m) {  // the table of build_tables in kf_capi.cu, bit for bit
-        long double a = twopi * (long double)m / (long double)N;
-        p.tw[m] = make_double2((double)cosl(a), (double)(-sinl(a)));
-    }
+    // plan 0's table: at most N entries for these N (16, 32 and 64 have two stages)
+    const std::vector<double> w = plan_twiddles<N, 0>();
+    static_assert(PlanV<N, 0>::radix[0] * PlanV<N, 0>::radix[1] == N, "two radix stages");
+    for (int m = 0; m < N; ++m) p.tw[m] = make_double2(w[2 * m], w[2 * m + 1]);
     double2 *mid = reinterpret_cast<double2 *>(scratch);
     p.z = ZJob{in, nullptr, out, nullptr, MUL_NONE, MUL_NONE};      // z: real rows -> half spectra (out)
     p.ay = AxisJob{out, mid, MUL_NONE, 0};                           // y: out -> scratch

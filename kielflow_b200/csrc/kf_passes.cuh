@@ -453,7 +453,6 @@ k_z_r2c(const ZJob *__restrict__ jobs, int njobs, int nrows,
     T2 *line = xch + l * LS;
     const PadAddr pa;
     PlanV<N, V>::template fft<T2, -1>(v, line, pa, p, tw);
-    __syncthreads();
 #pragma unroll
     for (int q = 0; q < E; ++q) line[pa(reg_row<N, P, PlanV<N, V>::RL>(p, q))] = v[q];
     __syncthreads();

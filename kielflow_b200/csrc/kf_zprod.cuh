@@ -84,6 +84,13 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
 #pragma unroll 1
     for (int rr = 0; rr < ZP_ROWS; ++rr) {
         const long off = (long)(r0 + rr) * NZC;
+        // the half spectra into the line's own buffer (A from 0, B from NZC), then
+        // the packed Hermitian line from there: element k and N - k share a load
+        for (int k = p; k < a.nkz; k += P) {
+            line[k] = __ldg(inA + off + k);
+            if (inB) line[NZC + k] = __ldg(inB + off + k);
+        }
+        __syncwarp();
         T2 v[E];
 #pragma unroll
         for (int q = 0; q < E; ++q) {
@@ -91,8 +98,8 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
             const int kk = k < NZC ? k : N - k;
             T2 x = mk<T2>((T)0, (T)0), y = x;
             if (kk < a.nkz) {
-                x = __ldg(inA + off + kk);
-                y = inB ? __ldg(inB + off + kk) : mul_ik(x, kv[kk]);
+                x = line[kk];
+                y = inB ? line[NZC + kk] : mul_ik(x, kv[kk]);
             }
             if (kk == 0 || 2 * kk == N) x.y = y.y = (T)0;  // as a c2r transform does
             if (k >= NZC) {
@@ -101,7 +108,8 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
             }
             v[q] = mk<T2>(x.x - y.y, x.y + y.x);  // A + iB
         }
-        PlanV<N, V>::template fft<T2, +1>(v, line, pa, p, tw);  // its last exchange ends with a barrier
+        __syncwarp();
+        PlanV<N, V>::template fft<T2, +1>(v, line, pa, p, tw);  // its last exchange ends with a warp barrier
 #pragma unroll
         for (int q = 0; q < E; ++q)
             line[reg_row<N, P, PlanV<N, V>::RL>(p, q)] = mk<T2>(v[q].x * a.scale, v[q].y * a.scale);
@@ -158,7 +166,7 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
     PlanV<N, V>::template fft<T2, -1>(v, line, pa, p, tw);
 #pragma unroll
     for (int q = 0; q < E; ++q) line[pa(reg_row<N, P, PlanV<N, V>::RL>(p, q))] = v[q];
-    __syncthreads();
+    __syncwarp();
     if (l >= 2 * ZP_ROWS) return;
     const long off = (long)(r0 + l / 2) * NZC;
     T2 *oA = a.out[2 * (l & 1)] + off, *oB = a.out[2 * (l & 1) + 1] + off;
@@ -253,7 +261,7 @@ k_z_phi(const double *__restrict__ phi, typename C2<T>::type *__restrict__ out,
     PlanV<N, V>::template fft<T2, -1>(v, line, pa, p, tw);
 #pragma unroll
     for (int q = 0; q < E; ++q) line[pa(reg_row<N, P, PlanV<N, V>::RL>(p, q))] = v[q];
-    __syncthreads();
+    __syncwarp();
     if (r >= N * N) return;
     T2 *oA = out + (long)r * NZC, *oB = oA + NZC;
     for (int k = p; k < nko; k += P) {
