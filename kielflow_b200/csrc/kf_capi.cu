@@ -115,7 +115,7 @@ struct kf_ctx {
     double *q2 = nullptr;
     int *pb = nullptr;  // x-pass 2/3-rule bounds per (j, kz) column (dealias_bounds)
     // the kept part of a masked half spectrum (AxTrunc)
-    int tr_nkz = 0, tr_nt = 0;
+    int tr_nkz = 0, tr_nt = 0, tr_mp = 0;  // tr_mp: elements per row of masked intermediates
     double tr_ball = 0., tr_disc = 0.;  // elements kept; elements of the active columns
     int *tr_jb = nullptr, *tr_tl = nullptr;
     double *stage64 = nullptr;
@@ -1346,8 +1346,9 @@ template <typename T, int N> struct Impl {
         }
         return v;
     }
-    static AxTrunc trunc(kf_ctx *c, int mode) {
-        AxTrunc A{AX_FULL, NZC, 0.f, nullptr, nullptr, 0, N};
+    // inv: an inverse x pass reads a state field, the forward one a masked intermediate
+    static AxTrunc trunc(kf_ctx *c, int mode, bool inv = true) {
+        AxTrunc A{AX_FULL, NZC, 0.f, nullptr, nullptr, 0, N, NZC, NZC};
         if (mode == AX_XB || mode == AX_YB) {
             A.mode = mode;
             A.r0 = mode == AX_XB ? c->bx_i0 : c->bx_j0;
@@ -1360,6 +1361,8 @@ template <typename T, int N> struct Impl {
         A.itpp = 1.f / (float)((c->tr_nkz + TC - 1) / TC);
         A.jb = c->tr_jb;
         A.tl = c->tr_tl;
+        A.ip = mode == AX_XM && inv ? NZC : c->tr_mp;
+        A.op = c->tr_mp;
         return A;
     }
     // kz extent of a z pass over masked fields
@@ -1410,22 +1413,20 @@ template <typename T, int N> struct Impl {
         const T sc = (T)(scale < 0. ? 1. / ((double)N * N * N) : scale);
         if (c->fftv)
             k_z_c2r<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        tw(c), sc, nkz(c, masked));
+                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr_mp : NZC);
         else
             k_z_c2r<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        tw(c), sc, nkz(c, masked));
+                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr_mp : NZC);
     }
-    static void zr2c(kf_ctx *c, int off, int njobs, bool masked = false) {
+    static void zr2c(kf_ctx *c, int off, int njobs) {
         const int nrows = N * N;
         const int ntiles = (nrows + LZ - 1) / LZ;
         const size_t smem = ZSmem<T, N, false>::bytes;
-        Launch L_(c, KC_Z_R2C, z_bytes(c, off, njobs, false, masked));
+        Launch L_(c, KC_Z_R2C, z_bytes(c, off, njobs, false, false));
         if (c->fftv)
-            k_z_r2c<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c),
-                                                                        nkz(c, masked));
+            k_z_r2c<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c));
         else
-            k_z_r2c<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c),
-                                                                        nkz(c, masked));
+            k_z_r2c<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c));
     }
     static RhsArgs<T> rargs(kf_ctx *c) {
         RhsArgs<T> a;
@@ -1457,10 +1458,10 @@ template <typename T, int N> struct Impl {
         Launch L_(c, KC_RHO, (double)N * N * nkz(c, true) * sizeof(T2) + (double)c->N * (c->rho_cs ? 24 : 16));
         if (c->fftv)
             k_z_rho<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, c->rho, c->rho_cs,
-                                                              tw(c), sc, nkz(c, true));
+                                                              tw(c), sc, nkz(c, true), c->tr_mp);
         else
             k_z_rho<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, c->rho, c->rho_cs,
-                                                              tw(c), sc, nkz(c, true));
+                                                              tw(c), sc, nkz(c, true), c->tr_mp);
         CK(cudaGetLastError());
     }
 
@@ -1503,7 +1504,9 @@ template <typename T, int N> struct Impl {
         a.scale = (T)(1. / ((double)N * N * N));
         a.terms = c->cfg.terms;
         a.nkz = nkz(c, true);
+        a.ip = c->tr_mp;
         a.nko = nkz(c, pen);
+        a.op = pen ? c->tr_mp : NZC;
         const size_t smem = ZProdSmem<T, N>::bytes;
         Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko) + 5. * a.bi * a.bj * N * sizeof(T));
         if (c->fftv)
@@ -1608,7 +1611,7 @@ template <typename T, int N> struct Impl {
 
     // the end of F: the forward x pass, K and its use in the RK4 stage
     static void stage(kf_ctx *c, bool pen) {
-        const AxTrunc A = trunc(c, pen ? AX_XM : AX_FULL);
+        const AxTrunc A = trunc(c, pen ? AX_XM : AX_FULL, false);
         StageArgs<T> a;
         for (int q = 0; q < 4; ++q) {
             a.in[q] = (const T2 *)c->CY[q];
@@ -1946,6 +1949,8 @@ void build_tables(kf_ctx *c) {
         const TruncTab t = trunc_table(pb, n, c->fp32 ? Tile<float>::TC : Tile<double>::TC);
         c->tr_nkz = t.nkz;
         c->tr_nt = (int)t.tl.size();
+        const int tc = c->fp32 ? Tile<float>::TC : Tile<double>::TC;
+        c->tr_mp = std::min((t.nkz + tc - 1) / tc * tc, nzc);
         for (int b : pb)
             if (b >= 0) {
                 c->tr_ball += 2 * b + 1;

@@ -120,8 +120,8 @@ template <typename T> struct AxisTile {
     typedef typename C2<T>::type T2;
     const T2 *in;
     T2 *out;
-    int base, rstride;  // element indices: n * n * (n/2 + 1) < 2^31 for every supported n
-    int obase;          // of the output (the input's base but for a packed window)
+    int base, rstride;   // element indices: n * n * (n/2 + 1) < 2^31 for every supported n
+    int obase, ostride;  // of the output
     int mul;
     int lb, sb;  // rows r with min(r, N - r) <= lb are loaded (the others are zero), <= sb stored
     bool valid;
@@ -140,18 +140,19 @@ __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ job
     G.mul = J.mul;
     G.lb = G.sb = N / 2;
     if (axis == 0) {
-        G.rstride = n * nzc;
+        G.rstride = n * A.ip;
+        G.ostride = n * A.op;
         if (A.mode == AX_XM) {
-            const int w = A.tl[tile];
-            const int kk = (w & 0xffff) + c;
-            G.base = (w >> 16) * nzc + kk;
-            G.lb = kk < A.nkz ? g.pb[G.base] : -1;
+            const int w = A.tl[tile], j = w >> 16, kk = (w & 0xffff) + c;
+            G.base = j * A.ip + kk;
+            G.obase = j * A.op + kk;
+            G.lb = kk < A.nkz ? g.pb[j * nzc + kk] : -1;
             G.valid = G.lb >= 0;
         } else {
             G.base = tile * TC + c;
             G.valid = G.base < n * nzc;
+            G.obase = A.mode == AX_XB ? G.base - A.r0 * n * nzc : G.base;
         }
-        G.obase = A.mode == AX_XB ? G.base - A.r0 * n * nzc : G.base;
     } else {
         constexpr int tpp = (nzc + TC - 1) / TC;
         int plane, kk;
@@ -170,9 +171,10 @@ __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ job
             else
                 G.sb = b;
         }
-        G.base = plane * n * nzc + kk;
-        G.rstride = nzc;
-        G.obase = A.mode == AX_YB ? (plane * A.rm - A.r0) * nzc + kk : G.base;
+        G.base = plane * n * A.ip + kk;
+        G.rstride = A.ip;
+        G.ostride = A.op;
+        G.obase = A.mode == AX_YB ? (plane * A.rm - A.r0) * nzc + kk : plane * n * A.op + kk;
     }
     return G;
 }
@@ -297,7 +299,7 @@ k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
             for (int q = 0; q < E; ++q) {
                 const int row = reg_row<N, P, PlanV<N, V>::RL>(p, q);
                 const bool st = A.mode >= AX_XB ? (unsigned)(row - A.r0) < (unsigned)A.rm : row_freq<N>(row) <= cur.sb;
-                if (st) cur.out[cur.obase + row * cur.rstride] = v[q];
+                if (st) cur.out[cur.obase + row * cur.ostride] = v[q];
             }
         }
     }
@@ -328,7 +330,7 @@ template <typename T, int N, bool C2R> struct ZSmem {
 template <typename T, int N, int V = 0>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P, (sizeof(T) == 4 && KF_ZC2R_MINB > 0 ? KF_ZC2R_MINB : 1))
 k_z_c2r(const ZJob *__restrict__ jobs, int njobs, int nrows, Geo<T> g,
-        const typename C2<T>::type *__restrict__ tw, T scale, int nkz) {
+        const typename C2<T>::type *__restrict__ tw, T scale, int nkz, int pitch) {
     typedef typename C2<T>::type T2;
     constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1;
     constexpr int LS = PadLen<N>::value;  // padded line of the exchange buffer
@@ -361,13 +363,14 @@ k_z_c2r(const ZJob *__restrict__ jobs, int njobs, int nrows, Geo<T> g,
             }
         }
     } else {
-        // spectra that are zero from kz = nkz on: only that part of each row
+        // spectra that are zero from kz = nkz on, rows of `pitch` elements
+        const long ro = (long)(r0 + l) * pitch;
         for (int k = p; k < nkz; k += P) {
             const int e = l * NZC + k;
-            if (e < lim) {
-                cp_async_copy(half + e, inA + off + e);
+            if (r0 + l < nrows) {
+                cp_async_copy(half + e, inA + ro + k);
                 if (inB)
-                    cp_async_copy(half + LZ * NZC + e, inB + off + e);
+                    cp_async_copy(half + LZ * NZC + e, inB + ro + k);
                 else
                     half[LZ * NZC + e] = mk<T2>((T)0, (T)0);
             } else {
@@ -426,7 +429,7 @@ k_z_c2r(const ZJob *__restrict__ jobs, int njobs, int nrows, Geo<T> g,
 template <typename T, int N, int V = 0>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
 k_z_r2c(const ZJob *__restrict__ jobs, int njobs, int nrows,
-        const typename C2<T>::type *__restrict__ tw, int nkz) {
+        const typename C2<T>::type *__restrict__ tw) {
     typedef typename C2<T>::type T2;
     constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1;
     constexpr int LS = PadLen<N>::value;
@@ -459,22 +462,15 @@ k_z_r2c(const ZJob *__restrict__ jobs, int njobs, int nrows,
     const int lim = (nrows - r0) * NZC;
     T2 *oA = static_cast<T2 *>(J.outA) + (long)r0 * NZC;
     T2 *oB = J.outB ? static_cast<T2 *>(J.outB) + (long)r0 * NZC : nullptr;
-    auto put = [&](int idx, int ll, int k) {
+    // the tile's LZ output rows of a half spectrum are one contiguous run of
+    // LZ * NZC elements from row r0
+    for (int idx = threadIdx.x; idx < LZ * NZC && idx < lim; idx += blockDim.x) {
+        const int ll = idx / NZC, k = idx - ll * NZC;
         const T2 zk = xch[ll * LS + pa(k)];
         const T2 zm = xch[ll * LS + pa(k == 0 ? 0 : N - k)];
         const T cr = zm.x, ci = -zm.y;  // conj(Z[N-k])
         oA[idx] = mk<T2>((T)0.5 * (zk.x + cr), (T)0.5 * (zk.y + ci));
         if (oB) oB[idx] = mk<T2>((T)0.5 * (zk.y - ci), (T)-0.5 * (zk.x - cr));
-    };
-    if (nkz == NZC) {
-        // the tile's LZ output rows of a half spectrum are one contiguous run
-        // of LZ * NZC elements from row r0
-        for (int idx = threadIdx.x; idx < LZ * NZC && idx < lim; idx += blockDim.x) {
-            const int ll = idx / NZC;
-            put(idx, ll, idx - ll * NZC);
-        }
-    } else {  // only kz < nkz is used by what follows
-        for (int k = p; k < nkz && l * NZC + k < lim; k += P) put(l * NZC + k, l, k);
     }
 }
 
@@ -512,21 +508,23 @@ k_xfwd_stage(const __grid_constant__ StageArgs<T> a, Geo<T> g, const typename C2
     const int q = blockIdx.x & 3, tile = blockIdx.x >> 2;
     const int c = threadIdx.x % TC, p = threadIdx.x / TC;
     constexpr int rstride = N * NZC;
-    int col = tile * TC + c, b = N / 2;
+    int col = tile * TC + c, icol = col, b = N / 2;
     bool valid = col < N * NZC;
     if (A.mode == AX_XM) {
         const int w = A.tl[tile];
         const int kk = (w & 0xffff) + c;
         col = (w >> 16) * NZC + kk;
+        icol = (w >> 16) * A.ip + kk;
         b = kk < A.nkz ? g.pb[col] : -1;
         valid = b >= 0;
     }
+    const int istride = N * A.ip;
     const T2 *__restrict__ in = a.in[q];
     T2 v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const int row = reg_row<N, P, PlanV<N, V>::R1>(p, e);
-        v[e] = valid ? in[col + row * rstride] : mk<T2>((T)0, (T)0);
+        v[e] = valid ? in[icol + row * istride] : mk<T2>((T)0, (T)0);
     }
     PlanV<N, V>::template fft<T2, -1>(v, sm + c, StrideAddr{TC}, p, tw);
     if (!valid) return;

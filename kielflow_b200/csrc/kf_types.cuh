@@ -72,6 +72,10 @@ struct AxTrunc {
     const int *jb;  // per kz < nkz: largest min(j, n - j) of an active column
     const int *tl;  // active x-pass tiles: (j << 16) | first kz
     int r0, rm;     // AX_XB, AX_YB: the window
+    // elements per (i, j) row of the input and the output: n/2 + 1, or for the
+    // masked passes' intermediates nkz rounded up to whole tiles, so that tiles are
+    // aligned 128-byte segments (a row of n/2 + 1 elements shifts them across lines)
+    int ip, op;
 };
 
 // sqrt is correctly rounded and monotone, so sqrt(s) < 2/3 holds exactly when

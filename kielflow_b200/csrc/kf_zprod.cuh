@@ -52,8 +52,8 @@ template <typename T> struct ZProdArgs {
     int i0, bi, j0, bj;
     T M, eta, scale;                    // scale: the 1/N of the c2r
     int terms;
-    int nkz;  // the inputs are zero from kz = nkz on
-    int nko;  // outputs are needed for kz < nko
+    int nkz, ip;  // the inputs are zero from kz = nkz on; elements per row
+    int nko, op;  // outputs are needed for kz < nko; elements per row
 };
 
 template <typename T, int N> struct ZProdSmem {
@@ -83,7 +83,7 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
     const bool adv = a.terms & T_ADVECTION, cont = a.terms & T_CONTINUITY;
 #pragma unroll 1
     for (int rr = 0; rr < ZP_ROWS; ++rr) {
-        const long off = (long)(r0 + rr) * NZC;
+        const long off = (long)(r0 + rr) * a.ip;
         // the half spectra into the line's own buffer (A from 0, B from NZC), then
         // the packed Hermitian line from there: element k and N - k share a load
         for (int k = p; k < a.nkz; k += P) {
@@ -168,7 +168,7 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
     for (int q = 0; q < E; ++q) line[pa(reg_row<N, P, PlanV<N, V>::RL>(p, q))] = v[q];
     __syncwarp();
     if (l >= 2 * ZP_ROWS) return;
-    const long off = (long)(r0 + l / 2) * NZC;
+    const long off = (long)(r0 + l / 2) * a.op;
     T2 *oA = a.out[2 * (l & 1)] + off, *oB = a.out[2 * (l & 1) + 1] + off;
     for (int k = p; k < a.nko; k += P) {
         const T2 zk = line[pa(k)];
@@ -189,14 +189,14 @@ template <typename T, int N, int V>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
 k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, const double *__restrict__ nd,
         double *__restrict__ rho, double *__restrict__ rcs, const typename C2<T>::type *__restrict__ tw, T scale,
-        int nkz) {
+        int nkz, int pitch) {
     typedef typename C2<T>::type T2;
     constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1, LS = PadLen<N>::value;
     extern __shared__ __align__(16) unsigned char kf_smem[];
     T2 *xch = reinterpret_cast<T2 *>(kf_smem);  // [LZ][LS]
     const int p = threadIdx.x % P, l = threadIdx.x / P;
     const int r = 2 * (blockIdx.x * LZ + l);
-    const long off = (long)r * NZC;
+    const long off = (long)r * pitch;
     T2 v[E];
 #pragma unroll
     for (int q = 0; q < E; ++q) {
@@ -205,7 +205,7 @@ k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, const d
         T2 x = mk<T2>((T)0, (T)0), y = x;
         if (kk < nkz && r < N * N) {
             x = __ldg(in + off + kk);
-            y = __ldg(in + off + NZC + kk);
+            y = __ldg(in + off + pitch + kk);
         }
         if (kk == 0 || 2 * kk == N) x.y = y.y = (T)0;
         if (k >= NZC) {
