@@ -191,6 +191,7 @@ struct kf_ctx {
     // what the end of the right-hand side does with K (k_xfwd_stage; 3: store it)
     int rk_mode = 3;
     double rk_c = 0.;
+    double stage_x = 0.;  // its time minus the step's (captured step)
     int stage_idx = 0;  // RK stage of the right-hand side being evaluated (0..3)
     // one RK4 step captured as a CUDA graph (FAS or no Poisson, profile off):
     // time / warm-start history and solve statistics live on the device
@@ -213,7 +214,7 @@ struct kf_ctx {
     cudaEvent_t ev_u = nullptr;
     double *stage64b = nullptr;  // FP32-bulk staging of the copy stream
     double step_dt = 0.;
-    long long step_kernels = 0, cycle_kernels = 0, head_kernels = 0;
+    long long step_kernels = 0, cycle_kernels = 0;
     int jV_x = 0, jV_y = 0, zV = 0, zW = 0, nWz = 0, nWf = 0, jW_y = 0, jW_x = 0, zS = 0, jS_y = 0, jS_x = 0;
     int jP_x = 0, jP_y = 0, zP = 0, jQ_x = 0, jQ_y = 0, zQ = 0;
 };
@@ -776,11 +777,11 @@ void smooth_split(kf_ctx *c, const LevelBuf &L, double *ph, const double *rh, in
 }
 
 // r = residual in split order, its max |r| into the d_max slots with_max
-void residual_split(kf_ctx *c, const LevelBuf &L, bool with_max, int cls) {
+void residual_split(kf_ctx *c, const LevelBuf &L, bool with_max, int cls, bool slots_zero = false) {
     const int n = L.n;
     const int Z = with_max ? (n >= 128 ? 4 : 2) : (n >= 128 ? 2 : 1);
     const dim3 b = split_block(c, n), g(1, (n + b.y - 1) / b.y, 2 * n / Z);
-    if (with_max) CK(cudaMemsetAsync(c->d_max, 0, 64 * sizeof(unsigned long long), c->st));
+    if (with_max && !slots_zero) CK(cudaMemsetAsync(c->d_max, 0, 64 * sizeof(unsigned long long), c->st));
     Launch L_(c, cls, 24. * n * n * n);
     if (with_max)
         k_residual_s<true><<<g, b, 0, c->st>>>(L.ph, L.rh, L.slev(), L.r, c->d_max, Z, *L.tab);
@@ -791,15 +792,16 @@ void residual_split(kf_ctx *c, const LevelBuf &L, bool with_max, int cls) {
 void vcycle(kf_ctx *c, int l);
 
 // First part of a V-cycle on level l (not the coarsest): pre-smoothing and the
-// residual L.r; with_max also leaves max |L.r| in the d_max slots.
-void vcycle_head(kf_ctx *c, int l, bool with_max) {
+// residual L.r; with_max also leaves max |L.r| in the d_max slots (slots_zero:
+// they are zero already).
+void vcycle_head(kf_ctx *c, int l, bool with_max, bool slots_zero = false) {
     LevelBuf &L = c->lv[l];
     const kf_config &cf = c->cfg;
     const int n = L.n;
     const long N = (long)n * n * n;
     if (split_on(c, l)) {
         smooth_split(c, L, L.ph, L.rh, cf.mg_pre, l == 0 ? KC_RBGS : KC_MG_COARSE);
-        residual_split(c, L, with_max, l == 0 ? KC_RESID : KC_MG_COARSE);
+        residual_split(c, L, with_max, l == 0 ? KC_RESID : KC_MG_COARSE, slots_zero);
         return;
     }
     if (march_ok(c, L) && cf.mg_pre >= 1) {
@@ -1134,33 +1136,32 @@ void poisson_captured(kf_ctx *c) {
     const bool sp = split_on(c, 0);
     if (extrap && sp) {
         Launch L_(c, KC_MISC, 32. * c->N);
-        k_guess_s<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(c->phi, c->phi_a, c->phi_cs, c->dtime, c->n);
+        k_guess_s<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(c->phi, c->phi_a, c->phi_cs, c->dtime, c->stage_x,
+                                                                             c->n);
     } else if (extrap) {
         Launch L_(c, KC_MISC, 24. * c->N);
-        k_guess<<<nblk(c->N, 256), 256, 0, c->st>>>(c->phi, c->phi_a, c->dtime, c->N);
+        k_guess<<<nblk(c->N, 256), 256, 0, c->st>>>(c->phi, c->phi_a, c->dtime, c->stage_x, c->N);
     } else if (sp) {
         split_field(c, c->phi, c->phi_cs);
     }
-    if (extrap) {
-        Launch L_(c, KC_MISC, 0.);
-        k_guess_post<<<1, 32, 0, c->st>>>(c->dtime);
-    }
     LevelBuf &L0 = c->lv[0];
     const bool fixed = !(cf.res_tol > 0.);
-    c->head_kernels = 0;
     if (!fixed && c->lv.size() > 1) {
-        // WHILE { head of the cycle (pre-smoothing, residual with its max);
-        //         k_fas_check_mid;  IF { rest of the cycle } }
+        // head of the cycle (pre-smoothing, residual with its max); k_fas_check;
+        // WHILE { rest of the cycle; head; k_fas_check }: as many passes as V-cycles.
+        // (WHILE { head; check; IF { rest } } took one pass more and an IF node in
+        // each; a pass costs about 7 us beside its kernels.)
         cudaStreamCaptureStatus cs;
         cudaGraph_t g = nullptr;
         CK(cudaStreamGetCaptureInfo(c->st, &cs, nullptr, &g, nullptr, nullptr));
-        cudaGraphConditionalHandle hw, hi;
+        cudaGraphConditionalHandle hw;
         CK(cudaGraphConditionalHandleCreate(&hw, g, 0, 0));
-        CK(cudaGraphConditionalHandleCreate(&hi, g, 0, 0));
-        {
+        auto head = [&](int first) {
+            vcycle_head(c, 0, true, !first);  // k_fas_check leaves the slots zero
             Launch L_(c, KC_MISC, 0.);
-            k_fas_begin<<<1, 32, 0, c->st>>>(c->dpois, hw);
-        }
+            k_fas_check<<<1, 32, 0, c->st>>>(c->d_max, c->dpois, cf.res_tol, cf.max_cycles, first, false, c->stage_idx, hw);
+        };
+        head(1);
         const cudaGraphNode_t *deps = nullptr;
         size_t ndeps = 0;
         CK(cudaStreamGetCaptureInfo(c->st, &cs, nullptr, &g, &deps, &ndeps));
@@ -1171,49 +1172,30 @@ void poisson_captured(kf_ctx *c) {
         cudaGraphNode_t wnode;
         CK(cudaGraphAddNode(&wnode, g, deps, ndeps, &wp));
         CK(cudaStreamUpdateCaptureDependencies(c->st, &wnode, 1, cudaStreamSetCaptureDependencies));
-        cudaGraph_t body = wp.conditional.phGraph_out[0];
-        const long long l0 = c->launches;
+        const long long l1 = c->launches;
         cudaStream_t outer = c->st;
         c->st = c->st_body;
-        cudaError_t e = cudaStreamBeginCaptureToGraph(c->st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        cudaError_t e = cudaStreamBeginCaptureToGraph(c->st, wp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                      cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
+            cudaGraph_t body_out = nullptr;
             try {
-                vcycle_head(c, 0, true);
-                {
-                    Launch L_(c, KC_MISC, 0.);
-                    k_fas_check_mid<<<1, 32, 0, c->st>>>(c->d_max, c->dpois, cf.res_tol, cf.max_cycles, c->stage_idx,
-                                                         hw, hi);
-                }
-                c->head_kernels = c->launches - l0;
-                cudaGraph_t gb = nullptr;
-                CK(cudaStreamGetCaptureInfo(c->st, &cs, nullptr, &gb, &deps, &ndeps));
-                cudaGraphNodeParams ip = {cudaGraphNodeTypeConditional};
-                ip.conditional.handle = hi;
-                ip.conditional.type = cudaGraphCondTypeIf;
-                ip.conditional.size = 1;
-                cudaGraphNode_t inode;
-                CK(cudaGraphAddNode(&inode, gb, deps, ndeps, &ip));
-                CK(cudaStreamUpdateCaptureDependencies(c->st, &inode, 1, cudaStreamSetCaptureDependencies));
-                cudaGraph_t body_out = nullptr;
-                CK(cudaStreamEndCapture(c->st, &body_out));
-                CK(cudaStreamBeginCaptureToGraph(c->st, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                 cudaStreamCaptureModeThreadLocal));
                 vcycle_tail(c, 0);
+                head(0);
                 e = cudaStreamEndCapture(c->st, &body_out);
             } catch (...) {
-                cudaGraph_t junk = nullptr;
-                cudaStreamEndCapture(c->st, &junk);
+                cudaStreamEndCapture(c->st, &body_out);
                 c->st = outer;
                 throw;
             }
         }
         c->st = outer;
         CK(e);
-        c->cycle_kernels = c->launches - l0;
+        c->cycle_kernels = c->launches - l1;
         solve_end(c);
         if (extrap) {
             Launch L_(c, KC_MISC, 0.);
-            k_hist_post<<<1, 32, 0, c->st>>>(c->dtime);
+            k_hist_post<<<1, 32, 0, c->st>>>(c->dtime, c->stage_x);
         }
         CK(cudaGetLastError());
         return;
@@ -1273,7 +1255,7 @@ void poisson_captured(kf_ctx *c) {
     solve_end(c);
     if (extrap) {
         Launch L_(c, KC_MISC, 0.);
-        k_hist_post<<<1, 32, 0, c->st>>>(c->dtime);
+        k_hist_post<<<1, 32, 0, c->st>>>(c->dtime, c->stage_x);
     }
     CK(cudaGetLastError());
 }
@@ -1924,11 +1906,14 @@ void build_tables(kf_ctx *c) {
         kv[i] = k_val_at(i, n, L);
         q2[i] = pow(kv[i] / kmax, 2.);
     }
+    // the tables depend on |kx|, |ky| and are the same with the two exchanged (the
+    // sums' first two terms): formed for n/2 >= i >= j, copied elsewhere
     std::vector<double> SV(c->Nc), PF(c->Nc);
-    for (int i = 0; i < n; ++i)
-        for (int j = 0; j < n; ++j)
+    auto at = [&](int i, int j) { return (size_t)nzc * ((size_t)j + (size_t)i * n); };
+    for (int i = 0; i <= n / 2; ++i)
+        for (int j = 0; j <= i; ++j)
             for (int k = 0; k < nzc; ++k) {
-                const size_t ijk = (size_t)k + nzc * ((size_t)j + (size_t)i * n);
+                const size_t ijk = at(i, j) + k;
                 const double kx = kv[i], ky = kv[j], kz = kv[k];
                 // rhs_standard.cpp:64-71 (field_SV), optional cut at sv_cut
                 const double knorm = sqrt(pow(kx / kmax, 2.) + pow(ky / kmax, 2.) + pow(kz / kmax, 2.));
@@ -1940,6 +1925,14 @@ void build_tables(kf_ctx *c) {
                 const double kq = sqrt(pow(kx / kmax, 2.) + pow(ky / kmax, 2.) + pow(kz / kzq, 2.));
                 PF[ijk] = exp(-2000. * pow(kq, 15.));
             }
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < n; ++j) {
+            const int a = std::min(i, n - i), b = std::min(j, n - j);
+            const size_t src = at(std::max(a, b), std::min(a, b)), dst = at(i, j);
+            if (src == dst) continue;
+            std::copy_n(&SV[src], nzc, &SV[dst]);
+            std::copy_n(&PF[src], nzc, &PF[dst]);
+        }
     c->q2 = dalloc<double>(c, sizeof(double) * n);
     CK(cudaMemcpy(c->q2, q2.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
     {
@@ -2537,11 +2530,12 @@ void capture_step(kf_ctx *c, double dt, bool wait_u, cudaGraphExec_t *out) {
     CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
     try {
         for (int i = 0; i < 4; ++i) {
-            {
+            if (!(pois && cf.phi_extrap)) {  // else with the solve's history (k_hist_post)
                 Launch L_(c, KC_MISC, 0.);
                 k_time<<<1, 32, 0, c->st>>>(c->dtime, xs[i], 0);
             }
             c->stage_idx = i;
+            c->stage_x = xs[i];
             rk_stage(c, cdt[i], mode[i]);
         }
         if (c->stretched) copy_state(c, c->Ys, c->Y);
@@ -2598,7 +2592,7 @@ void graph_end(kf_ctx *c) {
     c->tau_b = ht.tau_b;
     c->nhist = ht.nhist;
     const DevPois &o = c->hpois;
-    c->launches += (hp.total_cycles - o.total_cycles) * c->cycle_kernels + (hp.solves - o.solves) * c->head_kernels;
+    c->launches += (hp.total_cycles - o.total_cycles) * c->cycle_kernels;
     c->diag.solves += hp.solves - o.solves;
     c->diag.total_iterations += hp.total_cycles - o.total_cycles;
     if (hp.solves != o.solves) {

@@ -15,7 +15,7 @@ namespace kf {
 
 struct DevTime {
     double t, t_stage, tau_a, tau_b;
-    int nhist, newtime, pad0, pad1;
+    int nhist, pad0, pad1, pad2;
 };
 
 struct DevPois {
@@ -37,11 +37,11 @@ __global__ void k_time(DevTime *d, double x, int mode) {
         d->t = d->t + x;
 }
 
-// Start of a solve at t_stage (the host's phi_guess): extrapolate phi when
-// t_stage is a new time and two earlier solutions exist, or record phi.
+// Start of a solve at the stage time t + x (the host's phi_guess): extrapolate phi
+// when that is a new time and two earlier solutions exist, or record phi.
 __global__ void k_guess(double *__restrict__ phi, double *__restrict__ phi_a, const DevTime *__restrict__ d,
-                        long N) {
-    const double t = d->t_stage, ta = d->tau_a, tb = d->tau_b;
+                        double x, long N) {
+    const double t = d->t + x, ta = d->tau_a, tb = d->tau_b;
     const int nh = d->nhist;
     const bool newtime = nh == 0 || t != tb;
     if (!newtime || nh == 0) return;
@@ -55,32 +55,32 @@ __global__ void k_guess(double *__restrict__ phi, double *__restrict__ phi_a, co
     phi_a[i] = b;
 }
 
-// after k_guess: remember whether this solve is at a new time; shift tau_a
-__global__ void k_guess_post(DevTime *d) {
+// after the solve at the stage time t + x: a solve at a new time enters the history
+__global__ void k_hist_post(DevTime *d, double x) {
     if (threadIdx.x || blockIdx.x) return;
+    const double t = d->t + x;
     const int nh = d->nhist;
-    const bool newtime = nh == 0 || d->t_stage != d->tau_b;
-    d->newtime = newtime;
-    if (newtime && nh != 0) d->tau_a = d->tau_b;
-}
-
-// after the solve: a solve at a new time enters the history
-__global__ void k_hist_post(DevTime *d) {
-    if (threadIdx.x || blockIdx.x) return;
-    if (d->newtime) {
-        d->nhist = d->nhist < 2 ? d->nhist + 1 : 2;
-        d->tau_b = d->t_stage;
+    d->t_stage = t;
+    if (nh == 0 || t != d->tau_b) {
+        if (nh != 0) d->tau_a = d->tau_b;
+        d->nhist = nh < 2 ? nh + 1 : 2;
+        d->tau_b = t;
     }
 }
 
-// Convergence test of the FAS loop from the 64 max slots of k_resmax:
-// continue while r > tol and cyc < max_cycles (fixed: while cyc < max_cycles).
-// The loop is bounded by max_cycles whatever r is (NaN included).
-__global__ void k_fas_check(const unsigned long long *__restrict__ slots, DevPois *p, double tol, int max_cycles,
-                            int first, int fixed, int stage, cudaGraphConditionalHandle h) {
-    if (threadIdx.x || blockIdx.x) return;
-    unsigned long long m = 0;
-    for (int s = 0; s < 64; ++s) m = slots[s] > m ? slots[s] : m;
+// Convergence test of the FAS loop from the 64 max slots: continue while r > tol
+// and cyc < max_cycles (fixed: while cyc < max_cycles).  Adaptive solves test the
+// residual of the cycle's pre-smoothed iterate: the solve ends there when its max
+// |f| <= tol, so the returned phi carries the measured residual and no cycle ends
+// with a residual pass of its own.  The slots are left zero for the next pass.
+// The loop is bounded by max_cycles whatever r is (NaN included).  One warp.
+__global__ void k_fas_check(unsigned long long *__restrict__ slots, DevPois *p, double tol, int max_cycles, int first,
+                            int fixed, int stage, cudaGraphConditionalHandle h) {
+    const ulonglong2 v = reinterpret_cast<ulonglong2 *>(slots)[threadIdx.x];
+    reinterpret_cast<ulonglong2 *>(slots)[threadIdx.x] = make_ulonglong2(0, 0);
+    unsigned long long m = max(v.x, v.y);
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x) return;
     const double r = __longlong_as_double((long long)m);
     const int cyc = first ? 0 : p->cyc + 1;
     p->cyc = cyc;
@@ -98,43 +98,6 @@ __global__ void k_fas_check(const unsigned long long *__restrict__ slots, DevPoi
             p->not_converged += 1;
     }
     cudaGraphSetConditional(h, cont ? 1u : 0u);
-}
-
-// Adaptive FAS solve, one WHILE iteration = pre-smoothing and residual of the
-// finest level, this test, then (IF node) the rest of the V-cycle.  The test
-// uses the residual of the pre-smoothed iterate: the solve ends there when its
-// max |f| <= tol (or max_cycles cycles are done), so the returned phi carries
-// the measured residual and no cycle ends with a residual pass of its own.
-__global__ void k_fas_begin(DevPois *p, cudaGraphConditionalHandle hw) {
-    if (threadIdx.x || blockIdx.x) return;
-    p->cyc = 0;
-    cudaGraphSetConditional(hw, 1u);
-}
-
-__global__ void k_fas_check_mid(const unsigned long long *__restrict__ slots, DevPois *p, double tol, int max_cycles,
-                                int stage, cudaGraphConditionalHandle hw, cudaGraphConditionalHandle hi) {
-    if (threadIdx.x || blockIdx.x) return;
-    unsigned long long m = 0;
-    for (int s = 0; s < 64; ++s) m = slots[s] > m ? slots[s] : m;
-    const double r = __longlong_as_double((long long)m);
-    const int cyc = p->cyc;
-    p->r = r;
-    const bool cont = r > tol && cyc < max_cycles;
-    if (cont) {
-        p->cyc = cyc + 1;
-    } else {
-        p->solves += 1;
-        p->total_cycles += cyc;
-        p->last_cycles = cyc;
-        p->last_residual = r;
-        p->stage_cycles[stage & 3] += cyc;
-        if (r != r)
-            p->nans += 1;
-        else if (r > tol)
-            p->not_converged += 1;
-    }
-    cudaGraphSetConditional(hw, cont ? 1u : 0u);
-    cudaGraphSetConditional(hi, cont ? 1u : 0u);
 }
 
 }  // namespace kf

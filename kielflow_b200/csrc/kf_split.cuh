@@ -34,10 +34,11 @@ __global__ void __launch_bounds__(256) k_unsplit(const double *__restrict__ s, d
 // k_guess with the start of the solve in split order (and not in phi, which the
 // solve's end writes): blocks as k_split.
 __global__ void __launch_bounds__(256) k_guess_s(const double *__restrict__ phi, double *__restrict__ phi_a,
-                                                 double *__restrict__ s, const DevTime *__restrict__ d, int n) {
+                                                 double *__restrict__ s, const DevTime *__restrict__ d, double xt,
+                                                 int n) {
     const int k2 = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
     if (2 * k2 >= n || j >= n) return;
-    const double t = d->t_stage, ta = d->tau_a, tb = d->tau_b;
+    const double t = d->t + xt, ta = d->tau_a, tb = d->tau_b;
     const int nh = d->nhist;
     const int row = (i * n + j) * (n / 2) + k2, half = n * n * (n / 2), c0 = (i + j) & 1;
     double2 b = *reinterpret_cast<const double2 *>(phi + 2 * row);
