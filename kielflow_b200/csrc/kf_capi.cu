@@ -148,7 +148,8 @@ struct kf_ctx {
     int zS_I = 0, jS_Iy = 0, jS_Ix = 0, jS_Kx = 0, jS_Ky = 0, zS_K = 0, zS_Kf = 0, jS_Kfy = 0, jS_Kfx = 0;
     // Jacobi state carried between solves (solver_poisson_jacobi_nlin.hpp:66-95)
     double norm_max = 0., norm_sum = 0.;
-    JacState *d_js = nullptr, *h_js = nullptr;
+    JacState *d_js = nullptr, *h_js = nullptr;  // two on the device, taken in turn by the sweeps
+    JcStat *jc_part[2] = {};
     std::vector<JacGraph> jac;
     kf_diag_out diag{};
     // kernel profiling (CUDA events around each launch, when enabled)
@@ -481,12 +482,23 @@ double max_residual(kf_ctx *c, const LevelBuf &L, const double *phi, const doubl
     return r;
 }
 
-// One Jacobi sweep of level L, in -> out.
-void jacobi_sweep(kf_ctx *c, const LevelBuf &L, const double *in, double *out, const double *rho, const JacStop &S,
-                  int cond, cudaGraphConditionalHandle h) {
+// Blocks of a sweep: every block reads all of them (k_jacobi), so as few as fill
+// the chip; a thread takes several points from 64^3 on.
+int jac_blocks(long N) { return (int)std::min<long>((N + 255) / 256, N >= (1 << 20) ? 592 : 296); }
+
+// Sweep s of a run on level L (phi -> tmp for even s, back for odd).
+void jacobi_sweep(kf_ctx *c, const LevelBuf &L, double *phi, double *tmp, const double *rho, const JacStop &S, int s) {
     const long N = (long)L.n * L.n * L.n;
+    const int i = s & 1, o = i ^ 1;
     Launch L_(c, KC_JACOBI, 24. * N);
-    k_jacobi<RBS><<<red_blocks(N), RBS, 0, c->st>>>(in, out, rho, L.lev(), S, c->partial, c->d_js, cond, h);
+    k_jacobi<<<jac_blocks(N), 256, 0, c->st>>>(i ? tmp : phi, i ? phi : tmp, rho, L.lev(), S, c->jc_part[i],
+                                              c->jc_part[o], c->d_js + i, c->d_js + o);
+}
+// The record of a run after an even number of sweeps brought up to date.
+void jacobi_test(kf_ctx *c, const LevelBuf &L, const JacStop &S, int loop, cudaGraphConditionalHandle h) {
+    const long N = (long)L.n * L.n * L.n;
+    Launch L_(c, KC_JACOBI, 0.);
+    k_jacobi_test<<<1, 256, 0, c->st>>>(c->jc_part[0], jac_blocks(N), c->d_js, N, S, loop, h);
 }
 
 // The captured sweep loop: WHILE { JC_UNROLL sweeps phi -> tmp -> phi ... }, then
@@ -523,7 +535,8 @@ cudaGraphExec_t jacobi_graph(kf_ctx *c, const LevelBuf &L, double *phi, double *
         cudaGraph_t body = nullptr;
         try {
             for (int s = 0; s < JC_UNROLL; ++s)
-                jacobi_sweep(c, L, s & 1 ? tmp : phi, s & 1 ? phi : tmp, rho, S, s + 1 == JC_UNROLL, h);
+                jacobi_sweep(c, L, phi, tmp, rho, S, s);
+            jacobi_test(c, L, S, 1, h);
         } catch (...) {
             cudaStreamEndCapture(c->st, &body);
             throw;
@@ -561,12 +574,14 @@ int jacobi_solve(kf_ctx *c, const LevelBuf &L, double *phi, double *tmp, const d
     js.omega = 1.;
     if (S.max_it > 0) {
         cudaGraphExec_t exec = c->prof ? nullptr : jacobi_graph(c, L, phi, tmp, rho, S);
+        js.fresh = 1;
         CK(cudaMemcpyAsync(c->d_js, &js, sizeof(JacState), cudaMemcpyHostToDevice, c->st));
         if (exec) {
             CK(cudaGraphLaunch(exec, c->st));
-        } else {  // one sweep at a time, for the per-launch profile
-            for (int s = 0; !js.done; ++s) {
-                jacobi_sweep(c, L, s & 1 ? tmp : phi, s & 1 ? phi : tmp, rho, S, 0, 0);
+        } else {  // launched one by one, for the per-launch profile
+            while (!js.done) {
+                for (int s = 0; s < 2; ++s) jacobi_sweep(c, L, phi, tmp, rho, S, s);
+                jacobi_test(c, L, S, 0, 0);
                 CK(cudaGetLastError());
                 CK(cudaMemcpyAsync(&js, c->d_js, sizeof(JacState), cudaMemcpyDeviceToHost, c->st));
                 CK(cudaStreamSynchronize(c->st));
@@ -2384,7 +2399,11 @@ void create(kf_ctx *c) {
     CK(cudaMallocHost(&c->h_max, 64 * sizeof(unsigned long long)));
     if (cf.phi_extrap) c->phi_a = dalloc<double>(c, 8 * c->N);
     CK(cudaMallocHost(&c->h_red, sizeof(double) * 8));
-    c->d_js = dalloc<JacState>(c, sizeof(JacState));
+    c->d_js = dalloc<JacState>(c, 2 * sizeof(JacState));
+    for (auto &q : c->jc_part) {
+        q = dalloc<JcStat>(c, 592 * sizeof(JcStat));
+        CK(cudaMemset(q, 0, 592 * sizeof(JcStat)));
+    }
     CK(cudaMallocHost(&c->h_js, sizeof(JacState)));
     c->dtime = dalloc<DevTime>(c, sizeof(DevTime));
     c->dpois = dalloc<DevPois>(c, sizeof(DevPois));

@@ -1,13 +1,14 @@
 // kf_jacobi.cuh -- the reference's nonlinear Jacobi relaxation
 // (solver_poisson_jacobi_nlin.cpp:50-265) with its sweep loop on the device.
 //
-// A sweep is one kernel: the point updates, the sweep's statistics reduced in a
-// fixed order (block trees, then one tree over the blocks' partials by the block
-// that finishes last), Carre's over-relaxation factor and the stop test.  The
-// loop is a conditional WHILE node whose body holds JC_UNROLL sweeps, which
-// return at once when an earlier one has stopped; the host reads the record back
-// once per solve.  A host-driven sweep (two launches, a copy and a
-// synchronisation) took 27 us at 32^3.
+// A sweep is one kernel.  Its blocks leave their statistics (reduced in a fixed
+// order) in memory; every block of the next sweep reduces them again and forms
+// Carre's over-relaxation factor and the stop test from them, beside the update of
+// its points, of which only the last step needs the factor.  So a sweep waits for
+// no atomic, fence or last block: 6.8 -> 4 us at 32^3.  The loop is a conditional
+// WHILE node whose body holds JC_UNROLL sweeps, which return at once when an
+// earlier one has stopped; the host reads the record back once per solve.  A
+// host-driven sweep (two launches, a copy and a synchronisation) took 27 us.
 #pragma once
 
 #include "kf_poisson.cuh"
@@ -19,7 +20,7 @@ namespace kf {
 struct JacState {
     double norm_max, norm_sum, norm_max_old, norm_sum_old, sup, inf, omega, rlast;
     int iteration, done, converged, nan;
-    unsigned ticket, pad;
+    int fresh, pad;  // no sweep's statistics are to be taken in
 };
 
 struct JacStop {
@@ -36,19 +37,20 @@ __device__ __forceinline__ double div_by(double num, double den, double r) {
     return __fma_rn(__fma_rn(-q, den, num), r, q);
 }
 
-// point_coeffs: the same quotients and sums, the divisors' reciprocals from tables
-__device__ __forceinline__ void point_coeffs_div(const double *__restrict__ p, const double *__restrict__ rho,
+// point_coeffs: the same quotients and sums, the divisors' reciprocals from
+// tables; p: the plane i of the potential, pp and pm its neighbours
+__device__ __forceinline__ void point_coeffs_div(const double *pm, const double *p, const double *pp, double rho,
                                                  const Lev &L, int i, int j, int k, double &A, double &D) {
     const int n = L.n;
     D = __dadd_rn(__dadd_rn(L.dd[i], L.dd[j]), L.dd[k]);
-    A = div_by(p[lidx(wrapi(i + 1, n), j, k, n)], L.dp[i], L.rp[i]);
-    A = __dadd_rn(A, div_by(p[lidx(wrapi(i - 1, n), j, k, n)], L.dm[i], L.rm[i]));
-    A = __dadd_rn(A, div_by(p[lidx(i, wrapi(j + 1, n), k, n)], L.dp[j], L.rp[j]));
-    A = __dadd_rn(A, div_by(p[lidx(i, wrapi(j - 1, n), k, n)], L.dm[j], L.rm[j]));
-    A = __dadd_rn(A, div_by(p[lidx(i, j, wrapi(k + 1, n), n)], L.dp[k], L.rp[k]));
-    A = __dadd_rn(A, div_by(p[lidx(i, j, wrapi(k - 1, n), n)], L.dm[k], L.rm[k]));
+    A = div_by(pp[j * n + k], L.dp[i], L.rp[i]);
+    A = __dadd_rn(A, div_by(pm[j * n + k], L.dm[i], L.rm[i]));
+    A = __dadd_rn(A, div_by(p[wrapi(j + 1, n) * n + k], L.dp[j], L.rp[j]));
+    A = __dadd_rn(A, div_by(p[wrapi(j - 1, n) * n + k], L.dm[j], L.rm[j]));
+    A = __dadd_rn(A, div_by(p[j * n + wrapi(k + 1, n)], L.dp[k], L.rp[k]));
+    A = __dadd_rn(A, div_by(p[j * n + wrapi(k - 1, n)], L.dm[k], L.rm[k]));
     A = __dmul_rn(2., A);
-    A = __dadd_rn(A, rho[lidx(i, j, k, n)]);
+    A = __dadd_rn(A, rho);
 }
 
 // newton_method::solve (newton_method.hpp:16-63), eps 0.05, Nmax 20, g 0.8; f0 =
@@ -70,125 +72,167 @@ __device__ __forceinline__ double newton_point(double x, double A, double D, dou
     return __dsub_rn(x, dx);
 }
 
-// Block partials of a sweep's statistics: [0] max|dP|, [1] sum|dP|, [2] max P_new,
-// [3] min P_new, [4] max|f(P_old)|.  Tree over BS values per slot, t taking t + w
-// for w = BS/2, ..., 1, the last five levels by warp shuffle.
-template <int BS>
-__device__ __forceinline__ void jac_tree(double v[KF_RED], double (*sh)[BS]) {
-    const int t = threadIdx.x;
-    for (int s = 0; s < KF_RED; ++s) sh[s][t] = v[s];
-    __syncthreads();
-#pragma unroll
-    for (int w = BS / 2; w >= 32; w >>= 1) {
-        if (t < w) {
-            v[0] = nmax(v[0], sh[0][t + w]);
-            v[1] = __dadd_rn(v[1], sh[1][t + w]);
-            v[2] = nmax(v[2], sh[2][t + w]);
-            v[3] = nmin(v[3], sh[3][t + w]);
-            v[4] = nmax(v[4], sh[4][t + w]);
-            if (w > 32)
-                for (int s = 0; s < KF_RED; ++s) sh[s][t] = v[s];
-        }
-        if (w > 32) __syncthreads();
+// Statistics of a sweep over some points: sum and maximum of |dP|, maximum of
+// |f(P_old)|, extrema of P_new.  The sum's order is fixed: 256 values by a tree in
+// which t takes t + w for w = 128, 64, ..., 1; the others do not depend on it.
+struct JcStat {
+    double sum;
+    unsigned long long dmax, fmax;  // bit patterns (a NaN sorts above +inf)
+    double pmax, pmin;
+    __device__ __forceinline__ void join(const JcStat &o) {
+        sum = __dadd_rn(sum, o.sum);
+        dmax = max(dmax, o.dmax);
+        fmax = max(fmax, o.fmax);
+        pmax = ::fmax(pmax, o.pmax);
+        pmin = ::fmin(pmin, o.pmin);
     }
-    if (t < 32) {
-#pragma unroll
+    __device__ __forceinline__ void warp() {  // lane t takes t + 16, 8, ... 1: the result in lane 0
         for (int w = 16; w > 0; w >>= 1) {
-            v[0] = nmax(v[0], __shfl_down_sync(0xffffffffu, v[0], w));
-            v[1] = __dadd_rn(v[1], __shfl_down_sync(0xffffffffu, v[1], w));
-            v[2] = nmax(v[2], __shfl_down_sync(0xffffffffu, v[2], w));
-            v[3] = nmin(v[3], __shfl_down_sync(0xffffffffu, v[3], w));
-            v[4] = nmax(v[4], __shfl_down_sync(0xffffffffu, v[4], w));
+            JcStat o;
+            o.sum = __shfl_down_sync(0xffffffffu, sum, w);
+            o.dmax = __shfl_down_sync(0xffffffffu, dmax, w);
+            o.fmax = __shfl_down_sync(0xffffffffu, fmax, w);
+            o.pmax = __shfl_down_sync(0xffffffffu, pmax, w);
+            o.pmin = __shfl_down_sync(0xffffffffu, pmin, w);
+            join(o);
         }
     }
+};
+
+// The tree over a block's 256 values, by its first warp (the result in lane 0).
+__device__ __forceinline__ JcStat jac_tree(const JcStat &v, JcStat *sh) {
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    JcStat a[8];
+    if (threadIdx.x < 32) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) a[q] = sh[q * 32 + threadIdx.x];
+#pragma unroll
+        for (int w = 4; w > 0; w >>= 1)
+#pragma unroll
+            for (int q = 0; q < w; ++q) a[q].join(a[q + w]);
+        a[0].warp();
+    }
+    return a[0];
 }
 
-// One sweep in -> out.  cond: the last sweep of the loop's body sets the WHILE
-// condition h.
-template <int BS>
-__global__ void __launch_bounds__(BS) k_jacobi(const double *__restrict__ in, double *__restrict__ out,
-                                               const double *__restrict__ rho, Lev L, JacStop S,
-                                               double *__restrict__ partial, JacState *js, int cond,
-                                               cudaGraphConditionalHandle h) {
-    __shared__ double sh[KF_RED][BS];
-    __shared__ bool last;
-    if (js->done) {
-        if (cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
-        return;
-    }
-    const double omega = js->omega;
-    const int n = L.n;
-    const long N = (long)n * n * n;
-    double v[KF_RED] = {0., 0., -INFINITY, INFINITY, 0.};
-    if (blockIdx.x == 0 && threadIdx.x == 0) v[2] = v[3] = in[0];  // supremum = infinum = in.val[0] (:158-159)
-    for (long id = (long)blockIdx.x * BS + threadIdx.x; id < N; id += (long)gridDim.x * BS) {
-        const unsigned u = (unsigned)id;
-        const int k = (int)(u % (unsigned)n);
-        const unsigned r = u / (unsigned)n;
-        const int j = (int)(r % (unsigned)n), i = (int)(r / (unsigned)n);
-        double A, D;
-        point_coeffs_div(in, rho, L, i, j, k, A, D);
-        const double P_old = in[id];
-        double f0;
-        const double P_new = newton_point(P_old, A, D, f0);
-        const double delta = fabs(__dsub_rn(P_new, P_old));
-        out[id] = __dadd_rn(__dmul_rn(1. - omega, P_old), __dmul_rn(omega, P_new));
-        v[0] = nmax(v[0], delta);
-        v[1] = __dadd_rn(v[1], delta);
-        v[2] = nmax(v[2], P_new);
-        v[3] = nmin(v[3], P_new);
-        v[4] = nmax(v[4], fabs(f0));
-    }
-    jac_tree<BS>(v, sh);
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < KF_RED; ++s) partial[(long)blockIdx.x * KF_RED + s] = v[s];
-        __threadfence();
-        last = atomicAdd(&js->ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double w[KF_RED] = {0., 0., -INFINITY, INFINITY, 0.};
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += BS) {
-        const double *p = partial + (long)b * KF_RED;
-        w[0] = nmax(w[0], __ldcg(p));
-        w[1] = __dadd_rn(w[1], __ldcg(p + 1));
-        w[2] = nmax(w[2], __ldcg(p + 2));
-        w[3] = nmin(w[3], __ldcg(p + 3));
-        w[4] = nmax(w[4], __ldcg(p + 4));
-    }
-    __syncthreads();
-    jac_tree<BS>(w, sh);
-    if (threadIdx.x != 0) return;
-    js->ticket = 0;
-    const int iteration = js->iteration + 1;
-    js->norm_sum_old = js->norm_sum;
-    js->norm_max_old = js->norm_max;
-    js->sup = w[2];
-    js->inf = w[3];
-    js->rlast = w[4];
+// The record after a sweep with the statistics v.
+__device__ __forceinline__ void jac_finish(JacState &st, const JcStat &v, long N, const JacStop &S) {
+    const double w[5] = {__longlong_as_double((long long)v.dmax), v.sum, v.pmax, v.pmin,
+                         __longlong_as_double((long long)v.fmax)};
+    const int iteration = st.iteration + 1;
+    const double omega = st.omega;
+    st.norm_sum_old = st.norm_sum;
+    st.norm_max_old = st.norm_max;
+    st.sup = w[2];
+    st.inf = w[3];
+    st.rlast = w[4];
     const double norm_max = w[0], norm_sum = w[1] / (double)N;
-    bool nan = w[4] != w[4] || w[0] != w[0], done = nan, conv = false;
+    const bool nan = w[4] != w[4] || w[0] != w[0];
     // Carre's over-relaxation factor (:237-252)
     double om = .5;
-    if (norm_max < js->norm_max_old && iteration > 1) {
-        const double lambda = norm_sum / js->norm_sum_old;
+    if (norm_max < st.norm_max_old && iteration > 1) {
+        const double lambda = norm_sum / st.norm_sum_old;
         const double a = __dsub_rn(__dadd_rn(lambda, omega), 1.);
         om = 2. / __dadd_rn(1., sqrt(__dsub_rn(1., __dmul_rn(a, a) / __dmul_rn(lambda, __dmul_rn(omega, omega)))));
     }
     if (om != om) om = .5;
+    bool conv = false, done = nan;
     if (!nan) {
         conv = S.resstop ? w[4] <= S.tol : norm_max < __dmul_rn(S.limit, __dsub_rn(w[2], w[3]));
         done = conv || iteration >= S.max_it;
     }
-    js->norm_max = norm_max;
-    js->norm_sum = nan ? w[1] : norm_sum;
-    js->omega = om;
-    js->iteration = iteration;
-    js->converged = conv;
-    js->nan = nan;
-    js->done = done;
-    if (cond) cudaGraphSetConditional(h, done ? 0u : 1u);
+    st.norm_max = norm_max;
+    st.norm_sum = nan ? w[1] : norm_sum;
+    st.omega = om;
+    st.iteration = iteration;
+    st.converged = conv;
+    st.nan = nan;
+    st.done = done;
+}
+
+// The record with the last sweep's block statistics q[0 .. nq - 1] taken in, in
+// every thread: the loads (jac_load) are issued before, the result needs the block.
+__device__ __forceinline__ JcStat jac_load(const JcStat *q, int nq) {
+    JcStat v{0., 0ull, 0ull, -INFINITY, INFINITY};
+    for (int b = threadIdx.x; b < nq; b += 256) v.join(q[b]);
+    return v;
+}
+__device__ __forceinline__ void jac_record(const JcStat &v, const JacState *in, long N, const JacStop &S, JcStat *sh,
+                                           JacState *st) {
+    const JcStat w = jac_tree(v, sh);
+    if (threadIdx.x == 0) {
+        JacState s = *in;
+        if (!s.done && !s.fresh) jac_finish(s, w, N, S);
+        *st = s;
+    }
+    __syncthreads();
+}
+
+// One sweep in -> out; q, sin: the last sweep's statistics and the record before
+// it; p, sout: this one's statistics and the record before it.
+__global__ void __launch_bounds__(256) k_jacobi(const double *__restrict__ in, double *__restrict__ out,
+                                                const double *__restrict__ rho, Lev L, JacStop S,
+                                                const JcStat *__restrict__ q, JcStat *__restrict__ p,
+                                                const JacState *__restrict__ sin, JacState *__restrict__ sout) {
+    __shared__ JcStat sh[256];
+    __shared__ JacState st;
+    const int n = L.n, nn = n * n, t = threadIdx.x;
+    const long N = (long)nn * n;
+    const JcStat prev = jac_load(q, gridDim.x);
+    JcStat v{0., 0ull, 0ull, -INFINITY, INFINITY};
+    double omega = 1.;
+    bool have = false;
+    for (long id = (long)blockIdx.x * 256 + t; id < N || !have; id += (long)gridDim.x * 256) {
+        double P_old = 0., P_new = 0., f0 = 0.;
+        if (id < N) {
+            const unsigned u = (unsigned)id;
+            const int k = (int)(u % (unsigned)n);
+            const unsigned r = u / (unsigned)n;
+            const int j = (int)(r % (unsigned)n), i = (int)(r / (unsigned)n);
+            double A, D;
+            point_coeffs_div(in + wrapi(i - 1, n) * nn, in + i * nn, in + wrapi(i + 1, n) * nn, rho[id], L, i, j, k, A, D);
+            P_old = in[id];
+            P_new = newton_point(P_old, A, D, f0);
+        }
+        if (!have) {  // the factor, once the first point has come this far
+            have = true;
+            jac_record(prev, sin, N, S, sh, &st);
+            if (blockIdx.x == 0 && t == 0) {
+                JacState s = st;
+                s.fresh = 0;
+                *sout = s;
+            }
+            if (st.done) return;
+            omega = st.omega;
+            __syncthreads();  // sh is used again below
+        }
+        if (id >= N) break;
+        const double delta = fabs(__dsub_rn(P_new, P_old));
+        out[id] = __dadd_rn(__dmul_rn(1. - omega, P_old), __dmul_rn(omega, P_new));
+        v.join(JcStat{delta, (unsigned long long)__double_as_longlong(delta),
+                      (unsigned long long)__double_as_longlong(fabs(f0)), P_new, P_new});
+        if (id == 0) {  // supremum = infinum = in.val[0] at the start (:158-159)
+            v.pmax = fmax(v.pmax, P_old);
+            v.pmin = fmin(v.pmin, P_old);
+        }
+    }
+    v = jac_tree(v, sh);
+    if (t == 0) p[blockIdx.x] = v;
+}
+
+// After the body's sweeps: their last statistics into the record, the WHILE
+// condition h from it (loop == 0: not in a loop).  One block.
+__global__ void __launch_bounds__(256) k_jacobi_test(const JcStat *__restrict__ q, int nq, JacState *js, long N,
+                                                     JacStop S, int loop, cudaGraphConditionalHandle h) {
+    __shared__ JcStat sh[256];
+    __shared__ JacState st;
+    jac_record(jac_load(q, nq), js, N, S, sh, &st);
+    if (threadIdx.x) return;
+    JacState s = st;
+    s.fresh = 1;
+    *js = s;
+    if (loop) cudaGraphSetConditional(h, s.done ? 0u : 1u);
 }
 
 // phi <- tmp when the last sweep left the result there (an odd number of sweeps)
