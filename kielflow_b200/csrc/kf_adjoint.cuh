@@ -28,14 +28,15 @@ __device__ __forceinline__ void block_sum4(double v[4], double *sh, double *part
         for (int q = 0; q < 4; ++q) part[blockIdx.x * 4 + q] = sh[q * BS];
 }
 
-// acc[q] += sum over blocks of part[b*4 + q], fixed order (one thread).
+// acc[q] += sum over blocks of part[b*4 + q], fixed order, one thread per slot
+// (one thread for all four took 20 us at 1024 blocks).
 __global__ void k_accumulate4(const double *__restrict__ part, int nb, double *__restrict__ acc) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (int q = 0; q < 4; ++q) {
-        double s = 0.;
-        for (int b = 0; b < nb; ++b) s = __dadd_rn(s, part[b * 4 + q]);
-        acc[q] = __dadd_rn(acc[q], s);
-    }
+    const int q = threadIdx.x;
+    if (q >= 4 || blockIdx.x != 0) return;
+    double s = 0.;
+#pragma unroll 8
+    for (int b = 0; b < nb; ++b) s = __dadd_rn(s, part[b * 4 + q]);
+    acc[q] = __dadd_rn(acc[q], s);
 }
 
 // Transpose of the physical-space part of the right-hand side (k_products).
@@ -433,6 +434,39 @@ __global__ void __launch_bounds__(1024) k_coarse_solve_lin(double *__restrict__ 
     for (int id = threadIdx.x; id < N; id += blockDim.x) phi[id] = sp[id];
 }
 
+// Record of one adjoint Poisson solve: the source's maximum, the residual target
+// rtol max |b|, the last residual and the V-cycles done.
+struct DevAdj {
+    double bmax, tol, r;
+    int cyc, pad;
+};
+
+// the 64 slots' maximum in lane 0 of one warp, the slots left zero
+__device__ __forceinline__ double take_slots(unsigned long long *slots) {
+    const ulonglong2 v = reinterpret_cast<ulonglong2 *>(slots)[threadIdx.x];
+    reinterpret_cast<ulonglong2 *>(slots)[threadIdx.x] = make_ulonglong2(0, 0);
+    unsigned long long m = max(v.x, v.y);
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return __longlong_as_double((long long)m);
+}
+__global__ void k_adj_begin(unsigned long long *__restrict__ slots, DevAdj *d, double rtol) {
+    const double b = take_slots(slots);
+    if (threadIdx.x) return;
+    d->bmax = b;
+    d->tol = rtol * b;
+    d->cyc = 0;
+}
+// after a residual pass: go on while it is above the target (no source: not at all)
+__global__ void k_adj_check(unsigned long long *__restrict__ slots, DevAdj *d, int max_cycles, int first,
+                            cudaGraphConditionalHandle h) {
+    const double r = take_slots(slots);
+    if (threadIdx.x) return;
+    const int cyc = first ? 0 : d->cyc + 1;
+    d->cyc = cyc;
+    d->r = r;
+    cudaGraphSetConditional(h, d->bmax > 0. && r > d->tol && cyc < max_cycles ? 1u : 0u);
+}
+
 // Block sums of <b, bp> (slot 0) and <bp, bp> (slot 1): the least-squares
 // factor alpha = <b, bp> / <bp, bp> of the warm start alpha * psi_prev.
 template <int BS>
@@ -450,9 +484,9 @@ __global__ void __launch_bounds__(BS) k_dot2(const double *__restrict__ b, const
 
 // psi = alpha psi (alpha = sums[0] / sums[1], 0 when sums[1] == 0); bp = b
 __global__ void k_warm_scale(double *__restrict__ psi, double *__restrict__ bp, const double *__restrict__ b,
-                             const double *__restrict__ sums, long N) {
+                             const double *__restrict__ sums, const DevAdj *__restrict__ d, long N) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
+    if (i >= N || !(d->bmax > 0.)) return;  // no source (or a NaN in it): the record stays
     const double den = sums[1];
     const double alpha = den > 0. ? sums[0] / den : 0.;
     psi[i] *= alpha;

@@ -48,8 +48,9 @@ struct AdjState {
     std::vector<void *> segX;      // stage inputs of one segment: 16 per step
     std::vector<double *> segPhi;  // stage potentials of one segment: 4 per step
     std::vector<double *> allPhi;  // KF_ADJ_STORE_PHI: 4 per step of the whole run
-    cudaGraphExec_t graph = nullptr;
-    long long graph_kernels = 0;
+    cudaGraphExec_t graph = nullptr;  // a whole Poisson solve (adj_solve_body)
+    long long graph_kernels = 0, cycle_kernels = 0;
+    DevAdj *rec = nullptr, *h_rec = nullptr;
     long long cycles = 0;
     int solves = 0;
 };
@@ -202,6 +203,8 @@ void adj_init(kf_ctx *c) {
     a.part = dalloc<double>(c, sizeof(double) * 4 * 1184);
     a.acc = dalloc<double>(c, sizeof(double) * 4);
     CK(cudaMallocHost(&a.h_acc, sizeof(double) * 4));
+    a.rec = dalloc<DevAdj>(c, sizeof(DevAdj));
+    CK(cudaMallocHost(&a.h_rec, sizeof(DevAdj)));
     a.fin = snap_alloc(c);
     CK(cudaFuncSetAttribute(k_coarse_solve_lin, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     build_adj_jobs(c);
@@ -211,6 +214,7 @@ void adj_release(kf_ctx *c) {
     if (!c->adj) return;
     if (c->adj->graph) cudaGraphExecDestroy(c->adj->graph);
     if (c->adj->h_acc) cudaFreeHost(c->adj->h_acc);
+    if (c->adj->h_rec) cudaFreeHost(c->adj->h_rec);
     delete c->adj;  // device buffers are in c->allocs
     c->adj = nullptr;
 }
@@ -285,58 +289,26 @@ void avcycle(kf_ctx *c, int l) {
     CK(cudaGetLastError());
 }
 
-void run_avcycle(kf_ctx *c) {
-    AdjState &a = *c->adj;
-    if (c->prof) {
-        avcycle(c, 0);
-        return;
-    }
-    if (!a.graph) {
-        const long long l0 = c->launches;
-        CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-        avcycle(c, 0);
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamEndCapture(c->st, &g));
-        cudaError_t e = cudaGraphInstantiate(&a.graph, g, 0);
-        cudaGraphDestroy(g);
-        CK(e);
-        a.graph_kernels = c->launches - l0;
-        c->launches = l0;
-    }
-    CK(cudaGraphLaunch(a.graph, c->st));
-    c->launches += a.graph_kernels;
-}
-
-double read_max64(kf_ctx *c) {
-    CK(cudaMemcpyAsync(c->h_max, c->d_max, 64 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    unsigned long long m = 0;
-    for (int s = 0; s < 64; ++s) m = c->h_max[s] > m ? c->h_max[s] : m;
-    double r;
-    std::memcpy(&r, &m, sizeof(double));
-    return r;
-}
-
-double adj_resmax(kf_ctx *c) {
+// max |residual| of the finest level into the (zero) slots
+void adj_resmax(kf_ctx *c) {
     AdjState &a = *c->adj;
     LevelBuf &L = c->lv[0];
-    CK(cudaMemsetAsync(c->d_max, 0, 64 * sizeof(unsigned long long), c->st));
-    {
-        Launch L_(c, KC_ADJ_MG, 24. * c->N);
-        dim3 g = mg_grid(L.n, L.n);
-        g.z = L.n < 16 ? L.n : 16;
-        if (col_level(L.n))
-            k_residual_col<8, COL_PI, true, true, false><<<dim3(L.n / 64, L.n / 8, L.n / COL_PI), mg_block(), 0, c->st>>>(
-                a.rhob, a.phibar, L.lev(), nullptr, c->d_max, a.c0);
-        else
-            k_resmax_lin<<<g, mg_block(), 0, c->st>>>(a.rhob, a.phibar, a.c0, L.lev(), c->d_max);
-    }
+    Launch L_(c, KC_ADJ_MG, 24. * c->N);
+    dim3 g = mg_grid(L.n, L.n);
+    g.z = L.n < 16 ? L.n : 16;
+    if (col_level(L.n))
+        k_residual_col<8, COL_PI, true, true, false><<<dim3(L.n / 64, L.n / 8, L.n / COL_PI), mg_block(), 0, c->st>>>(
+            a.rhob, a.phibar, L.lev(), nullptr, c->d_max, a.c0);
+    else
+        k_resmax_lin<<<g, mg_block(), 0, c->st>>>(a.rhob, a.phibar, a.c0, L.lev(), c->d_max);
     CK(cudaGetLastError());
-    return read_max64(c);
 }
 
-// rhob <- (-lap_h + diag e^phi)^-1 phibar, phi = c->phi; warm start: rhob as it stands
-void adj_poisson(kf_ctx *c) {
+// The start of a solve: e^phi on every level, the source's maximum and the
+// target, the warm start (the previous solution times the least-squares factor of
+// this source on the previous one: consecutive stage sources are close to
+// proportional), the first residual.
+void adj_solve_begin(kf_ctx *c) {
     AdjState &a = *c->adj;
     const long N = c->N;
     {
@@ -353,41 +325,126 @@ void adj_poisson(kf_ctx *c) {
         Launch L_(c, KC_ADJ_MG, 8. * N);
         k_absmax<<<red_blocks(N), 256, 0, c->st>>>(a.phibar, N, c->d_max);
     }
-    const double bmax = read_max64(c);
-    if (bmax != bmax) throw KfError{KF_ERR_NAN, "NaN in the adjoint Poisson source"};
+    {
+        Launch L_(c, KC_ADJ_MG, 0.);
+        k_adj_begin<<<1, 32, 0, c->st>>>(c->d_max, a.rec, kAdjRtol);
+    }
+    const int nb = red_blocks(N);
+    {
+        Launch L_(c, KC_ADJ_MG, 16. * N);
+        k_dot2<RBS><<<nb, RBS, 0, c->st>>>(a.phibar, a.bprev, N, a.part);
+    }
+    CK(cudaMemsetAsync(a.sums, 0, 4 * sizeof(double), c->st));
+    {
+        Launch L_(c, KC_ADJ_MG, 32. * nb);
+        k_accumulate4<<<1, 32, 0, c->st>>>(a.part, nb, a.sums);
+    }
+    {
+        Launch L_(c, KC_ADJ_MG, 32. * N);
+        k_warm_scale<<<nblk(N, 256), 256, 0, c->st>>>(a.rhob, a.bprev, a.phibar, a.sums, a.rec, N);
+    }
+    adj_resmax(c);
+}
+
+void adj_check(kf_ctx *c, int first, cudaGraphConditionalHandle h) {
+    Launch L_(c, KC_ADJ_MG, 0.);
+    k_adj_check<<<1, 32, 0, c->st>>>(c->d_max, c->adj->rec, kAdjMaxCycles, first, h);
+}
+
+// The whole solve as a graph: adj_solve_begin, WHILE { V-cycle, residual, test }.
+void build_adj_graph(kf_ctx *c) {
+    AdjState &a = *c->adj;
+    const long long l0 = c->launches;
+    cudaStream_t outer = c->st;
+    cudaGraph_t g = nullptr;
+    CK(cudaStreamBeginCapture(outer, cudaStreamCaptureModeThreadLocal));
+    try {
+        cudaStreamCaptureStatus cs;
+        cudaGraph_t cg = nullptr;
+        CK(cudaStreamGetCaptureInfo(outer, &cs, nullptr, &cg, nullptr, nullptr));
+        cudaGraphConditionalHandle h;
+        CK(cudaGraphConditionalHandleCreate(&h, cg, 0, 0));
+        adj_solve_begin(c);
+        adj_check(c, 1, h);
+        const cudaGraphNode_t *deps = nullptr;
+        size_t ndeps = 0;
+        CK(cudaStreamGetCaptureInfo(outer, &cs, nullptr, &cg, &deps, &ndeps));
+        cudaGraphNodeParams wp = {cudaGraphNodeTypeConditional};
+        wp.conditional.handle = h;
+        wp.conditional.type = cudaGraphCondTypeWhile;
+        wp.conditional.size = 1;
+        cudaGraphNode_t wnode;
+        CK(cudaGraphAddNode(&wnode, cg, deps, ndeps, &wp));
+        CK(cudaStreamUpdateCaptureDependencies(outer, &wnode, 1, cudaStreamSetCaptureDependencies));
+        const long long l1 = c->launches;
+        c->st = c->st_body;
+        CK(cudaStreamBeginCaptureToGraph(c->st, wp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                         cudaStreamCaptureModeThreadLocal));
+        cudaGraph_t body = nullptr;
+        try {
+            avcycle(c, 0);
+            adj_resmax(c);
+            adj_check(c, 0, h);
+        } catch (...) {
+            cudaStreamEndCapture(c->st, &body);
+            throw;
+        }
+        CK(cudaStreamEndCapture(c->st, &body));
+        c->st = outer;
+        a.cycle_kernels = c->launches - l1;
+    } catch (...) {
+        c->st = outer;
+        cudaStreamEndCapture(outer, &g);
+        if (g) cudaGraphDestroy(g);
+        c->launches = l0;
+        throw;
+    }
+    CK(cudaStreamEndCapture(outer, &g));
+    const cudaError_t e = cudaGraphInstantiate(&a.graph, g, 0);
+    cudaGraphDestroy(g);
+    CK(e);
+    a.graph_kernels = c->launches - l0 - a.cycle_kernels;
+    c->launches = l0;
+}
+
+// rhob <- (-lap_h + diag e^phi)^-1 phibar, phi = c->phi; warm start: rhob as it stands
+void adj_poisson(kf_ctx *c) {
+    AdjState &a = *c->adj;
+    auto read = [&] {
+        CK(cudaMemcpyAsync(a.h_rec, a.rec, sizeof(DevAdj), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+    };
+    if (!c->prof) {
+        if (!a.graph) build_adj_graph(c);
+        CK(cudaGraphLaunch(a.graph, c->st));
+        read();
+        c->launches += a.graph_kernels + a.h_rec->cyc * a.cycle_kernels;
+    } else {  // launched one by one, for the per-launch profile
+        adj_solve_begin(c);
+        auto test = [&](int cyc) {
+            CK(cudaMemcpyAsync(c->h_max, c->d_max, 64 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->st));
+            read();
+            CK(cudaMemsetAsync(c->d_max, 0, 64 * sizeof(unsigned long long), c->st));
+            const unsigned long long m = *std::max_element(c->h_max, c->h_max + 64);
+            std::memcpy(&a.h_rec->r, &m, sizeof(double));
+            a.h_rec->cyc = cyc;
+            return a.h_rec->bmax > 0. && a.h_rec->r > a.h_rec->tol && cyc < kAdjMaxCycles;
+        };
+        for (int cyc = 0; test(cyc); ++cyc) {
+            avcycle(c, 0);
+            adj_resmax(c);
+        }
+    }
+    const DevAdj d = *a.h_rec;
+    if (d.bmax != d.bmax) throw KfError{KF_ERR_NAN, "NaN in the adjoint Poisson source"};
     a.solves++;
-    if (bmax == 0.) {
-        CK(cudaMemsetAsync(a.rhob, 0, 8 * N, c->st));
+    if (d.bmax == 0.) {
+        CK(cudaMemsetAsync(a.rhob, 0, 8 * c->N, c->st));
         return;
     }
-    // warm start: the previous solution times the least-squares factor of
-    // this source on the previous one (consecutive stage sources are close
-    // to proportional)
-    {
-        const int nb = red_blocks(N);
-        {
-            Launch L_(c, KC_ADJ_MG, 16. * N);
-            k_dot2<RBS><<<nb, RBS, 0, c->st>>>(a.phibar, a.bprev, N, a.part);
-        }
-        CK(cudaMemsetAsync(a.sums, 0, 4 * sizeof(double), c->st));
-        {
-            Launch L_(c, KC_ADJ_MG, 32. * nb);
-            k_accumulate4<<<1, 32, 0, c->st>>>(a.part, nb, a.sums);
-        }
-        Launch L_(c, KC_ADJ_MG, 32. * N);
-        k_warm_scale<<<nblk(N, 256), 256, 0, c->st>>>(a.rhob, a.bprev, a.phibar, a.sums, N);
-    }
-    const double tol = kAdjRtol * bmax;
-    double r = adj_resmax(c);
-    int cyc = 0;
-    while (r > tol && cyc < kAdjMaxCycles) {
-        run_avcycle(c);
-        ++cyc;
-        r = adj_resmax(c);
-    }
-    a.cycles += cyc;
-    if (r != r) throw KfError{KF_ERR_NAN, "NaN in the adjoint Poisson solve"};
-    if (r > tol) throw KfError{KF_ERR_NOT_CONVERGED, "adjoint Poisson solve did not reach its tolerance"};
+    a.cycles += d.cyc;
+    if (d.r != d.r) throw KfError{KF_ERR_NAN, "NaN in the adjoint Poisson solve"};
+    if (d.r > d.tol) throw KfError{KF_ERR_NOT_CONVERGED, "adjoint Poisson solve did not reach its tolerance"};
 }
 
 // ------------------------------------------------------------------ one stage VJP

@@ -164,9 +164,10 @@ struct kf_ctx {
     // the FAS V-cycle captured once as a CUDA graph (replayed every cycle)
     cudaGraphExec_t vgraph = nullptr;
     long long vgraph_kernels = 0;
-    // the part of a V-cycle after the finest level's residual (adaptive solves)
-    cudaGraphExec_t vgraph_tail = nullptr;
-    long long vgraph_tail_kernels = 0;
+    // an adaptive solve for the host-driven callers (fas_solve)
+    cudaGraphExec_t solve_graph = nullptr;
+    long long solve_kernels = 0, solve_cycle_kernels = 0;
+    DevPois *h_pois = nullptr;
     // per-(precision, n) entry points
     void (*rhs_fn)(kf_ctx *) = nullptr;
     void (*r2c_fn)(kf_ctx *) = nullptr;
@@ -965,28 +966,6 @@ void run_vcycle(kf_ctx *c) {
     c->launches += c->vgraph_kernels;
 }
 
-// vcycle_tail(c, 0), replayed from its own graph as run_vcycle does
-void run_vcycle_tail(kf_ctx *c) {
-    if (c->prof) {
-        vcycle_tail(c, 0);
-        return;
-    }
-    if (!c->vgraph_tail) {
-        const long long l0 = c->launches;
-        CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-        vcycle_tail(c, 0);
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamEndCapture(c->st, &g));
-        cudaError_t e = cudaGraphInstantiate(&c->vgraph_tail, g, 0);
-        cudaGraphDestroy(g);
-        CK(e);
-        c->vgraph_tail_kernels = c->launches - l0;
-        c->launches = l0;
-    }
-    CK(cudaGraphLaunch(c->vgraph_tail, c->st));
-    c->launches += c->vgraph_tail_kernels;
-}
-
 // max over the 64 d_max slots (IEEE bit patterns of non-negative doubles)
 double read_max_slots(kf_ctx *c) {
     CK(cudaMemcpyAsync(c->h_max, c->d_max, 64 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->st));
@@ -1017,6 +996,99 @@ void solve_end(kf_ctx *c) {
     Launch L_(c, KC_RHO, 16. * c->N);
     k_unsplit<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(c->phi_cs, c->phi, c->n);
     CK(cudaGetLastError());
+}
+
+// The adaptive FAS loop inside a capture on c->st: head of the cycle
+// (pre-smoothing, residual with its max); k_fas_check; WHILE { rest of the cycle;
+// head; k_fas_check }: as many passes as V-cycles.  (WHILE { head; check; IF { rest
+// } } took one pass more and an IF node in each; a pass costs about 7 us beside its
+// kernels.)  Returns the kernels of a pass.
+long long fas_loop(kf_ctx *c) {
+    const kf_config &cf = c->cfg;
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t g = nullptr;
+    CK(cudaStreamGetCaptureInfo(c->st, &cs, nullptr, &g, nullptr, nullptr));
+    cudaGraphConditionalHandle hw;
+    CK(cudaGraphConditionalHandleCreate(&hw, g, 0, 0));
+    auto head = [&](int first) {
+        vcycle_head(c, 0, true, !first);  // k_fas_check leaves the slots zero
+        Launch L_(c, KC_MISC, 0.);
+        k_fas_check<<<1, 32, 0, c->st>>>(c->d_max, c->dpois, cf.res_tol, cf.max_cycles, first, false, c->stage_idx, hw);
+    };
+    head(1);
+    const cudaGraphNode_t *deps = nullptr;
+    size_t ndeps = 0;
+    CK(cudaStreamGetCaptureInfo(c->st, &cs, nullptr, &g, &deps, &ndeps));
+    cudaGraphNodeParams wp = {cudaGraphNodeTypeConditional};
+    wp.conditional.handle = hw;
+    wp.conditional.type = cudaGraphCondTypeWhile;
+    wp.conditional.size = 1;
+    cudaGraphNode_t wnode;
+    CK(cudaGraphAddNode(&wnode, g, deps, ndeps, &wp));
+    CK(cudaStreamUpdateCaptureDependencies(c->st, &wnode, 1, cudaStreamSetCaptureDependencies));
+    const long long l1 = c->launches;
+    cudaStream_t outer = c->st;
+    c->st = c->st_body;
+    cudaError_t e = cudaStreamBeginCaptureToGraph(c->st, wp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                  cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        cudaGraph_t body_out = nullptr;
+        try {
+            vcycle_tail(c, 0);
+            head(0);
+            e = cudaStreamEndCapture(c->st, &body_out);
+        } catch (...) {
+            cudaStreamEndCapture(c->st, &body_out);
+            c->st = outer;
+            throw;
+        }
+    }
+    c->st = outer;
+    CK(e);
+    return c->launches - l1;
+}
+
+// A whole adaptive solve of the finest level from its own graph (fas_loop and the
+// way back from split order), for the host-driven callers: one launch and one
+// synchronisation.  Returns as poisson().
+int fas_solve(kf_ctx *c) {
+    const long long l0 = c->launches;
+    if (!c->solve_graph) {
+        CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
+        cudaGraph_t g = nullptr;
+        try {
+            c->solve_cycle_kernels = fas_loop(c);
+            solve_end(c);
+        } catch (...) {
+            cudaStreamEndCapture(c->st, &g);
+            if (g) cudaGraphDestroy(g);
+            c->launches = l0;
+            throw;
+        }
+        CK(cudaStreamEndCapture(c->st, &g));
+        const cudaError_t e = cudaGraphInstantiate(&c->solve_graph, g, 0);
+        cudaGraphDestroy(g);
+        CK(e);
+        c->solve_kernels = c->launches - l0 - c->solve_cycle_kernels;
+        c->launches = l0;
+    }
+    CK(cudaGraphLaunch(c->solve_graph, c->st));
+    CK(cudaMemcpyAsync(c->h_pois, c->dpois, sizeof(DevPois), cudaMemcpyDeviceToHost, c->st));
+    kerr_fetch(c);
+    CK(cudaStreamSynchronize(c->st));
+    kerr_check(c);
+    const DevPois &hp = *c->h_pois;
+    const int cyc = hp.last_cycles;
+    const bool nc = hp.not_converged != c->hpois.not_converged;
+    c->hpois = hp;
+    c->launches += c->solve_kernels + cyc * c->solve_cycle_kernels;
+    c->diag.last_iterations = cyc;
+    c->diag.stage_cycles[c->stage_idx & 3] += cyc;
+    c->diag.total_iterations += cyc;
+    c->diag.last_residual = hp.last_residual;
+    if (hp.last_residual != hp.last_residual) throw KfError{KF_ERR_NAN, "NaN in the multigrid solve"};
+    if (nc) c->diag.not_converged++;
+    return nc ? 1 : 0;
 }
 
 // Poisson solve on c->phi with source c->rho; split: whoever wrote c->rho wrote
@@ -1082,6 +1154,7 @@ int poisson(kf_ctx *c, bool split = false) {
         // test after each cycle's pre-smoothing on the residual the cycle
         // computes anyway; the rest of the cycle only when it fails
         solve_begin(c, split);
+        if (!c->prof) return fas_solve(c);
         double r = 0.;
         int cyc = 0;
         for (;;) {
@@ -1089,7 +1162,7 @@ int poisson(kf_ctx *c, bool split = false) {
             CK(cudaGetLastError());
             r = read_max_slots(c);
             if (!(r > cf.res_tol) || cyc >= cf.max_cycles) break;
-            run_vcycle_tail(c);
+            vcycle_tail(c, 0);
             ++cyc;
         }
         solve_end(c);
@@ -1162,51 +1235,7 @@ void poisson_captured(kf_ctx *c) {
     LevelBuf &L0 = c->lv[0];
     const bool fixed = !(cf.res_tol > 0.);
     if (!fixed && c->lv.size() > 1) {
-        // head of the cycle (pre-smoothing, residual with its max); k_fas_check;
-        // WHILE { rest of the cycle; head; k_fas_check }: as many passes as V-cycles.
-        // (WHILE { head; check; IF { rest } } took one pass more and an IF node in
-        // each; a pass costs about 7 us beside its kernels.)
-        cudaStreamCaptureStatus cs;
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamGetCaptureInfo(c->st, &cs, nullptr, &g, nullptr, nullptr));
-        cudaGraphConditionalHandle hw;
-        CK(cudaGraphConditionalHandleCreate(&hw, g, 0, 0));
-        auto head = [&](int first) {
-            vcycle_head(c, 0, true, !first);  // k_fas_check leaves the slots zero
-            Launch L_(c, KC_MISC, 0.);
-            k_fas_check<<<1, 32, 0, c->st>>>(c->d_max, c->dpois, cf.res_tol, cf.max_cycles, first, false, c->stage_idx, hw);
-        };
-        head(1);
-        const cudaGraphNode_t *deps = nullptr;
-        size_t ndeps = 0;
-        CK(cudaStreamGetCaptureInfo(c->st, &cs, nullptr, &g, &deps, &ndeps));
-        cudaGraphNodeParams wp = {cudaGraphNodeTypeConditional};
-        wp.conditional.handle = hw;
-        wp.conditional.type = cudaGraphCondTypeWhile;
-        wp.conditional.size = 1;
-        cudaGraphNode_t wnode;
-        CK(cudaGraphAddNode(&wnode, g, deps, ndeps, &wp));
-        CK(cudaStreamUpdateCaptureDependencies(c->st, &wnode, 1, cudaStreamSetCaptureDependencies));
-        const long long l1 = c->launches;
-        cudaStream_t outer = c->st;
-        c->st = c->st_body;
-        cudaError_t e = cudaStreamBeginCaptureToGraph(c->st, wp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                      cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) {
-            cudaGraph_t body_out = nullptr;
-            try {
-                vcycle_tail(c, 0);
-                head(0);
-                e = cudaStreamEndCapture(c->st, &body_out);
-            } catch (...) {
-                cudaStreamEndCapture(c->st, &body_out);
-                c->st = outer;
-                throw;
-            }
-        }
-        c->st = outer;
-        CK(e);
-        c->cycle_kernels = c->launches - l1;
+        c->cycle_kernels = fas_loop(c);
         solve_end(c);
         if (extrap) {
             Launch L_(c, KC_MISC, 0.);
@@ -2405,6 +2434,7 @@ void create(kf_ctx *c) {
         CK(cudaMemset(q, 0, 592 * sizeof(JcStat)));
     }
     CK(cudaMallocHost(&c->h_js, sizeof(JacState)));
+    CK(cudaMallocHost(&c->h_pois, sizeof(DevPois)));
     c->dtime = dalloc<DevTime>(c, sizeof(DevTime));
     c->dpois = dalloc<DevPois>(c, sizeof(DevPois));
     CK(cudaMemset(c->dtime, 0, sizeof(DevTime)));
@@ -2695,8 +2725,8 @@ void drop_graphs(kf_ctx *c) {
     CK(cudaStreamSynchronize(c->st));
     if (c->vgraph) cudaGraphExecDestroy(c->vgraph);
     c->vgraph = nullptr;
-    if (c->vgraph_tail) cudaGraphExecDestroy(c->vgraph_tail);
-    c->vgraph_tail = nullptr;
+    if (c->solve_graph) cudaGraphExecDestroy(c->solve_graph);
+    c->solve_graph = nullptr;
     if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
     c->step_graph = nullptr;
     if (c->step_graph_wait) cudaGraphExecDestroy(c->step_graph_wait);
@@ -2867,7 +2897,7 @@ int kf_ctx_destroy(kf_ctx *c) {
     }
     for (auto e : c->evfree) cudaEventDestroy(e);
     if (c->vgraph) cudaGraphExecDestroy(c->vgraph);
-    if (c->vgraph_tail) cudaGraphExecDestroy(c->vgraph_tail);
+    if (c->solve_graph) cudaGraphExecDestroy(c->solve_graph);
     if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
     if (c->step_graph_wait) cudaGraphExecDestroy(c->step_graph_wait);
     if (c->ev_u) cudaEventDestroy(c->ev_u);
@@ -2881,6 +2911,7 @@ int kf_ctx_destroy(kf_ctx *c) {
     for (void *p : c->allocs) cudaFree(p);
     for (auto &g : c->jac) cudaGraphExecDestroy(g.exec);
     if (c->h_js) cudaFreeHost(c->h_js);
+    if (c->h_pois) cudaFreeHost(c->h_pois);
     if (c->h_red) cudaFreeHost(c->h_red);
     if (c->h_max) cudaFreeHost(c->h_max);
     if (c->h_err) cudaFreeHost(c->h_err);
