@@ -299,6 +299,9 @@ int kf_set_overlap(kf_ctx *ctx, int on);
 /* interface_poisson_solver::solve (interface_poisson_solver.hpp:18): phi_io is
  * the initial guess and the result, rho is read only; host arrays, n^3 doubles. */
 int kf_poisson_solve(kf_ctx *ctx, double *phi_io, const double *rho);
+/* The same with the initial guess phi0 left as it is and the result in phi (which
+ * may be phi0: kf_poisson_solve). */
+int kf_poisson_solve_to(kf_ctx *ctx, const double *phi0, const double *rho, double *phi);
 
 /* diagnostics: Poisson statistics and FP64 conserved-quantity reductions */
 int kf_diag(kf_ctx *ctx, kf_diag_out *out);

@@ -133,7 +133,7 @@ def library_path() -> str:
 EXPORTS = [
     "kf_ctx_create", "kf_ctx_destroy", "kf_last_error", "kf_set_stream", "kf_synchronize", "kf_set_state",
     "kf_get_state", "kf_set_sources", "kf_set_phi", "kf_get_phi", "kf_rhs_eval", "kf_rk4_steps",
-    "kf_poisson_solve", "kf_diag", "kf_fft_r2c", "kf_fft_c2r", "kf_state_device_ptrs", "kf_launch_count",
+    "kf_poisson_solve", "kf_poisson_solve_to", "kf_diag", "kf_fft_r2c", "kf_fft_c2r", "kf_state_device_ptrs", "kf_launch_count",
     "kf_profile_enable", "kf_profile_read", "kf_profile_class_name", "kf_fft_r2c_noalloc", "kf_adjoint_run",
     "kf_batch_rk4_steps", "kf_set_state_linear", "kf_get_output", "kf_run", "kf_save", "kf_load",
     "kf_file_info_read", "kf_frontend_state", "kf_step_host", "kf_autotune", "kf_set_tuning",
@@ -168,6 +168,7 @@ def load_library():
     L.kf_rhs_eval.argtypes = [vp, ctypes.c_double]
     L.kf_rk4_steps.argtypes = [vp, ctypes.c_int, ctypes.c_double]
     L.kf_poisson_solve.argtypes = [vp, _D, _D]
+    L.kf_poisson_solve_to.argtypes = [vp, _D, _D, _D]
     L.kf_diag.argtypes = [vp, ctypes.POINTER(DiagOut)]
     L.kf_fft_r2c.argtypes = [vp, _D, _D]
     L.kf_fft_c2r.argtypes = [vp, _D, _D]
@@ -372,10 +373,11 @@ class Context:
         self._check(self.L.kf_rk4_steps(self.h, nsteps, dt))
 
     def poisson(self, phi, rho):
-        phi = np.array(phi, dtype=np.float64, order="C", copy=True)
+        phi = np.ascontiguousarray(phi, np.float64)
         rho = np.ascontiguousarray(rho, np.float64)
-        self._check(self.L.kf_poisson_solve(self.h, _ptr(phi), _ptr(rho)))
-        return phi
+        out = np.empty(phi.shape, np.float64)
+        self._check(self.L.kf_poisson_solve_to(self.h, _ptr(phi), _ptr(rho), _ptr(out)))
+        return out
 
     def adjoint(self, w, nsteps: int, dt: float, ckpt_every: int = 15, flags: int = 0,
                 want_dn0: bool = True, want_lam0: bool = False):

@@ -593,7 +593,7 @@ void adj_run(kf_ctx *c, int nsteps, double dt, int E, int flags, const double *w
         if (sphi)
             while ((int)a.allPhi.size() < 4 * nsteps) a.allPhi.push_back(dalloc<double>(c, 8 * N));
     }
-    CK(cudaMemcpyAsync(a.w, w, 8 * N, cudaMemcpyHostToDevice, c->st));
+    put_host(c, a.w, w, 8 * N);
     CK(cudaMemsetAsync(a.acc, 0, 4 * sizeof(double), c->st));
     a.cycles = 0;
     a.solves = 0;
@@ -664,11 +664,11 @@ void adj_run(kf_ctx *c, int nsteps, double dt, int E, int flags, const double *w
                 Launch L_(c, KC_ADJ_PW, 24. * N);
                 k_dn0<<<nblk(N, 256), 256, 0, c->st>>>(a.RB[0], a.RB[1], a.out, N);
             }
-            CK(cudaMemcpyAsync(dJ_dn0, a.out, 8 * N, cudaMemcpyDeviceToHost, c->st));
+            get_host(c, dJ_dn0, a.out, 8 * N);
         }
         if (lam0)
             for (int q = 0; q < 4; ++q)
-                CK(cudaMemcpyAsync(lam0 + 2 * c->Nc * q, a.lam[q], 16 * c->Nc, cudaMemcpyDeviceToHost, c->st));
+                get_host(c, lam0 + 2 * c->Nc * q, a.lam[q], 16 * c->Nc);
         snap_load(c, a.fin);
     }
     CK(cudaEventRecord(ev[2], c->st));

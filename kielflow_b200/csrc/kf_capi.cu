@@ -27,6 +27,7 @@
 #include "kf_adjoint.cuh"
 #include "kf_cluster.cuh"
 #include "kf_graph.cuh"
+#include "kf_hostpipe.hpp"
 #include "kf_jacobi.cuh"
 #include "kf_march.cuh"
 #include "kf_passes.cuh"
@@ -104,6 +105,7 @@ struct kf_ctx {
     std::string err;
     long long launches = 0;
     std::vector<void *> allocs;
+    HostPipe pipe;  // pageable host arrays (put_host, get_host)
 
     void *Y[4] = {}, *Ys[4] = {}, *ACC[4] = {}, *K[4] = {};
     void *CX[12] = {}, *CY[16] = {}, *R[24] = {}, *phihat = nullptr, *LIN[4] = {};
@@ -2445,12 +2447,16 @@ void create(kf_ctx *c) {
     CK(cudaDeviceSynchronize());
 }
 
+// The caller's host arrays to and from the device, on c->st
+void put_host(kf_ctx *c, void *dst, const void *src, size_t bytes) { CK(c->pipe.copy(dst, src, bytes, true, c->st)); }
+void get_host(kf_ctx *c, void *dst, const void *src, size_t bytes) { CK(c->pipe.copy(dst, src, bytes, false, c->st)); }
+
 // H2D of a host FP64 array of `count` doubles into a bulk-precision device array
 void put_bulk(kf_ctx *c, void *dst, const double *src, long count) {
     if (!c->fp32) {
-        CK(cudaMemcpyAsync(dst, src, 8 * count, cudaMemcpyHostToDevice, c->st));
+        put_host(c, dst, src, 8 * count);
     } else {
-        CK(cudaMemcpyAsync(c->stage64, src, 8 * count, cudaMemcpyHostToDevice, c->st));
+        put_host(c, c->stage64, src, 8 * count);
         Launch L_(c, KC_MISC, 12. * count);
         k_from_f64<float><<<nblk(count, 256), 256, 0, c->st>>>((float *)dst, c->stage64, count);
     }
@@ -2458,13 +2464,13 @@ void put_bulk(kf_ctx *c, void *dst, const double *src, long count) {
 
 void get_bulk(kf_ctx *c, double *dst, const void *src, long count) {
     if (!c->fp32) {
-        CK(cudaMemcpyAsync(dst, src, 8 * count, cudaMemcpyDeviceToHost, c->st));
+        get_host(c, dst, src, 8 * count);
     } else {
         {
             Launch L_(c, KC_MISC, 12. * count);
             k_to_f64<float><<<nblk(count, 256), 256, 0, c->st>>>(c->stage64, (const float *)src, count);
         }
-        CK(cudaMemcpyAsync(dst, c->stage64, 8 * count, cudaMemcpyDeviceToHost, c->st));
+        get_host(c, dst, c->stage64, 8 * count);
     }
 }
 
@@ -2962,7 +2968,7 @@ int kf_get_state(kf_ctx *c, double *ux, double *uy, double *uz, double *s) {
 
 int kf_set_sources(kf_ctx *c, const double *nd, const double *mask) {
     return guarded(c, [&] {
-        if (nd) CK(cudaMemcpyAsync(c->nd, nd, 8 * c->N, cudaMemcpyHostToDevice, c->st));
+        if (nd) put_host(c, c->nd, nd, 8 * c->N);
         if (mask) {
             put_bulk(c, c->H, mask, c->N);
             mask_box(c);
@@ -2973,7 +2979,7 @@ int kf_set_sources(kf_ctx *c, const double *nd, const double *mask) {
 
 int kf_set_phi(kf_ctx *c, const double *phi) {
     return guarded(c, [&] {
-        CK(cudaMemcpyAsync(c->phi, phi, 8 * c->N, cudaMemcpyHostToDevice, c->st));
+        put_host(c, c->phi, phi, 8 * c->N);
         c->nhist = 0;
         CK(cudaStreamSynchronize(c->st));
     });
@@ -2981,7 +2987,7 @@ int kf_set_phi(kf_ctx *c, const double *phi) {
 
 int kf_get_phi(kf_ctx *c, double *phi) {
     return guarded(c, [&] {
-        CK(cudaMemcpyAsync(phi, c->phi, 8 * c->N, cudaMemcpyDeviceToHost, c->st));
+        get_host(c, phi, c->phi, 8 * c->N);
         CK(cudaStreamSynchronize(c->st));
     });
 }
@@ -3108,18 +3114,19 @@ int kf_batch_rk4_steps(kf_ctx *const *ctxs, int nctx, int nsteps, const double *
     return rc;
 }
 
-int kf_poisson_solve(kf_ctx *c, double *phi_io, const double *rho) {
-    int rc = guarded(c, [&] {
-        if (!phi_io || !rho) throw KfError{KF_ERR_ARG, "null array"};
-        CK(cudaMemcpyAsync(c->phi, phi_io, 8 * c->N, cudaMemcpyHostToDevice, c->st));
-        CK(cudaMemcpyAsync(c->rho, rho, 8 * c->N, cudaMemcpyHostToDevice, c->st));
+int kf_poisson_solve_to(kf_ctx *c, const double *phi0, const double *rho, double *phi) {
+    return guarded(c, [&] {
+        if (!phi0 || !rho || !phi) throw KfError{KF_ERR_ARG, "null array"};
+        put_host(c, c->phi, phi0, 8 * c->N);
+        put_host(c, c->rho, rho, 8 * c->N);
         int r = poisson(c);
-        CK(cudaMemcpyAsync(phi_io, c->phi, 8 * c->N, cudaMemcpyDeviceToHost, c->st));
+        get_host(c, phi, c->phi, 8 * c->N);
         CK(cudaStreamSynchronize(c->st));
         if (r) throw KfError{KF_ERR_NOT_CONVERGED, "Poisson solve did not reach its tolerance"};
     });
-    return rc;
 }
+
+int kf_poisson_solve(kf_ctx *c, double *phi_io, const double *rho) { return kf_poisson_solve_to(c, phi_io, rho, phi_io); }
 
 int kf_diag(kf_ctx *c, kf_diag_out *out) {
     return guarded(c, [&] {

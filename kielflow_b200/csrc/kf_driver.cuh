@@ -307,7 +307,7 @@ int kf_get_output(kf_ctx *c, double *ux, double *uy, double *uz, double *n, doub
         out_fields(c);
         double *dst[5] = {ux, uy, uz, n, phihat};
         for (int q = 0; q < 5; ++q)
-            if (dst[q]) CK(cudaMemcpyAsync(dst[q], c->out->O[q], 16 * c->Nc, cudaMemcpyDeviceToHost, c->st));
+            if (dst[q]) get_host(c, dst[q], c->out->O[q], 16 * c->Nc);
         CK(cudaStreamSynchronize(c->st));
     });
 }
@@ -385,7 +385,7 @@ int kf_save(kf_ctx *c, const char *path, int kind, double t) {
         std::vector<std::vector<double>> h(5, std::vector<double>(cnt));
         double *f[5];
         for (int q = 0; q < 5; ++q) {
-            CK(cudaMemcpyAsync(h[q].data(), plane ? o.P[q] : o.F[q], 8 * cnt, cudaMemcpyDeviceToHost, c->st));
+            get_host(c, h[q].data(), plane ? o.P[q] : o.F[q], 8 * cnt);
             f[q] = h[q].data();
         }
         CK(cudaStreamSynchronize(c->st));
@@ -461,7 +461,7 @@ int kf_load(kf_ctx *c, const char *path, double *t_out) {
             CK(cudaMemcpyAsync(c->Y[q], c->CX[0], c->cs * c->Nc, cudaMemcpyDeviceToDevice, c->st));
             CK(cudaStreamSynchronize(c->st));  // the host source of put_bulk is reused
         }
-        CK(cudaMemcpyAsync(c->phi, e[4]->data.data(), 8 * c->N, cudaMemcpyHostToDevice, c->st));
+        put_host(c, c->phi, e[4]->data.data(), 8 * c->N);
         copy_state(c, c->Ys, c->Y);
         c->nhist = 0;
         CK(cudaStreamSynchronize(c->st));
