@@ -116,10 +116,15 @@ struct kf_ctx {
     void *tw[2] = {};  // twiddles of the two radix plans (plan_twiddles)
     double *q2 = nullptr;
     int *pb = nullptr;  // x-pass 2/3-rule bounds per (j, kz) column (dealias_bounds)
-    // the kept part of a masked half spectrum (AxTrunc)
-    int tr_nkz = 0, tr_nt = 0, tr_mp = 0;  // tr_mp: elements per row of masked intermediates
-    double tr_ball = 0., tr_disc = 0.;  // elements kept; elements of the active columns
-    int *tr_jb = nullptr, *tr_tl = nullptr;
+    // active columns of a half spectrum (AxTrunc): the 2/3 rule's, and those on which
+    // the phi filter table is not 0
+    struct Cols {
+        int nkz = 0, nt = 0, mp = 0;  // mp: elements per row of the intermediates
+        int *jb = nullptr, *tl = nullptr;
+        double cols = 0.;  // elements of the active columns
+    };
+    Cols tr, pf;
+    double tr_ball = 0.;  // elements the 2/3 rule keeps
     double *stage64 = nullptr;
     std::vector<LevelBuf> lv;
     double *partial = nullptr;
@@ -167,6 +172,7 @@ struct kf_ctx {
     cudaGraphExec_t vgraph = nullptr;
     long long vgraph_kernels = 0;
     // an adaptive solve for the host-driven callers (fas_solve)
+    long long host_solves = 0;  // adaptive FAS solves that the host drove
     cudaGraphExec_t solve_graph = nullptr;
     long long solve_kernels = 0, solve_cycle_kernels = 0;
     DevPois *h_pois = nullptr;
@@ -1156,7 +1162,9 @@ int poisson(kf_ctx *c, bool split = false) {
         // test after each cycle's pre-smoothing on the residual the cycle
         // computes anyway; the rest of the cycle only when it fails
         solve_begin(c, split);
-        if (!c->prof) return fas_solve(c);
+        // a context's first solve from here: making the graph takes as long as the
+        // launches and synchronisations that it saves in a few solves
+        if (!c->prof && c->host_solves++) return fas_solve(c);
         double r = 0.;
         int cyc = 0;
         for (;;) {
@@ -1217,28 +1225,35 @@ bool phi_guess(kf_ctx *c) {
     return newtime;
 }
 
+// Whether the right-hand side being formed solves by poisson_captured.
+bool captured_solve(const kf_ctx *c) {
+    return c->capturing && !c->phi_given && (c->cfg.terms & T_POISSON) && (c->cfg.terms & T_E_INT);
+}
+
 // The stage's Poisson solve inside the capture of a step graph: device-side
 // warm start, then the FAS loop as a conditional WHILE node whose body (one
-// V-cycle + the max-residual test) is captured on st_body.
+// V-cycle + the max-residual test) is captured on st_body.  On split levels phi
+// stays in split order from the first stage's start to the last stage's end: the
+// next stage's start and phi^ read it there.
 void poisson_captured(kf_ctx *c) {
     const kf_config &cf = c->cfg;
     const bool extrap = cf.phi_extrap != 0;
     const bool sp = split_on(c, 0);
     if (extrap && sp) {
         Launch L_(c, KC_MISC, 32. * c->N);
-        k_guess_s<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(c->phi, c->phi_a, c->phi_cs, c->dtime, c->stage_x,
-                                                                             c->n);
+        k_guess_s<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(c->stage_idx ? nullptr : c->phi, c->phi_a,
+                                                                     c->phi_cs, c->dtime, c->stage_x, c->n);
     } else if (extrap) {
         Launch L_(c, KC_MISC, 24. * c->N);
         k_guess<<<nblk(c->N, 256), 256, 0, c->st>>>(c->phi, c->phi_a, c->dtime, c->stage_x, c->N);
-    } else if (sp) {
+    } else if (sp && c->stage_idx == 0) {
         split_field(c, c->phi, c->phi_cs);
     }
     LevelBuf &L0 = c->lv[0];
     const bool fixed = !(cf.res_tol > 0.);
     if (!fixed && c->lv.size() > 1) {
         c->cycle_kernels = fas_loop(c);
-        solve_end(c);
+        if (c->stage_idx == 3) solve_end(c);
         if (extrap) {
             Launch L_(c, KC_MISC, 0.);
             k_hist_post<<<1, 32, 0, c->st>>>(c->dtime, c->stage_x);
@@ -1298,7 +1313,7 @@ void poisson_captured(kf_ctx *c) {
     c->st = outer;
     CK(e);
     c->cycle_kernels = c->launches - l0;
-    solve_end(c);
+    if (c->stage_idx == 3) solve_end(c);
     if (extrap) {
         Launch L_(c, KC_MISC, 0.);
         k_hist_post<<<1, 32, 0, c->st>>>(c->dtime, c->stage_x);
@@ -1336,12 +1351,13 @@ template <typename T, int N> struct Impl {
         CK(cudaFuncSetAttribute(k_z_r2c<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_zprod<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_rho<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        CK(cudaFuncSetAttribute(k_z_phi<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        CK(cudaFuncSetAttribute(k_z_phi<T, N, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        CK(cudaFuncSetAttribute(k_z_phi<T, N, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_xfwd_stage<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     }
 
     // distinct inputs and outputs of a launch, each as far as the mode moves it
-    static double job_bytes(kf_ctx *c, int off, int njobs, int mode = AX_FULL) {
+    static double job_bytes(kf_ctx *c, int off, int njobs, int mode, const kf_ctx::Cols &t) {
         std::vector<const void *> u;
         for (int j = 0; j < njobs; ++j) {
             const void *p = c->hj[off + j].in;
@@ -1350,11 +1366,12 @@ template <typename T, int N> struct Impl {
             if (!seen) u.push_back(p);
         }
         double fin = (double)c->Nc, fout = fin;
-        if (mode == AX_XM) fin = c->tr_ball, fout = c->tr_disc;
-        if (mode == AX_YI) fin = c->tr_disc, fout = (double)N * N * c->tr_nkz;
+        if (mode == AX_XM) fin = c->tr_ball, fout = t.cols;
+        if (mode == AX_YI) fin = t.cols, fout = (double)N * N * t.nkz;
         if (mode == AX_XB) fout = (double)c->bx_i * N * NZC;
         if (mode == AX_YB) fin = (double)c->bx_i * N * NZC, fout = (double)c->bx_i * c->bx_j * NZC;
-        if (mode == AX_YF) fin = (double)N * N * c->tr_nkz, fout = c->tr_disc;
+        if (mode == AX_XF) fin = fout = t.cols;
+        if (mode == AX_YF) fin = (double)N * N * t.nkz, fout = t.cols;
         return (u.size() * fin + njobs * fout) * sizeof(T2);
     }
     // resident blocks per SM x SMs of the pipelined pass (its grid)
@@ -1375,7 +1392,8 @@ template <typename T, int N> struct Impl {
         return v;
     }
     // inv: an inverse x pass reads a state field, the forward one a masked intermediate
-    static AxTrunc trunc(kf_ctx *c, int mode, bool inv = true) {
+    static AxTrunc trunc(kf_ctx *c, int mode, bool inv = true, const kf_ctx::Cols *cols = nullptr) {
+        const kf_ctx::Cols &t = cols ? *cols : c->tr;
         AxTrunc A{AX_FULL, NZC, 0.f, nullptr, nullptr, 0, N, NZC, NZC};
         if (mode == AX_XB || mode == AX_YB) {
             A.mode = mode;
@@ -1385,19 +1403,20 @@ template <typename T, int N> struct Impl {
         }
         if (mode == AX_FULL) return A;
         A.mode = mode;
-        A.nkz = c->tr_nkz;
-        A.itpp = 1.f / (float)((c->tr_nkz + TC - 1) / TC);
-        A.jb = c->tr_jb;
-        A.tl = c->tr_tl;
-        A.ip = mode == AX_XM && inv ? NZC : c->tr_mp;
-        A.op = c->tr_mp;
+        A.nkz = t.nkz;
+        A.itpp = 1.f / (float)((t.nkz + TC - 1) / TC);
+        A.jb = t.jb;
+        A.tl = t.tl;
+        A.ip = mode == AX_XM && inv ? NZC : t.mp;
+        A.op = mode == AX_XF ? NZC : t.mp;
         return A;
     }
     // kz extent of a z pass over masked fields
-    static int nkz(kf_ctx *c, bool masked) { return masked ? c->tr_nkz : NZC; }
-    template <int V> static void axis_v(kf_ctx *c, int off, int njobs, int ax, int sign, int mode) {
-        const AxTrunc A = trunc(c, mode);
-        const int ntiles = A.mode == AX_XM ? c->tr_nt
+    static int nkz(kf_ctx *c, bool masked) { return masked ? c->tr.nkz : NZC; }
+    template <int V>
+    static void axis_v(kf_ctx *c, int off, int njobs, int ax, int sign, int mode, const kf_ctx::Cols *cols) {
+        const AxTrunc A = trunc(c, mode, true, cols);
+        const int ntiles = A.mode == AX_XM || A.mode == AX_XF ? (cols ? cols->nt : c->tr.nt)
                            : ax == 0       ? (N * NZC + TC - 1) / TC
                                            : (A.mode == AX_YB ? c->bx_i : N) * ((A.nkz + TC - 1) / TC);
         const int total = njobs * ntiles, grid = std::min(total, pipe_grid<V>(sign));
@@ -1409,12 +1428,14 @@ template <typename T, int N> struct Impl {
             k_axis_pipe<T, N, +1, V><<<grid, TC * PV<V>, smem, c->st>>>(c->dj + off, njobs, ax, geo(c),
                                                                       tw(c), total, A);
     }
-    static void axis(kf_ctx *c, int off, int njobs, int ax, int sign, int mode = AX_FULL) {
-        Launch L_(c, sign > 0 ? KC_AXIS_INV : KC_AXIS_FWD, job_bytes(c, off, njobs, mode));
+    // cols: the active columns of a truncated mode (nullptr: the 2/3 rule's)
+    static void axis(kf_ctx *c, int off, int njobs, int ax, int sign, int mode = AX_FULL,
+                     const kf_ctx::Cols *cols = nullptr) {
+        Launch L_(c, sign > 0 ? KC_AXIS_INV : KC_AXIS_FWD, job_bytes(c, off, njobs, mode, cols ? *cols : c->tr));
         if (c->fftv)
-            axis_v<1>(c, off, njobs, ax, sign, mode);
+            axis_v<1>(c, off, njobs, ax, sign, mode, cols);
         else
-            axis_v<0>(c, off, njobs, ax, sign, mode);
+            axis_v<0>(c, off, njobs, ax, sign, mode, cols);
     }
     static double z_bytes(kf_ctx *c, int off, int njobs, bool c2r, bool masked, int nrows = N * N) {
         std::vector<const void *> u;
@@ -1441,10 +1462,10 @@ template <typename T, int N> struct Impl {
         const T sc = (T)(scale < 0. ? 1. / ((double)N * N * N) : scale);
         if (c->fftv)
             k_z_c2r<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr_mp : NZC);
+                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr.mp : NZC);
         else
             k_z_c2r<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr_mp : NZC);
+                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr.mp : NZC);
     }
     static void zr2c(kf_ctx *c, int off, int njobs) {
         const int nrows = N * N;
@@ -1483,26 +1504,42 @@ template <typename T, int N> struct Impl {
         const int nb = (N * N / 2 + LZ - 1) / LZ;
         const size_t smem = (size_t)LZ * PadLen<N>::value * sizeof(T2);
         const T sc = (T)(1. / ((double)N * N * N));
-        Launch L_(c, KC_RHO, (double)N * N * nkz(c, true) * sizeof(T2) + (double)c->N * (c->rho_cs ? 24 : 16));
+        double *rho = captured_solve(c) && split_on(c, 0) ? nullptr : c->rho;  // then only the split copy is read
+        Launch L_(c, KC_RHO, (double)N * N * nkz(c, true) * sizeof(T2) + (double)c->N * (8 + (rho ? 8 : 0) + (c->rho_cs ? 8 : 0)));
         if (c->fftv)
-            k_z_rho<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, c->rho, c->rho_cs,
-                                                              tw(c), sc, nkz(c, true), c->tr_mp);
+            k_z_rho<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, rho, c->rho_cs,
+                                                              tw(c), sc, nkz(c, true), c->tr.mp);
         else
-            k_z_rho<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, c->rho, c->rho_cs,
-                                                              tw(c), sc, nkz(c, true), c->tr_mp);
+            k_z_rho<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, rho, c->rho_cs,
+                                                              tw(c), sc, nkz(c, true), c->tr.mp);
         CK(cudaGetLastError());
     }
 
-    // CX[8] = z r2c of phi in the bulk precision
-    static void phi_pass(kf_ctx *c) {
+    // phi^ = r2c(phi) in the bulk precision.  With the pressure term phi^ is used
+    // times the filter table PF alone, which underflows to 0 for the larger wave
+    // numbers (kz above 0.4 n/2 in FP32): only the columns where it does not are
+    // formed, and phi^ is not read where it does.
+    static void phi_transform(kf_ctx *c) {
         const int nb = (N * N / 2 + LZ - 1) / LZ;
         const size_t smem = (size_t)LZ * PadLen<N>::value * sizeof(T2);
-        Launch L_(c, KC_Z_R2C, (double)c->N * 8 + (double)c->Nc * sizeof(T2));
-        if (c->fftv)
-            k_z_phi<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>(c->phi, (T2 *)c->CX[8], tw(c), NZC);
-        else
-            k_z_phi<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>(c->phi, (T2 *)c->CX[8], tw(c), NZC);
-        CK(cudaGetLastError());
+        const bool pf = (c->cfg.terms & T_PRESSURE) && c->pf.nkz;
+        const bool sp = captured_solve(c) && split_on(c, 0);  // (solve_end comes with the last stage)
+        const int nko = pf ? c->pf.nkz : NZC, pitch = pf ? c->pf.mp : NZC;
+        const double *phi = sp ? c->phi_cs : c->phi;
+        const int mode = pf ? AX_YF : AX_FULL;
+        {
+            Launch L_(c, KC_Z_R2C, (double)c->N * 8 + (double)N * N * nko * sizeof(T2));
+            auto go = [&](auto k, int threads) {
+                k<<<nb, threads, smem, c->st>>>(phi, (T2 *)c->CX[8], tw(c), nko, pitch);
+            };
+            if (c->fftv)
+                go(sp ? k_z_phi<T, N, 1, true> : k_z_phi<T, N, 1, false>, LZ * PV<1>);
+            else
+                go(sp ? k_z_phi<T, N, 0, true> : k_z_phi<T, N, 0, false>, LZ * PV<0>);
+            CK(cudaGetLastError());
+        }
+        axis(c, c->jB_y, 1, 1, -1, mode, &c->pf);
+        axis(c, c->jB_x, 1, 0, -1, pf ? AX_XF : AX_FULL, &c->pf);
     }
 
     // rounds D (z), E and the z part of F: k_zprod -> CX[0..3]
@@ -1532,9 +1569,9 @@ template <typename T, int N> struct Impl {
         a.scale = (T)(1. / ((double)N * N * N));
         a.terms = c->cfg.terms;
         a.nkz = nkz(c, true);
-        a.ip = c->tr_mp;
+        a.ip = c->tr.mp;
         a.nko = nkz(c, pen);
-        a.op = pen ? c->tr_mp : NZC;
+        a.op = pen ? c->tr.mp : NZC;
         const size_t smem = ZProdSmem<T, N>::bytes;
         Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko) + 5. * a.bi * a.bj * N * sizeof(T));
         if (c->fftv)
@@ -1603,9 +1640,7 @@ template <typename T, int N> struct Impl {
         if (c->capturing && c->capture_wait_u && c->stage_idx == 0)
             CK(cudaStreamWaitEvent(c->st, c->ev_u, cudaEventWaitExternal));
         if (Tm & T_E_INT) {
-            phi_pass(c);
-            axis(c, c->jB_y, 1, 1, -1);
-            axis(c, c->jB_x, 1, 0, -1);
+            phi_transform(c);
         }
         return forked;
     }
@@ -1652,10 +1687,10 @@ template <typename T, int N> struct Impl {
         a.c = (T)c->rk_c;
         a.mode = c->rk_mode;
         const bool act = A.mode == AX_XM;
-        const int ntiles = act ? c->tr_nt : (N * NZC + TC - 1) / TC;
+        const int ntiles = act ? c->tr.nt : (N * NZC + TC - 1) / TC;
         const double use = act ? c->tr_ball : (double)c->Nc;
         const size_t sm = (size_t)N * TC * sizeof(T2);
-        Launch L_(c, KC_XASM, 4. * sizeof(T2) * ((act ? c->tr_disc : use) + use * (a.mode == 3 ? 2 : a.mode == 0 ? 4 : 5)));
+        Launch L_(c, KC_XASM, 4. * sizeof(T2) * ((act ? c->tr.cols : use) + use * (a.mode == 3 ? 2 : a.mode == 0 ? 4 : 5)));
         if (c->fftv)
             k_xfwd_stage<T, N, 1><<<4 * ntiles, TC * PV<1>, sm, c->st>>>(a, geo(c), tw(c), A);
         else
@@ -1981,24 +2016,31 @@ void build_tables(kf_ctx *c) {
         }
     c->q2 = dalloc<double>(c, sizeof(double) * n);
     CK(cudaMemcpy(c->q2, q2.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+    auto cols = [&](const std::vector<int> &pb, kf_ctx::Cols &o) {
+        const int tc = c->fp32 ? Tile<float>::TC : Tile<double>::TC;
+        const TruncTab t = trunc_table(pb, n, tc);
+        o.nkz = t.nkz;
+        o.nt = (int)t.tl.size();
+        o.mp = std::min((t.nkz + tc - 1) / tc * tc, nzc);
+        for (int b : pb) o.cols += b >= 0 ? n : 0;
+        if (!o.nkz) return;
+        o.jb = dalloc<int>(c, sizeof(int) * t.jb.size());
+        o.tl = dalloc<int>(c, sizeof(int) * t.tl.size());
+        CK(cudaMemcpy(o.jb, t.jb.data(), sizeof(int) * t.jb.size(), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(o.tl, t.tl.data(), sizeof(int) * t.tl.size(), cudaMemcpyHostToDevice));
+    };
     {
         const std::vector<int> pb = dealias_bounds(q2, n, dealias_threshold());
         c->pb = dalloc<int>(c, sizeof(int) * pb.size());
         CK(cudaMemcpy(c->pb, pb.data(), sizeof(int) * pb.size(), cudaMemcpyHostToDevice));
-        const TruncTab t = trunc_table(pb, n, c->fp32 ? Tile<float>::TC : Tile<double>::TC);
-        c->tr_nkz = t.nkz;
-        c->tr_nt = (int)t.tl.size();
-        const int tc = c->fp32 ? Tile<float>::TC : Tile<double>::TC;
-        c->tr_mp = std::min((t.nkz + tc - 1) / tc * tc, nzc);
+        cols(pb, c->tr);
         for (int b : pb)
-            if (b >= 0) {
-                c->tr_ball += 2 * b + 1;
-                c->tr_disc += n;
-            }
-        c->tr_jb = dalloc<int>(c, sizeof(int) * t.jb.size());
-        c->tr_tl = dalloc<int>(c, sizeof(int) * t.tl.size());
-        CK(cudaMemcpy(c->tr_jb, t.jb.data(), sizeof(int) * t.jb.size(), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(c->tr_tl, t.tl.data(), sizeof(int) * t.tl.size(), cudaMemcpyHostToDevice));
+            if (b >= 0) c->tr_ball += 2 * b + 1;
+        // PF falls with every |k_d|, so a column's largest value is that of row 0
+        std::vector<int> pf((size_t)n * nzc);
+        for (size_t e = 0; e < pf.size(); ++e)
+            pf[e] = (c->fp32 ? (float)PF[e] != 0.f : PF[e] != 0.) ? 0 : -1;
+        cols(pf, c->pf);
     }
     if (c->fp32) {
         std::vector<float> kvf(n), SVf(c->Nc), PFf(c->Nc);

@@ -24,6 +24,10 @@ class HostPipe {
     static constexpr size_t kPiece = 256 << 10;  // bytes of a pinned piece
     static constexpr size_t kMin = 4 << 20;    // smaller arrays: one plain copy
     static constexpr int kThreads = 8;
+    // Pageable bytes after which the pieces are made: allocating them takes 2 to 5 ms,
+    // about what this many bytes lose by plain copies, so an object that is used
+    // once does not pay for them.
+    static constexpr size_t kAfter = 64 << 20;
 
     HostPipe() = default;
     HostPipe(const HostPipe &) = delete;
@@ -38,7 +42,7 @@ class HostPipe {
     // download's target is complete on return.
     cudaError_t copy(void *dst, const void *src, size_t bytes, bool up, cudaStream_t st) {
         const cudaMemcpyKind kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-        if (bytes < kMin || !pageable(up ? src : dst) || !ready()) return cudaMemcpyAsync(dst, src, bytes, kind, st);
+        if (bytes < kMin || !pageable(up ? src : dst) || !ready(bytes)) return cudaMemcpyAsync(dst, src, bytes, kind, st);
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
@@ -65,6 +69,7 @@ class HostPipe {
   private:
     std::vector<cudaEvent_t> ev_;  // two per thread: its pieces' last transfers
     char *buf_ = nullptr;
+    size_t seen_ = 0;  // pageable bytes asked for so far
 
     static bool pageable(const void *p) {
         cudaPointerAttributes a{};
@@ -75,9 +80,10 @@ class HostPipe {
         return a.type == cudaMemoryTypeUnregistered;
     }
 
-    // The pinned pieces and their events, on first use; false: plain copies.
-    bool ready() {
+    // The pinned pieces and their events, before a copy of `bytes`; false: plain copies.
+    bool ready(size_t bytes) {
         if (buf_) return true;
+        if ((seen_ += bytes) <= kAfter) return false;
         const int nt = std::min(kThreads, (int)std::thread::hardware_concurrency() / 2);
         if (nt < 2) return false;
         if (cudaMallocHost(&buf_, 2 * kPiece * nt) != cudaSuccess) {

@@ -127,6 +127,9 @@ template <typename T> struct AxisTile {
     bool valid;
 };
 
+// min(r, N - r), the |frequency| of row r
+template <int N> __device__ __forceinline__ int row_freq(int r) { return r <= N / 2 ? r : N - r; }
+
 // Tile `tile` of job `job` (global tile index tile * njobs + job), column c.
 template <typename T, int N>
 __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ jobs, int job, int tile, int axis,
@@ -148,6 +151,11 @@ __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ job
             G.obase = j * A.op + kk;
             G.lb = kk < A.nkz ? g.pb[j * nzc + kk] : -1;
             G.valid = G.lb >= 0;
+        } else if (A.mode == AX_XF) {
+            const int w = A.tl[tile], j = w >> 16, kk = (w & 0xffff) + c;
+            G.base = j * A.ip + kk;
+            G.obase = j * A.op + kk;
+            G.valid = kk < A.nkz && row_freq<N>(j) <= A.jb[kk];
         } else {
             G.base = tile * TC + c;
             G.valid = G.base < n * nzc;
@@ -178,9 +186,6 @@ __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ job
     }
     return G;
 }
-
-// min(r, N - r), the |frequency| of row r
-template <int N> __device__ __forceinline__ int row_freq(int r) { return r <= N / 2 ? r : N - r; }
 
 // Resident blocks per SM that the transform kernels ask the register
 // allocator for: as many as their shared memory allows (TILES tiles of
@@ -298,7 +303,8 @@ k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
 #pragma unroll
             for (int q = 0; q < E; ++q) {
                 const int row = reg_row<N, P, PlanV<N, V>::RL>(p, q);
-                const bool st = A.mode >= AX_XB ? (unsigned)(row - A.r0) < (unsigned)A.rm : row_freq<N>(row) <= cur.sb;
+                const bool st = A.mode == AX_XB || A.mode == AX_YB ? (unsigned)(row - A.r0) < (unsigned)A.rm
+                                                                 : row_freq<N>(row) <= cur.sb;
                 if (st) cur.out[cur.obase + row * cur.ostride] = v[q];
             }
         }

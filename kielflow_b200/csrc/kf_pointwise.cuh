@@ -95,8 +95,10 @@ __global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2
     T2 F1 = mk<T2>((T)0, (T)0);
     if (pres || eint) {
         if (eint) {
-            F1 = a.phihat[idx];
-            if (pres) { const T pf = a.PF[idx]; F1.x *= pf; F1.y *= pf; }
+            const T pf = pres ? a.PF[idx] : (T)1;
+            if (pf != (T)0) F1 = a.phihat[idx];  // (not formed where PF is 0)
+            F1.x *= pf;
+            F1.y *= pf;
         }
         if (pres) {
             F1.x += s.x / a.theta;

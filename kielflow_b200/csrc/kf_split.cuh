@@ -31,8 +31,8 @@ __global__ void __launch_bounds__(256) k_unsplit(const double *__restrict__ s, d
     *reinterpret_cast<double2 *>(x + 2 * row) = make_double2(s[c0 * half + row], s[(c0 ^ 1) * half + row]);
 }
 
-// k_guess with the start of the solve in split order (and not in phi, which the
-// solve's end writes): blocks as k_split.
+// k_guess with the start of the solve in split order, from phi or (phi == nullptr)
+// from the last solution in s: blocks as k_split.
 __global__ void __launch_bounds__(256) k_guess_s(const double *__restrict__ phi, double *__restrict__ phi_a,
                                                  double *__restrict__ s, const DevTime *__restrict__ d, double xt,
                                                  int n) {
@@ -41,8 +41,11 @@ __global__ void __launch_bounds__(256) k_guess_s(const double *__restrict__ phi,
     const double t = d->t + xt, ta = d->tau_a, tb = d->tau_b;
     const int nh = d->nhist;
     const int row = (i * n + j) * (n / 2) + k2, half = n * n * (n / 2), c0 = (i + j) & 1;
-    double2 b = *reinterpret_cast<const double2 *>(phi + 2 * row);
-    if (nh != 0 && t != tb) {
+    double2 b = phi ? *reinterpret_cast<const double2 *>(phi + 2 * row)
+                    : make_double2(s[c0 * half + row], s[(c0 ^ 1) * half + row]);
+    const bool newtime = nh != 0 && t != tb;
+    if (!phi && !newtime) return;
+    if (newtime) {
         double2 *pa = reinterpret_cast<double2 *>(phi_a + 2 * row);
         const double2 o = b;
         if (nh >= 2) {

@@ -57,12 +57,10 @@ __global__ void k_sl_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *l0, typen
     T2 F1 = mk<T2>((T)0, (T)0);
     const bool pres = Tm & T_PRESSURE, eint = Tm & T_E_INT;
     if (eint) {
-        F1 = a.phihat[idx];
-        if (pres) {
-            const T pf = a.PF[idx];
-            F1.x *= pf;
-            F1.y *= pf;
-        }
+        const T pf = pres ? a.PF[idx] : (T)1;
+        if (pf != (T)0) F1 = a.phihat[idx];  // (not formed where PF is 0)
+        F1.x *= pf;
+        F1.y *= pf;
     }
     if (pres) {
         F1.x += s.x / a.theta;

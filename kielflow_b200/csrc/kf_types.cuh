@@ -64,6 +64,7 @@ enum AxMode : int {
     AX_YF = 3,    // forward y pass whose x pass needs only active columns: every row -> rows within jb[kz]
     AX_XB = 4,    // x pass of which a window of planes is needed: every row -> rows r0 .. r0 + rm - 1, packed
     AX_YB = 5,    // y pass after AX_XB (rm0 planes): every row -> rows r0 .. r0 + rm - 1, packed
+    AX_XF = 6,    // forward x pass after AX_YF: active columns, every row
 };
 struct AxTrunc {
     int mode;

@@ -183,8 +183,8 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
 // line; ZTile<T>::LZ lines per block, n^2 / (2 LZ) blocks.
 //
 // Inverse, with the Poisson source as the epilogue: s_d = c2r(P s^) and
-// rho = e^{s_d} + n_d in FP64 (rhs_standard.cpp:108-111), into rho and, when
-// given, its colour-split copy (k_split's layout); sd is written when given.
+// rho = e^{s_d} + n_d in FP64 (rhs_standard.cpp:108-111), into rho and its
+// colour-split copy rcs (k_split's layout), each when given; so s_d into sd.
 template <typename T, int N, int V>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
 k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, const double *__restrict__ nd,
@@ -228,8 +228,10 @@ k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, const d
             sd[ia] = sa;
             sd[ib] = sb;
         }
-        rho[ia] = ra;
-        rho[ib] = rb;
+        if (rho) {
+            rho[ia] = ra;
+            rho[ib] = rb;
+        }
         if (rcs) {
             const int c = (c0 + z) & 1;
             rcs[c * half + (ia >> 1)] = ra;
@@ -239,11 +241,11 @@ k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, const d
 }
 
 // Forward, of the FP64 potential in the bulk precision: out = the half spectra
-// of phi's rows, kz < nko.
-template <typename T, int N, int V>
+// of phi's rows, kz < nko, rows of `pitch` elements.  SP: phi in split order.
+template <typename T, int N, int V, bool SP>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
 k_z_phi(const double *__restrict__ phi, typename C2<T>::type *__restrict__ out,
-        const typename C2<T>::type *__restrict__ tw, int nko) {
+        const typename C2<T>::type *__restrict__ tw, int nko, int pitch) {
     typedef typename C2<T>::type T2;
     constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1, LS = PadLen<N>::value;
     extern __shared__ __align__(16) unsigned char kf_smem[];
@@ -255,15 +257,23 @@ k_z_phi(const double *__restrict__ phi, typename C2<T>::type *__restrict__ out,
     T2 v[E];
 #pragma unroll
     for (int q = 0; q < E; ++q) {
-        const long i = (long)r * N + reg_row<N, P, PlanV<N, V>::R1>(p, q);
-        v[q] = r < N * N ? mk<T2>((T)phi[i], (T)phi[i + N]) : mk<T2>((T)0, (T)0);
+        const int z = reg_row<N, P, PlanV<N, V>::R1>(p, q);
+        const long i = (long)r * N + z;
+        if (SP) {
+            constexpr long half = (long)N * N * (N / 2);
+            const int c = (r / N + r % N + z) & 1;  // row r + 1: the other colour
+            v[q] = r < N * N ? mk<T2>((T)phi[c * half + (i >> 1)], (T)phi[(c ^ 1) * half + ((i + N) >> 1)])
+                             : mk<T2>((T)0, (T)0);
+        } else {
+            v[q] = r < N * N ? mk<T2>((T)phi[i], (T)phi[i + N]) : mk<T2>((T)0, (T)0);
+        }
     }
     PlanV<N, V>::template fft<T2, -1>(v, line, pa, p, tw);
 #pragma unroll
     for (int q = 0; q < E; ++q) line[pa(reg_row<N, P, PlanV<N, V>::RL>(p, q))] = v[q];
     __syncwarp();
     if (r >= N * N) return;
-    T2 *oA = out + (long)r * NZC, *oB = oA + NZC;
+    T2 *oA = out + (long)r * pitch, *oB = oA + pitch;
     for (int k = p; k < nko; k += P) {
         const T2 zk = line[pa(k)];
         const T2 zm = line[pa(k == 0 ? 0 : N - k)];

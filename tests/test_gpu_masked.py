@@ -84,3 +84,36 @@ def test_penalization_masks_vs_oracle(kind, prec):
     scale = max(np.abs(x).max() for x in r)
     err = max(np.abs(a - b).max() for a, b in zip(g, r)) / scale
     assert err < (1e-12 if prec == kf.KF_FP64 else 1e-5)
+
+
+@pytest.mark.parametrize("plan", [0, 1])
+@pytest.mark.parametrize("prec", [kf.KF_FP64, kf.KF_FP32_BULK])
+@pytest.mark.parametrize("filtered", [True, False])
+@pytest.mark.parametrize("n", [16, 64, 96, 128])
+def test_given_potential_vs_oracle(n, filtered, prec, plan):
+    """Of phi^ only the columns on which the phi filter is not 0 are formed (with
+    the pressure term, which applies it; all of them without): a white-noise
+    potential, taken as given."""
+    w = C.WORKLOADS["fas128"]
+    terms = kf.KF_T_ALL & ~kf.KF_T_POISSON & (-1 if filtered else ~kf.KF_T_PRESSURE)
+    cfg = C.config_for(w, n=n, precision=prec, terms=terms)
+    nd = I.gauss_charge(n, C.L_BOX, w["Q"], w["sigma"])
+    mask = I.sphere_mask(n, C.L_BOX, 2.0)
+    phi = 1e-2 * np.random.default_rng(n).standard_normal((n, n, n))
+    st = noise_state(n, n)
+    o = bind.Oracle(bind.KfoConfig(*[getattr(cfg, f) for f, _ in bind.KfoConfig._fields_]))
+    o.set_phi(phi)
+    o.set_state(st)
+    o.set_sources(nd, mask)
+    o.rhs()
+    r = o.get_state()
+    with kf.Context(cfg) as ctx:
+        ctx.set_tuning(plan, 8)
+        ctx.set_state(*st)
+        ctx.set_sources(nd, mask)
+        ctx.set_phi(phi)
+        ctx.rhs()
+        g = ctx.get_state()
+    scale = max(np.abs(x).max() for x in r)
+    err = max(np.abs(a - b).max() for a, b in zip(g, r)) / scale
+    assert err < (1e-12 if prec == kf.KF_FP64 else 1e-5)
