@@ -39,7 +39,7 @@ __global__ void k_accumulate4(const double *__restrict__ part, int nb, double *_
     acc[q] = __dadd_rn(acc[q], s);
 }
 
-// Transpose of the physical-space part of the right-hand side (k_products).
+// Transpose of the physical-space part of the right-hand side (k_zprod).
 //   pen: f_q = (1-H)(rl_q - pr_q) + H eta (qd_q - qfix_q), qd = (U, s_d), qfix_x = -M
 //   no pen: the products enter K through -r2c, fb_q carries c2r_u(Kbar_q / w)
 // Outputs the cotangents of U_c, dU[c][d], ds[d], s_d (penalization part), rl_q

@@ -148,11 +148,10 @@ struct kf_ctx {
     // sine-stretched axes: the chain-rule right-hand side's buffers, metric
     // tables and job lists (allocated only when cfg.stretch_m != 0)
     bool stretched = false;
-    void *SX[15] = {};
+    void *SX[12] = {};
     void *met = nullptr;    // filtered 1/dS per index (bulk precision)
     double *vol = nullptr;  // dS per index (cell widths / h) for the diagnostics
-    int jS_Dx = 0, jS_Dy = 0, zS_D = 0, zS_F = 0, jS_Fy = 0, jS_Fx = 0, jS_Gx = 0, jS_Gy = 0, zS_G = 0;
-    int zS_I = 0, jS_Iy = 0, jS_Ix = 0, jS_Kx = 0, jS_Ky = 0, zS_K = 0, zS_Kf = 0, jS_Kfy = 0, jS_Kfx = 0;
+    int jS_Dx = 0, jS_Dy = 0, zS_D = 0, zS_F = 0, jS_Fy = 0, jS_Gx = 0, jS_Gy = 0, zS_G = 0;
     // Jacobi state carried between solves (solver_poisson_jacobi_nlin.hpp:66-95)
     double norm_max = 0., norm_sum = 0.;
     JacState *d_js = nullptr, *h_js = nullptr;  // two on the device, taken in turn by the sweeps
@@ -256,7 +255,7 @@ enum KCls { KC_AXIS_INV, KC_AXIS_FWD, KC_Z_C2R, KC_Z_R2C, KC_XASM, KC_PROD, KC_L
             KC_MG_COARSE, KC_MARCH, KC_MARCH_RES,
             KC_N };
 const char *const kKClsName[KC_N] = {"k_axis_pass(inverse)", "k_axis_pass(forward)", "k_z_c2r", "k_z_r2c",
-                                     "k_xfwd_stage", "k_zprod/k_products", "k_lin", "k_rho", "k_rk", "k_jacobi",
+                                     "k_xfwd_stage", "k_zprod/k_sl_products", "k_lin", "k_rho", "-", "k_jacobi",
                                      "k_rbgs", "k_residual", "k_restrict/k_fas_rhs/k_prolong/k_inject",
                                      "k_coarse_solve/k_cc", "-", "conversion/diagnostics",
                                      "adjoint pointwise (k_prod_vjp/k_vjp_assemble/k_adj_stage/...)",
@@ -1354,6 +1353,7 @@ template <typename T, int N> struct Impl {
         CK(cudaFuncSetAttribute(k_z_phi<T, N, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_phi<T, N, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_xfwd_stage<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        CK(cudaFuncSetAttribute(k_x_filter<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     }
 
     // distinct inputs and outputs of a launch, each as far as the mode moves it
@@ -1467,15 +1467,17 @@ template <typename T, int N> struct Impl {
             k_z_c2r<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
                                                                         tw(c), sc, nkz(c, masked), masked ? c->tr.mp : NZC);
     }
-    static void zr2c(kf_ctx *c, int off, int njobs) {
+    // masked: only the rows' kept part, in rows of whole tiles
+    static void zr2c(kf_ctx *c, int off, int njobs, bool masked = false) {
+        const int pitch = masked ? c->tr.mp : NZC;
         const int nrows = N * N;
         const int ntiles = (nrows + LZ - 1) / LZ;
         const size_t smem = ZSmem<T, N, false>::bytes;
-        Launch L_(c, KC_Z_R2C, z_bytes(c, off, njobs, false, false));
+        Launch L_(c, KC_Z_R2C, z_bytes(c, off, njobs, false, masked));
         if (c->fftv)
-            k_z_r2c<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c));
+            k_z_r2c<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c), pitch);
         else
-            k_z_r2c<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c));
+            k_z_r2c<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, tw(c), pitch);
     }
     static RhsArgs<T> rargs(kf_ctx *c) {
         RhsArgs<T> a;
@@ -1700,16 +1702,19 @@ template <typename T, int N> struct Impl {
 
     // The right-hand side on sine-stretched axes: every derivative takes the
     // chain-rule path D_d F = r2c(m_d c2r(P i k_d F)) of
-    // OP_partial_derivative.cpp:104-136, so the derivative terms that
-    // rhs() folds into k-space become transform pairs:
+    // OP_partial_derivative.cpp:104-136.  What the right-hand side adds of them as
+    // they are it adds in physical space, to the products, and transforms once:
     //   C' linear parts, F1                 D' raw derivatives (15 c2r)
-    //   E' times the metric                 F' their r2c (15)
-    //   G' c2r(P D_d u'_c), c2r(P D_d s)    H' products (rhs_standard.cpp:323-436)
-    //   I' r2c of the products              J' assembly
-    //   K' penalization of the finished right-hand side, then the 2/3 filter
+    //   E' times the metric; sums S_q       c2r(-lin_q) on the mask's window
+    //   G' c2r(P D_d u'_c), c2r(P D_d s): 12 fields forward and back, filtered
+    //   H' S_q + products (rhs_standard.cpp:323-436), penalization
+    //   then the end of F, as rhs()
+    // (15 + 4 forward transforms of derivatives and products, their assembly in
+    // k-space and the penalization of the assembled right-hand side through
+    // another 4 back and forth before.)
     static void rhs_stretched(kf_ctx *c) {
         const int Tm = c->cfg.terms;
-        const bool pen = Tm & T_PENALIZATION;
+        const bool pen = Tm & T_PENALIZATION, win = pen && c->bx_i;
         const long Nc = c->Nc, Nr = c->N;
         const double cb = (double)Nc * sizeof(T2), rb = (double)Nr * sizeof(T);
         rounds_AB(c, false, pen);
@@ -1724,83 +1729,66 @@ template <typename T, int N> struct Impl {
         zc2r(c, c->zS_D, 10, true);
         {  // E'
             ScaleArgs<T> sa;
-            for (int j = 0; j < 15; ++j) sa.f[j] = (T *)c->R[4 + j];
+            for (int j = 0; j < 12; ++j) sa.f[j] = (T *)c->R[4 + j];
+            for (int j = 0; j < 3; ++j) sa.F1[j] = (const T *)c->R[16 + j];
+            for (int j = 0; j < 4; ++j) sa.S[j] = (T *)c->R[20 + j];
             sa.met = (const T *)c->met;
+            sa.M = (T)c->cfg.M;
+            sa.terms = Tm;
             sa.n = c->n;
             sa.N = Nr;
-            Launch L_(c, KC_PROD, 30. * rb);
+            Launch L_(c, KC_PROD, 31. * rb);
             k_sl_scale<T><<<nblk(Nr, 256), 256, 0, c->st>>>(sa);
         }
-        // F'
-        zr2c(c, c->zS_F, 8);
-        axis(c, c->jS_Fy, 15, 1, -1);
-        axis(c, c->jS_Fx, 15, 0, -1);
-        const bool prod = Tm & (T_ADVECTION | T_CONTINUITY);
-        if (prod) {
-            // G'
-            axis(c, c->jS_Gx, 12, 0, +1, AX_XM);
+        if (win) {
+            axis(c, c->jD_x + 6, 4, 0, +1, AX_XB);
+            axis(c, c->jD_y + 9, 4, 1, +1, AX_YB);
+            zc2r(c, c->zD + 8, 2, false, -1., c->bx_i * c->bx_j);
+        }
+        if (Tm & (T_ADVECTION | T_CONTINUITY)) {  // G'
+            zr2c(c, c->zS_F, 6, true);
+            axis(c, c->jS_Fy, 12, 1, -1, AX_YF);
+            x_filter(c, c->jS_Gx, 12);
             axis(c, c->jS_Gy, 12, 1, +1, AX_YI);
             zc2r(c, c->zS_G, 6, true);
-            {  // H'
-                ProdArgs<T> pa{};
-                for (int q = 0; q < 3; ++q) {
-                    pa.U[q] = (const T *)c->R[1 + q];
-                    pa.ds[q] = (const T *)c->R[13 + q];
-                    for (int d = 0; d < 3; ++d) pa.dU[q][d] = (const T *)c->R[4 + 3 * q + d];
-                }
-                for (int q = 0; q < 4; ++q) pa.out[q] = (T *)c->R[20 + q];
-                pa.M = (T)c->cfg.M;
-                pa.terms = Tm & (T_ADVECTION | T_CONTINUITY);
-                pa.N = Nr;
-                Launch L_(c, KC_PROD, 19. * rb);
-                k_products<T><<<nblk(Nr, 256), 256, 0, c->st>>>(pa);
-            }
-            // I'
-            zr2c(c, c->zS_I, 2);
-            axis(c, c->jS_Iy, 4, 1, -1);
-            axis(c, c->jS_Ix, 4, 0, -1);
         }
-        {  // J'
-            AsmArgs<T> aa;
+        {  // H'
+            SlProdArgs<T> pa{};
+            for (int q = 0; q < 3; ++q) {
+                pa.U[q] = (const T *)c->R[1 + q];
+                pa.ds[q] = (const T *)c->R[13 + q];
+                for (int d = 0; d < 3; ++d) pa.dU[q][d] = (const T *)c->R[4 + 3 * q + d];
+            }
             for (int q = 0; q < 4; ++q) {
-                aa.lin[q] = (const T2 *)c->LIN[q];
-                aa.pr[q] = prod ? (const T2 *)c->SX[8 + q] : nullptr;
-                aa.K[q] = (T2 *)c->K[q];
+                pa.out[q] = (T *)c->R[20 + q];
+                pa.rl[q] = (const T *)c->R[16 + q];
             }
-            for (int j = 0; j < 15; ++j) aa.dn[j] = (const T2 *)c->CY[j];
-            aa.M = (T)c->cfg.M;
-            aa.terms = Tm;
-            aa.Nc = Nc;
-            Launch L_(c, KC_XASM, 27 * cb);
-            k_sl_assemble<T><<<nblk(Nc, 256), 256, 0, c->st>>>(aa);
+            pa.sd = (const T *)c->R[0];
+            pa.H = (const T *)c->H;
+            pa.M = (T)c->cfg.M;
+            pa.eta = (T)c->cfg.pen_eta;
+            pa.i0 = c->bx_i0;
+            pa.bi = win ? c->bx_i : 0;
+            pa.j0 = c->bx_j0;
+            pa.bj = c->bx_j;
+            pa.terms = Tm;
+            pa.n = c->n;
+            pa.N = Nr;
+            Launch L_(c, KC_PROD, 23. * rb);
+            k_sl_products<T><<<nblk(Nr, 256), 256, 0, c->st>>>(pa);
         }
-        if (pen) {  // K'
-            axis(c, c->jS_Kx, 4, 0, +1);
-            axis(c, c->jS_Ky, 4, 1, +1);
-            zc2r(c, c->zS_K, 2);
-            {
-                ProdArgs<T> pa{};
-                for (int q = 0; q < 3; ++q) pa.U[q] = (const T *)c->R[1 + q];
-                for (int q = 0; q < 4; ++q) {
-                    pa.rl[q] = (const T *)c->R[20 + q];
-                    pa.out[q] = (T *)c->R[20 + q];
-                }
-                pa.sd = (const T *)c->R[0];
-                pa.H = (const T *)c->H;
-                pa.M = (T)c->cfg.M;
-                pa.eta = (T)c->cfg.pen_eta;
-                pa.terms = T_PENALIZATION;
-                pa.N = Nr;
-                Launch L_(c, KC_PROD, 13. * rb);
-                k_products<T><<<nblk(Nr, 256), 256, 0, c->st>>>(pa);
-            }
-            zr2c(c, c->zS_Kf, 2);
-            axis(c, c->jS_Kfy, 4, 1, -1);
-            axis(c, c->jS_Kfx, 4, 0, -1);
-            Launch L_(c, KC_MISC, 8 * cb);
-            k_sl_dealias4<T><<<nblk(Nc, 256), 256, 0, c->st>>>(geo(c), (T2 *)c->K[0], (T2 *)c->K[1],
-                                                                 (T2 *)c->K[2], (T2 *)c->K[3]);
-        }
+        zr2c(c, c->zF, 2, pen);
+        axis(c, c->jF_y, 4, 1, -1, pen ? AX_YF : AX_FULL);
+        stage(c, pen);
+    }
+    static void x_filter(kf_ctx *c, int off, int njobs) {
+        const AxTrunc A = trunc(c, AX_XM, false);
+        const size_t sm = (size_t)N * TC * sizeof(T2);
+        Launch L_(c, KC_AXIS_INV, 2. * njobs * c->tr.cols * sizeof(T2));
+        if (c->fftv)
+            k_x_filter<T, N, 1><<<njobs * c->tr.nt, TC * PV<1>, sm, c->st>>>(c->dj + off, njobs, geo(c), tw(c), A);
+        else
+            k_x_filter<T, N, 0><<<njobs * c->tr.nt, TC * PV<0>, sm, c->st>>>(c->dj + off, njobs, geo(c), tw(c), A);
         CK(cudaGetLastError());
     }
 
@@ -2353,44 +2341,17 @@ void build_jobs(kf_ctx *c) {
         zj(CY[0], MUL_IK, nullptr, 0, R[15], nullptr);
         zj(CY[14], MUL_NONE, CY[13], MUL_NONE, R[16], R[17]);
         zj(CY[12], MUL_IK, nullptr, 0, R[18], nullptr);
-        // F': r2c of the 15 scaled derivatives R[4..18] -> CY[0..14]
+        // G': the 12 scaled derivatives R[4..15], filtered (k_x_filter between the y passes)
         c->zS_F = (int)Z.size();
-        for (int j = 0; j < 14; j += 2) zj(R[4 + j], 0, R[5 + j], 0, CY[j], CY[j + 1]);
-        zj(R[18], 0, nullptr, 0, CY[14], nullptr);
+        for (int j = 0; j < 12; j += 2) zj(R[4 + j], 0, R[5 + j], 0, CY[j], CY[j + 1]);
         c->jS_Fy = (int)J.size();
-        for (int j = 0; j < 15; ++j) aj(CY[j], SX[j], MUL_NONE);
-        c->jS_Fx = (int)J.size();
-        for (int j = 0; j < 15; ++j) aj(SX[j], CY[j], MUL_NONE);
-        // G': c2r(P D_d u'_c), c2r(P D_d s) -> R[4..15] (the products' operands)
+        for (int j = 0; j < 12; ++j) aj(CY[j], SX[j], MUL_NONE);
         c->jS_Gx = (int)J.size();
-        for (int j = 0; j < 12; ++j) aj(CY[j], SX[j], MUL_P);
+        for (int j = 0; j < 12; ++j) aj(SX[j], CY[j], MUL_NONE);
         c->jS_Gy = (int)J.size();
-        for (int j = 0; j < 12; ++j) aj(SX[j], CX[j], MUL_NONE);
+        for (int j = 0; j < 12; ++j) aj(CY[j], SX[j], MUL_NONE);
         c->zS_G = (int)Z.size();
-        for (int j = 0; j < 12; j += 2) zj(CX[j], MUL_NONE, CX[j + 1], MUL_NONE, R[4 + j], R[5 + j]);
-        // I': r2c of the products R[20..23] -> SX[8..11]
-        c->zS_I = (int)Z.size();
-        zj(R[20], 0, R[21], 0, SX[0], SX[1]);
-        zj(R[22], 0, R[23], 0, SX[2], SX[3]);
-        c->jS_Iy = (int)J.size();
-        for (int q = 0; q < 4; ++q) aj(SX[q], SX[4 + q], MUL_NONE);
-        c->jS_Ix = (int)J.size();
-        for (int q = 0; q < 4; ++q) aj(SX[4 + q], SX[8 + q], MUL_NONE);
-        // K': penalization, K -> R[20..23] -> K
-        c->jS_Kx = (int)J.size();
-        for (int q = 0; q < 4; ++q) aj(c->K[q], SX[q], MUL_NONE);
-        c->jS_Ky = (int)J.size();
-        for (int q = 0; q < 4; ++q) aj(SX[q], SX[4 + q], MUL_NONE);
-        c->zS_K = (int)Z.size();
-        zj(SX[4], MUL_NONE, SX[5], MUL_NONE, R[20], R[21]);
-        zj(SX[6], MUL_NONE, SX[7], MUL_NONE, R[22], R[23]);
-        c->zS_Kf = (int)Z.size();
-        zj(R[20], 0, R[21], 0, SX[0], SX[1]);
-        zj(R[22], 0, R[23], 0, SX[2], SX[3]);
-        c->jS_Kfy = (int)J.size();
-        for (int q = 0; q < 4; ++q) aj(SX[q], SX[4 + q], MUL_NONE);
-        c->jS_Kfx = (int)J.size();
-        for (int q = 0; q < 4; ++q) aj(SX[4 + q], c->K[q], MUL_NONE);
+        for (int j = 0; j < 12; j += 2) zj(SX[j], MUL_NONE, SX[j + 1], MUL_NONE, R[4 + j], R[5 + j]);
     }
     c->hj = J;
     c->hz = Z;
@@ -2444,7 +2405,7 @@ void create(kf_ctx *c) {
     for (int i = 0; i < 16; ++i) c->CY[i] = dalloc<void>(c, cb);
     for (int i = 0; i < 24; ++i) c->R[i] = dalloc<void>(c, rb);
     if (c->stretched)
-        for (int i = 0; i < 15; ++i) c->SX[i] = dalloc<void>(c, cb);
+        for (int i = 0; i < 12; ++i) c->SX[i] = dalloc<void>(c, cb);
     c->phihat = dalloc<void>(c, cb);
     c->phi = dalloc<double>(c, 8 * c->N);
     c->rho = dalloc<double>(c, 8 * c->N);
@@ -2522,14 +2483,8 @@ void copy_state(kf_ctx *c, void *const *dst, void *const *src) {
 }
 
 // One stage: the right-hand side of Ys and the stage's combination, in the
-// right-hand side's last kernel or (stretched axes) in k_rk on its K.
-void rk_launch(kf_ctx *c, double cdt, int mode);
+// right-hand side's last kernel.
 void rk_stage(kf_ctx *c, double cdt, int mode) {
-    if (c->stretched) {
-        c->rhs_fn(c);
-        rk_launch(c, cdt, mode);
-        return;
-    }
     c->rk_mode = mode;
     c->rk_c = cdt;
     try {
@@ -2539,20 +2494,6 @@ void rk_stage(kf_ctx *c, double cdt, int mode) {
         throw;
     }
     c->rk_mode = 3;
-}
-
-void rk_launch(kf_ctx *c, double cdt, int mode) {
-    const long M = c->Nc;
-    for (int q = 0; q < 4; ++q) {
-        Launch L_(c, KC_RK, (double)M * c->cs * (mode == 1 ? 5 : 4));
-        if (c->fp32)
-            k_rk<float><<<nblk(M, 256), 256, 0, c->st>>>((float2 *)c->Y[q], (float2 *)c->ACC[q], (float2 *)c->Ys[q],
-                                                        (const float2 *)c->K[q], (float)cdt, mode, M);
-        else
-            k_rk<double><<<nblk(M, 256), 256, 0, c->st>>>((double2 *)c->Y[q], (double2 *)c->ACC[q], (double2 *)c->Ys[q],
-                                                         (const double2 *)c->K[q], cdt, mode, M);
-    }
-    CK(cudaGetLastError());
 }
 
 // One RK4 step (RKO4.cpp:105-238) on Y (== Ys on entry).  Optional hooks of
@@ -2578,7 +2519,6 @@ void rk4_step(kf_ctx *c, double dt, void *const *X, double *const *PH, double *c
         c->phi_given = false;
         if (PH) CK(cudaMemcpyAsync(PH[i], c->phi, 8 * c->N, cudaMemcpyDeviceToDevice, c->st));
     }
-    if (c->stretched) copy_state(c, c->Ys, c->Y);
     c->t = t0 + dt;
 }
 
@@ -2635,7 +2575,6 @@ void capture_step(kf_ctx *c, double dt, bool wait_u, cudaGraphExec_t *out) {
             c->stage_x = xs[i];
             rk_stage(c, cdt[i], mode[i]);
         }
-        if (c->stretched) copy_state(c, c->Ys, c->Y);
         {
             Launch L_(c, KC_MISC, 0.);
             k_time<<<1, 32, 0, c->st>>>(c->dtime, dt, 1);

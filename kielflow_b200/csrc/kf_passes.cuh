@@ -435,9 +435,9 @@ k_z_c2r(const ZJob *__restrict__ jobs, int njobs, int nrows, Geo<T> g,
 template <typename T, int N, int V = 0>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
 k_z_r2c(const ZJob *__restrict__ jobs, int njobs, int nrows,
-        const typename C2<T>::type *__restrict__ tw) {
+        const typename C2<T>::type *__restrict__ tw, int pitch) {
     typedef typename C2<T>::type T2;
-    constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1;
+    constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P;
     constexpr int LS = PadLen<N>::value;
     extern __shared__ __align__(16) unsigned char kf_smem[];
     T2 *xch = reinterpret_cast<T2 *>(kf_smem);  // [LZ][LS], padded lines
@@ -465,13 +465,13 @@ k_z_r2c(const ZJob *__restrict__ jobs, int njobs, int nrows,
 #pragma unroll
     for (int q = 0; q < E; ++q) line[pa(reg_row<N, P, PlanV<N, V>::RL>(p, q))] = v[q];
     __syncthreads();
-    const int lim = (nrows - r0) * NZC;
-    T2 *oA = static_cast<T2 *>(J.outA) + (long)r0 * NZC;
-    T2 *oB = J.outB ? static_cast<T2 *>(J.outB) + (long)r0 * NZC : nullptr;
-    // the tile's LZ output rows of a half spectrum are one contiguous run of
-    // LZ * NZC elements from row r0
-    for (int idx = threadIdx.x; idx < LZ * NZC && idx < lim; idx += blockDim.x) {
-        const int ll = idx / NZC, k = idx - ll * NZC;
+    const int lim = (nrows - r0) * pitch;
+    T2 *oA = static_cast<T2 *>(J.outA) + (long)r0 * pitch;
+    T2 *oB = J.outB ? static_cast<T2 *>(J.outB) + (long)r0 * pitch : nullptr;
+    // the tile's LZ output rows of `pitch` elements (of NZC) are one contiguous run
+    // from row r0
+    for (int idx = threadIdx.x; idx < LZ * pitch && idx < lim; idx += blockDim.x) {
+        const int ll = idx / pitch, k = idx - ll * pitch;
         const T2 zk = xch[ll * LS + pa(k)];
         const T2 zm = xch[ll * LS + pa(k == 0 ? 0 : N - k)];
         const T cr = zm.x, ci = -zm.y;  // conj(Z[N-k])

@@ -12,7 +12,7 @@
 
 namespace kf {
 
-// Linear spectral parts of FBuffer (no derivative; rhs_standard.cpp:119-140
+// -1 x the linear spectral parts of FBuffer (no derivative; rhs_standard.cpp:119-140
 // and the added diffusion) and the potential of the E-force/pressure term
 // F1 = PF phi^ + s^/theta (rhs_standard.cpp:218-240), one thread per
 // half-spectrum element.  Same order of operations as lin_term.
@@ -41,7 +41,7 @@ __global__ void k_sl_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *l0, typen
             fb.x += a.D * k2 * u.x;
             fb.y += a.D * k2 * u.y;
         }
-        o[q][idx] = fb;
+        o[q][idx] = mk<T2>(-fb.x, -fb.y);
     }
     const T2 s = a.Y[3][idx];
     {
@@ -52,7 +52,7 @@ __global__ void k_sl_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *l0, typen
             fb.x += a.D * k2 * s.x;
             fb.y += a.D * k2 * s.y;
         }
-        l3[idx] = fb;
+        l3[idx] = mk<T2>(-fb.x, -fb.y);
     }
     T2 F1 = mk<T2>((T)0, (T)0);
     const bool pres = Tm & T_PRESSURE, eint = Tm & T_E_INT;
@@ -69,112 +69,148 @@ __global__ void k_sl_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *l0, typen
     F1o[idx] = F1;
 }
 
-// The raw derivatives c2r(P i k_d F) times the metric of their direction, in
-// place (OP_partial_derivative.cpp:125-127).  f[j] is a derivative along axis
-// j % 3 (j = 3c + d for d_d u'_c, 9 + d for d_d s, 12 + d for d_d F1).
+// The raw derivatives c2r(P i k_d F) times the metric of their direction
+// (OP_partial_derivative.cpp:125-127): f[j] along axis j % 3 (j = 3c + d for
+// d_d u'_c, 9 + d for d_d s) in place, as the products want them projected once
+// more; and what the right-hand side adds of them as they are, before its one
+// transform of the sum (rhs_standard.cpp:218-319):
+//   S_c = D_c F1 + M D_x u'_c        S_3 = M D_x s + D_x u'_x + D_y u'_y + D_z u'_z
+// Memory-bound: 15 fields in, 16 out.
 template <typename T> struct ScaleArgs {
-    T *f[15];
-    const T *met;
-    int n;
+    T *f[12], *S[4];
+    const T *F1[3], *met;
+    T M;
+    int n, terms;
     long N;
 };
 
 template <typename T>
-__global__ void k_sl_scale(ScaleArgs<T> a) {
+__global__ void __launch_bounds__(256) k_sl_scale(ScaleArgs<T> a) {
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= a.N) return;
     const int k = (int)(idx % a.n);
     const long r = idx / a.n;
     const int j = (int)(r % a.n), i = (int)(r / a.n);
     const T m[3] = {a.met[i], a.met[j], a.met[k]};
+    const bool force = a.terms & (T_PRESSURE | T_E_INT), ext = a.terms & T_E_EXT;
+    T f[12], F1[3];
 #pragma unroll
-    for (int q = 0; q < 15; ++q) a.f[q][idx] = a.f[q][idx] * m[q % 3];
+    for (int q = 0; q < 12; ++q) f[q] = a.f[q][idx];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) F1[q] = force ? a.F1[q][idx] : (T)0;
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+        f[q] *= m[q % 3];
+        a.f[q][idx] = f[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) a.S[q][idx] = F1[q] * m[q] + (ext ? a.M * f[3 * q] : (T)0);
+    T s = ext ? a.M * f[9] : (T)0;
+    if (a.terms & T_CONTINUITY) s += f[0] + f[4] + f[8];
+    a.S[3][idx] = s;
 }
 
-// Assembly of the right-hand side from the linear parts, the chain-rule
-// derivatives dn[j] (spectral, numbered as ScaleArgs) and the transformed
-// products pr (advection, continuity), in the reference's order of
-// accumulation (rhs_standard.cpp:119-439) and sign (:538-560):
-//   u_c: lin_c + D_c F1 + M D_x u'_c + r2c(u . grad u_c)
-//   s  : lin_s + M D_x s + D_x u'_x + D_y u'_y + D_z u'_z + r2c(u . grad s)
-template <typename T> struct AsmArgs {
-    typedef typename C2<T>::type T2;
-    const T2 *lin[4];
-    const T2 *dn[15];
-    const T2 *pr[4];  // nullptr without advection and continuity
-    T2 *K[4];
-    T M;
-    int terms;
-    long Nc;
+// The physical part of the right-hand side, out_q (S_q on entry) ->
+//   t_c = S_c + u.grad u_c, t_3 = S_3 + u.grad s   (rhs_standard.cpp:323-436)
+// as -t_q or, where the mask H is not zero (on the window of rows that bounds it,
+// with l_q = c2r(-lin_q) there), the masking form (effect_penalization.cpp:35)
+//   (1-H)(l_q - t_q) + H eta (q_d - q_fix) - l_q,  q_fix = (-M, 0, 0, -10),
+// so that the right-hand side is -lin_q plus the transform of out_q.
+template <typename T> struct SlProdArgs {
+    const T *U[3], *dU[3][3], *ds[3];  // dU[c][d] = D_d U_c, ds[d] = D_d s
+    const T *sd, *H, *rl[4];           // penalization: c2r(P s^), the mask, l_q on the window
+    T *out[4];
+    T M, eta;
+    int i0, bi, j0, bj, terms, n;
+    long N;
 };
 
 template <typename T>
-__global__ void k_sl_assemble(AsmArgs<T> a) {
-    typedef typename C2<T>::type T2;
+__global__ void __launch_bounds__(256) k_sl_products(SlProdArgs<T> a) {
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= a.Nc) return;
-    const int Tm = a.terms;
-    const bool force = (Tm & T_PRESSURE) || (Tm & T_E_INT);
+    if (idx >= a.N) return;
+    const bool adv = a.terms & T_ADVECTION, cont = a.terms & T_CONTINUITY;
+    T t[4];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        T2 fb = a.lin[q][idx];
-        if (force) {
-            const T2 d = a.dn[12 + q][idx];
-            fb.x += d.x;
-            fb.y += d.y;
-        }
-        if (Tm & T_E_EXT) {
-            const T2 d = a.dn[3 * q][idx];
-            fb.x += a.M * d.x;
-            fb.y += a.M * d.y;
-        }
-        if (Tm & T_ADVECTION) {
-            const T2 d = a.pr[q][idx];
-            fb.x += d.x;
-            fb.y += d.y;
-        }
-        a.K[q][idx] = mk<T2>(-fb.x, -fb.y);
+    for (int q = 0; q < 4; ++q) t[q] = a.out[q][idx];
+    const int row = (int)(idx / a.n), bi = row / a.n - a.i0, bj = row % a.n - a.j0;
+    const bool box = (unsigned)bi < (unsigned)a.bi && (unsigned)bj < (unsigned)a.bj;
+    const T h = box ? a.H[idx] : (T)0;
+    T u[3] = {};
+    if (adv || cont || h != (T)0) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) u[d] = a.U[d][idx];
     }
-    T2 fb = a.lin[3][idx];
-    if (Tm & T_E_EXT) {
-        const T2 d = a.dn[9][idx];
-        fb.x += a.M * d.x;
-        fb.y += a.M * d.y;
-    }
-    if (Tm & T_CONTINUITY) {
+    if (adv) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const T2 d = a.dn[4 * c][idx];  // d_c u'_c
-            fb.x += d.x;
-            fb.y += d.y;
+            T s = u[0] * a.dU[c][0][idx];
+            s += u[1] * a.dU[c][1][idx];
+            s += u[2] * a.dU[c][2][idx];
+            t[c] += s;
         }
-        const T2 d = a.pr[3][idx];
-        fb.x += d.x;
-        fb.y += d.y;
     }
-    a.K[3][idx] = mk<T2>(-fb.x, -fb.y);
+    if (cont) {
+        T s = a.ds[0][idx] * u[0];
+        s += a.ds[1][idx] * u[1];
+        s += a.ds[2][idx] * u[2];
+        t[3] += s;
+    }
+    if (h != (T)0) {
+        const T qd[4] = {u[0], u[1], u[2], a.sd[idx]};
+        const T qfix[4] = {-a.M, (T)0, (T)0, (T)-10};
+        const long w = ((long)bi * a.bj + bj) * a.n + idx % a.n;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const T l = a.rl[q][w], r = l - t[q];
+            a.out[q][idx] = (((T)1 - h) * r + h * a.eta * (qd[q] - qfix[q])) - l;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a.out[q][idx] = -t[q];
+    }
 }
 
-// The 2/3 filter (OP_dealiasing.cpp:5-13) on four half spectra.
-template <typename T>
-__global__ void k_sl_dealias4(Geo<T> g, typename C2<T>::type *K0, typename C2<T>::type *K1,
-                              typename C2<T>::type *K2, typename C2<T>::type *K3) {
+// The 2/3 filter between the two x passes of P r2c(m c2r(..)): one block takes an
+// active column tile of one field through the forward transform, drops what the
+// rule does not keep and transforms back, so the spectrum itself is never stored.
+template <typename T, int N, int V = 0>
+__global__ void __launch_bounds__(Tile<T>::TC * PlanV<N, V>::P,
+                                  PipeMinBlocks<T, N, V, 1, sizeof(T) == 4 ? 4 : 2, 64>::value)
+k_x_filter(const AxisJob *__restrict__ jobs, int njobs, Geo<T> g, const typename C2<T>::type *__restrict__ tw,
+           AxTrunc A) {
     typedef typename C2<T>::type T2;
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long Nc = (long)g.n * g.n * g.nzc;
-    if (idx >= Nc) return;
-    const int k = (int)(idx % g.nzc);
-    const long r = idx / g.nzc;
-    const int j = (int)(r % g.n), i = (int)(r / g.n);
-    const T f = dealias_keep(g.q2, g.thr, i, j, k) ? (T)1 : (T)0;
-    T2 *o[4] = {K0, K1, K2, K3};
+    constexpr int TC = Tile<T>::TC, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1;
+    extern __shared__ __align__(16) unsigned char kf_smem[];
+    T2 *sm = reinterpret_cast<T2 *>(kf_smem);
+    const AxisJob J = jobs[blockIdx.x % njobs];
+    const int w = A.tl[blockIdx.x / njobs];
+    const int c = threadIdx.x % TC, p = threadIdx.x / TC;
+    const int kk = (w & 0xffff) + c, col = (w >> 16) * A.op + kk, rs = N * A.op;
+    const int b = kk < A.nkz ? g.pb[(w >> 16) * NZC + kk] : -1;
+    const T2 *in = static_cast<const T2 *>(J.in);
+    T2 v[E];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        T2 x = o[q][idx];
-        x.x *= f;
-        x.y *= f;
-        o[q][idx] = x;
+    for (int e = 0; e < E; ++e) {
+        const int row = reg_row<N, P, PlanV<N, V>::R1>(p, e);
+        v[e] = b >= 0 ? in[col + row * rs] : mk<T2>((T)0, (T)0);
     }
+    PlanV<N, V>::template fft<T2, -1>(v, sm + c, StrideAddr{TC}, p, tw);
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int row = reg_row<N, P, PlanV<N, V>::RL>(p, e);
+        sm[row * TC + c] = row_freq<N>(row) <= b ? v[e] : mk<T2>((T)0, (T)0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = sm[reg_row<N, P, PlanV<N, V>::R1>(p, e) * TC + c];
+    __syncthreads();
+    PlanV<N, V>::template fft<T2, +1>(v, sm + c, StrideAddr{TC}, p, tw);
+    if (b < 0) return;
+    T2 *out = static_cast<T2 *>(J.out);
+#pragma unroll
+    for (int e = 0; e < E; ++e) out[col + reg_row<N, P, PlanV<N, V>::RL>(p, e) * rs] = v[e];
 }
 
 }  // namespace kf

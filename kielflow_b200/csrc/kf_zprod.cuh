@@ -1,6 +1,7 @@
 // kf_zprod.cuh -- the z-local middle of the right-hand side in one kernel: the
 // inverse z transforms of u', s and their derivatives, the physical-space
-// products (k_products' terms) and the forward z transform of the four results,
+// products and the forward z transform of the four results,
+//   prod_c = u.grad u_c, prod_3 = u.grad s                     (rhs_standard.cpp:323-436)
 //   g_q = -prod_q                                             (H = 0)
 //   g_q = (1-H) (rl_q - prod_q) + H eta (q_d - q_fix) - rl_q   (H != 0)
 // so that the right-hand side is -lin_q + r2c(g_q) with the linear terms left in
@@ -17,7 +18,7 @@
 // transform of all rows' results at the end.
 //
 // 256^3 FP32, one right-hand side: the three passes it replaces (k_z_c2r 491 us,
-// k_products 305 us, k_z_r2c 74 us) wrote and read 40 real fields on the way.
+// the products 305 us, k_z_r2c 74 us) wrote and read 40 real fields on the way.
 #pragma once
 
 #include "kf_passes.cuh"
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
 k_z_phi(const double *__restrict__ phi, typename C2<T>::type *__restrict__ out,
         const typename C2<T>::type *__restrict__ tw, int nko, int pitch) {
     typedef typename C2<T>::type T2;
-    constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1, LS = PadLen<N>::value;
+    constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, LS = PadLen<N>::value;
     extern __shared__ __align__(16) unsigned char kf_smem[];
     T2 *xch = reinterpret_cast<T2 *>(kf_smem);  // [LZ][LS]
     const int p = threadIdx.x % P, l = threadIdx.x / P;
