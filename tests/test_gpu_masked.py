@@ -117,3 +117,33 @@ def test_given_potential_vs_oracle(n, filtered, prec, plan):
     scale = max(np.abs(x).max() for x in r)
     err = max(np.abs(a - b).max() for a, b in zip(g, r)) / scale
     assert err < (1e-12 if prec == kf.KF_FP64 else 1e-5)
+
+
+@pytest.mark.parametrize("plan", [0, 1])
+@pytest.mark.parametrize("prec", [kf.KF_FP64, kf.KF_FP32_BULK])
+@pytest.mark.parametrize("kind", [None, "ball", "across the box edge"])
+@pytest.mark.parametrize("n", [16, 32, 96, 128])
+def test_full_spectrum_stretched_rhs_vs_oracle(n, kind, prec, plan):
+    """On stretched axes: the filtered derivatives' passes (k_x_filter), the sums in
+    physical space and the penalization on the mask's window (kind None: without).
+    Four transforms follow one another, each good to a few rounding units of the
+    field's scale: 1e-5 and 1e-12 as above."""
+    w = C.WORKLOADS["fas128"]
+    L = I.L_DEFAULT
+    terms = NO_PHI if kind else NO_PHI & ~kf.KF_T_PENALIZATION
+    cfg = C.config_for(w, n=n, precision=prec, terms=terms, stretch_m=I.frontend_stretch(L))
+    nd = I.gauss_charge(n, C.L_BOX, w["Q"], w["sigma"])
+    mask = MASKS[kind or "ball"](n)
+    st = noise_state(n, n)
+    with kf.Context(cfg) as ctx:
+        ctx.set_tuning(plan, 8)
+        ctx.set_state(*noise_state(n, n + 1))
+        ctx.set_sources(nd, mask)
+        ctx.rhs()
+        ctx.set_state(*st)
+        ctx.rhs()
+        g = ctx.get_state()
+    r = oracle_rhs(cfg, st, nd, mask)
+    scale = max(np.abs(x).max() for x in r)
+    err = max(np.abs(a - b).max() for a, b in zip(g, r)) / scale
+    assert err < (1e-12 if prec == kf.KF_FP64 else 1e-5)
