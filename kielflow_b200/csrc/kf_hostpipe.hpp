@@ -13,7 +13,7 @@
 
 #include <algorithm>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -47,9 +47,10 @@ class HostPipe {
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
         const int nt = (int)ev_.size() / 2;
-        const size_t part = (bytes / nt + 4095) / 4096 * 4096;
+        const size_t part = ((bytes + nt - 1) / nt + 4095) / 4096 * 4096;  // nt parts hold all of it
         std::vector<cudaError_t> err(nt, cudaSuccess);
         std::vector<std::thread> th;
+        th.reserve(nt);
         int own = 0;  // ranges from here on are taken by this thread
         try {
             for (; own + 1 < nt; ++own)
@@ -57,7 +58,7 @@ class HostPipe {
                     err[own] = cudaSetDevice(dev);
                     if (err[own] == cudaSuccess) err[own] = range(own, part, dst, src, bytes, up, st);
                 });
-        } catch (const std::system_error &) {  // no thread to be had: fewer do it
+        } catch (const std::exception &) {  // no thread to be had: fewer do it
         }
         for (int k = own; k < nt; ++k) err[k] = range(k, part, dst, src, bytes, up, st);
         for (std::thread &t : th) t.join();
