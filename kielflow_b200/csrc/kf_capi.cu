@@ -5,8 +5,9 @@
 //   A  inverse x/y passes of s^ (P s^, i k_x P s^, i k_y P s^) and the z pass of
 //      P s^  ->  s_d;  rho = exp(s_d) + n_d;  Poisson solve -> phi
 //   B  phi^ = r2c(phi)                                    (E-force, :218-226)
-//   C  -lin_q in k-space (k_lin); with penalization also c2r(-lin_q) on the
-//      window of rows on which the mask is not zero
+//   C  -lin_q in k-space (k_lin); with penalization also the inverse x and y
+//      passes of -lin_q (FP32) or c2r(-lin_q) on the window of rows on which the
+//      mask is not zero (FP64)
 //   D  inverse x / y passes generating U_c, d_d U_c, d_d s
 //   E  k_zprod: their inverse z pass, the physical-space products (advection,
 //      u.grad s) [+ penalization] and the forward z pass of the results
@@ -1325,6 +1326,9 @@ template <typename T, int N> struct Impl {
     typedef typename C2<T>::type T2;
     static constexpr int TC = Tile<T>::TC, LZ = ZTile<T>::LZ, NZC = N / 2 + 1;
     template <int V> static constexpr int PV = PlanV<N, V>::P;
+    // with penalization the linear terms go through physical space whole (k_zprod):
+    // 256^3 FP32 bulk 14.2 ms a step against 13.1 with them in k-space
+    static constexpr bool RLINES = sizeof(T) == 4;
 
     static const T2 *tw(kf_ctx *c) { return (const T2 *)c->tw[c->fftv]; }
 
@@ -1348,7 +1352,9 @@ template <typename T, int N> struct Impl {
         CK(cudaFuncSetAttribute(k_axis_pipe<T, N, +1, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_c2r<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_r2c<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        CK(cudaFuncSetAttribute(k_zprod<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        CK(cudaFuncSetAttribute(k_zprod<T, N, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        if constexpr (RLINES)
+            CK(cudaFuncSetAttribute(k_zprod<T, N, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_rho<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_phi<T, N, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
         CK(cudaFuncSetAttribute(k_z_phi<T, N, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
@@ -1501,18 +1507,18 @@ template <typename T, int N> struct Impl {
     }
 
     // rho = exp(c2r(P s)) + n_d (and its colour-split copy) from round A's P s
-    // in CY[0]; sd: also s_d itself
-    static void rho_pass(kf_ctx *c, T *sd) {
-        const int nb = (N * N / 2 + LZ - 1) / LZ;
+    // in CY[0]; s_d itself into R[0] on the rows of sd
+    static void rho_pass(kf_ctx *c, RowBox sd) {
+        const int nb = zline_blocks<T, N>();
         const size_t smem = (size_t)LZ * PadLen<N>::value * sizeof(T2);
         const T sc = (T)(1. / ((double)N * N * N));
         double *rho = captured_solve(c) && split_on(c, 0) ? nullptr : c->rho;  // then only the split copy is read
         Launch L_(c, KC_RHO, (double)N * N * nkz(c, true) * sizeof(T2) + (double)c->N * (8 + (rho ? 8 : 0) + (c->rho_cs ? 8 : 0)));
         if (c->fftv)
-            k_z_rho<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, rho, c->rho_cs,
+            k_z_rho<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>((const T2 *)c->CY[0], (T *)c->R[0], sd, c->nd, rho, c->rho_cs,
                                                               tw(c), sc, nkz(c, true), c->tr.mp);
         else
-            k_z_rho<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>((const T2 *)c->CY[0], sd, c->nd, rho, c->rho_cs,
+            k_z_rho<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>((const T2 *)c->CY[0], (T *)c->R[0], sd, c->nd, rho, c->rho_cs,
                                                               tw(c), sc, nkz(c, true), c->tr.mp);
         CK(cudaGetLastError());
     }
@@ -1523,7 +1529,7 @@ template <typename T, int N> struct Impl {
     // formed, and phi^ is not read where it does.  (Together with phi staying in split
     // order between the stages: 2-4 % of a 256^3 step.)
     static void phi_transform(kf_ctx *c) {
-        const int nb = (N * N / 2 + LZ - 1) / LZ;
+        const int nb = zline_blocks<T, N>();
         const size_t smem = (size_t)LZ * PadLen<N>::value * sizeof(T2);
         const bool pf = (c->cfg.terms & T_PRESSURE) && c->pf.nkz;
         const bool sp = captured_solve(c) && split_on(c, 0);  // (solve_end comes with the last stage)
@@ -1546,7 +1552,8 @@ template <typename T, int N> struct Impl {
     }
 
     // rounds D (z), E and the z part of F: k_zprod -> CX[0..3]
-    static void zprod(kf_ctx *c, bool pen) {
+    // (RL: with the linear terms' lines)
+    template <bool RL> static void zprod(kf_ctx *c, bool pen) {
         ZProdArgs<T> a{};
         a.s0 = (const T2 *)c->CY[0];
         a.sy = (const T2 *)c->CY[1];
@@ -1559,7 +1566,9 @@ template <typename T, int N> struct Impl {
         for (int q = 0; q < 4; ++q) {
             a.out[q] = (T2 *)c->CX[q];
             a.rl[q] = (const T *)c->R[16 + q];
+            a.lin[q] = (const T2 *)c->CY[12 + q];
         }
+        a.sd = (const T *)c->R[0];
         a.H = (const T *)c->H;
         if (pen) {
             a.i0 = c->bx_i0;
@@ -1575,12 +1584,12 @@ template <typename T, int N> struct Impl {
         a.ip = c->tr.mp;
         a.nko = nkz(c, pen);
         a.op = pen ? c->tr.mp : NZC;
-        const size_t smem = ZProdSmem<T, N>::bytes;
-        Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko) + 5. * a.bi * a.bj * N * sizeof(T));
+        const size_t smem = ZProdSmem<T, N, RL>::bytes;
+        Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko + (RL ? 4. * NZC : 0.)) + (RL ? 2. : 6.) * a.bi * a.bj * N * sizeof(T));
         if (c->fftv)
-            k_zprod<T, N, 1><<<N * N / ZP_ROWS, ZP_LINES * PV<1>, smem, c->st>>>(a, (const T *)c->kv, tw(c));
+            k_zprod<T, N, 1, RL><<<N * N / ZP_ROWS, ZProdLines<RL>::value * PV<1>, smem, c->st>>>(a, (const T *)c->kv, tw(c));
         else
-            k_zprod<T, N, 0><<<N * N / ZP_ROWS, ZP_LINES * PV<0>, smem, c->st>>>(a, (const T *)c->kv, tw(c));
+            k_zprod<T, N, 0, RL><<<N * N / ZP_ROWS, ZProdLines<RL>::value * PV<0>, smem, c->st>>>(a, (const T *)c->kv, tw(c));
         CK(cudaGetLastError());
     }
 
@@ -1611,19 +1620,20 @@ template <typename T, int N> struct Impl {
         return true;
     }
 
-    // rounds A (P s, d_x s, d_y s, the Poisson source and, with keep_sd, s_d
-    // in R[0]), the Poisson solve and B (phi^ = r2c(phi)), shared by both
-    // right-hand sides
-    static bool rounds_AB(kf_ctx *c, bool fork, bool keep_sd) {
+    // rounds A (P s, d_x s, d_y s, the Poisson source and, with penalization, s_d
+    // in R[0] where the mask is not zero), the Poisson solve and B (phi^ =
+    // r2c(phi)), shared by both right-hand sides
+    static bool rounds_AB(kf_ctx *c, bool fork) {
         const int Tm = c->cfg.terms;
         const bool pois = (Tm & T_POISSON) && (Tm & T_E_INT);
         // A
         axis(c, c->jA_x, 2, 0, +1, AX_XM);
         axis(c, c->jA_y, 3, 1, +1, AX_YI);
         const bool solve = pois && !c->phi_given;
+        const RowBox box = (Tm & T_PENALIZATION) ? RowBox{c->bx_i0, c->bx_i, c->bx_j0, c->bx_j} : RowBox{0, 0, 0, 0};
         if (solve)
-            rho_pass(c, keep_sd ? (T *)c->R[0] : nullptr);
-        else if (keep_sd)
+            rho_pass(c, box);
+        else if (box.bi)
             zc2r(c, c->zA, 1, true);
         const bool forked = fork && fork_D(c);
         if (solve) {
@@ -1652,14 +1662,18 @@ template <typename T, int N> struct Impl {
     static void rhs(kf_ctx *c) {
         const int Tm = c->cfg.terms;
         const bool pen = Tm & T_PENALIZATION;
-        const bool forked = rounds_AB(c, true, false);
+        const bool forked = rounds_AB(c, true);
         // C
         {
             Launch L_(c, KC_LIN, (double)c->Nc * (9 * sizeof(T2) + 2 * sizeof(T)));
             k_lin<T><<<mg_grid(NZC, N), mg_block(), 0, c->st>>>(rargs(c), geo(c), (T2 *)c->LIN[0], (T2 *)c->LIN[1],
                                                                (T2 *)c->LIN[2], (T2 *)c->LIN[3]);
         }
-        if (pen && c->bx_i) {  // c2r(-lin_q) on the mask's window
+        const bool rl = RLINES && pen;
+        if (rl) {  // the linear terms' inverse x and y passes, whole
+            axis(c, c->jD_x + 6, 4, 0, +1);
+            axis(c, c->jD_y + 9, 4, 1, +1);
+        } else if (pen && c->bx_i) {  // c2r(-lin_q) on the mask's window
             axis(c, c->jD_x + 6, 4, 0, +1, AX_XB);
             axis(c, c->jD_y + 9, 4, 1, +1, AX_YB);
             zc2r(c, c->zD + 8, 2, false, -1., c->bx_i * c->bx_j);
@@ -1670,18 +1684,26 @@ template <typename T, int N> struct Impl {
         else
             CK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
         // z part of D, E, z part of F (with penalization only what the 2/3 rule keeps is formed)
-        zprod(c, pen);
+        if constexpr (RLINES) {
+            if (rl)
+                zprod<true>(c, pen);
+            else
+                zprod<false>(c, pen);
+        } else {
+            zprod<false>(c, pen);
+        }
         axis(c, c->jF_y, 4, 1, -1, pen ? AX_YF : AX_FULL);
-        stage(c, pen);
+        stage(c, pen, !rl);
     }
 
     // the end of F: the forward x pass, K and its use in the RK4 stage
-    static void stage(kf_ctx *c, bool pen) {
+    // (lin: with the linear terms of k_lin)
+    static void stage(kf_ctx *c, bool pen, bool lin) {
         const AxTrunc A = trunc(c, pen ? AX_XM : AX_FULL, false);
         StageArgs<T> a;
         for (int q = 0; q < 4; ++q) {
             a.in[q] = (const T2 *)c->CY[q];
-            a.lin[q] = (const T2 *)c->LIN[q];
+            a.lin[q] = lin ? (const T2 *)c->LIN[q] : nullptr;
             a.y[q] = (T2 *)c->Y[q];
             a.acc[q] = (T2 *)c->ACC[q];
             a.ys[q] = (T2 *)c->Ys[q];
@@ -1718,7 +1740,7 @@ template <typename T, int N> struct Impl {
         const bool pen = Tm & T_PENALIZATION, win = pen && c->bx_i;
         const long Nc = c->Nc, Nr = c->N;
         const double cb = (double)Nc * sizeof(T2), rb = (double)Nr * sizeof(T);
-        rounds_AB(c, false, pen);
+        rounds_AB(c, false);
         {  // C'
             Launch L_(c, KC_LIN, 4 * cb + 6 * cb + 2 * rb);
             k_sl_lin<T><<<nblk(Nc, 256), 256, 0, c->st>>>(rargs(c), geo(c), (T2 *)c->LIN[0], (T2 *)c->LIN[1],
@@ -1780,7 +1802,7 @@ template <typename T, int N> struct Impl {
         }
         zr2c(c, c->zF, 2, pen);
         axis(c, c->jF_y, 4, 1, -1, pen ? AX_YF : AX_FULL);
-        stage(c, pen);
+        stage(c, pen, true);
     }
     static void x_filter(kf_ctx *c, int off, int njobs) {
         const AxTrunc A = trunc(c, AX_XM, false);

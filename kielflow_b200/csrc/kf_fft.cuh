@@ -35,6 +35,9 @@ template <typename T2> __device__ __forceinline__ T2 csub(T2 a, T2 b) { return m
 template <typename T2> __device__ __forceinline__ T2 cmul(T2 a, T2 b) {
     return mk<T2>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+// a product that is rounded by itself, whatever it is added to
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 // multiply by SIGN*i :  (x + i y) * (SIGN i) = SIGN*(-y + i x)
 template <int SIGN, typename T2> __device__ __forceinline__ T2 mul_si(T2 a) {
     return SIGN < 0 ? mk<T2>(a.y, -a.x) : mk<T2>(-a.y, a.x);

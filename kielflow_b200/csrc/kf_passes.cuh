@@ -484,7 +484,8 @@ k_z_r2c(const ZJob *__restrict__ jobs, int njobs, int nrows,
 // One block transforms one column tile of one of the four fields and finishes
 // the right-hand side there,
 //   K_q = -lin_q + F_q                             (rhs_standard.cpp:538-560)
-// with -lin_q from k_lin and F_q the transform of the physical part (k_zprod);
+// with -lin_q from k_lin and F_q the transform of the physical part (k_zprod; lin[q]
+// == nullptr: that holds the linear terms, too);
 // with penalization F_q and -lin_q are needed inside the 2/3 rule only (the
 // filter after the physical-space penalization, rhs_standard.cpp:491-532): the
 // active columns (A.mode AX_XM), the rows within their bounds, K being zero
@@ -539,8 +540,11 @@ k_xfwd_stage(const __grid_constant__ StageArgs<T> a, Geo<T> g, const typename C2
         const int i = reg_row<N, P, PlanV<N, V>::RL>(p, e);
         if (row_freq<N>(i) > b) continue;
         const int idx = col + i * rstride;
-        const T2 l = a.lin[q][idx];
-        const T2 k = mk<T2>(l.x + v[e].x, l.y + v[e].y);
+        T2 k = v[e];
+        if (a.lin[q]) {
+            const T2 l = a.lin[q][idx];
+            k = mk<T2>(l.x + v[e].x, l.y + v[e].y);
+        }
         if (a.mode == 3) {
             a.K[q][idx] = k;
             continue;

@@ -15,6 +15,8 @@ namespace kf {
 //        (rhs_standard.cpp:135-139, 304-319)
 // Grid (ceil(nzc/32), n/8, n) of 32 x 8 blocks over (kz, j, i): no index
 // division; the four outputs of an element share its loads (state, phi^, tables).
+// The damping and diffusion sum's roundings are written out (k_zprod): in u_c the
+// diffusion product is rounded first with penalization, the damping one without.
 template <typename T>
 __global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *o0,
                                              typename C2<T>::type *o1, typename C2<T>::type *o2,
@@ -49,11 +51,13 @@ __global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         const T cf = diss && svo ? (a.tau + sv) : diss ? a.tau : svo ? sv : (T)0;
-        T2 fb = mk<T2>(cf * u[q].x, cf * u[q].y);
+        T2 fb = mk<T2>(mul_rn(cf, u[q].x), mul_rn(cf, u[q].y));
         if (Tm & T_DIFFUSION) {
-            const T k2 = kx * kx + ky * ky + kz * kz;
-            fb.x += a.D * k2 * u[q].x;
-            fb.y += a.D * k2 * u[q].y;
+            const T Dk = mul_rn(a.D, kx * kx + ky * ky + kz * kz);
+            if (Tm & T_PENALIZATION)
+                fb = mk<T2>(fma(cf, u[q].x, mul_rn(Dk, u[q].x)), fma(cf, u[q].y, mul_rn(Dk, u[q].y)));
+            else
+                fb = mk<T2>(fma(Dk, u[q].x, fb.x), fma(Dk, u[q].y, fb.y));
         }
         if (pres || eint) {
             const T kc = q == 0 ? kx : q == 1 ? ky : kz;
@@ -70,11 +74,10 @@ __global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2
     }
     {
         const T cf = (Tm & T_SVISCOSITY) ? sv : (T)0;
-        T2 fb = mk<T2>(cf * s.x, cf * s.y);
+        T2 fb = mk<T2>(mul_rn(cf, s.x), mul_rn(cf, s.y));
         if (Tm & T_DIFFUSION) {
-            const T k2 = kx * kx + ky * ky + kz * kz;
-            fb.x += a.D * k2 * s.x;
-            fb.y += a.D * k2 * s.y;
+            const T Dk = mul_rn(a.D, kx * kx + ky * ky + kz * kz);
+            fb = mk<T2>(fma(Dk, s.x, fb.x), fma(Dk, s.y, fb.y));
         }
         if ((Tm & T_E_EXT) && P) {
             const T2 d = mul_ik(s, kx);
