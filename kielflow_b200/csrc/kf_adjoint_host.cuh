@@ -55,14 +55,6 @@ struct AdjState {
     int solves = 0;
 };
 
-void dfree(kf_ctx *c, void *p) {
-    auto it = std::find(c->allocs.begin(), c->allocs.end(), p);
-    if (it != c->allocs.end()) {
-        c->allocs.erase(it);
-        cudaFree(p);
-    }
-}
-
 Geo<double> geo64(kf_ctx *c) {
     return Geo<double>{c->n, c->nzc, (const double *)c->kv, c->q2, dealias_threshold(), c->pb};
 }
@@ -97,7 +89,7 @@ void snap_load(kf_ctx *c, const Snap &s) {
 }
 
 // Job lists of the adjoint's transform passes (Impl::adj_pass), appended to
-// the context's lists, which are uploaded again.
+// the context's lists in new device arrays.
 void build_adj_jobs(kf_ctx *c) {
     AdjState &a = *c->adj;
     std::vector<AxisJob> &J = c->hj;
@@ -160,9 +152,7 @@ void build_adj_jobs(kf_ctx *c) {
     ZJob *dz = dalloc<ZJob>(c, sizeof(ZJob) * Z.size());
     CK(cudaMemcpy(dj, J.data(), sizeof(AxisJob) * J.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(dz, Z.data(), sizeof(ZJob) * Z.size(), cudaMemcpyHostToDevice));
-    CK(cudaStreamSynchronize(c->st));
-    dfree(c, c->dj);
-    dfree(c, c->dz);
+    // the lists without them stay as they are: captured steps hold their addresses
     c->dj = dj;
     c->dz = dz;
 }
