@@ -135,10 +135,14 @@ __global__ void __launch_bounds__(128) k_residual_s(const double *__restrict__ p
                                                 (unsigned long long)__double_as_longlong(fabs(v.y))));
                        });
     if constexpr (MAX) {
-        // per warp, by 32-bit halves; the lanes past the last row hold 0
-        const unsigned lanes = __activemask(), hi = (unsigned)(af >> 32), mh = __reduce_max_sync(lanes, hi);
+        // per warp, by 32-bit halves; the lanes past the last row hold 0.  Which lanes
+        // there are follows from the block's size: after the branch above a warp need
+        // not be together, and a part of it without lane 0 would not post its maximum
+        const int t = threadIdx.y * blockDim.x + threadIdx.x, left = (int)(blockDim.x * blockDim.y) - (t & ~31);
+        const unsigned lanes = left >= 32 ? 0xffffffffu : (1u << left) - 1u;
+        __syncwarp(lanes);
+        const unsigned hi = (unsigned)(af >> 32), mh = __reduce_max_sync(lanes, hi);
         const unsigned ml = __reduce_max_sync(lanes, hi == mh ? (unsigned)af : 0u);
-        const int t = threadIdx.y * blockDim.x + threadIdx.x;
         if ((t & 31) == 0)
             atomicMax(slots + ((blockIdx.y + blockIdx.z * gridDim.y + (t >> 5)) & 63),
                       ((unsigned long long)mh << 32) | ml);
