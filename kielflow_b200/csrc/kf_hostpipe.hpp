@@ -6,7 +6,8 @@
 // are taken one by one there.  Here a few threads each take a range of the array,
 // copy it through two pinned pieces of their own and queue their own transfers on
 // the stream, so that the host copies, the faults and the transfers overlap.
-// Page-locked or device-visible arrays, and small ones, take cudaMemcpyAsync.
+// Page-locked or device-visible arrays, small ones and the per-thread default stream
+// (whose handle names another stream in each thread) take cudaMemcpyAsync.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -42,7 +43,8 @@ class HostPipe {
     // download's target is complete on return.
     cudaError_t copy(void *dst, const void *src, size_t bytes, bool up, cudaStream_t st) {
         const cudaMemcpyKind kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-        if (bytes < kMin || !pageable(up ? src : dst) || !ready(bytes)) return cudaMemcpyAsync(dst, src, bytes, kind, st);
+        if (bytes < kMin || st == cudaStreamPerThread || !pageable(up ? src : dst) || !ready(bytes))
+            return cudaMemcpyAsync(dst, src, bytes, kind, st);
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
