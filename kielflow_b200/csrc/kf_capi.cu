@@ -1496,6 +1496,7 @@ template <typename T, int N> struct Impl {
         a.M = (T)c->cfg.M;
         a.D = (T)c->cfg.diff_D;
         a.terms = c->cfg.terms;
+        a.herm = (c->cfg.terms & T_PENALIZATION) && (c->stretched || !RLINES);
         return a;
     }
 

@@ -13,17 +13,14 @@ namespace kf {
 //        (rhs_standard.cpp:119-140, 218-248, 279-295)
 //   s  : SV s^ [+ D|k|^2 s^] + M i k_x P s^ + i k.P u^
 //        (rhs_standard.cpp:135-139, 304-319)
-// Grid (ceil(nzc/32), n/8, n) of 32 x 8 blocks over (kz, j, i): no index
+// k_lin: grid (ceil(nzc/32), n/8, n) of 32 x 8 blocks over (kz, j, i): no index
 // division; the four outputs of an element share its loads (state, phi^, tables).
 // The damping and diffusion sum's roundings are written out (k_zprod): in u_c the
 // diffusion product is rounded first with penalization, the damping one without.
 template <typename T>
-__global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *o0,
-                                             typename C2<T>::type *o1, typename C2<T>::type *o2,
-                                             typename C2<T>::type *o3) {
+__device__ __forceinline__ void lin_terms(const RhsArgs<T> &a, const Geo<T> &g, int i, int j, int k,
+                                          typename C2<T>::type *o) {
     typedef typename C2<T>::type T2;
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
-    if (k >= g.nzc || j >= g.n) return;
     const long idx = (long)k + (long)g.nzc * ((long)j + (long)i * g.n);
     const int Tm = a.terms;
     const bool P = dealias_keep(g.q2, g.thr, i, j, k);
@@ -47,7 +44,6 @@ __global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2
             F1.y += s.y / a.theta;
         }
     }
-    T2 *o[4] = {o0, o1, o2, o3};
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         const T cf = diss && svo ? (a.tau + sv) : diss ? a.tau : svo ? sv : (T)0;
@@ -70,7 +66,7 @@ __global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2
             fb.x += a.M * d.x;
             fb.y += a.M * d.y;
         }
-        o[q][idx] = mk<T2>(-fb.x, -fb.y);
+        o[q] = mk<T2>(-fb.x, -fb.y);
     }
     {
         const T cf = (Tm & T_SVISCOSITY) ? sv : (T)0;
@@ -92,8 +88,36 @@ __global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2
             fb.x += dy.x; fb.y += dy.y;
             fb.x += dz.x; fb.y += dz.y;
         }
-        o[3][idx] = mk<T2>(-fb.x, -fb.y);
+        o[3] = mk<T2>(-fb.x, -fb.y);
     }
+}
+
+// o: four values of element (i, j, k = 0); m: those of (-i, -j, 0)
+template <typename T2> __device__ __forceinline__ void hermitian_part(T2 *o, const T2 *m) {
+    typedef decltype(T2::x) T;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) o[q] = mk<T2>((T)0.5 * (o[q].x + m[q].x), (T)0.5 * (o[q].y - m[q].y));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *o0,
+                                             typename C2<T>::type *o1, typename C2<T>::type *o2,
+                                             typename C2<T>::type *o3) {
+    typedef typename C2<T>::type T2;
+    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
+    if (k >= g.nzc || j >= g.n) return;
+    T2 o[4];
+    lin_terms(a, g, i, j, k, o);
+    if (a.herm && k == 0 && dealias_keep(g.q2, g.thr, i, j, 0)) {
+        T2 m[4];
+        lin_terms(a, g, i ? g.n - i : 0, j ? g.n - j : 0, 0, m);
+        hermitian_part(o, m);
+    }
+    const long idx = (long)k + (long)g.nzc * ((long)j + (long)i * g.n);
+    o0[idx] = o[0];
+    o1[idx] = o[1];
+    o2[idx] = o[2];
+    o3[idx] = o[3];
 }
 
 // The (i, j) rows on which the penalization mask is not zero, as the window

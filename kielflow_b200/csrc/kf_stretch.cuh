@@ -8,6 +8,7 @@
 #pragma once
 
 #include "kf_passes.cuh"
+#include "kf_pointwise.cuh"
 #include "kf_types.cuh"
 
 namespace kf {
@@ -15,7 +16,30 @@ namespace kf {
 // -1 x the linear spectral parts of FBuffer (no derivative; rhs_standard.cpp:119-140
 // and the added diffusion) and the potential of the E-force/pressure term
 // F1 = PF phi^ + s^/theta (rhs_standard.cpp:218-240), one thread per
-// half-spectrum element.  Same order of operations as lin_term.
+// half-spectrum element.  Same order of operations as lin_terms.
+template <typename T>
+__device__ __forceinline__ void sl_lin_terms(const RhsArgs<T> &a, const Geo<T> &g, int i, int j, int k,
+                                             typename C2<T>::type *o) {
+    typedef typename C2<T>::type T2;
+    const long idx = (long)k + (long)g.nzc * ((long)j + (long)i * g.n);
+    const int Tm = a.terms;
+    const T kx = g.kv[i], ky = g.kv[j], kz = g.kv[k];
+    const T sv = a.SV[idx];
+    const bool diss = Tm & T_DISSIPATION, svo = Tm & T_SVISCOSITY;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const T2 y = a.Y[q][idx];
+        const T cf = q < 3 && diss ? (svo ? a.tau + sv : a.tau) : svo ? sv : (T)0;
+        T2 fb = mk<T2>(cf * y.x, cf * y.y);
+        if (Tm & T_DIFFUSION) {
+            const T k2 = kx * kx + ky * ky + kz * kz;
+            fb.x += a.D * k2 * y.x;
+            fb.y += a.D * k2 * y.y;
+        }
+        o[q] = mk<T2>(-fb.x, -fb.y);
+    }
+}
+
 template <typename T>
 __global__ void k_sl_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *l0, typename C2<T>::type *l1,
                          typename C2<T>::type *l2, typename C2<T>::type *l3, typename C2<T>::type *F1o) {
@@ -26,34 +50,19 @@ __global__ void k_sl_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *l0, typen
     const int k = (int)(idx % g.nzc);
     const long r = idx / g.nzc;
     const int j = (int)(r % g.n), i = (int)(r / g.n);
+    T2 o[4];
+    sl_lin_terms(a, g, i, j, k, o);
+    if (a.herm && k == 0 && dealias_keep(g.q2, g.thr, i, j, 0)) {
+        T2 m[4];
+        sl_lin_terms(a, g, i ? g.n - i : 0, j ? g.n - j : 0, 0, m);
+        hermitian_part(o, m);
+    }
+    l0[idx] = o[0];
+    l1[idx] = o[1];
+    l2[idx] = o[2];
+    l3[idx] = o[3];
     const int Tm = a.terms;
-    const T kx = g.kv[i], ky = g.kv[j], kz = g.kv[k];
-    const T sv = a.SV[idx];
-    T2 *o[3] = {l0, l1, l2};
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        const T2 u = a.Y[q][idx];
-        const bool diss = Tm & T_DISSIPATION, svo = Tm & T_SVISCOSITY;
-        const T cf = diss && svo ? (a.tau + sv) : diss ? a.tau : svo ? sv : (T)0;
-        T2 fb = mk<T2>(cf * u.x, cf * u.y);
-        if (Tm & T_DIFFUSION) {
-            const T k2 = kx * kx + ky * ky + kz * kz;
-            fb.x += a.D * k2 * u.x;
-            fb.y += a.D * k2 * u.y;
-        }
-        o[q][idx] = mk<T2>(-fb.x, -fb.y);
-    }
     const T2 s = a.Y[3][idx];
-    {
-        const T cf = (Tm & T_SVISCOSITY) ? sv : (T)0;
-        T2 fb = mk<T2>(cf * s.x, cf * s.y);
-        if (Tm & T_DIFFUSION) {
-            const T k2 = kx * kx + ky * ky + kz * kz;
-            fb.x += a.D * k2 * s.x;
-            fb.y += a.D * k2 * s.y;
-        }
-        l3[idx] = mk<T2>(-fb.x, -fb.y);
-    }
     T2 F1 = mk<T2>((T)0, (T)0);
     const bool pres = Tm & T_PRESSURE, eint = Tm & T_E_INT;
     if (eint) {
