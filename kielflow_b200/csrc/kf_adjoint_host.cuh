@@ -404,12 +404,12 @@ void adj_poisson(kf_ctx *c) {
         CK(cudaMemcpyAsync(a.h_rec, a.rec, sizeof(DevAdj), cudaMemcpyDeviceToHost, c->st));
         CK(cudaStreamSynchronize(c->st));
     };
-    if (!c->prof) {
+    if (!host_driven(c)) {
         if (!a.graph) build_adj_graph(c);
         CK(cudaGraphLaunch(a.graph, c->st));
         read();
         c->launches += a.graph_kernels + a.h_rec->cyc * a.cycle_kernels;
-    } else {  // launched one by one, for the per-launch profile
+    } else {  // launched one by one
         adj_solve_begin(c);
         auto test = [&](int cyc) {
             CK(cudaMemcpyAsync(c->h_max, c->d_max, 64 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->st));

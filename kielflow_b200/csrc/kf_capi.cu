@@ -314,6 +314,16 @@ struct Launch {
     }
 };
 
+// Whether everything is launched kernel by kernel: for the per-launch profile, and
+// with KIELFLOW_B200_NO_GRAPH=1, for tools that do not see into captured graphs.
+bool host_driven(const kf_ctx *c) {
+    static const bool off = [] {
+        const char *e = std::getenv("KIELFLOW_B200_NO_GRAPH");
+        return e && e[0] == '1';
+    }();
+    return c->prof || off;
+}
+
 // ------------------------------------------------------------------ host tables
 double k_val_at(int i, int n, double L) {  // axis_EqSt.cpp:57-61
     double pi = acos(-1.);
@@ -582,12 +592,12 @@ int jacobi_solve(kf_ctx *c, const LevelBuf &L, double *phi, double *tmp, const d
     js.norm_sum = c->norm_sum;
     js.omega = 1.;
     if (S.max_it > 0) {
-        cudaGraphExec_t exec = c->prof ? nullptr : jacobi_graph(c, L, phi, tmp, rho, S);
+        cudaGraphExec_t exec = host_driven(c) ? nullptr : jacobi_graph(c, L, phi, tmp, rho, S);
         js.fresh = 1;
         CK(cudaMemcpyAsync(c->d_js, &js, sizeof(JacState), cudaMemcpyHostToDevice, c->st));
         if (exec) {
             CK(cudaGraphLaunch(exec, c->st));
-        } else {  // launched one by one, for the per-launch profile
+        } else {  // launched one by one
             while (!js.done) {
                 for (int s = 0; s < 2; ++s) jacobi_sweep(c, L, phi, tmp, rho, S, s);
                 jacobi_test(c, L, S, 0, 0);
@@ -951,10 +961,10 @@ void vcycle(kf_ctx *c, int l) {
 }
 
 // One FAS V-cycle on the finest level: replayed from a CUDA graph captured on
-// first use (one launch instead of ~70), or launched kernel by kernel while
-// the per-launch profile is on.
+// first use (one launch instead of ~70), or launched kernel by kernel
+// (host_driven).
 void run_vcycle(kf_ctx *c) {
-    if (c->prof) {
+    if (host_driven(c)) {
         vcycle(c, 0);
         return;
     }
@@ -1164,7 +1174,7 @@ int poisson(kf_ctx *c, bool split = false) {
         solve_begin(c, split);
         // a context's first solve from here: making the graph takes as long as the
         // launches and synchronisations that it saves in a few solves
-        if (!c->prof && c->host_solves++) return fas_solve(c);
+        if (!host_driven(c) && c->host_solves++) return fas_solve(c);
         double r = 0.;
         int cyc = 0;
         for (;;) {
@@ -2546,17 +2556,11 @@ void rk4_step(kf_ctx *c, double dt, void *const *X, double *const *PH, double *c
     c->t = t0 + dt;
 }
 
-// Whether kf_rk4_steps replays a captured step graph: every decision of the
-// step can be taken on the device (FAS or no Poisson solve; the Jacobi and
-// cascadic solvers steer their sweeps from the host) and the per-launch
-// profile is off.  KIELFLOW_B200_NO_GRAPH=1 forces the host-driven path.
+// Whether kf_rk4_steps replays a captured step graph: FAS or no Poisson solve (the
+// Jacobi and cascadic solves, graphs of their own, are launched from the host).
 bool graph_path(kf_ctx *c) {
     const kf_config &cf = c->cfg;
-    static const bool off = [] {
-        const char *e = std::getenv("KIELFLOW_B200_NO_GRAPH");
-        return e && e[0] == '1';
-    }();
-    if (c->prof || off) return false;
+    if (host_driven(c)) return false;
     const bool pois = (cf.terms & T_POISSON) && (cf.terms & T_E_INT);
     return !pois || cf.poisson_mode == KF_PS_FAS;
 }
