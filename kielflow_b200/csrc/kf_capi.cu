@@ -1009,11 +1009,13 @@ void solve_begin(kf_ctx *c, bool rho_done) {
     if (!rho_done) split_field(c, c->rho, c->rho_cs);
     split_field(c, c->phi, c->phi_cs);
 }
-void solve_end(kf_ctx *c) {
-    if (!split_on(c, 0)) return;
+void unsplit_field(kf_ctx *c, const double *s, double *x) {
     Launch L_(c, KC_RHO, 16. * c->N);
-    k_unsplit<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(c->phi_cs, c->phi, c->n);
+    k_unsplit<<<mg_grid(c->n / 2, c->n), mg_block(), 0, c->st>>>(s, x, c->n);
     CK(cudaGetLastError());
+}
+void solve_end(kf_ctx *c) {
+    if (split_on(c, 0)) unsplit_field(c, c->phi_cs, c->phi);
 }
 
 // The adaptive FAS loop inside a capture on c->st: head of the cycle
@@ -2207,6 +2209,7 @@ void build_levels(kf_ctx *c) {
             if (l == 0) {
                 c->phi_cs = dalloc<double>(c, bytes);
                 c->rho_cs = dalloc<double>(c, bytes);
+                CK(cudaMemset(c->rho_cs, 0, bytes));  // kf_autotune reads it, with or without a solve before
             }
             L.ph = l == 0 ? c->phi_cs : L.phi;
             L.rh = l == 0 ? c->rho_cs : L.rho;
@@ -2448,6 +2451,7 @@ void create(kf_ctx *c) {
     c->phiT = c->fp32 ? dalloc<void>(c, rb) : (void *)c->phi;
     c->stage64 = dalloc<double>(c, (size_t)16 * (c->Nc > c->N ? c->Nc : c->N));
     CK(cudaMemset(c->phi, 0, 8 * c->N));
+    CK(cudaMemset(c->rho, 0, 8 * c->N));
     CK(cudaMemset(c->nd, 0, 8 * c->N));
     CK(cudaMemset(c->H, 0, rb));
     for (int q = 0; q < 4; ++q) {
@@ -2839,7 +2843,12 @@ void autotune(kf_ctx *c, int reps, kf_tune_out *o) {
         double *tmp = nullptr;
         CK(cudaMalloc(&tmp, 8 * (size_t)c->N));
         try {
-            if (c->phi_cs) split_field(c, c->rho, c->rho_cs);
+            // the last solve's source in both orders (a captured solve leaves it in
+            // split order only, one with the streaming smoother in natural order)
+            if (split_on(c, 0))
+                unsplit_field(c, c->rho_cs, c->rho);
+            else if (c->rho_cs)
+                split_field(c, c->rho, c->rho_cs);
             int best = -1;
             for (int k = 0; k < 4; ++k) {
                 c->rbgs_by = rows[k];
