@@ -2146,8 +2146,8 @@ void build_levels(kf_ctx *c) {
             dm[i] = H[i] * (H[i + 1] + H[i]);
             ip[i] = 2. / dp[i];
             im[i] = 2. / dm[i];
-            rp[i] = 1. / dp[i];
-            rm[i] = 1. / dm[i];
+            rp[i] = div_reciprocal(dp[i]);
+            rm[i] = div_reciprocal(dm[i]);
         }
         for (int m = 1; m < n; m += 2) {  // OP_hto2h gamma on this (fine) axis
             const double x1 = val_at(m - 1, n, Lb, sm), x2 = val_at(m + 1, n, Lb, sm), x = val_at(m, n, Lb, sm);

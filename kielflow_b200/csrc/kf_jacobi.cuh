@@ -11,6 +11,7 @@
 // host-driven sweep (two launches, a copy and a synchronisation) took 27 us.
 #pragma once
 
+#include "kf_div.hpp"
 #include "kf_poisson.cuh"
 
 namespace kf {
@@ -28,13 +29,16 @@ struct JacStop {
     double limit, tol;  // relative-update limit; residual target (resstop)
 };
 
-// num / den with r = 1 / den rounded to nearest: Markstein's correction
-// (P. Markstein, IBM J. Res. Dev. 34, 1990): with q within an ulp,
-// q + r (num - q den) is num / den correctly rounded; one step brings num r there.
-__device__ __forceinline__ double div_by(double num, double den, double r) {
-    double q = __dmul_rn(num, r);
-    q = __fma_rn(__fma_rn(-q, den, num), r, q);
-    return __fma_rn(__fma_rn(-q, den, num), r, q);
+// The sum A of point_coeffs by divisions
+__device__ __noinline__ double point_sum(const double *pm, const double *p, const double *pp, const Lev &L, int i, int j,
+                                         int k) {
+    const int n = L.n;
+    double A = pp[j * n + k] / L.dp[i];
+    A = __dadd_rn(A, pm[j * n + k] / L.dm[i]);
+    A = __dadd_rn(A, p[wrapi(j + 1, n) * n + k] / L.dp[j]);
+    A = __dadd_rn(A, p[wrapi(j - 1, n) * n + k] / L.dm[j]);
+    A = __dadd_rn(A, p[j * n + wrapi(k + 1, n)] / L.dp[k]);
+    return __dadd_rn(A, p[j * n + wrapi(k - 1, n)] / L.dm[k]);
 }
 
 // point_coeffs: the same quotients and sums, the divisors' reciprocals from
@@ -49,6 +53,7 @@ __device__ __forceinline__ void point_coeffs_div(const double *pm, const double 
     A = __dadd_rn(A, div_by(p[wrapi(j - 1, n) * n + k], L.dm[j], L.rm[j]));
     A = __dadd_rn(A, div_by(p[j * n + wrapi(k + 1, n)], L.dp[k], L.rp[k]));
     A = __dadd_rn(A, div_by(p[j * n + wrapi(k - 1, n)], L.dm[k], L.rm[k]));
+    if (A != A) A = point_sum(pm, p, pp, L, i, j, k);
     A = __dmul_rn(2., A);
     A = __dadd_rn(A, rho);
 }
