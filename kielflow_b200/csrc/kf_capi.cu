@@ -1508,7 +1508,7 @@ template <typename T, int N> struct Impl {
         a.M = (T)c->cfg.M;
         a.D = (T)c->cfg.diff_D;
         a.terms = c->cfg.terms;
-        a.herm = (c->cfg.terms & T_PENALIZATION) && (c->stretched || !RLINES);
+        a.herm = (c->cfg.terms & T_PENALIZATION) && window_launches(c);
         return a;
     }
 
@@ -1520,18 +1520,18 @@ template <typename T, int N> struct Impl {
     }
 
     // rho = exp(c2r(P s)) + n_d (and its colour-split copy) from round A's P s
-    // in CY[0]; s_d itself into R[0] on the rows of sd
-    static void rho_pass(kf_ctx *c, RowBox sd) {
+    // in CY[0]; s_d itself into R[0] on the rows of the window
+    static void rho_pass(kf_ctx *c, const int *window) {
         const int nb = zline_blocks<T, N>();
         const size_t smem = (size_t)LZ * PadLen<N>::value * sizeof(T2);
         const T sc = (T)(1. / ((double)N * N * N));
         double *rho = captured_solve(c) && split_on(c, 0) ? nullptr : c->rho;  // then only the split copy is read
         Launch L_(c, KC_RHO, (double)N * N * nkz(c, true) * sizeof(T2) + (double)c->N * (8 + (rho ? 8 : 0) + (c->rho_cs ? 8 : 0)));
         if (c->fftv)
-            k_z_rho<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>((const T2 *)c->CY[0], (T *)c->R[0], sd, c->nd, rho, c->rho_cs,
+            k_z_rho<T, N, 1><<<nb, LZ * PV<1>, smem, c->st>>>((const T2 *)c->CY[0], (T *)c->R[0], window, c->nd, rho, c->rho_cs,
                                                               tw(c), sc, nkz(c, true), c->tr.mp);
         else
-            k_z_rho<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>((const T2 *)c->CY[0], (T *)c->R[0], sd, c->nd, rho, c->rho_cs,
+            k_z_rho<T, N, 0><<<nb, LZ * PV<0>, smem, c->st>>>((const T2 *)c->CY[0], (T *)c->R[0], window, c->nd, rho, c->rho_cs,
                                                               tw(c), sc, nkz(c, true), c->tr.mp);
         CK(cudaGetLastError());
     }
@@ -1583,12 +1583,7 @@ template <typename T, int N> struct Impl {
         }
         a.sd = (const T *)c->R[0];
         a.H = (const T *)c->H;
-        if (pen) {
-            a.i0 = c->bx_i0;
-            a.bi = c->bx_i;
-            a.j0 = c->bx_j0;
-            a.bj = c->bx_j;
-        }
+        a.box = pen ? c->d_box : nullptr;
         a.M = (T)c->cfg.M;
         a.eta = (T)c->cfg.pen_eta;
         a.scale = (T)(1. / ((double)N * N * N));
@@ -1598,7 +1593,7 @@ template <typename T, int N> struct Impl {
         a.nko = nkz(c, pen);
         a.op = pen ? c->tr.mp : NZC;
         const size_t smem = ZProdSmem<T, N, RL>::bytes;
-        Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko + (RL ? 4. * NZC : 0.)) + (RL ? 2. : 6.) * a.bi * a.bj * N * sizeof(T));
+        Launch L_(c, KC_PROD, (double)N * N * sizeof(T2) * (12. * a.nkz + 4. * a.nko + (RL ? 4. * NZC : 0.)) + (pen ? (RL ? 2. : 6.) * c->bx_i * c->bx_j * N : 0.) * sizeof(T));
         if (c->fftv)
             k_zprod<T, N, 1, RL><<<N * N / ZP_ROWS, ZProdLines<RL>::value * PV<1>, smem, c->st>>>(a, (const T *)c->kv, tw(c));
         else
@@ -1633,6 +1628,9 @@ template <typename T, int N> struct Impl {
         return true;
     }
 
+    // Whether launches of the right-hand side depend on the mask's window
+    static bool window_launches(const kf_ctx *c) { return c->stretched || !RLINES; }
+
     // rounds A (P s, d_x s, d_y s, the Poisson source and, with penalization, s_d
     // in R[0] where the mask is not zero), the Poisson solve and B (phi^ =
     // r2c(phi)), shared by both right-hand sides
@@ -1643,10 +1641,10 @@ template <typename T, int N> struct Impl {
         axis(c, c->jA_x, 2, 0, +1, AX_XM);
         axis(c, c->jA_y, 3, 1, +1, AX_YI);
         const bool solve = pois && !c->phi_given;
-        const RowBox box = (Tm & T_PENALIZATION) ? RowBox{c->bx_i0, c->bx_i, c->bx_j0, c->bx_j} : RowBox{0, 0, 0, 0};
+        const bool pen = Tm & T_PENALIZATION;
         if (solve)
-            rho_pass(c, box);
-        else if (box.bi)
+            rho_pass(c, pen ? c->d_box : nullptr);
+        else if (pen && (c->bx_i || !window_launches(c)))
             zc2r(c, c->zA, 1, true);
         const bool forked = fork && fork_D(c);
         if (solve) {
@@ -2464,6 +2462,7 @@ void create(kf_ctx *c) {
     c->red = dalloc<double>(c, sizeof(double) * 8);
     c->d_sweeps = dalloc<int>(c, sizeof(int) * 4);
     c->d_box = dalloc<int>(c, sizeof(int) * 4);
+    CK(cudaMemset(c->d_box, 0xff, sizeof(int) * 4));  // max i = -1: no row
     c->d_err = dalloc<int>(c, sizeof(int));
     CK(cudaMemset(c->d_err, 0, sizeof(int)));
     CK(cudaMallocHost(&c->h_err, sizeof(int)));
@@ -2740,23 +2739,27 @@ namespace {
 
 // Captured graphs hold the kernel variants they were captured with; dropped
 // when the variants change and rebuilt by their next use.
-void drop_graphs(kf_ctx *c) {
+void drop_step_graphs(kf_ctx *c) {
     CK(cudaStreamSynchronize(c->st));
-    if (c->vgraph) cudaGraphExecDestroy(c->vgraph);
-    c->vgraph = nullptr;
-    if (c->solve_graph) cudaGraphExecDestroy(c->solve_graph);
-    c->solve_graph = nullptr;
     if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
     c->step_graph = nullptr;
     if (c->step_graph_wait) cudaGraphExecDestroy(c->step_graph_wait);
     c->step_graph_wait = nullptr;
+}
+void drop_graphs(kf_ctx *c) {
+    drop_step_graphs(c);
+    if (c->vgraph) cudaGraphExecDestroy(c->vgraph);
+    c->vgraph = nullptr;
+    if (c->solve_graph) cudaGraphExecDestroy(c->solve_graph);
+    c->solve_graph = nullptr;
     if (c->adj && c->adj->graph) {
         cudaGraphExecDestroy(c->adj->graph);
         c->adj->graph = nullptr;
     }
 }
 
-// The mask's window of rows; the captured steps hold it, so a change drops them.
+// The mask's window of rows; captured steps whose launches depend on it are dropped
+// when it changes (Impl::window_launches).
 void mask_box(kf_ctx *c) {
     const int n = c->n;
     int b[4] = {n, -1, n, -1};
@@ -2779,7 +2782,7 @@ void mask_box(kf_ctx *c) {
     c->bx_i = bi;
     c->bx_j0 = j0;
     c->bx_j = bj;
-    drop_graphs(c);
+    if ((c->cfg.terms & T_PENALIZATION) && (c->stretched || !c->fp32)) drop_step_graphs(c);
 }
 
 // milliseconds per call of f: two untimed calls, then reps calls between

@@ -52,18 +52,37 @@ template <typename T, int N, int V, bool RL> struct ZProdMinBlocks {
     static constexpr int value = by_regs < 12 ? by_regs : 12;
 };
 
+// The window of rows (i, j) on which the mask is not zero, as k_mask_box leaves it
+// (min i, max i, min j, max j; nullptr: none).  Kernels of the captured step read
+// it from there, so that a mask that moves does not cost a new capture.
+struct RowBox {
+    int i0, bi, j0, bj;
+    __device__ __forceinline__ explicit RowBox(const int *__restrict__ b) : i0(0), bi(0), j0(0), bj(0) {
+        if (b && b[1] >= 0) {
+            i0 = b[0];
+            bi = b[1] - b[0] + 1;
+            j0 = b[2];
+            bj = b[3] - b[2] + 1;
+        }
+    }
+    __device__ __forceinline__ bool has(int i, int j) const {
+        return (unsigned)(i - i0) < (unsigned)bi && (unsigned)(j - j0) < (unsigned)bj;
+    }
+    __device__ __forceinline__ int row(int i, int j) const { return (i - i0) * bj + j - j0; }
+};
+
 template <typename T> struct ZProdArgs {
     typedef typename C2<T>::type T2;
     const T2 *s0, *sy, *sx;             // y-passed spectra of P s, d_y s, d_x s
     const T2 *u[3], *uy[3], *ux[3];     // of U_c, d_y U_c, d_x U_c
     T2 *out[4];                         // z-transformed results, half spectra
-    // penalization: the mask, the window of rows on which it is not zero
-    // (k_mask_box; bi = 0: none), s_d, and c2r(-lin_q) on that window's rows (RL: the
-    // y-passed spectra of -lin_q, of every row)
+    // penalization: the mask, the window of rows on which it is not zero (RowBox), s_d,
+    // and c2r(-lin_q) on that window's rows (RL: the y-passed spectra of -lin_q, of
+    // every row)
     const T *H, *sd;
+    const int *box;
     const T *rl[4];
     const T2 *lin[4];
-    int i0, bi, j0, bj;
     T M, eta, scale;                    // scale: the 1/N of the c2r
     int terms;
     int nkz, ip;  // the inputs are zero from kz = nkz on; elements per row
@@ -103,6 +122,7 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
     T2 *line = xch + l * LS;
     const PadAddr pa;
     const bool adv = a.terms & T_ADVECTION, cont = a.terms & T_CONTINUITY;
+    const RowBox box(a.box);
 #pragma unroll 1
     for (int rr = 0; rr < ZP_ROWS; ++rr) {
         const long off = (long)(r0 + rr) * ip;
@@ -140,8 +160,8 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
         for (int q = 0; q < E; ++q)
             line[reg_row<N, P, PlanV<N, V>::RL>(p, q)] = mk<T2>(v[q].x * a.scale, v[q].y * a.scale);
         __syncthreads();
-        const int bi = (r0 + rr) / N - a.i0, bj = (r0 + rr) % N - a.j0, brow = bi * a.bj + bj;
-        const bool box = (unsigned)bi < (unsigned)a.bi && (unsigned)bj < (unsigned)a.bj;
+        const bool inbox = box.has((r0 + rr) / N, (r0 + rr) % N);
+        const int brow = box.row((r0 + rr) / N, (r0 + rr) % N);
         for (int z = threadIdx.x; z < N; z += NT) {
             const T2 U0 = xch[z], U1 = xch[LS + z], U2 = xch[2 * LS + z];  // (U_c, d_z U_c)
             const T ux = U0.x, uy = U1.x, uz = U2.x;
@@ -165,7 +185,7 @@ k_zprod(const __grid_constant__ ZProdArgs<T> a, const T *__restrict__ kv,
                 rl[2] = l1.x;
                 rl[3] = l1.y;
             }
-            const T h = box ? a.H[(long)(r0 + rr) * N + z] : (T)0;
+            const T h = inbox ? a.H[(long)(r0 + rr) * N + z] : (T)0;
             if (h != (T)0) {
                 const T qd[4] = {ux, uy, uz, a.sd[(long)(r0 + rr) * N + z]};
                 const T qfix[4] = {-a.M, (T)0, (T)0, (T)-10};
@@ -218,17 +238,10 @@ template <typename T, int N> inline int zline_blocks() {
 // Inverse, with the Poisson source as the epilogue: s_d = c2r(P s^) and
 // rho = e^{s_d} + n_d in FP64 (rhs_standard.cpp:108-111), into rho and its
 // colour-split copy rcs (k_split's layout), each when given; and s_d into sd on the
-// window of rows i0 <= i < i0 + bi, j0 <= j < j0 + bj (bi = 0: nowhere).
-struct RowBox {
-    int i0, bi, j0, bj;
-    __device__ __forceinline__ bool has(int i, int j) const {
-        return (unsigned)(i - i0) < (unsigned)bi && (unsigned)(j - j0) < (unsigned)bj;
-    }
-};
-
+// rows of the window.
 template <typename T, int N, int V>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P)
-k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, RowBox box, const double *__restrict__ nd,
+k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, const int *__restrict__ window, const double *__restrict__ nd,
         double *__restrict__ rho, double *__restrict__ rcs, const typename C2<T>::type *__restrict__ tw, T scale,
         int nkz, int pitch) {
     typedef typename C2<T>::type T2;
@@ -258,6 +271,7 @@ k_z_rho(const typename C2<T>::type *__restrict__ in, T *__restrict__ sd, RowBox 
     }
     PlanV<N, V>::template fft<T2, +1>(v, xch + l * LS, PadAddr{}, p, tw);
     if (r >= N * N) return;
+    const RowBox box(window);
     constexpr long half = (long)N * N * (N / 2);
     auto put = [&](int row, int z, T s) {
         const long i = (long)row * N + z;
