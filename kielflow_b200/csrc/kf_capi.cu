@@ -194,10 +194,10 @@ struct kf_ctx {
     int cc_level = -1;         // entry level of k_cc, or -1 (cc_setup)
     int cc_ctas = 0;           // its cluster size
     ClusterCycle ccyc{};
-    // window of rows (i, j) on which the penalization mask is not zero
-    // (k_mask_box; bi = 0: none)
-    int bx_i0 = 0, bx_i = 0, bx_j0 = 0, bx_j = 0;
+    // window of rows (i, j) on which the penalization mask is not zero (RowBox), and
+    // its size
     int *d_box = nullptr;
+    int bx_i = 0, bx_j = 0;
     // what the end of the right-hand side does with K (k_xfwd_stage; 3: store it)
     int rk_mode = 3;
     double rk_c = 0.;
@@ -1412,11 +1412,10 @@ template <typename T, int N> struct Impl {
     // inv: an inverse x pass reads a state field, the forward one a masked intermediate
     static AxTrunc trunc(kf_ctx *c, int mode, bool inv = true, const kf_ctx::Cols *cols = nullptr) {
         const kf_ctx::Cols &t = cols ? *cols : c->tr;
-        AxTrunc A{AX_FULL, NZC, 0.f, nullptr, nullptr, 0, N, NZC, NZC};
+        AxTrunc A{AX_FULL, NZC, 0.f, nullptr, nullptr, nullptr, NZC, NZC};
         if (mode == AX_XB || mode == AX_YB) {
             A.mode = mode;
-            A.r0 = mode == AX_XB ? c->bx_i0 : c->bx_j0;
-            A.rm = mode == AX_XB ? c->bx_i : c->bx_j;
+            A.win = c->d_box;
             return A;
         }
         if (mode == AX_FULL) return A;
@@ -1436,7 +1435,7 @@ template <typename T, int N> struct Impl {
         const AxTrunc A = trunc(c, mode, true, cols);
         const int ntiles = A.mode == AX_XM || A.mode == AX_XF ? (cols ? cols->nt : c->tr.nt)
                            : ax == 0       ? (N * NZC + TC - 1) / TC
-                                           : (A.mode == AX_YB ? c->bx_i : N) * ((A.nkz + TC - 1) / TC);
+                                           : N * ((A.nkz + TC - 1) / TC);
         const int total = njobs * ntiles, grid = std::min(total, pipe_grid<V>(sign));
         const size_t smem = axis_pipe_smem<T, N>(njobs);
         if (sign < 0)
@@ -1473,17 +1472,19 @@ template <typename T, int N> struct Impl {
     }
     // scale < 0: the 1/N of c2r; otherwise the given factor (1 for transposes)
     // masked: the half spectra come from masked x / y passes (zero from kz = nkz on)
-    static void zc2r(kf_ctx *c, int off, int njobs, bool masked = false, double scale = -1., int nrows = N * N) {
-        const int ntiles = (nrows + LZ - 1) / LZ;
+    // window: rows of the mask's window, packed
+    static void zc2r(kf_ctx *c, int off, int njobs, bool masked = false, double scale = -1., bool window = false) {
+        const int nrows = N * N, ntiles = (nrows + LZ - 1) / LZ;
+        const int *win = window ? c->d_box : nullptr;
         const size_t smem = ZSmem<T, N, true>::bytes;
-        Launch L_(c, KC_Z_C2R, z_bytes(c, off, njobs, true, masked, nrows));
+        Launch L_(c, KC_Z_C2R, z_bytes(c, off, njobs, true, masked, window ? c->bx_i * c->bx_j : nrows));
         const T sc = (T)(scale < 0. ? 1. / ((double)N * N * N) : scale);
         if (c->fftv)
             k_z_c2r<T, N, 1><<<njobs * ntiles, LZ * PV<1>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr.mp : NZC);
+                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr.mp : NZC, win);
         else
             k_z_c2r<T, N, 0><<<njobs * ntiles, LZ * PV<0>, smem, c->st>>>(c->dz + off, njobs, nrows, geo(c),
-                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr.mp : NZC);
+                                                                        tw(c), sc, nkz(c, masked), masked ? c->tr.mp : NZC, win);
     }
     // masked: only the rows' kept part, in rows of whole tiles
     static void zr2c(kf_ctx *c, int off, int njobs, bool masked = false) {
@@ -1508,7 +1509,7 @@ template <typename T, int N> struct Impl {
         a.M = (T)c->cfg.M;
         a.D = (T)c->cfg.diff_D;
         a.terms = c->cfg.terms;
-        a.herm = (c->cfg.terms & T_PENALIZATION) && window_launches(c);
+        a.herm = (c->cfg.terms & T_PENALIZATION) && (c->stretched || !RLINES);
         return a;
     }
 
@@ -1628,9 +1629,6 @@ template <typename T, int N> struct Impl {
         return true;
     }
 
-    // Whether launches of the right-hand side depend on the mask's window
-    static bool window_launches(const kf_ctx *c) { return c->stretched || !RLINES; }
-
     // rounds A (P s, d_x s, d_y s, the Poisson source and, with penalization, s_d
     // in R[0] where the mask is not zero), the Poisson solve and B (phi^ =
     // r2c(phi)), shared by both right-hand sides
@@ -1644,7 +1642,7 @@ template <typename T, int N> struct Impl {
         const bool pen = Tm & T_PENALIZATION;
         if (solve)
             rho_pass(c, pen ? c->d_box : nullptr);
-        else if (pen && (c->bx_i || !window_launches(c)))
+        else if (pen)
             zc2r(c, c->zA, 1, true);
         const bool forked = fork && fork_D(c);
         if (solve) {
@@ -1684,10 +1682,10 @@ template <typename T, int N> struct Impl {
         if (rl) {  // the linear terms' inverse x and y passes, whole
             axis(c, c->jD_x + 6, 4, 0, +1);
             axis(c, c->jD_y + 9, 4, 1, +1);
-        } else if (pen && c->bx_i) {  // c2r(-lin_q) on the mask's window
+        } else if (pen) {  // c2r(-lin_q) on the mask's window
             axis(c, c->jD_x + 6, 4, 0, +1, AX_XB);
             axis(c, c->jD_y + 9, 4, 1, +1, AX_YB);
-            zc2r(c, c->zD + 8, 2, false, -1., c->bx_i * c->bx_j);
+            zc2r(c, c->zD + 8, 2, false, -1., true);
         }
         // D: the u', s part, unless forked
         if (!forked)
@@ -1748,7 +1746,7 @@ template <typename T, int N> struct Impl {
     // another 4 back and forth before.)
     static void rhs_stretched(kf_ctx *c) {
         const int Tm = c->cfg.terms;
-        const bool pen = Tm & T_PENALIZATION, win = pen && c->bx_i;
+        const bool pen = Tm & T_PENALIZATION;
         const long Nc = c->Nc, Nr = c->N;
         const double cb = (double)Nc * sizeof(T2), rb = (double)Nr * sizeof(T);
         rounds_AB(c, false);
@@ -1774,10 +1772,10 @@ template <typename T, int N> struct Impl {
             Launch L_(c, KC_PROD, 31. * rb);
             k_sl_scale<T><<<nblk(Nr, 256), 256, 0, c->st>>>(sa);
         }
-        if (win) {
+        if (pen) {
             axis(c, c->jD_x + 6, 4, 0, +1, AX_XB);
             axis(c, c->jD_y + 9, 4, 1, +1, AX_YB);
-            zc2r(c, c->zD + 8, 2, false, -1., c->bx_i * c->bx_j);
+            zc2r(c, c->zD + 8, 2, false, -1., true);
         }
         if (Tm & (T_ADVECTION | T_CONTINUITY)) {  // G'
             zr2c(c, c->zS_F, 6, true);
@@ -1801,10 +1799,7 @@ template <typename T, int N> struct Impl {
             pa.H = (const T *)c->H;
             pa.M = (T)c->cfg.M;
             pa.eta = (T)c->cfg.pen_eta;
-            pa.i0 = c->bx_i0;
-            pa.bi = win ? c->bx_i : 0;
-            pa.j0 = c->bx_j0;
-            pa.bj = c->bx_j;
+            pa.box = pen ? c->d_box : nullptr;
             pa.terms = Tm;
             pa.n = c->n;
             pa.N = Nr;
@@ -2739,15 +2734,12 @@ namespace {
 
 // Captured graphs hold the kernel variants they were captured with; dropped
 // when the variants change and rebuilt by their next use.
-void drop_step_graphs(kf_ctx *c) {
+void drop_graphs(kf_ctx *c) {
     CK(cudaStreamSynchronize(c->st));
     if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
     c->step_graph = nullptr;
     if (c->step_graph_wait) cudaGraphExecDestroy(c->step_graph_wait);
     c->step_graph_wait = nullptr;
-}
-void drop_graphs(kf_ctx *c) {
-    drop_step_graphs(c);
     if (c->vgraph) cudaGraphExecDestroy(c->vgraph);
     c->vgraph = nullptr;
     if (c->solve_graph) cudaGraphExecDestroy(c->solve_graph);
@@ -2758,8 +2750,7 @@ void drop_graphs(kf_ctx *c) {
     }
 }
 
-// The mask's window of rows; captured steps whose launches depend on it are dropped
-// when it changes (Impl::window_launches).
+// The mask's window of rows (RowBox), with its size for the profile's bytes
 void mask_box(kf_ctx *c) {
     const int n = c->n;
     int b[4] = {n, -1, n, -1};
@@ -2775,14 +2766,8 @@ void mask_box(kf_ctx *c) {
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(b, c->d_box, sizeof(b), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    const bool any = b[1] >= 0;
-    const int i0 = any ? b[0] : 0, bi = any ? b[1] - b[0] + 1 : 0, j0 = any ? b[2] : 0, bj = any ? b[3] - b[2] + 1 : 0;
-    if (i0 == c->bx_i0 && bi == c->bx_i && j0 == c->bx_j0 && bj == c->bx_j) return;
-    c->bx_i0 = i0;
-    c->bx_i = bi;
-    c->bx_j0 = j0;
-    c->bx_j = bj;
-    if ((c->cfg.terms & T_PENALIZATION) && (c->stretched || !c->fp32)) drop_step_graphs(c);
+    c->bx_i = b[1] >= 0 ? b[1] - b[0] + 1 : 0;
+    c->bx_j = b[1] >= 0 ? b[3] - b[2] + 1 : 0;
 }
 
 // milliseconds per call of f: two untimed calls, then reps calls between

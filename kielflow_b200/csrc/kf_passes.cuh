@@ -159,7 +159,7 @@ __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ job
         } else {
             G.base = tile * TC + c;
             G.valid = G.base < n * nzc;
-            G.obase = A.mode == AX_XB ? G.base - A.r0 * n * nzc : G.base;
+            G.obase = A.mode == AX_XB ? G.base - __ldg(A.win) * n * nzc : G.base;
         }
     } else {
         constexpr int tpp = (nzc + TC - 1) / TC;
@@ -182,7 +182,11 @@ __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ job
         G.base = plane * n * A.ip + kk;
         G.rstride = A.ip;
         G.ostride = A.op;
-        G.obase = A.mode == AX_YB ? (plane * A.rm - A.r0) * nzc + kk : plane * n * A.op + kk;
+        G.obase = plane * n * A.op + kk;
+        if (A.mode == AX_YB) {
+            const RowBox w(A.win);
+            G.obase = (plane * w.bj - w.j0) * nzc + kk;
+        }
     }
     return G;
 }
@@ -238,13 +242,22 @@ __global__ void __launch_bounds__(Tile<T>::TC * PlanV<N, V>::P,
 k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
             const typename C2<T>::type *__restrict__ tw, int total, AxTrunc A) {
     typedef typename C2<T>::type T2;
-    constexpr int TC = Tile<T>::TC, P = PlanV<N, V>::P, E = N / P;
+    constexpr int TC = Tile<T>::TC, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1;
     constexpr int D = KF_PIPE_DEPTH;
     extern __shared__ __align__(16) unsigned char kf_smem[];
     T2 *sm = reinterpret_cast<T2 *>(kf_smem);  // exchange [N][TC]
     T2 *stg0 = sm + N * TC;                     // staging  [D][N][TC]
     const int c = threadIdx.x % TC, p = threadIdx.x / TC;
     int t = blockIdx.x;
+    // the rows that the window modes store
+    const bool win = A.mode == AX_XB || A.mode == AX_YB;
+    int w0 = 0, wn = N;
+    if (win) {
+        const RowBox w(A.win);
+        w0 = A.mode == AX_XB ? w.i0 : w.j0;
+        wn = A.mode == AX_XB ? w.bi : w.bj;
+        if (A.mode == AX_YB || w.bi == 0) total = njobs * w.bi * ((NZC + TC - 1) / TC);
+    }
     if (t >= total) return;
     // (job, tile) of global tile t = tile * njobs + job, advanced by the grid
     // stride without a division per tile: for the tile being transformed (c*)
@@ -303,9 +316,7 @@ k_axis_pipe(const AxisJob *__restrict__ jobs, int njobs, int axis, Geo<T> g,
 #pragma unroll
             for (int q = 0; q < E; ++q) {
                 const int row = reg_row<N, P, PlanV<N, V>::RL>(p, q);
-                const bool st = A.mode == AX_XB || A.mode == AX_YB ? (unsigned)(row - A.r0) < (unsigned)A.rm
-                                                                 : row_freq<N>(row) <= cur.sb;
-                if (st) cur.out[cur.obase + row * cur.ostride] = v[q];
+                if (win ? (unsigned)(row - w0) < (unsigned)wn : row_freq<N>(row) <= cur.sb) cur.out[cur.obase + row * cur.ostride] = v[q];
             }
         }
     }
@@ -336,7 +347,7 @@ template <typename T, int N, bool C2R> struct ZSmem {
 template <typename T, int N, int V = 0>
 __global__ void __launch_bounds__(ZTile<T>::LZ * PlanV<N, V>::P, (sizeof(T) == 4 && KF_ZC2R_MINB > 0 ? KF_ZC2R_MINB : 1))
 k_z_c2r(const ZJob *__restrict__ jobs, int njobs, int nrows, Geo<T> g,
-        const typename C2<T>::type *__restrict__ tw, T scale, int nkz, int pitch) {
+        const typename C2<T>::type *__restrict__ tw, T scale, int nkz, int pitch, const int *__restrict__ win) {
     typedef typename C2<T>::type T2;
     constexpr int LZ = ZTile<T>::LZ, P = PlanV<N, V>::P, E = N / P, NZC = N / 2 + 1;
     constexpr int LS = PadLen<N>::value;  // padded line of the exchange buffer
@@ -344,8 +355,13 @@ k_z_c2r(const ZJob *__restrict__ jobs, int njobs, int nrows, Geo<T> g,
     T2 *half = reinterpret_cast<T2 *>(kf_smem);  // [2][LZ][NZC], staging of the half spectra
     T2 *xch = half;                              // [LZ][LS], reused by the transform once staged
     const int job = blockIdx.x % njobs, tile = blockIdx.x / njobs;
-    const ZJob J = jobs[job];
     const int r0 = tile * LZ;
+    if (win) {  // the window's rows, packed
+        const RowBox w(win);
+        nrows = w.bi * w.bj;
+        if (r0 >= nrows) return;
+    }
+    const ZJob J = jobs[job];
     const T2 *inA = static_cast<const T2 *>(J.inA);
     const T2 *inB = static_cast<const T2 *>(J.inB);
     const int p = threadIdx.x % P, l = threadIdx.x / P;

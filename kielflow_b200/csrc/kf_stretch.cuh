@@ -131,7 +131,8 @@ template <typename T> struct SlProdArgs {
     const T *sd, *H, *rl[4];           // penalization: c2r(P s^), the mask, l_q on the window
     T *out[4];
     T M, eta;
-    int i0, bi, j0, bj, terms, n;
+    const int *box;  // the mask's window (RowBox)
+    int terms, n;
     long N;
 };
 
@@ -143,9 +144,9 @@ __global__ void __launch_bounds__(256) k_sl_products(SlProdArgs<T> a) {
     T t[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) t[q] = a.out[q][idx];
-    const int row = (int)(idx / a.n), bi = row / a.n - a.i0, bj = row % a.n - a.j0;
-    const bool box = (unsigned)bi < (unsigned)a.bi && (unsigned)bj < (unsigned)a.bj;
-    const T h = box ? a.H[idx] : (T)0;
+    const int row = (int)(idx / a.n), i = row / a.n, j = row % a.n;
+    const RowBox box(a.box);
+    const T h = box.has(i, j) ? a.H[idx] : (T)0;
     T u[3] = {};
     if (adv || cont || h != (T)0) {
 #pragma unroll
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(256) k_sl_products(SlProdArgs<T> a) {
     if (h != (T)0) {
         const T qd[4] = {u[0], u[1], u[2], a.sd[idx]};
         const T qfix[4] = {-a.M, (T)0, (T)0, (T)-10};
-        const long w = ((long)bi * a.bj + bj) * a.n + idx % a.n;
+        const long w = (long)box.row(i, j) * a.n + idx % a.n;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const T l = a.rl[q][w], r = l - t[q];

@@ -62,17 +62,36 @@ enum AxMode : int {
     AX_XM = 1,    // x pass, masked input: active columns, rows within the column's bound -> every row
     AX_YI = 2,    // y pass after AX_XM: columns kz < nkz, rows j within jb[kz] -> every row
     AX_YF = 3,    // forward y pass whose x pass needs only active columns: every row -> rows within jb[kz]
-    AX_XB = 4,    // x pass of which a window of planes is needed: every row -> rows r0 .. r0 + rm - 1, packed
-    AX_YB = 5,    // y pass after AX_XB (rm0 planes): every row -> rows r0 .. r0 + rm - 1, packed
+    AX_XB = 4,    // x pass of which the window's planes are needed: every row -> these, packed
+    AX_YB = 5,    // y pass after AX_XB, on the window's planes: every row -> the window's rows, packed
     AX_XF = 6,    // forward x pass after AX_YF: active columns, every row
 };
+// The window of rows (i, j) on which the mask is not zero, as k_mask_box leaves it
+// (min i, max i, min j, max j; nullptr: none).  Kernels read it from there, so
+// that captured steps do not depend on it.
+struct RowBox {
+    int i0, bi, j0, bj;
+    __device__ __forceinline__ explicit RowBox(const int *__restrict__ b) : i0(0), bi(0), j0(0), bj(0) {
+        if (b && __ldg(b + 1) >= 0) {
+            i0 = __ldg(b);
+            bi = __ldg(b + 1) - i0 + 1;
+            j0 = __ldg(b + 2);
+            bj = __ldg(b + 3) - j0 + 1;
+        }
+    }
+    __device__ __forceinline__ bool has(int i, int j) const {
+        return (unsigned)(i - i0) < (unsigned)bi && (unsigned)(j - j0) < (unsigned)bj;
+    }
+    __device__ __forceinline__ int row(int i, int j) const { return (i - i0) * bj + j - j0; }
+};
+
 struct AxTrunc {
     int mode;
     int nkz;        // columns kz < nkz are active
     float itpp;     // 1 / column tiles per plane of AX_YI, AX_YF
     const int *jb;  // per kz < nkz: largest min(j, n - j) of an active column
     const int *tl;  // active x-pass tiles: (j << 16) | first kz
-    int r0, rm;     // AX_XB, AX_YB: the window
+    const int *win; // AX_XB, AX_YB: the window's planes i, rows j (RowBox)
     // elements per (i, j) row of the input and the output: n/2 + 1, or for the
     // masked passes' intermediates nkz rounded up to whole tiles, so that tiles are
     // aligned 128-byte segments (a row of n/2 + 1 elements shifts them across lines)

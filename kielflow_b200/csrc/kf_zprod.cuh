@@ -52,25 +52,6 @@ template <typename T, int N, int V, bool RL> struct ZProdMinBlocks {
     static constexpr int value = by_regs < 12 ? by_regs : 12;
 };
 
-// The window of rows (i, j) on which the mask is not zero, as k_mask_box leaves it
-// (min i, max i, min j, max j; nullptr: none).  Kernels of the captured step read
-// it from there, so that a mask that moves does not cost a new capture.
-struct RowBox {
-    int i0, bi, j0, bj;
-    __device__ __forceinline__ explicit RowBox(const int *__restrict__ b) : i0(0), bi(0), j0(0), bj(0) {
-        if (b && b[1] >= 0) {
-            i0 = b[0];
-            bi = b[1] - b[0] + 1;
-            j0 = b[2];
-            bj = b[3] - b[2] + 1;
-        }
-    }
-    __device__ __forceinline__ bool has(int i, int j) const {
-        return (unsigned)(i - i0) < (unsigned)bi && (unsigned)(j - j0) < (unsigned)bj;
-    }
-    __device__ __forceinline__ int row(int i, int j) const { return (i - i0) * bj + j - j0; }
-};
-
 template <typename T> struct ZProdArgs {
     typedef typename C2<T>::type T2;
     const T2 *s0, *sy, *sx;             // y-passed spectra of P s, d_y s, d_x s
