@@ -246,12 +246,6 @@ __global__ void __launch_bounds__(BS) k_poisson_vjp_tail(const double *__restric
     block_sum4<BS>(acc, sh, part);
 }
 
-// y = a x + b y over interleaved complex (real coordinates), four fields via a grid dimension
-__global__ void k_axpby(double *__restrict__ y, const double *__restrict__ x, double a, double b, long M) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < M) y[i] = __dadd_rn(__dmul_rn(a, x[i]), __dmul_rn(b, y[i]));
-}
-
 // c = exp(phi)
 __global__ void k_exp(const double *__restrict__ phi, double *__restrict__ c, long N) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -281,21 +275,7 @@ __global__ void __launch_bounds__(BS) k_dot_w(const double *__restrict__ w, cons
 // is linear, so the "Newton step" is the exact point solve psi = A / (D + c),
 // over-relaxed by om as the forward smoother (om = 1: the point solve itself).
 
-template <int BY = 8>
-__global__ void __launch_bounds__(32 * BY) k_rbgs_lin(double *__restrict__ phi, const double *__restrict__ rho,
-                                                      const double *__restrict__ cl, Lev L, int color, double om) {
-    const int n = L.n;
-    const int k2 = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * BY + threadIdx.y, i = blockIdx.z;
-    if (2 * k2 >= n || j >= n) return;
-    const int k = 2 * k2 + ((i + j + color) & 1);
-    double A, D;
-    point_coeffs_fast(phi, rho, L, i, j, k, A, D);
-    const long q = lidx(i, j, k, n);
-    const double y = A / __dadd_rn(D, cl[q]);
-    phi[q] = om == 1. ? y : __dadd_rn(phi[q], __dmul_rn(om, __dsub_rn(y, phi[q])));
-}
-
-// The same linear half sweep indexed as k_rbgs_t: one 32-bit index with
+// The linear half sweep, indexed as k_rbgs_t: one 32-bit index with
 // wrapped neighbour offsets, the i and j axis tables from the constant bank;
 // the loads, the sum and its order are point_coeffs_fast's.
 template <int BY = 8>

@@ -66,18 +66,11 @@ struct LevelBuf {
     double *ddk = nullptr, *ipk = nullptr, *imk = nullptr;
     double *ph = nullptr, *rh = nullptr;
     SLev slev() const { return SLev{n, dd, ip, im, ddk, ipk, imk}; }
-    std::shared_ptr<AxTab> tab;  // host copy of dd, ip, im for k_rbgs_t (n <= KF_TAB_N)
+    std::shared_ptr<AxTab> tab;  // host copy of dd, ip, im (kernel parameter of the half sweeps)
     Lev lev() const { return Lev{n, dd, dp, dm, ip, im, rp, rm}; }
 };
 
 constexpr int RBS = 256;  // reduction block size
-
-// Half sweeps with the i and j axis tables passed as a kernel parameter
-// (k_rbgs_t; 0: k_rbgs reads them from global memory).
-#ifndef KF_RBGS_TAB
-#define KF_RBGS_TAB 1
-#endif
-
 
 // Sweeps in the body of the Jacobi loop's WHILE node (even: they alternate
 // between the two potentials).
@@ -112,7 +105,7 @@ struct kf_ctx {
     void *CX[12] = {}, *CY[16] = {}, *R[24] = {}, *phihat = nullptr, *LIN[4] = {};
     double *phi = nullptr, *rho = nullptr, *nd = nullptr;
     double *rho_cs = nullptr, *phi_cs = nullptr;  // the finest rho and phi in split order
-    void *H = nullptr, *phiT = nullptr;
+    void *H = nullptr;
     void *kv = nullptr, *SV = nullptr, *PF = nullptr;
     void *tw[2] = {};  // twiddles of the two radix plans (plan_twiddles)
     double *q2 = nullptr;
@@ -143,8 +136,8 @@ struct kf_ctx {
     AxisJob *dj = nullptr;
     ZJob *dz = nullptr;
     // job-list offsets (into dj / dz) and counts
-    int jA_x = 0, jA_y = 0, zA = 0, zB = 0, jB_y = 0, jB_x = 0, jD_x = 0, nD_x = 0, jD_y = 0, nD_y = 0;
-    int zD = 0, nzD = 0, zF = 0, jF_y = 0, jF_x = 0, jT_x = 0, jT_y = 0, zT = 0, jTf_y = 0, jTf_x = 0;
+    int jA_x = 0, jA_y = 0, zA = 0, jB_y = 0, jB_x = 0, jD_x = 0, jD_y = 0;
+    int zD = 0, zF = 0, jF_y = 0, jT_x = 0, jT_y = 0, zT = 0, jTf_y = 0, jTf_x = 0;
     int jG_x = 0, jG_y = 0, zG = 0;
     // sine-stretched axes: the chain-rule right-hand side's buffers, metric
     // tables and job lists (allocated only when cfg.stretch_m != 0)
@@ -188,7 +181,7 @@ struct kf_ctx {
     OutState *out = nullptr;
     bool phi_given = false;
     int fftv = 0;     // radix-plan variant of the transform kernels (kf_autotune)
-    int rbgs_by = 8;  // smoother variant (kf_autotune): k_rbgs rows per block, or 0 for k_rbgs_march
+    int rbgs_by = 8;  // smoother variant (kf_autotune): half-sweep block size, or 0 for k_rbgs_march
     bool march_maps = false;  // the driver's tensor-map encoder is available
     bool coarse_block = true;  // the coarse levels of a V-cycle in one k_cc cluster (kf_set_coarse_block)
     int cc_level = -1;         // entry level of k_cc, or -1 (cc_setup)
@@ -710,8 +703,8 @@ void smooth(kf_ctx *c, LevelBuf &L, double *phi, const double *rho, const double
     smooth_plain(c, L, phi, rho, cc, sweeps, cls);
 }
 
-// `sweeps` red-black sweeps as two half-sweep launches each (k_rbgs, or
-// k_rbgs_lin with the adjoint's e^phi).  (Sweeping a level larger than L2 in
+// `sweeps` red-black sweeps as two half-sweep launches each (k_rbgs_t, or
+// k_rbgs_lin_t with the adjoint's e^phi).  (Sweeping a level larger than L2 in
 // chunks of i-planes, black one plane behind red so that the black half finds
 // its data in L2, gives the same potentials bit for bit but measured slower at
 // 256^3: 156 / 169 / 181 / 214 us per sweep for 1 / 2 / 4 / 8 chunks.  So did
@@ -719,7 +712,6 @@ void smooth(kf_ctx *c, LevelBuf &L, double *phi, const double *rho, const double
 // tables and the planes between their points: 20.4 / 20.2 ms against 18.9 ms
 // for 240 half sweeps; L1 use fell from 89 to 62 %, but occupancy halved and
 // the DRAM throughput, 4.5 TB/s on 1.33x the algorithmic bytes, stayed.)
-
 void smooth_plain(kf_ctx *c, LevelBuf &L, double *phi, const double *rho, const double *cc, int sweeps, int cls) {
     const int n = L.n;
     const long N = (long)n * n * n;
@@ -729,34 +721,20 @@ void smooth_plain(kf_ctx *c, LevelBuf &L, double *phi, const double *rho, const 
     for (int s = 0; s < sweeps; ++s)
         for (int color = 0; color < 2; ++color) {
             Launch L_(c, cls, 16. * N);
-            if (cc && L.tab) {
+            if (cc) {
                 if (by == 4)
                     k_rbgs_lin_t<4><<<g, b, 0, c->st>>>(phi, rho, cc, L.lev(), color, om, *L.tab);
                 else if (by == 16)
                     k_rbgs_lin_t<16><<<g, b, 0, c->st>>>(phi, rho, cc, L.lev(), color, om, *L.tab);
                 else
                     k_rbgs_lin_t<8><<<g, b, 0, c->st>>>(phi, rho, cc, L.lev(), color, om, *L.tab);
-            } else if (cc) {
-                if (by == 4)
-                    k_rbgs_lin<4><<<g, b, 0, c->st>>>(phi, rho, cc, L.lev(), color, om);
-                else if (by == 16)
-                    k_rbgs_lin<16><<<g, b, 0, c->st>>>(phi, rho, cc, L.lev(), color, om);
-                else
-                    k_rbgs_lin<8><<<g, b, 0, c->st>>>(phi, rho, cc, L.lev(), color, om);
-            } else if (L.tab) {
+            } else {
                 if (by == 4)
                     k_rbgs_t<4><<<g, b, 0, c->st>>>(phi, rho, L.lev(), color, om, *L.tab);
                 else if (by == 16)
                     k_rbgs_t<16><<<g, b, 0, c->st>>>(phi, rho, L.lev(), color, om, *L.tab);
                 else
                     k_rbgs_t<8><<<g, b, 0, c->st>>>(phi, rho, L.lev(), color, om, *L.tab);
-            } else {
-                if (by == 4)
-                    k_rbgs<4><<<g, b, 0, c->st>>>(phi, rho, L.lev(), color, om);
-                else if (by == 16)
-                    k_rbgs<16><<<g, b, 0, c->st>>>(phi, rho, L.lev(), color, om);
-                else
-                    k_rbgs<8><<<g, b, 0, c->st>>>(phi, rho, L.lev(), color, om);
             }
         }
 }
@@ -2162,13 +2140,11 @@ void build_levels(kf_ctx *c) {
         CK(cudaMemcpy(L.dp, dp.data(), 8 * n, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(L.dm, dm.data(), 8 * n, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(L.gam, gam.data(), 8 * n, cudaMemcpyHostToDevice));
-        if (KF_RBGS_TAB && n <= KF_TAB_N) {
-            L.tab = std::make_shared<AxTab>();
-            for (int m = 0; m < n; ++m) {
-                L.tab->dd[m] = dd[m];
-                L.tab->ip[m] = ip[m];
-                L.tab->im[m] = im[m];
-            }
+        L.tab = std::make_shared<AxTab>();  // n <= KF_TAB_N for every grid size
+        for (int m = 0; m < n; ++m) {
+            L.tab->dd[m] = dd[m];
+            L.tab->ip[m] = ip[m];
+            L.tab->im[m] = im[m];
         }
         const size_t bytes = sizeof(double) * (size_t)n * n * n;
         L.r = dalloc<double>(c, bytes);
@@ -2186,7 +2162,7 @@ void build_levels(kf_ctx *c) {
             L.phi0 = dalloc<double>(c, bytes);
         }
         // above the sizes that the cluster takes, where bandwidth counts
-        L.sp = cf.poisson_mode == KF_PS_FAS && nl > 1 && l + 1 < nl && n > CC_MAX_N && n % 16 == 0 && L.tab;
+        L.sp = cf.poisson_mode == KF_PS_FAS && nl > 1 && l + 1 < nl && n > CC_MAX_N && n % 16 == 0;
         if (L.sp) {
             std::vector<double> t(3 * n);
             for (int k = 0; k < n; ++k) {
@@ -2284,9 +2260,7 @@ void build_jobs(kf_ctx *c) {
     c->zA = (int)Z.size();
     zj(CY[0], MUL_NONE, nullptr, 0, R[0], nullptr);
     // B
-    c->zB = (int)Z.size();
-    zj(c->phiT, 0, nullptr, 0, CX[8], nullptr);  // CX[8], CY[12]: not written by round D's u', s part
-    c->jB_y = (int)J.size();
+    c->jB_y = (int)J.size();  // CX[8], CY[12]: not written by round D's u', s part
     aj(CX[8], CY[12], MUL_NONE);
     c->jB_x = (int)J.size();
     aj(CY[12], c->phihat, MUL_NONE);
@@ -2319,8 +2293,6 @@ void build_jobs(kf_ctx *c) {
     zj(R[22], 0, R[23], 0, CX[2], CX[3]);
     c->jF_y = (int)J.size();
     for (int q = 0; q < 4; ++q) aj(CX[q], CY[q], MUL_NONE);
-    c->jF_x = (int)J.size();
-    for (int q = 0; q < 4; ++q) aj(CY[q], c->K[q], MUL_NONE);
     // standalone transforms: r2c R[0] -> CX[0] ; c2r CX[0] -> R[0]
     c->zT = (int)Z.size();
     zj(R[0], 0, nullptr, 0, CX[1], nullptr);
@@ -2441,7 +2413,6 @@ void create(kf_ctx *c) {
     c->rho = dalloc<double>(c, 8 * c->N);
     c->nd = dalloc<double>(c, 8 * c->N);
     c->H = dalloc<void>(c, rb);
-    c->phiT = c->fp32 ? dalloc<void>(c, rb) : (void *)c->phi;
     c->stage64 = dalloc<double>(c, (size_t)16 * (c->Nc > c->N ? c->Nc : c->N));
     CK(cudaMemset(c->phi, 0, 8 * c->N));
     CK(cudaMemset(c->rho, 0, 8 * c->N));

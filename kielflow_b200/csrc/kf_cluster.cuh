@@ -9,7 +9,7 @@
 // and, when it updates a point of its first or last plane, writes it into the
 // neighbour's copy as well (distributed shared memory); a cluster barrier (0.2
 // us) ends each phase.  Points, operations and their order are those of the
-// level-by-level kernels (k_fas_rhs, k_rbgs, k_residual, k_restrict,
+// level-by-level kernels (k_fas_rhs, k_rbgs_t, k_residual, k_restrict,
 // k_coarse_solve, k_correction, k_prolong_add), so the potentials are the same
 // bit for bit.
 //

@@ -2,11 +2,11 @@
 // sweep (FP64): TMA-staged tiles, temporal blocking of the two colour
 // half-sweeps in shared memory, and the residual fused into the last pass.
 //
-// The arithmetic per point is the one of k_rbgs / k_residual (kf_poisson.cuh):
+// The arithmetic per point is the one of k_rbgs_t / k_residual (kf_poisson.cuh):
 // the 7-point operator of the axis spacings H[i] (solver_poisson_jacobi_nlin.cpp
 // :177-211, weights 2/den precomputed) and one over-relaxed Newton step on
 // A - D x - e^x = 0, in the same order of operations, so a launch of this kernel
-// gives the potentials of two k_rbgs launches bit for bit.
+// gives the potentials of two k_rbgs_t launches bit for bit.
 //
 // Layout.  A CTA owns a tile of TK = 64 (k, contiguous) x TJ (j) points and a
 // chunk of CI i-planes.  It streams the planes i0 - H ... i0 + CI + H - 1 of phi

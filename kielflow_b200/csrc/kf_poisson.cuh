@@ -79,9 +79,8 @@ __device__ __forceinline__ double f_point(double A, double D, double x) {
 // ------------------------------------------------------------ reductions
 constexpr int KF_RED = 5;  // slots of a block's partials (kf_jacobi.cuh)
 
-// NaN-propagating max / min (fmax alone would drop a NaN)
+// NaN-propagating max (fmax alone would drop a NaN)
 __device__ __forceinline__ double nmax(double a, double b) { return (a != a || b != b) ? a + b : fmax(a, b); }
-__device__ __forceinline__ double nmin(double a, double b) { return (a != a || b != b) ? a + b : fmin(a, b); }
 
 // Launch geometry of the multigrid kernels: block (32, 8), grid
 // (ceil(nx/32), ceil(n/8), n) over (k or k/2, j, i) -- no index division.
@@ -162,42 +161,13 @@ __global__ void k_extrap(double *__restrict__ phi, double *__restrict__ phi_a, d
     phi_a[i] = b;
 }
 
-// Red-black Gauss-Seidel-Newton half sweep (colour (i+j+k)%2): one Newton
-// step per point; grid over (k/2, j, i), blocks of 32 x BY (the tile shape
-// kf_autotune chooses; the arithmetic does not depend on it).
-// The axis tables of a level of at most 256 points per axis, passed by value
-// as a kernel parameter: entries read with a warp-uniform index (the i and j
-// of a half-sweep warp) come from the constant bank instead of L1.
+// The axis tables of a level (at most 256 points per axis), passed by value as a
+// kernel parameter: entries read with a warp-uniform index (the i and j of a
+// half-sweep warp) come from the constant bank instead of L1.
 constexpr int KF_TAB_N = 256;
 struct AxTab {
     double dd[KF_TAB_N], ip[KF_TAB_N], im[KF_TAB_N];
 };
-
-// The point's index and its six periodic neighbours' are one 32-bit base and
-// wrapped offsets (n^3 < 2^31 for every supported n <= 256): the loads, the
-// sum and its order are point_coeffs_fast's, with fewer integer instructions.
-template <int BY = 8>
-__global__ void __launch_bounds__(32 * BY) k_rbgs(double *__restrict__ phi, const double *__restrict__ rho, Lev L,
-                                                  int color, double om) {
-    const int n = L.n;
-    const int k2 = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * BY + threadIdx.y, i = blockIdx.z;
-    if (2 * k2 >= n || j >= n) return;
-    const int k = 2 * k2 + ((i + j + color) & 1);
-    const int nn = n * n;
-    const int q = (i * n + j) * n + k;
-    const int oip = i == n - 1 ? -(n - 1) * nn : nn, oim = i == 0 ? (n - 1) * nn : -nn;
-    const int ojp = j == n - 1 ? -(n - 1) * n : n, ojm = j == 0 ? (n - 1) * n : -n;
-    const int okp = k == n - 1 ? -(n - 1) : 1, okm = k == 0 ? n - 1 : -1;
-    const double D = __dadd_rn(__dadd_rn(L.dd[i], L.dd[j]), L.dd[k]);
-    double A = __dmul_rn(phi[q + oip], L.ip[i]);
-    A = __dadd_rn(A, __dmul_rn(phi[q + oim], L.im[i]));
-    A = __dadd_rn(A, __dmul_rn(phi[q + ojp], L.ip[j]));
-    A = __dadd_rn(A, __dmul_rn(phi[q + ojm], L.im[j]));
-    A = __dadd_rn(A, __dmul_rn(phi[q + okp], L.ip[k]));
-    A = __dadd_rn(A, __dmul_rn(phi[q + okm], L.im[k]));
-    A = __dadd_rn(A, rho[q]);
-    phi[q] = newton_step(phi[q], A, D, om);
-}
 
 // A level's field split by colour: the point of colour c at k = 2 k2 + ((i + j +
 // c) & 1) is element c n^3/2 + (i n + j) n/2 + k2 (kf_split.cuh).
@@ -211,7 +181,12 @@ __global__ void __launch_bounds__(256) k_split(const double *__restrict__ x, dou
     s[(c0 ^ 1) * half + row] = v.y;
 }
 
-// The same half sweep with the i and j tables from the constant bank (AxTab).
+// Red-black Gauss-Seidel-Newton half sweep (colour (i+j+k)%2) in natural order: one
+// Newton step per point; grid over (k/2, j, i), blocks of 32 x BY (the tile shape
+// kf_autotune chooses; the arithmetic does not depend on it).  The point's index
+// and its six periodic neighbours' are one 32-bit base and wrapped offsets (n^3 <
+// 2^31 for every supported n <= 256): the loads, the sum and its order are
+// point_coeffs_fast's, with fewer integer instructions.
 template <int BY = 8>
 __global__ void __launch_bounds__(32 * BY) k_rbgs_t(double *__restrict__ phi, const double *__restrict__ rho, Lev L,
                                                     int color, double om, const __grid_constant__ AxTab T) {
@@ -353,7 +328,7 @@ __device__ __forceinline__ double block_nmax(double m, double *sh) {
     return res;
 }
 
-// One red-black half sweep (k_rbgs's point update) of a level the block holds.
+// One red-black half sweep (k_rbgs_t's point update) of a level the block holds.
 __device__ __forceinline__ void block_half_sweep(double *sp, const double *sr, const Lev &Ls, int color,
                                                  double om) {
     const int n = Ls.n;

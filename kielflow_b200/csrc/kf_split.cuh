@@ -101,7 +101,7 @@ __device__ __forceinline__ void split_pair(const double *__restrict__ phi, const
     f(color * H + q, x, A0, A1, __dadd_rn(dij, dk.x), __dadd_rn(dij, dk.y));
 }
 
-// One red-black half sweep (k_rbgs's point update).
+// One red-black half sweep (k_rbgs_t's point update).
 __global__ void __launch_bounds__(128) k_rbgs_s(double *phi, const double *__restrict__ rho, SLev L, int color,
                                                 double om, const __grid_constant__ AxTab T) {
     const int j = blockIdx.y * blockDim.y + threadIdx.y, i = blockIdx.z;
