@@ -770,8 +770,9 @@ void coarse_cluster(kf_ctx *c, double *phi, double *phi0, const double *r, const
 // Whether level l's cycle runs in split order (not with the streaming smoother)
 bool split_on(const kf_ctx *c, int l) { return c->lv[l].sp && c->rbgs_by != 0; }
 
-// Blocks of the split-order kernels: 64 threads where the level streams from
-// memory, 128 where it lies in L2 (split_pair), halved or doubled by rbgs_rows 4, 16.
+// Blocks of the split-order kernels: 128 threads where the level lies in L2, 64
+// where it streams from memory and both serve (split_pair); halved, at least a row,
+// by rbgs_rows 4 and doubled, at most 128, by 16.
 dim3 split_block(const kf_ctx *c, int n) {
     const int want = std::min(128, (n >= 256 ? 8 : 16) * c->rbgs_by), tx = n / 4;
     return dim3(tx, std::max(1, want / tx));
@@ -2649,7 +2650,9 @@ void rk4_steps_graph(kf_ctx *c, int nsteps, double dt) {
 // interface_ode_solver::solve with the state in host arrays, in place: the
 // upload of s goes first on the compute stream; u' is uploaded on a copy
 // stream while stage 1's Poisson solve runs (the captured step of the first
-// step waits for it just before it needs u'); the result is copied back.
+// step waits for it just before it needs u'); the result is copied back.  That
+// order hides the upload for page-locked arrays; a pageable u' holds the host until
+// it is staged, before the step is launched.
 void step_host(kf_ctx *c, int nsteps, double dt, double *const *host) {
     if (!c->st_copy) {
         CK(cudaStreamCreateWithFlags(&c->st_copy, cudaStreamNonBlocking));

@@ -3,10 +3,11 @@
 // The host driver decides three things per stage that depend on run-time
 // values: the stage time, the start of the Poisson solve (linear extrapolation
 // of the last two solutions at distinct times) and whether the FAS V-cycles
-// have converged.  For a captured step these decisions are taken by the
-// one-thread kernels below on a small device-resident record, with the same
-// arithmetic as the host path (so both paths give identical results), and the
-// convergence loop is a conditional WHILE node driven by k_fas_check.
+// have converged.  For a captured step these decisions are taken by the kernels
+// below (one thread, one warp or, where a field is extrapolated, a whole grid) on
+// a small device-resident record, with the same arithmetic as the host path (so
+// both paths give identical results), and the convergence loop is a conditional
+// WHILE node driven by k_fas_check.
 #pragma once
 
 #include <cuda_runtime.h>

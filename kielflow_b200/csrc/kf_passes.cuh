@@ -196,7 +196,8 @@ __device__ __forceinline__ AxisTile<T> axis_tile(const AxisJob *__restrict__ job
 // N x TC elements per block), at most CAP, and no more than leave FLOOR
 // registers per thread.  Without this bound the allocator spends 128-224
 // registers per thread on the 256-point transforms and two blocks fit; with
-// it the same code fits 64-85 registers (FP32) without spilling.
+// it the same code fits 64-85 registers (FP32) without spilling (k_x_filter with the
+// first plan, two transforms in one kernel, spills 60 bytes at 64 registers).
 template <typename T, int N, int V, int TILES, int CAP, int FLOOR> struct PipeMinBlocks {
     static constexpr long threads = (long)Tile<T>::TC * PlanV<N, V>::P;
     static constexpr long smem = (long)TILES * N * Tile<T>::TC * sizeof(typename C2<T>::type);

@@ -62,12 +62,12 @@ __global__ void __launch_bounds__(256) k_guess_s(const double *__restrict__ phi,
 
 // One colour of a level, two points of a row per thread (elements k2 = 2 t and
 // 2 t + 1: 16-byte loads, two independent chains of Newton steps or residuals).
-// Block (n / 4, rows), grid (1, ceil(n / rows), n).  256^3: 56 us for the half
-// sweep, 4.8 TB/s, in blocks of 64 threads (61 us in blocks of 128: their warps
-// load and compute in step; natural order: 72 us); threads that march 2-16 planes
-// with the i-neighbours in registers and the next plane prefetched took 68-88 us,
-// for their 93-128 registers leave fewer warps.  Up to 128^3, in L2, blocks of 128
-// threads are as fast or faster (128^3 8.8 us, 96^3 5.3, 64^3 2.8).
+// Block (n / 4, rows), grid (1, ceil(n / rows), n).  256^3: 51 us for the half
+// sweep, 5.2 TB/s, in blocks of 64 threads as of 128 (51.3 and 50.7 us; natural
+// order: 72 us); threads that march 2-16 planes with the i-neighbours in registers
+// and the next plane prefetched took 68-88 us, for their 93-128 registers leave
+// fewer warps.  Up to 128^3, in L2, blocks of 128 threads are faster (128^3: 8.3 us
+// against 9.3 in blocks of 64; a 96^3 step 1.71 ms against 1.76).
 template <typename F>
 __device__ __forceinline__ void split_pair(const double *__restrict__ phi, const double *__restrict__ rho,
                                            const SLev &L, const AxTab &T, int color, int i, int j, F f) {
