@@ -1488,7 +1488,6 @@ template <typename T, int N> struct Impl {
         a.M = (T)c->cfg.M;
         a.D = (T)c->cfg.diff_D;
         a.terms = c->cfg.terms;
-        a.herm = (c->cfg.terms & T_PENALIZATION) && (c->stretched || !RLINES);
         return a;
     }
 
@@ -1654,8 +1653,9 @@ template <typename T, int N> struct Impl {
         // C
         {
             Launch L_(c, KC_LIN, (double)c->Nc * (9 * sizeof(T2) + 2 * sizeof(T)));
-            k_lin<T><<<mg_grid(NZC, N), mg_block(), 0, c->st>>>(rargs(c), geo(c), (T2 *)c->LIN[0], (T2 *)c->LIN[1],
-                                                               (T2 *)c->LIN[2], (T2 *)c->LIN[3]);
+            const auto k = pen && !RLINES ? k_lin<T, !RLINES> : k_lin<T, false>;
+            k<<<mg_grid(NZC, N), mg_block(), 0, c->st>>>(rargs(c), geo(c), (T2 *)c->LIN[0], (T2 *)c->LIN[1],
+                                                         (T2 *)c->LIN[2], (T2 *)c->LIN[3]);
         }
         const bool rl = RLINES && pen;
         if (rl) {  // the linear terms' inverse x and y passes, whole
@@ -1732,7 +1732,7 @@ template <typename T, int N> struct Impl {
         {  // C'
             Launch L_(c, KC_LIN, 4 * cb + 6 * cb + 2 * rb);
             k_sl_lin<T><<<nblk(Nc, 256), 256, 0, c->st>>>(rargs(c), geo(c), (T2 *)c->LIN[0], (T2 *)c->LIN[1],
-                                                            (T2 *)c->LIN[2], (T2 *)c->LIN[3], (T2 *)c->CX[10]);
+                                                            (T2 *)c->LIN[2], (T2 *)c->LIN[3], (T2 *)c->CX[10], pen);
         }
         // D'
         axis(c, c->jS_Dx, 8, 0, +1, AX_XM);

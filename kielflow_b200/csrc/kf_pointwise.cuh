@@ -92,32 +92,41 @@ __device__ __forceinline__ void lin_terms(const RhsArgs<T> &a, const Geo<T> &g, 
     }
 }
 
-// o: four values of element (i, j, k = 0); m: those of (-i, -j, 0)
+// The Hermitian part of the kz = 0 plane, which is what a way through physical
+// space leaves of it (penalization): o holds four values of element (i, j, 0), m
+// those of (-i, -j, 0)
 template <typename T2> __device__ __forceinline__ void hermitian_part(T2 *o, const T2 *m) {
     typedef decltype(T2::x) T;
 #pragma unroll
     for (int q = 0; q < 4; ++q) o[q] = mk<T2>((T)0.5 * (o[q].x + m[q].x), (T)0.5 * (o[q].y - m[q].y));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *o0,
+// HERM: with the Hermitian part of the kz = 0 plane (hermitian_part) inside the 2/3
+// rule, where the result is used.
+template <typename T, bool HERM>
+__global__ void __launch_bounds__(256, HERM ? 4 : 1) k_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *o0,
                                              typename C2<T>::type *o1, typename C2<T>::type *o2,
                                              typename C2<T>::type *o3) {
     typedef typename C2<T>::type T2;
     const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
     if (k >= g.nzc || j >= g.n) return;
-    T2 o[4];
-    lin_terms(a, g, i, j, k, o);
-    if (a.herm && k == 0 && dealias_keep(g.q2, g.thr, i, j, 0)) {
-        T2 m[4];
-        lin_terms(a, g, i ? g.n - i : 0, j ? g.n - j : 0, 0, m);
-        hermitian_part(o, m);
-    }
     const long idx = (long)k + (long)g.nzc * ((long)j + (long)i * g.n);
-    o0[idx] = o[0];
-    o1[idx] = o[1];
-    o2[idx] = o[2];
-    o3[idx] = o[3];
+    // Where the Hermitian part is formed, the mirror's values go through the
+    // element's own place, so that few registers live across the terms' code
+    const bool h = HERM && k == 0 && dealias_keep(g.q2, g.thr, i, j, 0);
+#pragma unroll 1
+    for (int mirror = h ? 1 : 0; mirror >= 0; --mirror) {
+        T2 o[4];
+        lin_terms(a, g, mirror && i ? g.n - i : i, mirror && j ? g.n - j : j, k, o);
+        if (h && !mirror) {
+            const T2 m[4] = {o0[idx], o1[idx], o2[idx], o3[idx]};
+            hermitian_part(o, m);
+        }
+        o0[idx] = o[0];
+        o1[idx] = o[1];
+        o2[idx] = o[2];
+        o3[idx] = o[3];
+    }
 }
 
 // The (i, j) rows on which the penalization mask is not zero, as the window

@@ -17,6 +17,7 @@ namespace kf {
 // and the added diffusion) and the potential of the E-force/pressure term
 // F1 = PF phi^ + s^/theta (rhs_standard.cpp:218-240), one thread per
 // half-spectrum element.  Same order of operations as lin_terms.
+// herm: with the Hermitian part of the kz = 0 plane, as k_lin.
 template <typename T>
 __device__ __forceinline__ void sl_lin_terms(const RhsArgs<T> &a, const Geo<T> &g, int i, int j, int k,
                                              typename C2<T>::type *o) {
@@ -42,7 +43,7 @@ __device__ __forceinline__ void sl_lin_terms(const RhsArgs<T> &a, const Geo<T> &
 
 template <typename T>
 __global__ void k_sl_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *l0, typename C2<T>::type *l1,
-                         typename C2<T>::type *l2, typename C2<T>::type *l3, typename C2<T>::type *F1o) {
+                         typename C2<T>::type *l2, typename C2<T>::type *l3, typename C2<T>::type *F1o, bool herm) {
     typedef typename C2<T>::type T2;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long Nc = (long)g.n * g.n * g.nzc;
@@ -52,7 +53,7 @@ __global__ void k_sl_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *l0, typen
     const int j = (int)(r % g.n), i = (int)(r / g.n);
     T2 o[4];
     sl_lin_terms(a, g, i, j, k, o);
-    if (a.herm && k == 0 && dealias_keep(g.q2, g.thr, i, j, 0)) {
+    if (herm && k == 0 && dealias_keep(g.q2, g.thr, i, j, 0)) {
         T2 m[4];
         sl_lin_terms(a, g, i ? g.n - i : 0, j ? g.n - j : 0, 0, m);
         hermitian_part(o, m);

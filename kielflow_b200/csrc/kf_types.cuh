@@ -136,10 +136,6 @@ template <typename T> struct RhsArgs {
     const T *PF;        // phi filter exp(-2000 |k~_Q1|^15) (operations.hpp:20-46)
     T tau, theta, M, D;
     int terms;
-    // the Hermitian part of the kz = 0 plane, as a way through physical space leaves
-    // it (inside the 2/3 rule, where the result is used): penalization with the
-    // linear terms in k-space
-    int herm;
 };
 
 }  // namespace kf
