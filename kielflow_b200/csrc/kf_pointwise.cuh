@@ -104,7 +104,7 @@ template <typename T2> __device__ __forceinline__ void hermitian_part(T2 *o, con
 // HERM: with the Hermitian part of the kz = 0 plane (hermitian_part) inside the 2/3
 // rule, where the result is used.
 template <typename T, bool HERM>
-__global__ void __launch_bounds__(256, HERM ? 4 : 1) k_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *o0,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4) k_lin(RhsArgs<T> a, Geo<T> g, typename C2<T>::type *o0,
                                              typename C2<T>::type *o1, typename C2<T>::type *o2,
                                              typename C2<T>::type *o3) {
     typedef typename C2<T>::type T2;
